@@ -61,7 +61,7 @@ class ActionModel(nn.Module):
             from ..ops.lstm import persistent_ok
             layer = self.lstm.layers[0]
             b, t, e = frame_embeddings.shape
-            if persistent_ok(b, layer.hidden) and e % 8 == 0:
+            if b <= 8 and persistent_ok(b, layer.hidden) and e % 8 == 0:
                 from ..ops.streaming import streaming_lstm_head_ce
                 return streaming_lstm_head_ce(frame_embeddings.transpose(0, 1).contiguous(), layer.weights_ih,
                                               layer.weights_hh, layer.bias_ih, layer.bias_hh, layer.h0, layer.c0,

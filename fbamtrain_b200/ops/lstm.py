@@ -2,7 +2,7 @@
 
 Forward: one tensor-core GEMM computes the input projection of all time steps
 (``X·W_ihᵀ + b_ih + b_hh``, fp32 out), then one persistent cooperative kernel runs the recurrence
-with ``W_hh`` resident in registers (``csrc/lstm.cu``).  Backward: one persistent kernel does BPTT and
+with ``W_hh`` resident on chip (``csrc/lstm.cu``).  Backward: one persistent kernel does BPTT and
 emits ``dGates`` for every step; the weight and input gradients are then three large GEMMs over all
 ``T·B`` rows (``dX = dGates·W_ih``, ``dW_ih = dGatesᵀ·X``, ``dW_hh = dGatesᵀ·H_prev``) and a column sum.
 The reference performs the same mathematics one step at a time with a GEMM per step and recomputes
@@ -10,7 +10,7 @@ the gates in the backward pass (reference: ``tensorlib/src/streaming_lstm_fwd.cp
 ``streaming_lstm_bwd.cpp:1218-1307``); here the activated gates are kept (in the buffer that held the
 pre-activations), so nothing is recomputed.
 
-Shapes beyond the persistent kernels' limits (hidden > 2048 or batch > 8) run step by step: a GEMM
+Shapes beyond the persistent kernels' limits (hidden > 2048 or not a multiple of 16) run step by step: a GEMM
 per step against ``W_hh`` followed by the same gate arithmetic.
 """
 from __future__ import annotations
@@ -24,18 +24,11 @@ from . import native as nv
 from . import reference as ref
 from .native_ops import gemm, gemm_nn, gemm_tn
 
-_scratch = {}
-
-
-def _counter(device) -> torch.Tensor:
-    key = ("ctr", device.index)
-    if key not in _scratch:
-        _scratch[key] = torch.zeros(1, dtype=torch.int32, device=device)
-    return _scratch[key]
-
 
 def persistent_ok(batch: int, hidden: int) -> bool:
-    return batch <= 8 and hidden % 16 == 0 and hidden <= nv.lib().fbam_lstm_persistent_max_hidden()
+    """Any batch: 32 rows per launch.  (Batch 32, 256 steps, H 1024, forward + backward: 2.9 ms against 107.9 ms
+    with a GEMM per step.)"""
+    return batch >= 1 and hidden % 16 == 0 and hidden <= nv.lib().fbam_lstm_persistent_max_hidden()
 
 
 class _LstmSequence(torch.autograd.Function):
@@ -50,11 +43,10 @@ class _LstmSequence(torch.autograd.Function):
         gates = gemm(x2, wi, bias=bias, out_dtype=torch.float32).view(t_len, b, 4 * h)
         y = torch.empty(t_len, b, h, dtype=x.dtype, device=dev)
         c_all = torch.empty(t_len, b, h, dtype=torch.float32, device=dev)
-        hbuf = torch.empty(2 * 8 * h, dtype=x.dtype, device=dev)
         h0f, c0f = h0.float().contiguous(), c0.float().contiguous()
         per_sample = int(h0.dim() == 2)
         nv.check(nv.lib(wh).fbam_lstm_fwd_ex(nv.ptr(gates), nv.ptr(wh), nv.ptr(h0f), nv.ptr(c0f), nv.ptr(y),
-                                           nv.ptr(c_all), nv.ptr(hbuf), nv.ptr(_counter(dev)),
+                                           nv.ptr(c_all), None, None,
                                            nv.ptr(nv.status_word(dev)), t_len, b, h, per_sample, nv.stream_ptr()),
                  "fbam_lstm_fwd")
         flops.add(2.0 * t_len * b * h * 4 * h)          # the recurrent product; the input projection is a counted GEMM
@@ -77,8 +69,8 @@ class _LstmSequence(torch.autograd.Function):
         dcl = None if dc_last is None else dc_last.float().contiguous()
         nv.check(nv.lib(wh).fbam_lstm_bwd_ex(nv.ptr(gates), nv.ptr(c_all), nv.ptr(c0f), nv.ptr(dy), nv.ptr(wh_t),
                                            nv.ptr(dgates), nv.ptr(dh0), nv.ptr(dc0), nv.ptr(dhl), nv.ptr(dcl),
-                                           nv.ptr(_counter(dev)), nv.ptr(nv.status_word(dev)), t_len, b, h,
-                                           ctx.per_sample, nv.stream_ptr()), "fbam_lstm_bwd")
+                                           None, nv.ptr(nv.status_word(dev)), t_len, b, h, ctx.per_sample,
+                                           nv.stream_ptr()), "fbam_lstm_bwd")
         flops.add(2.0 * t_len * b * h * 4 * h)
         dg2 = dgates.view(t_len * b, 4 * h)
         dx = gemm_nn(dg2, wi).view(t_len, b, i_dim) if ctx.needs_input_grad[0] else None

@@ -30,7 +30,7 @@ GEMM_ACC_NONE, GEMM_ACC_RMW, GEMM_ACC_ATOMIC = 0, 1, 2
 _ERRORS = {1: "unsupported shape", 2: "operand not 16-byte aligned", 3: "tensor-map encode failed",
            4: "driver entry point unavailable", 5: "kernel launch failed",
            101: "TMA producer wait timed out", 102: "MMA wait timed out", 103: "epilogue wait timed out",
-           201: "LSTM grid barrier timed out"}
+           201: "LSTM step exchange timed out"}
 
 
 class ConvGeom(C.Structure):

@@ -29,13 +29,12 @@ from . import native as nv
 from .native_ops import _colsum, gemm, gemm_nn, gemm_tn
 
 
-def _fwd_chunk(x2, wi, wh, bias, h_state, c_state, t_len, b, h, dev, counter):
+def _fwd_chunk(x2, wi, wh, bias, h_state, c_state, t_len, b, h, dev):
     gates = gemm(x2, wi, bias=bias, out_dtype=torch.float32).view(t_len, b, 4 * h)
     y = torch.empty(t_len, b, h, dtype=wh.dtype, device=dev)
     c_all = torch.empty(t_len, b, h, dtype=torch.float32, device=dev)
-    hbuf = torch.empty(2 * 8 * h, dtype=wh.dtype, device=dev)
     nv.check(nv.lib(wh).fbam_lstm_fwd_ex(nv.ptr(gates), nv.ptr(wh), nv.ptr(h_state), nv.ptr(c_state), nv.ptr(y),
-                                       nv.ptr(c_all), nv.ptr(hbuf), nv.ptr(counter), nv.ptr(nv.status_word(dev)),
+                                       nv.ptr(c_all), None, None, nv.ptr(nv.status_word(dev)),
                                        t_len, b, h, 1, nv.stream_ptr()), "fbam_lstm_fwd")
     return gates, y, c_all
 
@@ -49,7 +48,6 @@ class _StreamingLstmHeadCe(torch.autograd.Function):
         elem = w_head.dtype                       # the model's 16-bit compute type
         wi, wh = w_ih.to(elem), w_hh.to(elem)
         bias = (b_ih.float() + b_hh.float()).contiguous()
-        counter = torch.zeros(1, dtype=torch.int32, device=dev)
         h_state = h0.float().unsqueeze(0).expand(b, h).contiguous()
         c_state = c0.float().unsqueeze(0).expand(b, h).contiguous()
         loss = torch.zeros(1, dtype=torch.float32, device=dev)
@@ -65,7 +63,7 @@ class _StreamingLstmHeadCe(torch.autograd.Function):
             n = hi - lo
             boundary.append((h_state, c_state))
             x2 = x_c.to(elem).reshape(n * b, i_dim)
-            _, y, c_all = _fwd_chunk(x2, wi, wh, bias, h_state, c_state, n, b, h, dev, counter)
+            _, y, c_all = _fwd_chunk(x2, wi, wh, bias, h_state, c_state, n, b, h, dev)
             h_state, c_state = y[-1].float(), c_all[-1].clone()
             # per-chunk hook on its own stream: LM head + CE forward/backward for this chunk
             ce_stream.wait_stream(torch.cuda.current_stream())
@@ -97,7 +95,6 @@ class _StreamingLstmHeadCe(torch.autograd.Function):
         t_total, b, i_dim, h, chunk, offload = ctx.meta
         dev = wi.device
         x, dy_store = ctx.x, ctx.dy_store
-        counter = torch.zeros(1, dtype=torch.int32, device=dev)
         wh_t = wh.t().contiguous()
         dw_ih = torch.zeros(4 * h, i_dim, dtype=torch.float32, device=dev)
         dw_hh = torch.zeros(4 * h, h, dtype=torch.float32, device=dev)
@@ -114,14 +111,14 @@ class _StreamingLstmHeadCe(torch.autograd.Function):
             h_start, c_start = ctx.boundary[k]
             x2 = x_c.to(wi.dtype).reshape(n * b, i_dim)
             with flops.not_useful():                  # recomputation of what a resident run would have kept
-                gates, y, c_all = _fwd_chunk(x2, wi, wh, bias, h_start, c_start, n, b, h, dev, counter)
+                gates, y, c_all = _fwd_chunk(x2, wi, wh, bias, h_start, c_start, n, b, h, dev)
             dgates = torch.empty(n, b, 4 * h, dtype=wi.dtype, device=dev)
             dh0 = torch.empty(b, h, dtype=torch.float32, device=dev)
             dc0 = torch.empty(b, h, dtype=torch.float32, device=dev)
             nv.check(nv.lib(wh_t).fbam_lstm_bwd_ex(nv.ptr(gates), nv.ptr(c_all), nv.ptr(c_start), nv.ptr(dy_c.contiguous()),
                                                nv.ptr(wh_t), nv.ptr(dgates), nv.ptr(dh0), nv.ptr(dc0),
-                                               nv.ptr(dh_carry), nv.ptr(dc_carry), nv.ptr(counter),
-                                               nv.ptr(nv.status_word(dev)), n, b, h, 1, nv.stream_ptr()),
+                                               nv.ptr(dh_carry), nv.ptr(dc_carry), None, nv.ptr(nv.status_word(dev)),
+                                               n, b, h, 1, nv.stream_ptr()),
                      "fbam_lstm_bwd")
             dh_carry, dc_carry = dh0, dc0
             dg2 = dgates.view(n * b, 4 * h)

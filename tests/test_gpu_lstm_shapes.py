@@ -1,0 +1,106 @@
+"""The persistent recurrence at the edges of its launch rules — batch rows that fill groups of eight partly, several
+groups per block, several launches, hidden sizes on both sides of every block shape — and with a buffer that rules out
+the wide loads, against the fp32 PyTorch definition."""
+import math
+
+import pytest
+import torch
+
+from fbamtrain_b200.ops import reference as ref
+from fbamtrain_b200.utils.testing import assert_similar
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _problem(t_len, b, i_dim, h, dtype, per_sample=False):
+    g = torch.Generator(device=DEV).manual_seed(t_len * 1000 + b * 10 + h)
+    k = 1.0 / math.sqrt(h)
+
+    def uniform(*shape):
+        return ((torch.rand(shape, device=DEV, generator=g) * 2 - 1) * k).requires_grad_(True)
+
+    x = torch.randn(t_len, b, i_dim, device=DEV, generator=g).to(dtype).requires_grad_(True)
+    state = (b, h) if per_sample else (h,)
+    h0, c0 = ((0.1 * torch.randn(state, device=DEV, generator=g)).requires_grad_(True) for _ in range(2))
+    return (x, uniform(4 * h, i_dim), uniform(4 * h, h), uniform(4 * h), uniform(4 * h), h0, c0), g
+
+
+def _rel(a, e):
+    return float((a.float() - e).norm() / e.norm().clamp_min(1e-20))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("t_len,b,h", [
+    (1, 1, 16), (2, 3, 48), (5, 9, 16), (6, 17, 256), (4, 32, 256), (5, 33, 240),      # 8 units, up to four groups
+    (6, 8, 272), (5, 16, 272), (4, 25, 512), (7, 31, 496),                             # 16 units above one group
+    (5, 8, 528), (6, 9, 528), (5, 24, 1024), (9, 32, 1024), (4, 41, 1008),             # two groups, one or two turns
+    (4, 8, 1040), (5, 13, 1072), (4, 20, 2048), (6, 32, 2048),                         # one group, up to four turns
+])
+def test_batch_and_hidden_edges(t_len, b, h, dtype):
+    from fbamtrain_b200.ops import lstm as L, native as nv
+    params, g = _problem(t_len, b, 64, h, dtype)
+    assert L.persistent_ok(b, h)
+    y, h_n, c_n = L.lstm_sequence(*params, dtype)
+    dy = torch.randn(y.shape, device=DEV, generator=g).to(dtype)
+    got = torch.autograd.grad((y.float() * dy.float()).sum() + c_n.sum() + h_n.float().sum(), params)
+    nv.check_status(y.device)
+    fp = [p.detach().float().requires_grad_(True) for p in params]
+    yf, hf, cf = ref.lstm_sequence(*fp, torch.float32)
+    exp = torch.autograd.grad((yf * dy.float()).sum() + cf.sum() + hf.sum(), fp)
+    assert_similar(yf.to(dtype), y, 3e-2)
+    assert_similar(cf, c_n, 3e-2)
+    # weights, h and the gate gradients are rounded to the 16-bit type once per step (bf16: 2^-9 relative each)
+    for name, a, e in zip(["dx", "dw_ih", "dw_hh", "db_ih", "db_hh", "dh0", "dc0"], got, exp):
+        assert _rel(a, e) < 4e-2, (name, _rel(a, e))
+
+
+@pytest.mark.parametrize("b,h", [(3, 64), (12, 528)])
+def test_carried_state_per_sample(b, h):
+    from fbamtrain_b200.ops import lstm as L
+    params, _ = _problem(8, b, 64, h, torch.bfloat16, per_sample=True)
+    y, _, c_n = L.lstm_sequence(*params, torch.bfloat16)
+    head = [p.detach() for p in params]
+    y1, _, c1 = L.lstm_sequence(head[0][:5].contiguous(), *head[1:], torch.bfloat16)
+    y2, _, c2 = L.lstm_sequence(head[0][5:].contiguous(), *head[1:5], y1[-1].float(), c1, torch.bfloat16)
+    assert torch.equal(torch.cat([y1, y2]), y) and torch.equal(c2, c_n)
+
+
+def test_output_rows_without_16_byte_alignment():
+    """The C entry takes y and dGates at any element offset: two bytes off, the vectors are exchanged element by
+    element, with the same bits as a result."""
+    from fbamtrain_b200.ops import native as nv
+    t_len, b, h = 7, 5, 80
+    g = torch.Generator(device=DEV).manual_seed(3)
+    pre = torch.randn(t_len, b, 4 * h, device=DEV, generator=g)
+    whh = (torch.randn(4 * h, h, device=DEV, generator=g) / math.sqrt(h)).bfloat16()
+    h0, c0 = torch.randn(2, h, device=DEV, generator=g).unbind(0)
+    dy = torch.randn(t_len, b, h, device=DEV, generator=g).bfloat16()
+    status = nv.status_word(pre.device)
+    results = []
+    for shift in (0, 1):
+        gates = pre.clone()
+        y = torch.zeros(t_len * b * h + 8, dtype=torch.bfloat16, device=DEV)[shift:shift + t_len * b * h]
+        dg = torch.zeros(4 * t_len * b * h + 8, dtype=torch.bfloat16, device=DEV)[shift:shift + 4 * t_len * b * h]
+        c_all = torch.empty(t_len, b, h, device=DEV)
+        dh0, dc0 = torch.empty(2, b, h, device=DEV).unbind(0)
+        assert nv.lib().fbam_lstm_fwd(nv.ptr(gates), nv.ptr(whh), nv.ptr(h0), nv.ptr(c0), nv.ptr(y), nv.ptr(c_all), None,
+                                      None, nv.ptr(status), t_len, b, h, nv.stream_ptr()) == 0
+        whh_t = whh.t().contiguous()
+        assert nv.lib().fbam_lstm_bwd(nv.ptr(gates), nv.ptr(c_all), nv.ptr(c0), nv.ptr(dy), nv.ptr(whh_t), nv.ptr(dg),
+                                      nv.ptr(dh0), nv.ptr(dc0), None, None, None, nv.ptr(status), t_len, b, h,
+                                      nv.stream_ptr()) == 0
+        nv.check_status(pre.device)
+        results.append([t.clone() for t in (gates, y, c_all, dg, dh0, dc0)])
+    for a, e in zip(results[1], results[0]):
+        assert torch.equal(a, e)
+
+
+def test_nan_travels_through_the_exchange():
+    """A NaN hidden value is data, not an unwritten word: the recurrence goes on and the NaN reaches the outputs."""
+    from fbamtrain_b200.ops import lstm as L, native as nv
+    params, _ = _problem(6, 2, 64, 64, torch.bfloat16)
+    params[0].data[2, 1] = float("nan")
+    y, _, c_n = L.lstm_sequence(*params, torch.bfloat16)
+    nv.check_status(y.device)
+    assert torch.isfinite(y[:, 0].float()).all() and torch.isnan(y[2:, 1].float()).all() and torch.isnan(c_n[1]).all()
