@@ -10,11 +10,10 @@
 // O ← O·exp2(m_old − m_new) + P·V.  The log-sum-exp per row is stored for the backward pass.
 //
 // Backward: one CTA per (batch, head, block of 128 keys) walks the query blocks that attend to it and, per
-// block, issues five tcgen05 GEMMs: S = Q·Kᵀ and dP = dO·Vᵀ into TMEM, then — after the 128 threads rebuilt
-// P = exp2(scale·S − lse) and dS = P∘(dP − δ) in shared memory — dV += Pᵀ·dO, dK += dSᵀ·Q (accumulating in
-// TMEM across query blocks; P and dS are read as MN-major A operands, i.e. transposed for free) and
-// dQ_block = dS·K, which is added into an fp32 dQ buffer with atomics.  δ = rowsum(dO∘O) comes from a small
-// pre-pass kernel.
+// block, issues five tcgen05 GEMMs: S = Q·Kᵀ and dP = dO·Vᵀ into TMEM, then — from P = exp2(scale·S − lse) and
+// dS = P∘(dP − δ) in shared memory — dV += Pᵀ·dO, dK += dSᵀ·Q (accumulating in TMEM across query blocks; P and dS
+// are read as MN-major A operands, i.e. transposed for free) and dQ_block = dS·K, which is added into an fp32 dQ
+// buffer with vector reductions.  δ = rowsum(dO∘O) comes from a small pre-pass kernel.
 //
 // Q/K/V/O/dO are addressed as (B, T, H, D) views with arbitrary batch / row / head strides (the fused QKV
 // projection output is used in place).  All mbarrier waits are bounded.
@@ -54,6 +53,13 @@ __device__ __forceinline__ float fast_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+
+// Arrival of a whole warp (one per warp: 32 arrivals on one barrier would be served one after the other): every lane
+// has fenced its own accesses before.
+__device__ __forceinline__ void warp_arrive(uint64_t* bar) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
 }
 
 // Address of element (row, col8 = 8-element group index) in a [rows x 64]-bf16 panel with 128-byte swizzle.
@@ -284,6 +290,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 // accumulators stay in tensor memory for the whole key loop (every P·V product adds to them); the softmax threads
 // rescale them there only when a row's reference maximum moves (see below), so a group goes from one block's softmax
 // straight to the next while its P·V product is still running.
+// A group's scores are read from TMEM once and masked in a pass of their own; with masks inside the loops and two reads
+// the kernel took 123 us at B8 T1024 H16 D64 causal (now 65) and 56 us at B16 T480 H8 D128 (now 36).
 template <int D>
 __global__ void __launch_bounds__(288, 1)
 attn_fwd2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -336,7 +344,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     mbar_init(v_empty, 1);
     for (int g = 0; g < 2; ++g) {
       mbar_init(&s_full[g], 1);
-      mbar_init(&p_ready[g], 128);
+      mbar_init(&p_ready[g], 4);
       mbar_init(&pv_full[g], 1);
     }
     mbar_fence_init();
@@ -454,27 +462,24 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       if (!mbar_wait(&s_full[g], kb & 1)) { ok = false; break; }
       fence_after_sync();
       const int k0 = kb * BKV;
-      const bool need_mask = (p.causal && kb == qb) || (k0 + BKV > p.T);
-      // row maximum of this block: two 32-column chunks per TMEM round trip, four independent comparison chains
-      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll 1
-      for (int c0 = 0; c0 < BKV; c0 += 64) {
-        uint32_t ra[32], rb[32];
-        tmem_ld_32x32(tmem_s + lane_addr + c0, ra);
-        tmem_ld_32x32(tmem_s + lane_addr + c0 + 32, rb);
-        tmem_ld_wait();
+      // keys of this block that the row sees: [0, vis)
+      int vis = BKV;
+      if ((p.causal && kb == qb) || (k0 + BKV > p.T)) vis = min(BKV, (p.causal ? min(p.T, t_q + 1) : p.T) - k0);
+      // The row's scores, read from tensor memory once (registers for all 128).  Masking is a pass of its own that
+      // only the last blocks of a row take: as a condition inside the loops below it cost every block four
+      // instructions per score.
+      uint32_t r[BKV];
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          float sa = __uint_as_float(ra[j]), sb = __uint_as_float(rb[j]);
-          if (need_mask) {
-            const int tk = k0 + c0 + j;
-            if (tk >= p.T || (p.causal && tk > t_q)) sa = -INFINITY;
-            if (tk + 32 >= p.T || (p.causal && tk + 32 > t_q)) sb = -INFINITY;
-          }
-          mx4[j & 1] = fmaxf(mx4[j & 1], sa);
-          mx4[2 + (j & 1)] = fmaxf(mx4[2 + (j & 1)], sb);
-        }
+      for (int c0 = 0; c0 < BKV; c0 += 32) tmem_ld_32x32(tmem_s + lane_addr + c0, *reinterpret_cast<uint32_t(*)[32]>(r + c0));
+      tmem_ld_wait();
+      if (vis < BKV) {
+#pragma unroll
+        for (int j = 0; j < BKV; ++j)
+          if (j >= vis) r[j] = 0xff800000u;      // -inf
       }
+      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int j = 0; j < BKV; ++j) mx4[j & 3] = fmaxf(mx4[j & 3], __uint_as_float(r[j]));
       const float m_blk = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
       const bool grow = (m_blk - m) * p.scale_log2 > 8.0f;      // true on the first block (m = -inf) of any visible key
       float alpha = 1.0f;
@@ -492,16 +497,16 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         const float2 a2 = make_float2(alpha, alpha);
 #pragma unroll 1
         for (int c0 = 0; c0 < D; c0 += 32) {
-          uint32_t r[32];
-          tmem_ld_32x32(tmem_pv + lane_addr + c0, r);
+          uint32_t ro[32];
+          tmem_ld_32x32(tmem_pv + lane_addr + c0, ro);
           tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 32; j += 2) {
-            const float2 v = __fmul2_rn(make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), a2);
-            r[j] = __float_as_uint(v.x);
-            r[j + 1] = __float_as_uint(v.y);
+            const float2 v = __fmul2_rn(make_float2(__uint_as_float(ro[j]), __uint_as_float(ro[j + 1])), a2);
+            ro[j] = __float_as_uint(v.x);
+            ro[j + 1] = __float_as_uint(v.y);
           }
-          tmem_st_32x32(tmem_pv + lane_addr + c0, r);
+          tmem_st_32x32(tmem_pv + lane_addr + c0, ro);
         }
         tmem_st_wait();
       }
@@ -511,37 +516,23 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       const float nm = -m_use * p.scale_log2;
       const float2 nm2 = make_float2(nm, nm);
       float2 rs2 = make_float2(0.0f, 0.0f), rs2b = make_float2(0.0f, 0.0f);
-#pragma unroll 1
-      for (int c0 = 0; c0 < BKV; c0 += 32) {
-        uint32_t r[32];
-        tmem_ld_32x32(tmem_s + lane_addr + c0, r);
-        tmem_ld_wait();
 #pragma unroll
-        for (int j8 = 0; j8 < 4; ++j8) {
-          __align__(16) elem2_t hh[4];
+      for (int chunk = 0; chunk < BKV / 8; ++chunk) {
+        __align__(16) elem2_t hh[4];
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int j = j8 * 8 + 2 * q;
-            float2 sv = make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1]));
-            if (need_mask) {
-              const int tk = k0 + c0 + j;
-              if (tk >= p.T || (p.causal && tk > t_q)) sv.x = -INFINITY;
-              if (tk + 1 >= p.T || (p.causal && tk + 1 > t_q)) sv.y = -INFINITY;
-            }
-            const float2 e = __ffma2_rn(sv, sc2, nm2);
-            const float2 pe = make_float2(fast_exp2(e.x), fast_exp2(e.y));
-            if (q & 1) rs2b = __fadd2_rn(rs2b, pe); else rs2 = __fadd2_rn(rs2, pe);
-            hh[q] = f22e2(pe);
-          }
-          const int chunk = (c0 >> 3) + j8;
-          uint8_t* dst = sPg + (chunk >> 3) * BQ * 128 + swz(row, chunk & 7);
-          *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<uint4*>(hh);
+        for (int q = 0; q < 4; ++q) {
+          const int j = chunk * 8 + 2 * q;
+          const float2 e = __ffma2_rn(make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), sc2, nm2);
+          const float2 pe = make_float2(fast_exp2(e.x), fast_exp2(e.y));
+          if (q & 1) rs2b = __fadd2_rn(rs2b, pe); else rs2 = __fadd2_rn(rs2, pe);
+          hh[q] = f22e2(pe);
         }
+        *reinterpret_cast<uint4*>(sPg + (chunk >> 3) * BQ * 128 + swz(row, chunk & 7)) = *reinterpret_cast<uint4*>(hh);
       }
       l = l * alpha + ((rs2.x + rs2.y) + (rs2b.x + rs2b.y));
       fence_proxy_async();
       fence_before_sync();
-      mbar_arrive(&p_ready[g]);
+      warp_arrive(&p_ready[g]);
     }
     if (ok && my_nkb > 0) {
       // the last P·V product completes the output rows in tensor memory: divide by the row sum and store
@@ -581,141 +572,242 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 }
 
 // -------------------------------------------------------------------------------------------------
-// backward pre-pass: delta[b,h,t] = sum_d dO*O
+// backward pre-pass: delta[b,h,t] = sum_d dO*O.  D / 8 lanes per row, 16-byte loads: DRAM-bound (the two tensors are
+// read once).  28 us -> 9 us at B8 T1024 H16 D64 (a warp per row with 4-byte loads before).
 // -------------------------------------------------------------------------------------------------
+template <int D>
 __global__ void attn_delta_kernel(const elem_t* __restrict__ o, const elem_t* __restrict__ d_o, float* __restrict__ delta,
-                                  int B, int T, int H, int D, long long do_sb, long long do_st, long long do_sh) {
-  const long long idx = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);   // (b, t, h) row
-  const int lane = threadIdx.x & 31;
-  if (idx >= (long long)B * T * H) return;
+                                  int B, int T, int H, long long do_sb, long long do_st, long long do_sh) {
+  constexpr int kLanes = D / 8;
+  const long long idx = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / kLanes;   // (b, t, h) row
+  const int part = threadIdx.x % kLanes;
+  const bool on = idx < (long long)B * T * H;
+  float s = 0.0f;
   const int hh = (int)(idx % H);
   const long long bt = idx / H;
-  const int t = (int)(bt % T);
-  const int b = (int)(bt / T);
-  const elem_t* orow = o + idx * D;
-  const elem_t* drow = d_o + b * do_sb + t * do_st + hh * do_sh;
-  float s = 0.0f;
-  for (int d = lane * 2; d < D; d += 64) {
-    const float2 a = e22ff(*reinterpret_cast<const elem2_t*>(orow + d));
-    const float2 g = e22ff(*reinterpret_cast<const elem2_t*>(drow + d));
-    s += a.x * g.x + a.y * g.y;
+  const int t = (int)(bt % T), b = (int)(bt / T);
+  if (on) {
+    const uint4 ov = *reinterpret_cast<const uint4*>(o + idx * D + part * 8);
+    const uint4 gv = *reinterpret_cast<const uint4*>(d_o + b * do_sb + t * do_st + hh * do_sh + part * 8);
+    const elem2_t* oe = reinterpret_cast<const elem2_t*>(&ov);
+    const elem2_t* ge = reinterpret_cast<const elem2_t*>(&gv);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 x = e22ff(oe[i]), y = e22ff(ge[i]);
+      s += x.x * y.x + x.y * y.y;
+    }
   }
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-  if (lane == 0) delta[((long long)b * H + hh) * T + t] = s;
+  for (int off = kLanes / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+  if (on && part == 0) delta[((long long)b * H + hh) * T + t] = s;
+}
+
+// The fp32 sums of dQ are kept by (batch, head, query block) as [D / 4 pieces][128 rows][4]: the threads that add to them
+// own one row each, and in this order a warp's 16-byte reductions cover 512 consecutive bytes.  In row order they touch
+// 32 different lines per instruction, which kept the load/store unit busy for 2700 (D = 64) and 5700 cycles per block
+// and delayed every shared-memory store behind it.  This kernel turns a block into 16-bit rows of a strided view.
+template <int D>
+__global__ void __launch_bounds__(256) attn_dq_store_kernel(const float4* __restrict__ src, elem_t* __restrict__ dst, int T, int H,
+                                                            int nqb, long long sb, long long st, long long sh) {
+  constexpr int kLd = D + 8;   // 16-byte pieces of 8 rows on different banks
+  __shared__ __align__(16) elem_t tile[128 * kLd];
+  const int qb = blockIdx.x % nqb;
+  const long long bh = blockIdx.x / nqb;
+  const float4* in = src + (long long)blockIdx.x * (D / 4) * 128;
+#pragma unroll
+  for (int i = threadIdx.x; i < 128 * D / 4; i += 256) {
+    const float4 v = in[i];
+    __align__(8) elem2_t e[2] = {ff2e2(v.x, v.y), ff2e2(v.z, v.w)};
+    *reinterpret_cast<uint2*>(tile + (i % 128) * kLd + (i / 128) * 4) = *reinterpret_cast<uint2*>(e);
+  }
+  __syncthreads();
+  elem_t* out = dst + bh / H * sb + bh % H * sh;
+#pragma unroll
+  for (int i = threadIdx.x; i < 128 * D / 8; i += 256) {
+    const int row = i / (D / 8), d = i % (D / 8) * 8, t = qb * 128 + row;
+    if (t < T) *reinterpret_cast<uint4*>(out + t * st + d) = *reinterpret_cast<const uint4*>(tile + row * kLd + d);
+  }
 }
 
 // -------------------------------------------------------------------------------------------------
 // backward main kernel
 // -------------------------------------------------------------------------------------------------
+// One CTA per (batch, head, 128 keys) walks the query blocks.  The five products of a block and the point-wise work
+// between them form a cycle; what bounds the kernel is how much of that cycle overlaps.  Roles:
+//   warp 21     TMA: K, V once; Q two blocks deep; dO two blocks deep (D = 64) or one (D = 128: shared memory is full)
+//   warp 20     MMA issue, in the order  S(i+1), dV(i)  once P(i) is stored, then  dP(i+1), dQ(i), dK(i)  (D = 64) or
+//               dQ(i), dK(i), dP(i+1)  (D = 128, where dQ borrows dP's columns) once dS(i) is stored: while the tensor
+//               core works on block i, the point-wise warps already have S(i+1)
+//   warps 4-19  point-wise: P = exp2(scale·S − lse) -> shared memory, then dS = P∘(dP − δ)·scale -> shared memory; four
+//               threads per query row, 32 keys each, and the row statistics fetched one block ahead
+//   warps 0-3   drain dQ from tensor memory into the fp32 sums (16-byte reductions), off everybody else's path
+// Every barrier that a role waits on can complete its next phase only after that role has gone on (Q and dO have one
+// "free" barrier per stage for this reason), so a wait by phase parity cannot miss a phase.
+// Tensor memory: S 128 | dP 128 | dV D | dK D | (D = 64) dQ 64 columns.
+//
+// Before, one group of four warps did load, products, point-wise work and drain in turn: at B8 T1024 H16 D64 causal
+// 291 us, now 108 us; at B16 T480 H8 D128 197 us, now 82 us.
 struct AttnBwdParams {
-  int B, T, H, D;
+  int B, T, H;
   int causal;
   float scale_log2, scale;
   const float* lse;    // (B, H, T)
   const float* delta;  // (B, H, T)
-  float* dq;           // (B, T, H, D) fp32, zero-initialised; atomically accumulated
-  elem_t* dk;            // (B, T, H, D) contiguous
+  float4* dq;          // (B, H, query block, D / 4, 128 rows) fp32, zero-initialised; accumulated with reductions
+  elem_t* dk;          // (B, T, H, D) views with strides g_sb, g_st, g_sh
   elem_t* dv;
+  long long g_sb, g_st, g_sh;
   int* status;
 };
 
+constexpr int kBwdWarps = 22, kBwdThreads = kBwdWarps * 32;
+
 template <int D>
-__global__ void __launch_bounds__(160, 1)
+constexpr int kBwdDoStages = D == 64 ? 2 : 1;
+template <int D>
+constexpr int kBwdPBuffers = D == 64 ? 2 : 1;
+template <int D>
+constexpr int bwd_smem_bytes() { return (4 + kBwdDoStages<D>) * 128 * D * 2 + (1 + kBwdPBuffers<D>) * 128 * 128 * 2 + 256 + 1024; }
+
+template <int D>
+__global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                 const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
                 const AttnBwdParams p) {
   constexpr int DP = D / 64;
   constexpr int kTile = 128 * D * 2;           // a 128-row x D operand tile
   constexpr int kSq = 128 * 128 * 2;           // P / dS tiles
-  // TMEM columns: S [0,128) — reused for dQ after S has been read; dP [128,256); dV [256,256+D); dK [256+D, 256+2D)
+  constexpr int kDoStages = kBwdDoStages<D>;
+  constexpr int kPBuffers = kBwdPBuffers<D>;
+  constexpr bool kOwnDq = D == 64;             // dQ has tensor-memory columns of its own
   constexpr uint32_t kTmemCols = 512;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sK = smem;
   uint8_t* sV = sK + kTile;
-  uint8_t* sQ = sV + kTile;
-  uint8_t* sDO = sQ + kTile;
-  uint8_t* sP = sDO + kTile;
-  uint8_t* sDS = sP + kSq;
+  uint8_t* sQ = sV + kTile;                    // two stages
+  uint8_t* sDO = sQ + 2 * kTile;               // kDoStages stages
+  uint8_t* sP = sDO + kDoStages * kTile;
+  uint8_t* sDS = sP + kPBuffers * kSq;         // P: kPBuffers buffers
   uint64_t* bars = reinterpret_cast<uint64_t*>(sDS + kSq);
   uint64_t* kv_full = bars;
-  uint64_t* qdo_full = bars + 1;
-  uint64_t* sdp_full = bars + 2;    // S and dP are in TMEM
-  uint64_t* pds_ready = bars + 3;   // P and dS are in smem (128 arrivals)
-  uint64_t* dq_full = bars + 4;     // dV/dK accumulated, dQ block in TMEM
-  uint64_t* dq_read = bars + 5;     // 128 arrivals: dQ consumed, operands may be overwritten
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 6);
+  uint64_t* q_full = bars + 1;      // [2]
+  uint64_t* do_full = bars + 3;     // [2]
+  uint64_t* q_free = bars + 5;      // [2] dK(i) has read the stage
+  uint64_t* do_free = bars + 7;     // [2] dV(i) has read the stage
+  uint64_t* s_full = bars + 9;      // S(i) in tensor memory
+  uint64_t* dp_full = bars + 10;    // dP(i) in tensor memory
+  uint64_t* p_ready = bars + 11;    // P(i) stored, S(i) read (16 warps)
+  uint64_t* ds_ready = bars + 12;   // dS(i) stored, dP(i) read (16 warps)
+  uint64_t* dv_done = bars + 13;    // [2] dV(i) has read the P buffer
+  uint64_t* dq_full = bars + 15;    // dQ(i) in tensor memory
+  uint64_t* dq_read = bars + 16;    // dQ(i) drained (4 warps)
+  uint64_t* dk_done = bars + 17;    // dQ(i) and dK(i) have read dS; all products so far are complete
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kb = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  // causal: the key blocks with the most query blocks first, over all heads
+  const int kb = p.causal ? blockIdx.z : blockIdx.x;
+  const int h = p.causal ? blockIdx.x : blockIdx.y;
+  const int b = p.causal ? blockIdx.y : blockIdx.z;
   const int k0 = kb * BKV;
-  const int nqb = (p.T + BQ - 1) / BQ;
-  const int qb_begin = p.causal ? kb : 0;
+  const int qb0 = p.causal ? kb : 0;
+  const int nqb = (p.T + BQ - 1) / BQ, n = nqb - qb0;     // query blocks; at least one of them ours
 
   if (threadIdx.x == 0) {
     prefetch_tensormap(&map_q); prefetch_tensormap(&map_k); prefetch_tensormap(&map_v); prefetch_tensormap(&map_do);
-    mbar_init(kv_full, 1); mbar_init(qdo_full, 1); mbar_init(sdp_full, 1);
-    mbar_init(pds_ready, 128); mbar_init(dq_full, 1); mbar_init(dq_read, 128);
+    for (int i = 0; i < 18; ++i) mbar_init(&bars[i], i == 11 || i == 12 ? 16 : i == 16 ? 4 : 1);
     mbar_fence_init();
   }
-  if (warp == 0) { tmem_alloc(tmem_slot, kTmemCols); tmem_relinquish(); }
+  if (warp == 20) { tmem_alloc(tmem_slot, kTmemCols); tmem_relinquish(); }
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t tm_s = tmem, tm_dp = tmem + 128, tm_dv = tmem + 256, tm_dk = tmem + 256 + D, tm_dq = tmem;
+  const uint32_t tm_s = tmem, tm_dp = tmem + 128, tm_dv = tmem + 256, tm_dk = tmem + 256 + D;
+  const uint32_t tm_dq = kOwnDq ? tmem + 256 + 2 * D : tm_dp;
 
-  if (warp == 0) {
+  if (warp == 21) {
     if (elect_one()) {
       bool ok = true;
-      mbar_expect_tx(kv_full, 2 * kTile);
+      auto load = [&](uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int t) {
 #pragma unroll
-      for (int j = 0; j < DP; ++j) {
-        tma_load_attn(sK + j * 128 * 128, &map_k, kv_full, j * 64, h, k0, b);
-        tma_load_attn(sV + j * 128 * 128, &map_v, kv_full, j * 64, h, k0, b);
+        for (int j = 0; j < DP; ++j) tma_load_attn(dst + j * 128 * 128, map, bar, j * 64, h, t, b);
+      };
+      auto load_q = [&](int i) {
+        if (i >= 2 && !mbar_wait(&q_free[i & 1], ((i >> 1) - 1) & 1)) { ok = false; return; }
+        mbar_expect_tx(&q_full[i & 1], kTile);
+        load(sQ + (i & 1) * kTile, &map_q, &q_full[i & 1], (qb0 + i) * BQ);
+      };
+      auto load_do = [&](int i) {
+        const int s = i % kDoStages;
+        if (i >= kDoStages && !mbar_wait(&do_free[s], (i / kDoStages - 1) & 1)) { ok = false; return; }
+        mbar_expect_tx(&do_full[s], kTile);
+        load(sDO + s * kTile, &map_do, &do_full[s], (qb0 + i) * BQ);
+      };
+      mbar_expect_tx(kv_full, 2 * kTile);
+      load(sK, &map_k, kv_full, k0);
+      load_q(0);
+      load(sV, &map_v, kv_full, k0);
+      load_do(0);
+      if (n > 1) load_q(1);
+      for (int i = 1; i < n && ok; ++i) {
+        load_do(i);
+        if (ok && i + 1 < n) load_q(i + 1);
       }
+      if (!ok) atomicExch(p.status, ATT_ERR_TIMEOUT);
+    }
+  } else if (warp == 20) {
+    if (elect_one()) {
+      bool ok = true;
       const uint32_t id_s = make_idesc_f16kind(128, 128, false, false);   // S = Q Kᵀ, dP = dO Vᵀ
       const uint32_t id_t = make_idesc_f16kind(128, D, true, true);       // dV = Pᵀ dO, dK = dSᵀ Q (A, B MN-major)
       const uint32_t id_q = make_idesc_f16kind(128, D, false, true);      // dQ = dS K (B MN-major)
+      const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aP = smem_u32(sP), aDS = smem_u32(sDS);
+      auto scores = [&](uint32_t d, uint32_t a, uint32_t bb) {            // both operands K-major over D
+#pragma unroll
+        for (int k = 0; k < D / 16; ++k) {
+          const uint32_t off = (k / 4) * 128 * 128 + (k % 4) * 32;
+          mma_f16_ss(d, make_smem_desc_sw128(a + off, 16, 1024), make_smem_desc_sw128(bb + off, 16, 1024), id_s, k != 0);
+        }
+      };
+      auto transposed = [&](uint32_t d, uint32_t a, uint32_t bb, bool first) {
+        // K dimension = queries, 16 rows per step.  A (P or dS) is [query rows][keys]: as an MN-major operand its M =
+        // keys; two 64-key panels, LBO = panel
+#pragma unroll
+        for (int k = 0; k < 128 / 16; ++k)
+          mma_f16_ss(d, make_smem_desc_sw128(a + k * 16 * 128, 128 * 128, 1024),
+                     make_smem_desc_sw128(bb + k * 16 * 128, 128 * 128, 1024), id_t, !first || k != 0);
+      };
+      auto issue_s = [&](int i) {
+        if (!mbar_wait(&q_full[i & 1], (i >> 1) & 1)) { ok = false; return; }
+        fence_after_sync();
+        scores(tm_s, smem_u32(sQ + (i & 1) * kTile), aK);
+        mma_commit(s_full);
+      };
+      auto issue_dp = [&](int i) {
+        if (!mbar_wait(&do_full[i % kDoStages], (i / kDoStages) & 1)) { ok = false; return; }
+        fence_after_sync();
+        scores(tm_dp, smem_u32(sDO + (i % kDoStages) * kTile), aV);
+        mma_commit(dp_full);
+      };
       ok = mbar_wait(kv_full, 0);
-      int it = 0;
-      for (int qb = qb_begin; qb < nqb && ok; ++qb, ++it) {
-        if (it > 0 && !mbar_wait(dq_read, (it - 1) & 1)) { ok = false; break; }   // previous block fully consumed
-        mbar_expect_tx(qdo_full, 2 * kTile);
-#pragma unroll
-        for (int j = 0; j < DP; ++j) {
-          tma_load_attn(sQ + j * 128 * 128, &map_q, qdo_full, j * 64, h, qb * BQ, b);
-          tma_load_attn(sDO + j * 128 * 128, &map_do, qdo_full, j * 64, h, qb * BQ, b);
-        }
-        if (!mbar_wait(qdo_full, it & 1)) { ok = false; break; }
+      if (ok) issue_s(0);
+      if (ok) issue_dp(0);
+      for (int i = 0; i < n && ok; ++i) {
+        if (!mbar_wait(p_ready, i & 1)) { ok = false; break; }
         fence_after_sync();
-        const uint32_t aQ = smem_u32(sQ), aK = smem_u32(sK), aV = smem_u32(sV), aDO = smem_u32(sDO);
-        const uint32_t aP = smem_u32(sP), aDS = smem_u32(sDS);
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t off = (k / 4) * 128 * 128 + (k % 4) * 32;
-          mma_f16_ss(tm_s, make_smem_desc_sw128(aQ + off, 16, 1024), make_smem_desc_sw128(aK + off, 16, 1024), id_s,
-                     k != 0);
-        }
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t off = (k / 4) * 128 * 128 + (k % 4) * 32;
-          mma_f16_ss(tm_dp, make_smem_desc_sw128(aDO + off, 16, 1024), make_smem_desc_sw128(aV + off, 16, 1024), id_s,
-                     k != 0);
-        }
-        mma_commit(sdp_full);
-        if (!mbar_wait(pds_ready, it & 1)) { ok = false; break; }
+        if (i + 1 < n) issue_s(i + 1);
+        if (!ok) break;
+        transposed(tm_dv, aP + (i % kPBuffers) * kSq, smem_u32(sDO + (i % kDoStages) * kTile), i == 0);
+        mma_commit(&dv_done[i % kPBuffers]);
+        mma_commit(&do_free[i % kDoStages]);
+        if (!mbar_wait(ds_ready, i & 1)) { ok = false; break; }
         fence_after_sync();
-#pragma unroll
-        for (int k = 0; k < 128 / 16; ++k) {   // K dimension = queries: 16 rows of P / dS / dO / Q per step
-          // A (P or dS) is [query rows][keys]: as an MN-major operand its M = keys; two 64-key panels, LBO = panel
-          const uint64_t a_p = make_smem_desc_sw128(aP + k * 16 * 128, 128 * 128, 1024);
-          const uint64_t a_ds = make_smem_desc_sw128(aDS + k * 16 * 128, 128 * 128, 1024);
-          const uint64_t b_do = make_smem_desc_sw128(aDO + k * 16 * 128, 128 * 128, 1024);
-          const uint64_t b_q = make_smem_desc_sw128(aQ + k * 16 * 128, 128 * 128, 1024);
-          mma_f16_ss(tm_dv, a_p, b_do, id_t, (it | k) != 0);
-          mma_f16_ss(tm_dk, a_ds, b_q, id_t, (it | k) != 0);
+        if (kOwnDq) {
+          if (i + 1 < n) issue_dp(i + 1);
+          if (!ok || (i > 0 && !mbar_wait(dq_read, (i - 1) & 1))) { ok = false; break; }
+          fence_after_sync();
         }
 #pragma unroll
         for (int k = 0; k < 128 / 16; ++k) {   // dQ = dS (K-major over keys) · K (MN-major: key rows, D contiguous)
@@ -724,109 +816,156 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           mma_f16_ss(tm_dq, a_ds, b_k, id_q, k != 0);
         }
         mma_commit(dq_full);
+        transposed(tm_dk, aDS, smem_u32(sQ + (i & 1) * kTile), i == 0);
+        mma_commit(dk_done);
+        mma_commit(&q_free[i & 1]);
+        if (!kOwnDq && i + 1 < n) {
+          if (!mbar_wait(dq_read, i & 1)) { ok = false; break; }
+          fence_after_sync();
+          issue_dp(i + 1);
+        }
       }
       if (!ok) atomicExch(p.status, ATT_ERR_TIMEOUT);
     }
-  } else {
-    const int lane_group = warp & 3;
+  } else if (warp >= 4) {
+    // ---------------------------------------------------------------- point-wise: one query row, 32 keys per thread
+    const int lane_group = warp & 3, part = (warp - 4) >> 2;
     const int row = lane_group * 32 + lane;
     const uint32_t lane_addr = uint32_t(lane_group * 32) << 16;
+    const long long stat0 = ((long long)b * p.H + h) * p.T;
+    const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
+    uint8_t* pRow = sP + (part >> 1) * 128 * 128;      // the 64-key panel
+    uint8_t* dsRow = sDS + (part >> 1) * 128 * 128;
+    const int chunk0 = (part & 1) * 4;                 // first 16-byte piece of the panel row
     bool ok = true;
-    int it = 0;
-    for (int qb = qb_begin; qb < nqb; ++qb, ++it) {
-      const int t_q = qb * BQ + row;
+    float lse_next = 0.0f, dl_next = 0.0f;             // statistics of the next block: fetched one block ahead
+    if (qb0 * BQ + row < p.T) {
+      lse_next = p.lse[stat0 + qb0 * BQ + row];
+      dl_next = p.delta[stat0 + qb0 * BQ + row];
+    }
+    for (int i = 0; i < n; ++i) {
+      const int t_q = (qb0 + i) * BQ + row;
       const bool row_ok = t_q < p.T;
-      const long long stat_idx = ((long long)b * p.H + h) * p.T + t_q;
-      const float lse = row_ok ? p.lse[stat_idx] : 0.0f;
-      const float dl = row_ok ? p.delta[stat_idx] : 0.0f;
-      if (!mbar_wait(sdp_full, it & 1)) { ok = false; break; }
+      const float lse = lse_next, dl = dl_next;
+      if (t_q + BQ < p.T) {
+        lse_next = p.lse[stat0 + t_q + BQ];
+        dl_next = p.delta[stat0 + t_q + BQ];
+      }
+      const float nl = -lse * 1.4426950408889634f;
+      const float2 nl2 = make_float2(nl, nl);
+      // keys of this thread that the row sees: [0, vis)
+      int vis = 32;
+      if ((p.causal && i == 0) || (k0 + BKV > p.T) || !row_ok) {
+        const int lim = !row_ok ? 0 : (p.causal ? min(p.T, t_q + 1) : p.T);
+        vis = min(32, max(0, lim - (k0 + part * 32)));
+      }
+      if (!mbar_wait(s_full, i & 1)) { ok = false; break; }
       fence_after_sync();
-      const bool need_mask = (p.causal && qb == kb) || (k0 + BKV > p.T) || !row_ok;
-#pragma unroll 1
-      for (int c0 = 0; c0 < BKV; c0 += 32) {
-        uint32_t rs[32], rd[32];
-        tmem_ld_32x32(tm_s + lane_addr + c0, rs);
-        tmem_ld_32x32(tm_dp + lane_addr + c0, rd);
-        tmem_ld_wait();
+      uint32_t r[32];
+      float pr[32];
+      tmem_ld_32x32(tm_s + lane_addr + part * 32, r);
+      tmem_ld_wait();
 #pragma unroll
-        for (int j8 = 0; j8 < 4; ++j8) {
-          __align__(16) elem2_t hp[4], hd[4];
+      for (int j = 0; j < 32; j += 2) {
+        const float2 e = __ffma2_rn(make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), sc2, nl2);
+        pr[j] = fast_exp2(e.x);
+        pr[j + 1] = fast_exp2(e.y);
+      }
+      if (vis < 32) {
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            float pe[2], de[2];
+        for (int j = 0; j < 32; ++j)
+          if (j >= vis) pr[j] = 0.0f;
+      }
+      // dV(i - kPBuffers) has read the buffer
+      if (i >= kPBuffers && !mbar_wait(&dv_done[i % kPBuffers], (i / kPBuffers - 1) & 1)) { ok = false; break; }
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const int j = j8 * 8 + 2 * q + e;
-              const int tk = k0 + c0 + j;
-              float pr = fast_exp2(__uint_as_float(rs[j]) * p.scale_log2 - lse * 1.4426950408889634f);
-              if (need_mask && (!row_ok || tk >= p.T || (p.causal && tk > t_q))) pr = 0.0f;
-              pe[e] = pr;
-              de[e] = pr * (__uint_as_float(rd[j]) - dl) * p.scale;
-            }
-            hp[q] = ff2e2(pe[0], pe[1]);
-            hd[q] = ff2e2(de[0], de[1]);
-          }
-          const int chunk = (c0 >> 3) + j8;
-          const uint32_t off = (chunk >> 3) * 128 * 128 + swz(row, chunk & 7);
-          *reinterpret_cast<uint4*>(sP + off) = *reinterpret_cast<uint4*>(hp);
-          *reinterpret_cast<uint4*>(sDS + off) = *reinterpret_cast<uint4*>(hd);
-        }
+      for (int j8 = 0; j8 < 4; ++j8) {
+        __align__(16) elem2_t hp[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) hp[q] = ff2e2(pr[j8 * 8 + 2 * q], pr[j8 * 8 + 2 * q + 1]);
+        *reinterpret_cast<uint4*>(pRow + (i % kPBuffers) * kSq + swz(row, chunk0 + j8)) = *reinterpret_cast<uint4*>(hp);
       }
       fence_proxy_async();
       fence_before_sync();
-      mbar_arrive(pds_ready);
-      if (!mbar_wait(dq_full, it & 1)) { ok = false; break; }
+      warp_arrive(p_ready);
+      if (!mbar_wait(dp_full, i & 1)) { ok = false; break; }
+      fence_after_sync();
+      tmem_ld_32x32(tm_dp + lane_addr + part * 32, r);
+      tmem_ld_wait();
+      if (i > 0 && !mbar_wait(dk_done, (i - 1) & 1)) { ok = false; break; }   // dQ(i-1), dK(i-1) have read dS
+#pragma unroll
+      for (int j8 = 0; j8 < 4; ++j8) {
+        __align__(16) elem2_t hd[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int j = j8 * 8 + 2 * q;
+          hd[q] = ff2e2(pr[j] * (__uint_as_float(r[j]) - dl) * p.scale, pr[j + 1] * (__uint_as_float(r[j + 1]) - dl) * p.scale);
+        }
+        *reinterpret_cast<uint4*>(dsRow + swz(row, chunk0 + j8)) = *reinterpret_cast<uint4*>(hd);
+      }
+      fence_proxy_async();
+      fence_before_sync();
+      warp_arrive(ds_ready);
+    }
+    // dV (parts 0, 1) and dK (parts 2, 3) of this key block, half of the columns each
+    if (ok && mbar_wait(dk_done, (n - 1) & 1)) {
+      fence_after_sync();
+      const int t_k = k0 + row;
+      elem_t* dst = (part < 2 ? p.dv : p.dk) + (long long)b * p.g_sb + (long long)t_k * p.g_st + (long long)h * p.g_sh;
+      const uint32_t src = part < 2 ? tm_dv : tm_dk;
+#pragma unroll 1
+      for (int c0 = (part & 1) * (D / 2); c0 < ((part & 1) + 1) * (D / 2); c0 += 32) {
+        uint32_t r[32];
+        tmem_ld_32x32(src + lane_addr + c0, r);
+        tmem_ld_wait();
+        if (t_k < p.T) {
+#pragma unroll
+          for (int j = 0; j < 32; j += 8) {
+            __align__(16) elem2_t hh[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              hh[q] = ff2e2(__uint_as_float(r[j + 2 * q]), __uint_as_float(r[j + 2 * q + 1]));
+            *reinterpret_cast<uint4*>(dst + c0 + j) = *reinterpret_cast<uint4*>(hh);
+          }
+        }
+      }
+    } else {
+      ok = false;
+    }
+    if (!ok && lane == 0) atomicExch(p.status, ATT_ERR_TIMEOUT);
+  } else {
+    // ---------------------------------------------------------------- dQ drain: one query row per thread
+    const int row = warp * 32 + lane;
+    const uint32_t lane_addr = uint32_t(warp * 32) << 16;
+    bool ok = true;
+    for (int i = 0; i < n; ++i) {
+      const int t_q = (qb0 + i) * BQ + row;
+      float4* dst = p.dq + (((long long)b * p.H + h) * nqb + qb0 + i) * (D / 4) * 128 + row;
+      if (!mbar_wait(dq_full, i & 1)) { ok = false; break; }
       fence_after_sync();
 #pragma unroll 1
       for (int c0 = 0; c0 < D; c0 += 32) {
         uint32_t r[32];
         tmem_ld_32x32(tm_dq + lane_addr + c0, r);
         tmem_ld_wait();
-        if (row_ok) {
-          float* dst = p.dq + (((long long)b * p.T + t_q) * p.H + h) * D + c0;
+        if (c0 + 32 == D) {      // all of dQ(i) has been read: the columns may be written again
+          fence_before_sync();
+          warp_arrive(dq_read);
+        }
+        if (t_q < p.T) {
 #pragma unroll
-          for (int j = 0; j < 32; j += 4)       // 16-byte vector reductions: a quarter of the instructions of scalar adds
-            atomicAdd(reinterpret_cast<float4*>(dst + j),
+          for (int j = 0; j < 32; j += 4)
+            atomicAdd(dst + (c0 + j) / 4 * 128,
                       make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]),
                                   __uint_as_float(r[j + 3])));
         }
       }
-      fence_before_sync();
-      mbar_arrive(dq_read);
-    }
-    // dK, dV of this key block
-    if (ok && it > 0) {
-      const int t_k = k0 + row;
-#pragma unroll 1
-      for (int which = 0; which < 2; ++which) {
-        elem_t* base = which == 0 ? p.dv : p.dk;
-        const uint32_t src = which == 0 ? tm_dv : tm_dk;
-#pragma unroll 1
-        for (int c0 = 0; c0 < D; c0 += 32) {
-          uint32_t r[32];
-          tmem_ld_32x32(src + lane_addr + c0, r);
-          tmem_ld_wait();
-          if (t_k < p.T) {
-            elem_t* dst = base + (((long long)b * p.T + t_k) * p.H + h) * D + c0;
-#pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              __align__(16) elem2_t hh[4];
-#pragma unroll
-              for (int q = 0; q < 4; ++q)
-                hh[q] = ff2e2(__uint_as_float(r[j + 2 * q]), __uint_as_float(r[j + 2 * q + 1]));
-              *reinterpret_cast<uint4*>(dst + j) = *reinterpret_cast<uint4*>(hh);
-            }
-          }
-        }
-      }
-    } else if (ok && it == 0) {
-      // no query block attends to this key block (cannot happen for causal self-attention with T_q = T_k)
     }
     if (!ok && lane == 0) atomicExch(p.status, ATT_ERR_TIMEOUT);
   }
   fence_before_sync();
   __syncthreads();
-  if (warp == 0) { fence_after_sync(); tmem_dealloc(tmem, kTmemCols); }
+  if (warp == 20) { fence_after_sync(); tmem_dealloc(tmem, kTmemCols); }
 }
 
 // -------------------------------------------------------------------------------------------------
@@ -929,34 +1068,46 @@ int fbam_attn_fwd2(const void* q, const void* k, const void* v, long long sb, lo
   return cudaGetLastError() == cudaSuccess ? 0 : 5;
 }
 
-// d_o: (B, T, H, D) view with its own strides; o: contiguous forward output; dq: fp32 zero-initialised (B,T,H,D);
-// dk/dv: contiguous bf16 (B,T,H,D); delta: (B,H,T) scratch.
+// d_o: (B, T, H, D) view with its own strides; o: contiguous forward output; dq32: fp32 scratch for the sums of dQ,
+// B * H * D * (T rounded up to 128) values; dq/dk/dv: 16-bit (B, T, H, D) views that share the strides g_*; delta: (B, H, T) scratch.
 int fbam_attn_bwd(const void* q, const void* k, const void* v, long long sb, long long st, long long sh, const void* o,
                   const void* d_o, long long do_sb, long long do_st, long long do_sh, const float* lse, float* delta,
-                  float* dq, void* dk, void* dv, int B, int T, int H, int D, int causal, float scale, int* status,
-                  void* stream) {
+                  float* dq32, void* dq, void* dk, void* dv, long long g_sb, long long g_st, long long g_sh, int B, int T,
+                  int H, int D, int causal, float scale, int* status, void* stream) {
   if ((D != 64 && D != 128) || B < 1 || T < 1 || H < 1) return 1;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  const long long rows = (long long)B * T * H;
-  attn_delta_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, s>>>((const elem_t*)o, (const elem_t*)d_o, delta, B, T, H, D,
-                                                               do_sb, do_st, do_sh);
-  if (cudaGetLastError() != cudaSuccess) return 5;
   CUtensorMap mq, mk, mv, mdo;
   int e;
   if ((e = encode_bthd(&mq, q, B, T, H, D, sb, st, sh))) return e;
   if ((e = encode_bthd(&mk, k, B, T, H, D, sb, st, sh))) return e;
   if ((e = encode_bthd(&mv, v, B, T, H, D, sb, st, sh))) return e;
   if ((e = encode_bthd(&mdo, d_o, B, T, H, D, do_sb, do_st, do_sh))) return e;
-  AttnBwdParams p{B, T, H, D, causal, scale * 1.4426950408889634f, scale, lse, delta, dq, (elem_t*)dk, (elem_t*)dv, status};
-  dim3 grid((T + BKV - 1) / BKV, H, B);
-  const int smem = 4 * 128 * D * 2 + 2 * 128 * 128 * 2 + 256 + 1024;
+  const uintptr_t outs = (uintptr_t)dq | (uintptr_t)dk | (uintptr_t)dv | (uintptr_t)o | (uintptr_t)dq32;
+  if ((outs & 15) || g_sb % 8 || g_st % 8 || g_sh % 8) return 2;
+  const long long rows = (long long)B * T * H, pieces = rows * (D / 8);
+  const unsigned nkb = (T + BKV - 1) / BKV;      // also the query blocks
+  if ((long long)B * H * nkb > 0x7fffffffll) return 1;
+  if (cudaMemsetAsync(dq32, 0, (size_t)B * H * nkb * 128 * D * sizeof(float), s) != cudaSuccess) return 5;
+  const unsigned blocks = (unsigned)((pieces + 255) / 256);
+  if (D == 64)
+    attn_delta_kernel<64><<<blocks, 256, 0, s>>>((const elem_t*)o, (const elem_t*)d_o, delta, B, T, H, do_sb, do_st, do_sh);
+  else
+    attn_delta_kernel<128><<<blocks, 256, 0, s>>>((const elem_t*)o, (const elem_t*)d_o, delta, B, T, H, do_sb, do_st, do_sh);
+  AttnBwdParams p{B, T, H, causal, scale * 1.4426950408889634f, scale, lse, delta, reinterpret_cast<float4*>(dq32), (elem_t*)dk, (elem_t*)dv,
+                  g_sb, g_st, g_sh, status};
+  const dim3 grid = causal ? dim3(H, B, nkb) : dim3(nkb, H, B);
   if (D == 64) {
-    if (set_smem(attn_bwd_kernel<64>, smem)) return 5;
-    attn_bwd_kernel<64><<<grid, 160, smem, s>>>(mq, mk, mv, mdo, p);
+    if (set_smem(attn_bwd_kernel<64>, bwd_smem_bytes<64>())) return 5;
+    attn_bwd_kernel<64><<<grid, kBwdThreads, bwd_smem_bytes<64>(), s>>>(mq, mk, mv, mdo, p);
   } else {
-    if (set_smem(attn_bwd_kernel<128>, smem)) return 5;
-    attn_bwd_kernel<128><<<grid, 160, smem, s>>>(mq, mk, mv, mdo, p);
+    if (set_smem(attn_bwd_kernel<128>, bwd_smem_bytes<128>())) return 5;
+    attn_bwd_kernel<128><<<grid, kBwdThreads, bwd_smem_bytes<128>(), s>>>(mq, mk, mv, mdo, p);
   }
+  const unsigned tiles = (unsigned)B * H * nkb;
+  if (D == 64)
+    attn_dq_store_kernel<64><<<tiles, 256, 0, s>>>((const float4*)dq32, (elem_t*)dq, T, H, nkb, g_sb, g_st, g_sh);
+  else
+    attn_dq_store_kernel<128><<<tiles, 256, 0, s>>>((const float4*)dq32, (elem_t*)dq, T, H, nkb, g_sb, g_st, g_sh);
   return cudaGetLastError() == cudaSuccess ? 0 : 5;
 }
 

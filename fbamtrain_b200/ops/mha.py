@@ -37,8 +37,8 @@ class _FlashAttention(torch.autograd.Function):
         lse = torch.empty(b, h, t, dtype=torch.float32, device=q.device)
         scale = 1.0 / math.sqrt(d)
         sb, st, sh = q.stride(0), q.stride(1), q.stride(2)
-        # Two query tiles per CTA (one tile's softmax overlaps the other's MMAs): 0.131 ms against 0.215 ms for one
-        # tile per CTA at B8 H8 T1024 D128.  FBAMTRAIN_ATTENTION_FWD2=0 selects the one-tile kernel (same results).
+        # Two query tiles per CTA (one tile's softmax overlaps the other's MMAs): 0.055 ms against 0.215 ms for one
+        # tile per CTA at B8 H8 T1024 D128 causal.  FBAMTRAIN_ATTENTION_FWD2=0 selects the one-tile kernel (same results).
         fwd = nv.lib(q).fbam_attn_fwd if os.environ.get("FBAMTRAIN_ATTENTION_FWD2", "1") == "0" else nv.lib(q).fbam_attn_fwd2
         nv.check(fwd(nv.ptr(q), nv.ptr(k), nv.ptr(v), C.c_longlong(sb), C.c_longlong(st), C.c_longlong(sh),
                      nv.ptr(out), nv.ptr(lse), b, t, h, d, int(causal), C.c_float(scale),
@@ -49,23 +49,28 @@ class _FlashAttention(torch.autograd.Function):
         return out
 
     @staticmethod
-    def backward(ctx, d_out, raw_dq=False):
-        q, k, v, out, lse = ctx.saved_tensors
-        b, t, h, d = q.shape
-        if d_out.stride(3) != 1:
-            d_out = d_out.contiguous()
-        dq32 = torch.zeros(b, t, h, d, dtype=torch.float32, device=q.device)
-        dk = torch.empty(b, t, h, d, dtype=q.dtype, device=q.device)
-        dv = torch.empty(b, t, h, d, dtype=q.dtype, device=q.device)
-        delta = torch.empty(b, h, t, dtype=torch.float32, device=q.device)
-        nv.check(nv.lib(q).fbam_attn_bwd(
-            nv.ptr(q), nv.ptr(k), nv.ptr(v), C.c_longlong(q.stride(0)), C.c_longlong(q.stride(1)),
-            C.c_longlong(q.stride(2)), nv.ptr(out), nv.ptr(d_out), C.c_longlong(d_out.stride(0)),
-            C.c_longlong(d_out.stride(1)), C.c_longlong(d_out.stride(2)), nv.ptr(lse), nv.ptr(delta), nv.ptr(dq32),
-            nv.ptr(dk), nv.ptr(dv), b, t, h, d, int(ctx.causal), C.c_float(ctx.scale),
-            nv.ptr(nv.status_word(q.device)), nv.stream_ptr()), "fbam_attn_bwd")
-        flops.add(10.0 * b * h * t * t * d * (0.5 if ctx.causal else 1.0))   # 2.5 x forward
-        return (dq32 if raw_dq else dq32.to(q.dtype)), dk, dv, None
+    def backward(ctx, d_out):
+        dq, dk, dv = (torch.empty_like(ctx.saved_tensors[3]) for _ in range(3))
+        _backward(ctx, d_out, dq, dk, dv)
+        return dq, dk, dv, None
+
+
+def _backward(ctx, d_out, dq, dk, dv):
+    """Fills ``dq``, ``dk``, ``dv``: ``(B, T, H, D)`` views of one layout."""
+    q, k, v, out, lse = ctx.saved_tensors
+    b, t, h, d = q.shape
+    if d_out.stride(3) != 1:
+        d_out = d_out.contiguous()
+    dq32 = torch.empty(b, h, (t + 127) // 128 * 128, d, dtype=torch.float32, device=q.device)
+    delta = torch.empty(b, h, t, dtype=torch.float32, device=q.device)
+    nv.check(nv.lib(q).fbam_attn_bwd(
+        nv.ptr(q), nv.ptr(k), nv.ptr(v), C.c_longlong(q.stride(0)), C.c_longlong(q.stride(1)),
+        C.c_longlong(q.stride(2)), nv.ptr(out), nv.ptr(d_out), C.c_longlong(d_out.stride(0)),
+        C.c_longlong(d_out.stride(1)), C.c_longlong(d_out.stride(2)), nv.ptr(lse), nv.ptr(delta), nv.ptr(dq32),
+        nv.ptr(dq), nv.ptr(dk), nv.ptr(dv), C.c_longlong(dq.stride(0)), C.c_longlong(dq.stride(1)),
+        C.c_longlong(dq.stride(2)), b, t, h, d, int(ctx.causal), C.c_float(ctx.scale),
+        nv.ptr(nv.status_word(q.device)), nv.stream_ptr()), "fbam_attn_bwd")
+    flops.add(10.0 * b * h * t * t * d * (0.5 if ctx.causal else 1.0))   # 2.5 x forward
 
 
 class _FlashAttentionQkv(torch.autograd.Function):
@@ -81,11 +86,8 @@ class _FlashAttentionQkv(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, d_out):
-        dq, dk, dv, _ = _FlashAttention.backward(ctx, d_out, raw_dq=True)
-        dqkv = torch.empty(ctx.qkv_shape, dtype=dk.dtype, device=d_out.device)
-        dqkv[:, :, 0].copy_(dq)            # fp32 accumulator -> 16-bit, straight into its slice
-        dqkv[:, :, 1].copy_(dk)
-        dqkv[:, :, 2].copy_(dv)
+        dqkv = torch.empty(ctx.qkv_shape, dtype=ctx.saved_tensors[0].dtype, device=d_out.device)
+        _backward(ctx, d_out, dqkv[:, :, 0], dqkv[:, :, 1], dqkv[:, :, 2])
         return dqkv, None
 
 
