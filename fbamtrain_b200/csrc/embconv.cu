@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(256, 3) embconv_fwd_kernel(const int* __restri
                                                              const float* __restrict__ pos, elem_t* __restrict__ z,
                                                              elem_t* __restrict__ y, long long frames, int vocab, int O,
                                                              EmbConvGeom g, int seg_len, int nseg, int z_has_input,
-                                                             int apply_gelu) {
+                                                             int apply_gelu, int write_z) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int p_out = g.oh * g.ow;
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(256, 3) embconv_fwd_kernel(const int* __restri
         Pack8 out;
 #pragma unroll
         for (int j = 0; j < 4; ++j) out.h[j] = f22e2(v[j]);
-        *reinterpret_cast<Pack8*>(z + off + u * z_step) = out;
+        if (write_z) *reinterpret_cast<Pack8*>(z + off + u * z_step) = out;
         if (y != nullptr) {
           if (apply_gelu) {
 #pragma unroll
@@ -334,10 +334,10 @@ extern "C" int fbam_embconv_features(const void* cells, void* feat, long long fr
 }
 
 // table: bf16 [vocab][9][O]; pos: fp32 [oh*ow][O] or null; z: bf16 [frames][oh*ow][O], read (when z_has_input) and
-// overwritten with the pre-activation; y: bf16 like z or null, receives GELU(z) (or z itself without apply_gelu).
+// overwritten with the pre-activation (left alone without write_z); y: bf16 like z or null, receives GELU(z) (or z itself without apply_gelu).
 extern "C" int fbam_embconv_fwd(const void* cells, const void* table, const void* pos, void* z, void* y,
                                 long long frames, int vocab, int O, int rows, int cols, int oh, int ow, int stride,
-                                int pad, int dil, int seg_len, int z_has_input, int apply_gelu, void* stream) {
+                                int pad, int dil, int seg_len, int z_has_input, int apply_gelu, int write_z, void* stream) {
   const EmbConvGeom g{rows, cols, oh, ow, stride, pad, dil};
   if (!geom_ok(g) || frames < 0 || vocab < 1 || O < 8 || O % 8 != 0 || seg_len < 1) return 1;
   if (reinterpret_cast<uintptr_t>(table) % 16 != 0 || reinterpret_cast<uintptr_t>(z) % 16 != 0 ||
@@ -352,7 +352,7 @@ extern "C" int fbam_embconv_fwd(const void* cells, const void* table, const void
   embconv_fwd_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       reinterpret_cast<const int*>(cells), reinterpret_cast<const elem_t*>(table), reinterpret_cast<const float*>(pos),
       reinterpret_cast<elem_t*>(z), reinterpret_cast<elem_t*>(y), frames, vocab, O, g, seg_len, nseg, z_has_input,
-      apply_gelu);
+      apply_gelu, write_z);
   return launch_result();
 }
 

@@ -133,14 +133,14 @@ def features_native(cells: torch.Tensor, rows: int, cols: int, stride: int, pad:
 
 
 def forward_native(cells, table, pos, z, y, rows, cols, stride, pad, dil, z_has_input=True, apply_gelu=True,
-                   seg_len: int = SEGMENT_FRAMES) -> None:
+                   seg_len: int = SEGMENT_FRAMES, write_z=True) -> None:
     """``z (N, P_out, O)`` bf16 holds the colour term on entry (when ``z_has_input``) and the pre-activation on
-    return; ``y`` receives ``GELU(z)``."""
+    return (only a backward pass reads it: ``write_z=False`` leaves it alone); ``y`` receives ``GELU(z)``."""
     from . import native as nv
     vocab, _, o = table.shape
     nv.check(nv.lib(table).fbam_embconv_fwd(nv.ptr(cells), nv.ptr(table), nv.ptr(pos), nv.ptr(z), nv.ptr(y),
                                        C.c_longlong(cells.shape[0]), vocab, o, *_geom_args(rows, cols, stride, pad, dil),
-                                       seg_len, int(z_has_input), int(apply_gelu), nv.stream_ptr()),
+                                       seg_len, int(z_has_input), int(apply_gelu), int(write_z), nv.stream_ptr()),
              "fbam_embconv_fwd")
 
 
@@ -202,8 +202,9 @@ def _tables_native(cp_embed, pos_embed, colour, w, rows, cols, stride, pad, dil)
 # =================================================================================================
 # first layer, forward and backward
 # =================================================================================================
-def first_layer_forward_native(cells, cp_embed, pos_embed, colour, w, rows, cols, stride, pad, dil):
-    """→ ``y = GELU(z)``, ``z`` (both bf16 ``(N, OH, OW, O)``) and the colour features kept for the backward."""
+def first_layer_forward_native(cells, cp_embed, pos_embed, colour, w, rows, cols, stride, pad, dil, need_grad=True):
+    """→ ``y = GELU(z)``, ``z`` (both bf16 ``(N, OH, OW, O)``) and the colour features kept for the backward (``z`` is not
+    the pre-activation without ``need_grad``)."""
     from . import native_ops as no
     o = w.shape[0]
     n = cells.shape[0]
@@ -213,7 +214,7 @@ def first_layer_forward_native(cells, cp_embed, pos_embed, colour, w, rows, cols
     # colour term: K = 64 makes this GEMM all epilogue; the CTA-pair kernel writes its tiles with TMA stores
     z = no.gemm(feat.view(n * oh * ow, FEATURES), cc_t, two_cta=True)
     y = torch.empty_like(z)
-    forward_native(cells, table, pos_out, z, y, rows, cols, stride, pad, dil)
+    forward_native(cells, table, pos_out, z, y, rows, cols, stride, pad, dil, write_z=need_grad)
     return y.view(n, oh, ow, o), z.view(n, oh, ow, o), feat
 
 

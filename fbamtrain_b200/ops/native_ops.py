@@ -522,23 +522,28 @@ class _CellConvGeluStackPool(torch.autograd.Function):
     reductions turn into the gradients of the tables and of the first filter."""
 
     @staticmethod
-    def forward(ctx, cells, cp_embed, pos_embed, colour, rows, cols, stride, paddings, dilations, *weights):
+    def forward(ctx, need_grad, cells, cp_embed, pos_embed, colour, rows, cols, stride, paddings, dilations, *weights):
         from . import embconv
         cells = cells.contiguous()
         y1, z1, feat = embconv.first_layer_forward_native(cells, cp_embed, pos_embed, colour, weights[0], rows, cols,
-                                                          stride, paddings[0], dilations[0])
+                                                          stride, paddings[0], dilations[0], need_grad)
         ys, zs = [y1], [z1]
         for w, pad, dil in zip(weights[1:], paddings[1:], dilations[1:]):
-            oh, ow = conv_out_hw(ys[-1].shape[1], ys[-1].shape[2], stride, pad, dil)
-            z = debug.fresh((cells.shape[0], oh, ow, w.shape[0]), y1.dtype, cells.device)
+            z = None
+            if need_grad:
+                oh, ow = conv_out_hw(ys[-1].shape[1], ys[-1].shape[2], stride, pad, dil)
+                z = debug.fresh((cells.shape[0], oh, ow, w.shape[0]), y1.dtype, cells.device)
             ys.append(conv2d_fprop(ys[-1], w, stride, pad, dil, act="gelu", preact_out=z))
+            if not need_grad:
+                ys = ys[-1:]
             zs.append(z)
         last = ys[-1]
         n, h, wd, c = last.shape
         vec = torch.empty(n, c, dtype=last.dtype, device=cells.device)
         nv.check(nv.lib(last).fbam_global_avgpool(nv.ptr(last), nv.ptr(vec), C.c_longlong(n), h * wd, c, 0, None,
                                               nv.stream_ptr()), "fbam_global_avgpool")
-        ctx.save_for_backward(cells, feat, cp_embed, pos_embed, colour, *ys[:-1], *zs, *weights)
+        if need_grad:
+            ctx.save_for_backward(cells, feat, cp_embed, pos_embed, colour, *ys[:-1], *zs, *weights)
         ctx.cfg = (rows, cols, stride, tuple(paddings), tuple(dilations), len(weights))
         return vec
 
@@ -559,20 +564,22 @@ class _CellConvGeluStackPool(torch.autograd.Function):
         dws = [None] * nb
         for i in range(nb - 1, 0, -1):
             x_in, w = ys[i - 1], weights[i]
-            if ctx.needs_input_grad[9 + i]:
+            if ctx.needs_input_grad[10 + i]:
                 dws[i] = conv2d_wgrad(x_in, dz, w.shape, stride, paddings[i], dilations[i])
             dz = conv2d_dgrad(dz, w, (x_in.shape[1], x_in.shape[2]), stride, paddings[i], dilations[i],
                               gelu_grad_in=zs[i - 1])
         d_cp, d_pos, d_col, dws[0] = embconv.first_layer_backward_native(
             cells, feat, dz, cp_embed, pos_embed, colour, weights[0], rows, cols, stride, paddings[0], dilations[0])
-        return (None, d_cp.to(cp_embed.dtype), d_pos.to(pos_embed.dtype), d_col.to(colour.dtype), None, None, None, None,
-                None, *dws)
+        return (None, None, d_cp.to(cp_embed.dtype), d_pos.to(pos_embed.dtype), d_col.to(colour.dtype), None, None, None,
+                None, None, *dws)
 
 
 def cell_conv_gelu_stack_pool(cells, cp_embed, pos_embed, colour, rows, cols, weights, stride, paddings, dilations):
     _need_elem(*weights)
-    return _CellConvGeluStackPool.apply(cells, cp_embed, pos_embed, colour, rows, cols, stride, tuple(paddings),
-                                        tuple(dilations), *weights)
+    # what only a backward pass reads (pre-activations, colour features) is not written without one
+    need_grad = torch.is_grad_enabled() and any(t.requires_grad for t in (cp_embed, pos_embed, colour, *weights))
+    return _CellConvGeluStackPool.apply(need_grad, cells, cp_embed, pos_embed, colour, rows, cols, stride,
+                                        tuple(paddings), tuple(dilations), *weights)
 
 
 def conv_gelu_stack_pool(x, weights, stride, paddings, dilations):
