@@ -251,6 +251,16 @@ def _gelu_bwd(preact: torch.Tensor, dy: torch.Tensor) -> torch.Tensor:
     return out
 
 
+def _gelu_bwd_colsum(preact: torch.Tensor, dy: torch.Tensor):
+    """``dz = dy · gelu'(preact)`` and its fp32 column sums in one pass."""
+    rows, cols = preact.shape
+    dz = torch.empty_like(dy)
+    out = torch.zeros(cols, dtype=torch.float32, device=dy.device)
+    nv.check(nv.lib(preact).fbam_gelu_bwd_colsum(nv.ptr(preact), nv.ptr(dy), nv.ptr(dz), nv.ptr(out),
+                                                 C.c_longlong(rows), cols, nv.stream_ptr()), "fbam_gelu_bwd_colsum")
+    return dz, out
+
+
 class _Linear(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias, act, residual=None):
@@ -278,18 +288,21 @@ class _Linear(torch.autograd.Function):
         dy2 = dy.reshape(-1, dy.shape[-1])
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
-        if ctx.act == "gelu":
+        want_db = ctx.has_bias and ctx.needs_input_grad[2]
+        dx = dw = db = None
+        if ctx.act == "gelu" and want_db:
+            dy2, db = _gelu_bwd_colsum(preact, dy2)
+        elif ctx.act == "gelu":
             dy2 = _gelu_bwd(preact, dy2)
         elif ctx.act == "relu":
             dy2 = dy2 * (preact > 0)
-        dx = dw = db = None
         if ctx.needs_input_grad[0]:
             dx = gemm_nn(dy2, weight).view(ctx.in_shape)
         if ctx.needs_input_grad[1]:
             n_out, n_in = dy2.shape[1], x2.shape[1]
             dw = gemm_tn(dy2, x2, splits=weight_grad_splits(n_out, n_in, dy2.shape[0]) if USE_MN_MAJOR else 0)
-        if ctx.has_bias and ctx.needs_input_grad[2]:
-            db = _colsum(dy2).to(dy2.dtype)
+        if want_db:
+            db = (_colsum(dy2) if db is None else db).to(dy2.dtype)
         d_res = dy if len(ctx.needs_input_grad) > 4 and ctx.needs_input_grad[4] else None
         return dx, dw, db, None, d_res
 

@@ -1,0 +1,47 @@
+"""The row-wise and column-wise kernels at the edges of their launch rules: single rows, partial rounds of the warps of a
+block, more rows than one pass of the grid, and column counts on both sides of every vector width."""
+import pytest
+import torch
+
+from fbamtrain_b200.ops import reference as ref
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _rel(a, e):
+    return float((a.detach().double() - e).norm() / e.norm().clamp_min(1e-30))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,dim", [(1, 8), (3, 64), (65, 256), (9, 264), (700, 512), (33, 1000), (20000, 128), (9001, 1024),
+                                      (17, 2048), (5, 4096)])
+def test_rmsnorm_backward(rows, dim, dtype):
+    from fbamtrain_b200.ops import native_ops as no
+    g = torch.Generator(device=DEV).manual_seed(rows + dim)
+    x = torch.randn(rows, dim, device=DEV, generator=g).to(dtype).requires_grad_(True)
+    w = (1 + 0.1 * torch.randn(dim, device=DEV, generator=g)).to(dtype).requires_grad_(True)
+    dy = torch.randn(rows, dim, device=DEV, generator=g).to(dtype)
+    dx, dw = torch.autograd.grad(no.rms_norm(x, w, 1e-5), (x, w), dy)
+    xd, wd = x.detach().double().requires_grad_(True), w.detach().double().requires_grad_(True)
+    y = xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-5) * wd
+    ex, ew = torch.autograd.grad(y, (xd, wd), dy.double())
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11       # one rounding of the result, relative to its norm
+    assert _rel(dx, ex) < eps and _rel(dw, ew) < eps
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,cols", [(1, 8), (7, 64), (64, 264), (65, 256), (511, 1024), (600, 248), (5000, 520)])
+def test_gelu_backward_with_column_sums(rows, cols, dtype):
+    from fbamtrain_b200.ops import native_ops as no
+    g = torch.Generator(device=DEV).manual_seed(rows * 3 + cols)
+    z, dy = (torch.randn(rows, cols, device=DEV, generator=g).to(dtype) for _ in range(2))
+    dz, sums = no._gelu_bwd_colsum(z, dy)
+    exp = dy.double() * ref.gelu_grad(z.double())
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    assert _rel(dz, exp) < eps
+    assert torch.equal(dz, no._gelu_bwd(z, dy))
+    # fp32 sums of the rounded values: at most rows roundings of a partial sum
+    bound = rows * 2.0 ** -24 * dz.double().abs().sum(0) + 1e-6
+    assert bool(((sums.double() - dz.double().sum(0)).abs() <= bound).all())
+    assert bool(((no._colsum(dz).double() - dz.double().sum(0)).abs() <= bound).all())
