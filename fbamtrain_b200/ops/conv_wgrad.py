@@ -60,7 +60,7 @@ def wgrad_pass(x, dy, o: int, c: int, taps, stride: int, out_dtype=None, splits:
     p.alpha = 1.0
     p.out_fp32 = 1
     p.splits, p.bn, p.bm = splits, bn, bm
-    with debug.label(f"wgrad c{c} o{o} taps{nt}"):
+    with debug.label(lambda: f"wgrad c{c} o{o} taps{nt}"):
         code = nv.lib(dy).fbam_conv_wgrad(nv.ptr(dy), o, nv.ptr(x), ih, iw, c, C.byref(p), nv.stream_ptr())
     nv.check(code, "fbam_conv_wgrad")
     flops.add(2.0 * b * oh * ow * o * nt * c)

@@ -147,7 +147,9 @@ def check(code: int, what: str) -> None:
 
 
 def stream_ptr() -> C.c_void_p:
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current stream of the current device (without the stream object that ``torch.cuda.current_stream`` builds,
+    which is several times the cost of the launch that follows)."""
+    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def ptr(t: Optional[torch.Tensor]) -> C.c_void_p:

@@ -12,6 +12,7 @@ time: the autograd Functions pick the epilogue and operand form of each launch.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import math
 import os
 from typing import Optional, Tuple
@@ -95,7 +96,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             raise ValueError("split-K takes no epilogue options")
         return _gemm_split_k(a, b, a_mn, b_mn, m, n, k, out, out_dtype or a.dtype, splits, bm, bn)
     if (bm == 0 and bn == 0 and max_ctas == 0 and two_cta is None and ready_flags is None and rs_out is None and
-            ce_stats is None and ce_grad is None):
+            ce_stats is None and ce_grad is None and tuning.active()):
         tuned = tuning.lookup(tuning.gemm_key(m, n, k, a_mn, b_mn), {"m": m, "n": n, "k": k, "a_mn": a_mn, "b_mn": b_mn})
         if tuned is not None:
             bm, bn, max_ctas = tuned.get("bm", 0), tuned.get("bn", 0), tuned.get("max_ctas", 0)
@@ -154,7 +155,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         pair = (n >= 256 and n % 16 == 0 and bm != 128 and
                 ((m + 255) // 256) * ((n + 255) // 256) >= 148)
     fn = nv.lib(a).fbam_gemm2 if pair else nv.lib(a).fbam_gemm
-    with debug.label(f"gemm{'2' if pair else ''} m{m} n{n} k{k} {'T' if a_mn else 'N'}{'T' if b_mn else 'N'}"):
+    with debug.label(lambda: f"gemm{'2' if pair else ''} m{m} n{n} k{k} {'T' if a_mn else 'N'}{'T' if b_mn else 'N'}"):
         code = fn(nv.ptr(a), C.c_longlong(a.stride(0)), int(a_mn), nv.ptr(b), C.c_longlong(b.stride(0)), int(b_mn),
                   m, n, k, C.byref(p), nv.stream_ptr())
     nv.check(code, "fbam_gemm")
@@ -171,7 +172,7 @@ def _gemm_split_k(a, b, a_mn, b_mn, m, n, k, out, out_dtype, splits, bm, bn) -> 
     p.split_workspace, p.split_stride = work.data_ptr(), m * n
     p.status = nv.status_word(a.device).data_ptr()
     p.alpha, p.out_fp32, p.splits, p.bn, p.bm = 1.0, 1, splits, bn, bm
-    with debug.label(f"gemm m{m} n{n} k{k} {'T' if a_mn else 'N'}{'T' if b_mn else 'N'} split{splits}"):
+    with debug.label(lambda: f"gemm m{m} n{n} k{k} {'T' if a_mn else 'N'}{'T' if b_mn else 'N'} split{splits}"):
         code = nv.lib(a).fbam_gemm(nv.ptr(a), C.c_longlong(a.stride(0)), int(a_mn), nv.ptr(b), C.c_longlong(b.stride(0)),
                                    int(b_mn), m, n, k, C.byref(p), nv.stream_ptr())
     nv.check(code, "fbam_gemm")
@@ -315,6 +316,7 @@ def linear(x, weight, bias=None, act="none", residual=None):
 # =================================================================================================
 # convolution (implicit GEMM)
 # =================================================================================================
+@functools.lru_cache(maxsize=4096)
 def _brick(n: int, h: int, w: int, total: int = 128) -> Tuple[int, int, int]:
     """Splits the `total` rows of a tile into (tn, th, tw) positions with the least padding waste."""
     best, best_cost = (1, 1, total), None
@@ -345,7 +347,7 @@ def conv_pass(x: torch.Tensor, wmat: torch.Tensor, n_out: int, out: torch.Tensor
     b, ih, iw, c = x.shape
     if classes is not None:
         two_cta, tile_rows, bn = True, 0, 0
-    elif bn == 0 and tile_rows == 0 and two_cta is None:
+    elif bn == 0 and tile_rows == 0 and two_cta is None and tuning.active():
         tuned = tuning.lookup(tuning.conv_key(b, grid_hw[0], grid_hw[1], c, n_out, len(taps), in_mul, out_mul),
                               {"batch": b, "in_h": ih, "in_w": iw, "c": c, "n_out": n_out, "grid_hw": list(grid_hw),
                                "in_mul": in_mul, "out_mul": out_mul, "taps": [list(t) for t in taps],
@@ -395,7 +397,7 @@ def conv_pass(x: torch.Tensor, wmat: torch.Tensor, n_out: int, out: torch.Tensor
     if gelu_grad_in is not None:
         p.gelu_grad_in = gelu_grad_in.data_ptr()
     fn = nv.lib(x).fbam_conv2 if pair else nv.lib(x).fbam_conv
-    with debug.label(f"conv{'2' if pair else ''} c{c} n{n_out} taps{len(taps)} in_mul{in_mul} out_mul{out_mul} {act}"
+    with debug.label(lambda: f"conv{'2' if pair else ''} c{c} n{n_out} taps{len(taps)} in_mul{in_mul} out_mul{out_mul} {act}"
                      + (f" classes{len(classes)}" if classes is not None else "")):
         code = fn(nv.ptr(x), ih, iw, c, nv.ptr(wmat), C.c_longlong(wmat.stride(0)), n_out, C.byref(p),
                   nv.stream_ptr())

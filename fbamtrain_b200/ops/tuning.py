@@ -92,6 +92,11 @@ def _current() -> Optional[Dict[str, dict]]:
     return _table
 
 
+def active() -> bool:
+    """Whether :func:`lookup` can do anything: callers skip building keys and shapes otherwise."""
+    return _recording is not None or _loaded_from == "<set_table>" or bool(os.environ.get("FBAMTRAIN_TUNING_FILE"))
+
+
 def lookup(key: str, shape: Optional[dict] = None) -> Optional[dict]:
     """The tuned configuration for ``key`` (None: use the launcher's rule).  While :func:`recording` is active the
     key and ``shape`` (what the tuner needs to rebuild the launch) are noted as well."""

@@ -210,9 +210,11 @@ class Trainer:
                     recompute = None                  # None: as configured
                     for i, lo in enumerate(range(0, b * t, chunk)):
                         torch.cuda.current_stream().wait_event(events[i])
-                        before = torch.cuda.memory_allocated(self.device)
+                        # the first chunk's growth decides for the rest: nothing to ask when there is no rest
+                        probe = recompute is None and not self.model.cfg.frame_head_recompute and i + 1 < n_chunks
+                        before = torch.cuda.memory_allocated(self.device) if probe else 0
                         parts.append(self.model.frame_head_chunk(flat[lo:lo + chunk], recompute))
-                        if recompute is None and not self.model.cfg.frame_head_recompute:
+                        if probe:
                             # Activations kept for the backward grow by about the same amount per chunk.  When
                             # the rest would not fit, the remaining chunks keep only their inputs and are run
                             # again in the backward (the alternative is running out of memory).

@@ -15,6 +15,7 @@
 """
 from __future__ import annotations
 
+import contextlib
 import os
 import sys
 
@@ -52,12 +53,13 @@ def fresh(shape, dtype, device) -> torch.Tensor:
     return t
 
 
-def label(name: str):
-    """Profiler range around a native launch (only when FBAMTRAIN_PROFILE_LABELS is set)."""
-    if PROFILE_LABELS:
-        return torch.profiler.record_function(name)
-    import contextlib
-    return contextlib.nullcontext()
+_NO_LABEL = contextlib.nullcontext()
+
+
+def label(name):
+    """Profiler range around a native launch (only when FBAMTRAIN_PROFILE_LABELS is set; ``name`` is a function so that
+    the text is only built then)."""
+    return torch.profiler.record_function(name()) if PROFILE_LABELS else _NO_LABEL
 
 
 def after_launch(name: str, *args) -> None:
