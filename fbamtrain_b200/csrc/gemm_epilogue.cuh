@@ -186,14 +186,14 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, long long roff,
   #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                   float2 f = e22ff(h[q]);
-                  v[j + 2 * q] += f.x;
-                  v[j + 2 * q + 1] += f.y;
+                  v[j + 2 * q] = fmaf(p.residual_scale, f.x, v[j + 2 * q]);
+                  v[j + 2 * q + 1] = fmaf(p.residual_scale, f.y, v[j + 2 * q + 1]);
                 }
               }
             } else {
   #pragma unroll
               for (int j = 0; j < 32; ++j)
-                if (valid && n0 + j < p.N) v[j] += e2f(ri[j]);
+                if (valid && n0 + j < p.N) v[j] = fmaf(p.residual_scale, e2f(ri[j]), v[j]);
             }
           }
           if constexpr (STAGE) {

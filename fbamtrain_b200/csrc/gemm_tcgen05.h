@@ -40,12 +40,13 @@ struct GemmParams {
   void* D;                          // output, bf16 or fp32, row pitch ldd elements
   long long ldd;
   const void* bias;                 // [N] or null
-  const elem_t* residual;    // [M, N] pitch ldr, added after the activation, or null
+  const elem_t* residual;    // [M, N] pitch ldr, times residual_scale added after the activation, or null
   long long ldr;
   elem_t* preact_out;        // [M, N] pitch ldd: value before the activation, or null
   const elem_t* gelu_grad_in;  // [M, N] pitch ldd: result is multiplied by gelu'(this), or null
   int* status;                      // device word, receives an error code on a timed-out wait
   float alpha;
+  float residual_scale;             // the residual is multiplied by this
   int out_fp32, bias_fp32, act, accumulate;
   int bn;                           // 0 = choose from N; else 64 / 128 / 256
   int bm;                           // 0 = choose from the tile count; else 128 / 256 (plain GEMM and wgrad)

@@ -55,7 +55,7 @@ class GemmParams(C.Structure):
                 ("preact_out", C.c_void_p),
                 ("gelu_grad_in", C.c_void_p),
                 ("status", C.c_void_p),
-                ("alpha", C.c_float),
+                ("alpha", C.c_float), ("residual_scale", C.c_float),
                 ("out_fp32", C.c_int), ("bias_fp32", C.c_int), ("act", C.c_int), ("accumulate", C.c_int),
                 ("bn", C.c_int), ("bm", C.c_int), ("max_ctas", C.c_int), ("splits", C.c_int),
                 ("split_workspace", C.c_void_p), ("split_stride", C.c_longlong),

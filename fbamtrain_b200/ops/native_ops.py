@@ -56,7 +56,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
          bn: int = 0, bm: int = 0, max_ctas: int = 0, ready_flags: Optional[torch.Tensor] = None,
          flag_rows: int = 0, flag_on_b: bool = False, flag_epoch: int = 0, flag_spin_limit: int = 0,
          rs_out=None, rs_rows_per_rank: int = 0, tile_m_rotate: int = 0, two_cta=None,
-         rs_slot: int = -1, rs_row_stores: bool = False, ce_stats=None, ce_grad=None, splits: int = 0) -> torch.Tensor:
+         rs_slot: int = -1, rs_row_stores: bool = False, ce_stats=None, ce_grad=None, splits: int = 0,
+         residual_scale: float = 1.0) -> torch.Tensor:
     """``D[M, N] = epilogue(A · Bᵀ)``.
 
     ``a``: ``(M, K)`` (or ``(K, M)`` when ``a_mn``); ``b``: ``(N, K)`` (or ``(K, N)`` when ``b_mn``).
@@ -125,7 +126,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     p.bias_fp32 = int(bias is not None and bias.dtype == torch.float32)
     if residual is not None:
         _need_elem(residual)
-        p.residual, p.ldr = residual.data_ptr(), residual.stride(0)
+        p.residual, p.ldr, p.residual_scale = residual.data_ptr(), residual.stride(0), residual_scale
     if preact_out is not None:
         if preact_out.stride(0) != out.stride(0):
             raise ValueError("preact_out must share the output's row pitch")
@@ -941,12 +942,47 @@ def newton_schulz(g: torch.Tensor, steps: int = 5, dtype: torch.dtype = BF16, no
         from ..optim.muon import newton_schulz as ns_ref
         return ns_ref(g, steps, dtype)
     nrm = x.float().norm() if norm is None else norm
-    x = (x.float() / (nrm + 1e-7)).to(BF16).contiguous()
-    for _ in range(steps):
-        a = gemm(x, x)                                            # X Xᵀ           (r x r)
-        b = gemm(a, a, alpha=NS_C, residual=(a * NS_B))           # c·A A + b·A   (A is symmetric: A Aᵀ = A A)
-        x = gemm(b, x, b_mn=True, residual=(x * NS_A))            # B X + a·X
+    x = _ns_iterate((x.float() / (nrm + 1e-7)).to(BF16).contiguous(), steps)
     return (x.t() if transposed else x).to(dtype)
+
+
+def _ns_iterate(x: torch.Tensor, steps: int) -> torch.Tensor:
+    for _ in range(steps):
+        a = gemm(x, x)                                                      # X Xᵀ           (r x r)
+        b = gemm(a, a, alpha=NS_C, residual=a, residual_scale=NS_B)         # c·A A + b·A   (A is symmetric: A Aᵀ = A A)
+        x = gemm(b, x, b_mn=True, residual=x, residual_scale=NS_A)          # B X + a·X
+    return x
+
+
+_MUON_TYPES = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
+
+
+def muon_step_supported(grad: torch.Tensor, rows: int, cols: int, buf: torch.Tensor, master: torch.Tensor,
+                        param: torch.Tensor) -> bool:
+    """Contiguous operands, rows and columns in multiples of 8, an fp32 master (or fp32 parameter)."""
+    return (grad.is_cuda and rows % 8 == 0 and cols % 8 == 0 and rows > 0 and cols > 0 and grad.dtype in _MUON_TYPES
+            and buf.dtype == torch.float32 and master.dtype == torch.float32
+            and all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (grad, buf, master, param)))
+
+
+def muon_step(grad, buf, master, param, rows: int, cols: int, mu: float, nesterov: bool, steps: int, lr: float,
+              weight_decay: float) -> None:
+    """One Muon step of a matrix: momentum, normalisation, Newton–Schulz, update of ``master`` and (when it is another
+    tensor) of the 16-bit ``param``."""
+    dev = grad.device
+    lib = nv.lib(BF16)
+    x = torch.empty(rows, cols, dtype=BF16, device=dev)
+    xn = torch.empty(min(rows, cols), max(rows, cols), dtype=BF16, device=dev)
+    partial = torch.empty(lib.fbam_muon_partials(), dtype=torch.float32, device=dev)
+    nv.check(lib.fbam_muon_prepare(nv.ptr(grad), _MUON_TYPES[grad.dtype], nv.ptr(buf), nv.ptr(x), nv.ptr(partial),
+                                   nv.ptr(xn), rows, cols, C.c_float(mu), int(nesterov), nv.stream_ptr()),
+             "fbam_muon_prepare")
+    u = _ns_iterate(xn, steps)
+    rounded = None if param.data_ptr() == master.data_ptr() else param
+    nv.check(lib.fbam_muon_apply(nv.ptr(u), nv.ptr(master), nv.ptr(rounded),
+                                 0 if rounded is None else _MUON_TYPES[param.dtype], rows, cols,
+                                 C.c_float(1.0 - lr * weight_decay), C.c_float(lr),
+                                 C.c_float(max(1.0, rows / cols) ** 0.5), nv.stream_ptr()), "fbam_muon_apply")
 
 
 # =================================================================================================

@@ -77,6 +77,22 @@ class MuonOptimizer(Optimizer):
                 return native_ns
         return newton_schulz
 
+    def _native_step(self, name: str, p: torch.nn.Parameter, w: torch.Tensor) -> bool:
+        """The whole step on the native kernels (on a GPU, when the layout allows and nobody replaced the iterations)."""
+        if not p.is_cuda or self.ns_fn is not newton_schulz:
+            return False
+        from ..ops import dispatch
+        if dispatch.get_backend() != "auto":
+            return False
+        from ..ops import native_ops as no
+        buf, rows = self.state[name]["momentum"], p.shape[0]
+        cols = p.numel() // rows if rows else 0
+        if not no.muon_step_supported(p.grad, rows, cols, buf, w, p.data):
+            return False
+        no.muon_step(p.grad, buf, w, p.data, rows, cols, self.momentum, self.nesterov, self.ns_steps, self.lr,
+                     self.weight_decay)
+        return True
+
     def apply_update(self, name: str, p: torch.nn.Parameter, u2d: torch.Tensor) -> None:
         """``p ← p·(1 − lr·wd) − lr·scale·U`` on the master copy; ``u2d`` is the orthogonalised ``(out, rest)`` update."""
         w = self._master(name, p)
@@ -96,6 +112,8 @@ class MuonOptimizer(Optimizer):
             if p.grad is None:
                 continue
             w = self._master(name, p)
+            if self._native_step(name, p, w):
+                continue
             g2 = p.grad.float().reshape(p.shape[0], -1)
             u = muon_update(g2, self.state[name]["momentum"].view_as(g2), self.momentum, self.nesterov,
                             self.ns_steps, self._ns(p.device))
