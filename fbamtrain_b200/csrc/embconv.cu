@@ -102,7 +102,10 @@ __device__ __forceinline__ void add_row(float2* acc, const elem_t* row, float si
   for (int j = 0; j < 4; ++j) acc[j] = __ffma2_rn(s2, e22ff(r.h[j]), acc[j]);
 }
 
-__global__ void __launch_bounds__(256, 3) embconv_fwd_kernel(const int* __restrict__ cells, const elem_t* __restrict__ table,
+// Blocks of 128 threads, five per SM (no spills; 256 and three: 817 us against 798 per 1024 frames of 24 x 80 pixels and
+// 256 channels with 5 % of the cells changing).
+constexpr int kFwdThreads = 128;
+__global__ void __launch_bounds__(kFwdThreads, 5) embconv_fwd_kernel(const int* __restrict__ cells, const elem_t* __restrict__ table,
                                                              const float* __restrict__ pos, elem_t* __restrict__ z,
                                                              elem_t* __restrict__ y, long long frames, int vocab, int O,
                                                              EmbConvGeom g, int seg_len, int nseg, int z_has_input,
@@ -346,10 +349,10 @@ extern "C" int fbam_embconv_fwd(const void* cells, const void* table, const void
   if (frames == 0) return 0;
   const int nseg = (int)((frames + seg_len - 1) / seg_len);
   const long long items = (long long)oh * ow * nseg;
-  const long long blocks = (items + 7) / 8;
+  const long long blocks = (items + kFwdThreads / 32 - 1) / (kFwdThreads / 32);
   if (blocks > 0x7fffffffll) return 1;
   dim3 grid((unsigned)blocks, (unsigned)((O + 255) / 256));
-  embconv_fwd_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+  embconv_fwd_kernel<<<grid, kFwdThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       reinterpret_cast<const int*>(cells), reinterpret_cast<const elem_t*>(table), reinterpret_cast<const float*>(pos),
       reinterpret_cast<elem_t*>(z), reinterpret_cast<elem_t*>(y), frames, vocab, O, g, seg_len, nseg, z_has_input,
       apply_gelu, write_z);

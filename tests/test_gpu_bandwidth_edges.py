@@ -45,3 +45,22 @@ def test_gelu_backward_with_column_sums(rows, cols, dtype):
     bound = rows * 2.0 ** -24 * dz.double().abs().sum(0) + 1e-6
     assert bool(((sums.double() - dz.double().sum(0)).abs() <= bound).all())
     assert bool(((no._colsum(dz).double() - dz.double().sum(0)).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("n,pix,c", [(1, 1, 8), (3, 7, 64), (5, 480, 512), (2, 33, 528), (1, 1000, 2048), (2, 5, 2056),
+                                     (66000, 2, 8)])
+def test_mean_pool_backward_with_gelu(n, pix, c, dtype):
+    import ctypes as C
+    from fbamtrain_b200.ops import native as nv
+    g = torch.Generator(device=DEV).manual_seed(n + pix + c)
+    z = torch.randn(n, pix, c, device=DEV, generator=g).to(dtype)
+    dy = torch.randn(n, c, device=DEV, generator=g).to(dtype)
+    for with_z in (True, False):
+        dx = torch.empty_like(z)
+        nv.check(nv.lib(z).fbam_global_avgpool(nv.ptr(dy), nv.ptr(dx), C.c_longlong(n), pix, c, 1,
+                                               nv.ptr(z if with_z else None), nv.stream_ptr()), "fbam_global_avgpool")
+        exp = (dy.double() / pix).unsqueeze(1).expand(n, pix, c)
+        if with_z:
+            exp = exp * ref.gelu_grad(z.double())
+        assert _rel(dx, exp) < (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11)
