@@ -54,6 +54,8 @@ class DownsampleBlock(nn.Module):
         if self.ln is not None:
             x = self.ln(x)
         x = ops.conv2d_nhwc(x, self.conv_weight, self.stride, self.padding, self.dilation)
+        if self.mode != "geglu" and self.stride == 1:
+            return ops.gelu_avg_pool2x2_nhwc(x)
         x = ops.geglu(x) if self.mode == "geglu" else ops.gelu(x)
         if self.stride == 1:
             x = ops.avg_pool2x2_nhwc(x)

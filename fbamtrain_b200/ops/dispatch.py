@@ -127,6 +127,14 @@ def avg_pool2x2_nhwc(x):
     return ref.avg_pool2x2_nhwc(x)
 
 
+def gelu_avg_pool2x2_nhwc(x):
+    """``avg_pool2x2_nhwc(gelu(x))``; one pass on the native path."""
+    if _native(x) and x.shape[3] % 8 == 0:
+        from .native_ops import gelu_avg_pool2x2_nhwc as f
+        return f(x)
+    return avg_pool2x2_nhwc(gelu(x))
+
+
 def global_avg_pool_nhwc(x):
     """``(N, H, W, C)`` → ``(N, C)`` mean over the spatial positions (fp32 accumulate)."""
     if _native(x):

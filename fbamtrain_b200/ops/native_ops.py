@@ -777,6 +777,35 @@ def avg_pool2x2_nhwc(x):
     return _AvgPool2x2.apply(x)
 
 
+class _GeluAvgPool2x2(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, z):
+        z = z.contiguous()
+        n, h, w, c = z.shape
+        y = torch.empty(n, h // 2, w // 2, c, dtype=z.dtype, device=z.device)
+        nv.check(nv.lib(z).fbam_gelu_avgpool2x2(nv.ptr(z), None, nv.ptr(y), C.c_longlong(n), h // 2, w // 2, c,
+                                               nv.stream_ptr()), "fbam_gelu_avgpool2x2")
+        ctx.save_for_backward(z)
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        (z,) = ctx.saved_tensors
+        n, h, w, c = z.shape
+        dz = torch.empty_like(z)
+        dy = dy.contiguous()
+        nv.check(nv.lib(z).fbam_gelu_avgpool2x2(nv.ptr(z), nv.ptr(dy), nv.ptr(dz), C.c_longlong(n), h // 2, w // 2, c,
+                                               nv.stream_ptr()), "fbam_gelu_avgpool2x2")
+        return dz
+
+
+def gelu_avg_pool2x2_nhwc(z):
+    _need_elem(z)
+    if z.shape[1] % 2 or z.shape[2] % 2:
+        raise ValueError("2x2 pooling needs even height and width")
+    return _GeluAvgPool2x2.apply(z)
+
+
 class _GlobalAvgPool(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x):

@@ -64,3 +64,21 @@ def test_mean_pool_backward_with_gelu(n, pix, c, dtype):
         if with_z:
             exp = exp * ref.gelu_grad(z.double())
         assert _rel(dx, exp) < (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("n,h,w,c", [(1, 2, 2, 8), (3, 6, 10, 24), (2, 48, 20, 256), (5, 4, 2, 1032)])
+def test_gelu_with_2x2_mean_pool(n, h, w, c, dtype):
+    from fbamtrain_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(n + h + w + c)
+    z = torch.randn(n, h, w, c, device=DEV, generator=g).to(dtype).requires_grad_(True)
+    dy = torch.randn(n, h // 2, w // 2, c, device=DEV, generator=g).to(dtype)
+    y = ops.gelu_avg_pool2x2_nhwc(z)
+    (dz,) = torch.autograd.grad(y, z, dy.transpose(1, 2).contiguous().transpose(1, 2))      # a strided gradient
+    zd = z.detach().double().requires_grad_(True)
+    e = torch.nn.functional.gelu(zd).view(n, h // 2, 2, w // 2, 2, c).mean(dim=(2, 4))
+    (edz,) = torch.autograd.grad(e, zd, dy.double())
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    assert _rel(y, e) < eps and _rel(dz, edz) < eps
+    with pytest.raises(ValueError):
+        ops.gelu_avg_pool2x2_nhwc(z[:, :h - 1])
