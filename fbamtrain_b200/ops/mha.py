@@ -50,14 +50,16 @@ class _FlashAttention(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, d_out):
-        dq, dk, dv = (torch.empty_like(ctx.saved_tensors[3]) for _ in range(3))
-        _backward(ctx, d_out, dq, dk, dv)
+        saved = ctx.saved_tensors
+        dq, dk, dv = (torch.empty_like(saved[3]) for _ in range(3))
+        _backward(ctx, saved, d_out, dq, dk, dv)
         return dq, dk, dv, None
 
 
-def _backward(ctx, d_out, dq, dk, dv):
-    """Fills ``dq``, ``dk``, ``dv``: ``(B, T, H, D)`` views of one layout."""
-    q, k, v, out, lse = ctx.saved_tensors
+def _backward(ctx, saved, d_out, dq, dk, dv):
+    """Fills ``dq``, ``dk``, ``dv``: ``(B, T, H, D)`` views of one layout.  ``saved``: ``ctx.saved_tensors``, which the
+    caller reads once: every access runs the unpack hooks (a checkpoint refuses a second one, an offload copies again)."""
+    q, k, v, out, lse = saved
     b, t, h, d = q.shape
     if d_out.stride(3) != 1:
         d_out = d_out.contiguous()
@@ -86,8 +88,9 @@ class _FlashAttentionQkv(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, d_out):
-        dqkv = torch.empty(ctx.qkv_shape, dtype=ctx.saved_tensors[0].dtype, device=d_out.device)
-        _backward(ctx, d_out, dqkv[:, :, 0], dqkv[:, :, 1], dqkv[:, :, 2])
+        saved = ctx.saved_tensors
+        dqkv = torch.empty(ctx.qkv_shape, dtype=saved[0].dtype, device=d_out.device)
+        _backward(ctx, saved, d_out, dqkv[:, :, 0], dqkv[:, :, 1], dqkv[:, :, 2])
         return dqkv, None
 
 
