@@ -1004,7 +1004,7 @@ def muon_step(grad, buf, master, param, rows: int, cols: int, mu: float, nestero
     xn = torch.empty(min(rows, cols), max(rows, cols), dtype=BF16, device=dev)
     partial = torch.empty(lib.fbam_muon_partials(), dtype=torch.float32, device=dev)
     nv.check(lib.fbam_muon_prepare(nv.ptr(grad), _MUON_TYPES[grad.dtype], nv.ptr(buf), nv.ptr(x), nv.ptr(partial),
-                                   nv.ptr(xn), rows, cols, C.c_float(mu), int(nesterov), nv.stream_ptr()),
+                                   nv.ptr(xn), rows, cols, C.c_float(mu), C.c_float(1.0 - mu), int(nesterov), nv.stream_ptr()),
              "fbam_muon_prepare")
     u = _ns_iterate(xn, steps)
     rounded = None if param.data_ptr() == master.data_ptr() else param

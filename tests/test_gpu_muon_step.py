@@ -61,3 +61,19 @@ def test_other_layouts_take_the_general_path(shape):
     a.step()
     b.step()
     assert torch.equal(p.data, q.data)
+
+
+@pytest.mark.parametrize("nesterov", [True, False])
+@pytest.mark.parametrize("momentum", [0.9, 0.95, 0.999, 0.9999])
+def test_momentum_has_no_bias(momentum, nesterov):
+    """One step from a zero buffer leaves ``(1 - momentum) * grad`` with one rounding of the complement and one of the
+    product, 2^-24 each; a complement formed from the rounded momentum is off by up to 2^-25 / (1 - momentum)."""
+    from fbamtrain_b200.optim.muon import MuonOptimizer
+    g = torch.Generator(device=DEV).manual_seed(3)
+    p = torch.nn.Parameter(0.05 * torch.randn(64, 128, device=DEV, generator=g))
+    opt = MuonOptimizer([("w", p)], "o", 1e-2, momentum, nesterov, 0.0)
+    p.grad = torch.randn(64, 128, device=DEV, generator=g)
+    opt.step()
+    exact = (1.0 - momentum) * p.grad.double()
+    err = (opt.state["w"]["momentum"].double() - exact).abs() / exact.abs()
+    assert float(err.max()) < 2 * 2.0 ** -24 * 1.01
