@@ -147,7 +147,6 @@ rmsnorm_bwd_kernel(const elem_t* __restrict__ dy, const elem_t* __restrict__ x, 
   for (int i = 0; i < VEC_PER_LANE; ++i)
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
-  const float inv_dim = 1.0f / dim;
   const long long step = (long long)gridDim.x * warps * ROWS;
   for (long long row0 = ((long long)blockIdx.x * warps + (threadIdx.x >> 5)) * ROWS; row0 < rows; row0 += step) {
     Pack8 xp[ROWS][VEC_PER_LANE], dp[ROWS][VEC_PER_LANE];
@@ -184,7 +183,7 @@ rmsnorm_bwd_kernel(const elem_t* __restrict__ dy, const elem_t* __restrict__ x, 
           }
         }
       }
-      dot = warp_sum(dot) * inv_dim;
+      dot = warp_sum(dot) / dim;  // not times a rounded 1 / dim: one rounding, also when dim is no power of two
 #pragma unroll
       for (int i = 0; i < VEC_PER_LANE; ++i) {
         const int c = (i * 32 + lane) * 8;

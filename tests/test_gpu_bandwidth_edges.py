@@ -31,6 +31,21 @@ def test_rmsnorm_backward(rows, dim, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("dim", [24, 328, 488, 656, 1312, 2624])
+def test_rmsnorm_backward_mean_is_a_division(dim, dtype):
+    """Rows of ones: the mean is dim / dim = 1 and the gradient exactly zero.  dim times a rounded 1 / dim is not 1 for
+    most of these sizes, and leaves 6e-8."""
+    import ctypes as C
+    from fbamtrain_b200.ops import native as nv
+    x = torch.ones(3, dim, device=DEV, dtype=dtype)
+    w, rstd = torch.ones(dim, device=DEV, dtype=dtype), torch.ones(3, device=DEV)
+    dx, dw = torch.full_like(x, 7.0), torch.zeros(dim, device=DEV)
+    nv.check(nv.lib(x).fbam_rmsnorm_bwd(nv.ptr(x), nv.ptr(x), nv.ptr(w), nv.ptr(rstd), nv.ptr(dx), nv.ptr(dw),
+                                        C.c_longlong(3), dim, nv.stream_ptr()), "fbam_rmsnorm_bwd")
+    assert int(torch.count_nonzero(dx)) == 0 and bool((dw == 3).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("rows,cols", [(1, 8), (7, 64), (64, 264), (65, 256), (511, 1024), (600, 248), (5000, 520)])
 def test_gelu_backward_with_column_sums(rows, cols, dtype):
     from fbamtrain_b200.ops import native_ops as no
