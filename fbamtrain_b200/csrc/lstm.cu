@@ -552,6 +552,7 @@ int fbam_lstm_fwd_ex(float* gates, const void* whh, const float* h0, const float
   (void)hbuf;
   (void)counter;
   if (B < 1 || H < 16 || H % 16 != 0 || H > 2048 || T < 1) return 1;
+  if (reinterpret_cast<uintptr_t>(whh) % 4 != 0) return 2;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   const size_t exchanged = (size_t)(T - 1) * B * H * sizeof(elem_t);  // nobody reads the last step's y
   if (exchanged != 0 && cudaMemsetAsync(y, 0xff, exchanged, s) != cudaSuccess) return 5;
@@ -577,6 +578,7 @@ int fbam_lstm_bwd_ex(const float* gates, const float* c_all, const float* c0, co
                      unsigned* counter, int* status, int T, int B, int H, int per_sample, void* stream) {
   (void)counter;
   if (B < 1 || H < 16 || H % 16 != 0 || H > 2048 || T < 1) return 1;
+  if (reinterpret_cast<uintptr_t>(whh_t) % 4 != 0) return 2;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (cudaMemsetAsync(dgates, 0xff, (size_t)T * B * 4 * H * sizeof(elem_t), s) != cudaSuccess) return 5;
   int vec = reinterpret_cast<uintptr_t>(dgates) % 16 == 0;
@@ -613,6 +615,7 @@ const char* fbam_lstm_fwd_noalloc_strerror(int code) {
   switch (code) {
     case 0: return "ok";
     case 1: return "unsupported shape: need 1 <= B <= 8, H a multiple of 16, T >= 1";
+    case 2: return "recurrent weight not 4-byte aligned";
     case 5: return "kernel launch failed";
     case FBAM_LSTM_NOALLOC_ERR_TOO_LARGE:
       return "hidden size exceeds FBAM_LSTM_NOALLOC_MAX_HIDDEN (1024): use fbam_lstm_fwd instead";

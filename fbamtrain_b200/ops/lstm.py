@@ -31,6 +31,15 @@ def persistent_ok(batch: int, hidden: int) -> bool:
     return hidden % 16 == 0 and hidden <= nv.lib().fbam_lstm_persistent_max_hidden()
 
 
+def recurrent_weight(w_hh: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+    """``w_hh (4H, H)`` as the persistent kernels read it: dense rows, loaded 4 bytes at a time (a GEMM per step took any
+    row pitch and copied what started at an odd element)."""
+    if w_hh.shape[0] != 4 * w_hh.shape[1]:
+        raise ValueError(f"recurrent weight of shape {tuple(w_hh.shape)} is not (4H, H)")
+    w = w_hh.to(dtype).contiguous()
+    return w if w.data_ptr() % 4 == 0 else w.clone()
+
+
 class _LstmSequence(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w_ih, w_hh, b_ih, b_hh, h0, c0):
@@ -38,13 +47,14 @@ class _LstmSequence(torch.autograd.Function):
         h = w_hh.shape[1]
         dev = x.device
         x2 = x.reshape(t_len * b, i_dim).contiguous()
-        wi, wh = w_ih.to(x.dtype), w_hh.to(x.dtype)
-        bias = (b_ih.float() + b_hh.float()).contiguous()
+        wi, wh = w_ih.to(x.dtype), recurrent_weight(w_hh, x.dtype)
+        bias = (b_ih.float() + b_hh.float()).expand(4 * h).contiguous()
         gates = gemm(x2, wi, bias=bias, out_dtype=torch.float32).view(t_len, b, 4 * h)
         y = torch.empty(t_len, b, h, dtype=x.dtype, device=dev)
         c_all = torch.empty(t_len, b, h, dtype=torch.float32, device=dev)
-        h0f, c0f = h0.float().contiguous(), c0.float().contiguous()
         per_sample = int(h0.dim() == 2)
+        shape = (b, h) if per_sample else (h,)
+        h0f, c0f = h0.float().expand(shape).contiguous(), c0.float().expand(shape).contiguous()
         nv.check(nv.lib(wh).fbam_lstm_fwd_ex(nv.ptr(gates), nv.ptr(wh), nv.ptr(h0f), nv.ptr(c0f), nv.ptr(y),
                                            nv.ptr(c_all), None, None,
                                            nv.ptr(nv.status_word(dev)), t_len, b, h, per_sample, nv.stream_ptr()),

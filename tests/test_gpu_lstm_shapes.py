@@ -104,3 +104,29 @@ def test_nan_travels_through_the_exchange():
     y, _, c_n = L.lstm_sequence(*params, torch.bfloat16)
     nv.check_status(y.device)
     assert torch.isfinite(y[:, 0].float()).all() and torch.isnan(y[2:, 1].float()).all() and torch.isnan(c_n[1]).all()
+
+
+@pytest.mark.parametrize("b", [3, 9])
+def test_operand_layouts_and_sizes(b):
+    """Batches above 8 used to run a GEMM per step, which takes a recurrent weight of any row pitch and start and
+    broadcasts one-element states and biases: dense copies give the same bits, and sizes that do not fit are refused."""
+    from fbamtrain_b200.ops import lstm as L
+    h, dtype = 64, torch.bfloat16
+    params, g = _problem(4, b, 64, h, dtype)
+    x, w_ih, w_hh, b_ih, b_hh, h0, c0 = [p.detach() for p in params]
+    w_hh = w_hh.to(dtype)
+    expected = L.lstm_sequence(x, w_ih, w_hh, b_ih, b_hh, h0, c0, dtype)[0]
+    pitched = torch.zeros(4 * h, h + 8, dtype=dtype, device=DEV)
+    pitched[:, :h] = w_hh
+    odd = torch.zeros(4 * h * h + 1, dtype=dtype, device=DEV)
+    odd[1:] = w_hh.flatten()
+    for w in (pitched[:, :h], odd[1:].view(4 * h, h), w_hh.t().contiguous().t()):
+        assert torch.equal(L.lstm_sequence(x, w_ih, w, b_ih, b_hh, h0, c0, dtype)[0], expected)
+    one = torch.full((1,), 0.25, device=DEV)
+    a = L.lstm_sequence(x, w_ih, w_hh, one, one, one, one, dtype)[0]
+    full = [torch.full((n,), 0.25, device=DEV) for n in (4 * h, 4 * h, h, h)]
+    assert torch.equal(a, L.lstm_sequence(x, w_ih, w_hh, *full, dtype)[0])
+    for wrong in ((w_ih, w_hh[:-1], b_ih, b_hh, h0, c0), (w_ih, w_hh, b_ih[:-1], b_hh[:-1], h0, c0),
+                  (w_ih, w_hh, b_ih, b_hh, h0[:-1], c0), (w_ih, w_hh, b_ih, b_hh, h0, c0[:-1])):
+        with pytest.raises((ValueError, RuntimeError)):
+            L.lstm_sequence(x, *wrong, dtype)
