@@ -988,9 +988,11 @@ _MUON_TYPES = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
 
 def muon_step_supported(grad: torch.Tensor, rows: int, cols: int, buf: torch.Tensor, master: torch.Tensor,
                         param: torch.Tensor) -> bool:
-    """Contiguous operands, rows and columns in multiples of 8, an fp32 master (or fp32 parameter)."""
+    """Contiguous operands, rows and columns in multiples of 8, an fp32 master with a 16-bit parameter beside it (or an
+    fp32 parameter that is its own master)."""
     return (grad.is_cuda and rows % 8 == 0 and cols % 8 == 0 and rows > 0 and cols > 0 and grad.dtype in _MUON_TYPES
             and buf.dtype == torch.float32 and master.dtype == torch.float32
+            and (param.dtype in nv.ELEM_DTYPES or param.data_ptr() == master.data_ptr())
             and all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (grad, buf, master, param)))
 
 

@@ -63,6 +63,19 @@ def test_other_layouts_take_the_general_path(shape):
     assert torch.equal(p.data, q.data)
 
 
+def test_parameter_widened_beside_its_master():
+    """A model that was widened after its optimizer was built (``model.float()``): fp32 parameter, separate fp32 master."""
+    ((p, a), (q, b)), g = _optimizers((64, 128), torch.bfloat16, 0.95, True)
+    b._native_step = lambda *args: False
+    for t in (p, q):
+        t.data = t.data.float()
+    p.grad = torch.randn(64, 128, device=DEV, generator=g)
+    q.grad = p.grad.clone()
+    a.step()
+    b.step()
+    assert torch.equal(p.data, q.data) and torch.equal(p.data, a._master("w", p))
+
+
 @pytest.mark.parametrize("nesterov", [True, False])
 @pytest.mark.parametrize("momentum", [0.9, 0.95, 0.999, 0.9999])
 def test_momentum_has_no_bias(momentum, nesterov):
