@@ -602,30 +602,35 @@ __global__ void attn_delta_kernel(const elem_t* __restrict__ o, const elem_t* __
   if (on && part == 0) delta[((long long)b * H + hh) * T + t] = s;
 }
 
-// The fp32 sums of dQ are kept by (batch, head, query block) as [D / 4 pieces][128 rows][4]: the threads that add to them
+// The fp32 sums of dQ are kept by (batch, head, query block) as [D / 4 pieces][rows][4]: the threads that add to them
 // own one row each, and in this order a warp's 16-byte reductions cover 512 consecutive bytes.  In row order they touch
 // 32 different lines per instruction, which kept the load/store unit busy for 2700 (D = 64) and 5700 cycles per block
-// and delayed every shared-memory store behind it.  This kernel turns a block into 16-bit rows of a strided view.
+// and delayed every shared-memory store behind it.  A block has 128 rows, the last one of a sequence what is left: the
+// scratch, its zero fill and this pass are as large as dQ also where a sequence is a few tokens.  This kernel turns a
+// block into 16-bit rows of a strided view.
 template <int D>
 __global__ void __launch_bounds__(256) attn_dq_store_kernel(const float4* __restrict__ src, elem_t* __restrict__ dst, int T, int H,
                                                             int nqb, long long sb, long long st, long long sh) {
   constexpr int kLd = D + 8;   // 16-byte pieces of 8 rows on different banks
   __shared__ __align__(16) elem_t tile[128 * kLd];
-  const int qb = blockIdx.x % nqb;
+  const int qb = blockIdx.x % nqb, rows = min(128, T - qb * 128);
   const long long bh = blockIdx.x / nqb;
-  const float4* in = src + (long long)blockIdx.x * (D / 4) * 128;
+  const float4* in = src + (bh * T + qb * 128) * (D / 4);
+  const int in_row = threadIdx.x % 128;
+  if (in_row < rows) {
 #pragma unroll
-  for (int i = threadIdx.x; i < 128 * D / 4; i += 256) {
-    const float4 v = in[i];
-    __align__(8) elem2_t e[2] = {ff2e2(v.x, v.y), ff2e2(v.z, v.w)};
-    *reinterpret_cast<uint2*>(tile + (i % 128) * kLd + (i / 128) * 4) = *reinterpret_cast<uint2*>(e);
+    for (int piece = threadIdx.x / 128; piece < D / 4; piece += 2) {
+      const float4 v = in[piece * rows + in_row];
+      __align__(8) elem2_t e[2] = {ff2e2(v.x, v.y), ff2e2(v.z, v.w)};
+      *reinterpret_cast<uint2*>(tile + in_row * kLd + piece * 4) = *reinterpret_cast<uint2*>(e);
+    }
   }
   __syncthreads();
   elem_t* out = dst + bh / H * sb + bh % H * sh;
 #pragma unroll
   for (int i = threadIdx.x; i < 128 * D / 8; i += 256) {
     const int row = i / (D / 8), d = i % (D / 8) * 8, t = qb * 128 + row;
-    if (t < T) *reinterpret_cast<uint4*>(out + t * st + d) = *reinterpret_cast<const uint4*>(tile + row * kLd + d);
+    if (row < rows) *reinterpret_cast<uint4*>(out + t * st + d) = *reinterpret_cast<const uint4*>(tile + row * kLd + d);
   }
 }
 
@@ -653,7 +658,7 @@ struct AttnBwdParams {
   float scale_log2, scale;
   const float* lse;    // (B, H, T)
   const float* delta;  // (B, H, T)
-  float4* dq;          // (B, H, query block, D / 4, 128 rows) fp32, zero-initialised; accumulated with reductions
+  float4* dq;          // (B, H, query block, D / 4, rows) fp32, zero-initialised; accumulated with reductions
   elem_t* dk;          // (B, T, H, D) views with strides g_sb, g_st, g_sh
   elem_t* dv;
   long long g_sb, g_st, g_sh;
@@ -939,8 +944,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     const uint32_t lane_addr = uint32_t(warp * 32) << 16;
     bool ok = true;
     for (int i = 0; i < n; ++i) {
-      const int t_q = (qb0 + i) * BQ + row;
-      float4* dst = p.dq + (((long long)b * p.H + h) * nqb + qb0 + i) * (D / 4) * 128 + row;
+      const int t_0 = (qb0 + i) * BQ, t_q = t_0 + row, rows = min(BQ, p.T - t_0);
+      float4* dst = p.dq + (((long long)b * p.H + h) * p.T + t_0) * (D / 4) + row;
       if (!mbar_wait(dq_full, i & 1)) { ok = false; break; }
       fence_after_sync();
 #pragma unroll 1
@@ -955,7 +960,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         if (t_q < p.T) {
 #pragma unroll
           for (int j = 0; j < 32; j += 4)
-            atomicAdd(dst + (c0 + j) / 4 * 128,
+            atomicAdd(dst + (c0 + j) / 4 * rows,
                       make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]),
                                   __uint_as_float(r[j + 3])));
         }
@@ -1069,7 +1074,7 @@ int fbam_attn_fwd2(const void* q, const void* k, const void* v, long long sb, lo
 }
 
 // d_o: (B, T, H, D) view with its own strides; o: contiguous forward output; dq32: fp32 scratch for the sums of dQ,
-// B * H * D * (T rounded up to 128) values; dq/dk/dv: 16-bit (B, T, H, D) views that share the strides g_*; delta: (B, H, T) scratch.
+// B * T * H * D values; dq/dk/dv: 16-bit (B, T, H, D) views that share the strides g_*; delta: (B, H, T) scratch.
 int fbam_attn_bwd(const void* q, const void* k, const void* v, long long sb, long long st, long long sh, const void* o,
                   const void* d_o, long long do_sb, long long do_st, long long do_sh, const float* lse, float* delta,
                   float* dq32, void* dq, void* dk, void* dv, long long g_sb, long long g_st, long long g_sh, int B, int T,
@@ -1087,7 +1092,7 @@ int fbam_attn_bwd(const void* q, const void* k, const void* v, long long sb, lon
   const long long rows = (long long)B * T * H, pieces = rows * (D / 8);
   const unsigned nkb = (T + BKV - 1) / BKV;      // also the query blocks
   if ((long long)B * H * nkb > 0x7fffffffll) return 1;
-  if (cudaMemsetAsync(dq32, 0, (size_t)B * H * nkb * 128 * D * sizeof(float), s) != cudaSuccess) return 5;
+  if (cudaMemsetAsync(dq32, 0, (size_t)rows * D * sizeof(float), s) != cudaSuccess) return 5;
   const unsigned blocks = (unsigned)((pieces + 255) / 256);
   if (D == 64)
     attn_delta_kernel<64><<<blocks, 256, 0, s>>>((const elem_t*)o, (const elem_t*)d_o, delta, B, T, H, do_sb, do_st, do_sh);

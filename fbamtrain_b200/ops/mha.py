@@ -63,7 +63,7 @@ def _backward(ctx, saved, d_out, dq, dk, dv):
     b, t, h, d = q.shape
     if d_out.stride(3) != 1:
         d_out = d_out.contiguous()
-    dq32 = torch.empty(b, h, (t + 127) // 128 * 128, d, dtype=torch.float32, device=q.device)
+    dq32 = torch.empty(b, h, t, d, dtype=torch.float32, device=q.device)
     delta = torch.empty(b, h, t, dtype=torch.float32, device=q.device)
     nv.check(nv.lib(q).fbam_attn_bwd(
         nv.ptr(q), nv.ptr(k), nv.ptr(v), C.c_longlong(q.stride(0)), C.c_longlong(q.stride(1)),

@@ -39,3 +39,33 @@ def test_forward_and_gradients(t, d, causal, fused, dtype):
         err = (got[:, :, i].float() - ef[:, :, i]).norm()
         # a single token has dq = dk = 0 up to rounding: measured against all three gradients
         assert float(err / ef.norm()) < eps and float(err) <= 3 * eps * float(ef[:, :, i].norm()) + 1e-3 * float(ef.norm()), name
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("t", [1, 24, 127, 128, 130, 300])
+def test_gradient_scratch_is_as_large_as_the_gradient(t, d):
+    """The fp32 sums of dQ take B·T·H·D values: what lies behind them stays as it was (rounded up to whole tiles they
+    were 128 times as much at one token)."""
+    import ctypes as C
+    from fbamtrain_b200.ops import native as nv
+    b, h = 2, 3
+    g = torch.Generator(device=DEV).manual_seed(t + d)
+    q, k, v, d_out = (torch.randn(b, t, h, d, device=DEV, generator=g).bfloat16() for _ in range(4))
+    out, dq, dk, dv = (torch.empty_like(q) for _ in range(4))
+    lse, delta = (torch.empty(b, h, t, device=DEV) for _ in range(2))
+    room = b * h * d * ((t + 127) // 128 * 128 + 128)
+    dq32 = torch.full((room,), 7.0, device=DEV)
+    strides = [C.c_longlong(n) for n in q.stride()[:3]]
+    status, scale = nv.status_word(q.device), d ** -0.5
+    nv.check(nv.lib(q).fbam_attn_fwd2(nv.ptr(q), nv.ptr(k), nv.ptr(v), *strides, nv.ptr(out), nv.ptr(lse), b, t, h, d, 0,
+                                      C.c_float(scale), nv.ptr(status), nv.stream_ptr()), "fbam_attn_fwd2")
+    nv.check(nv.lib(q).fbam_attn_bwd(nv.ptr(q), nv.ptr(k), nv.ptr(v), *strides, nv.ptr(out), nv.ptr(d_out), *strides,
+                                     nv.ptr(lse), nv.ptr(delta), nv.ptr(dq32), nv.ptr(dq), nv.ptr(dk), nv.ptr(dv), *strides,
+                                     b, t, h, d, 0, C.c_float(scale), nv.ptr(status), nv.stream_ptr()), "fbam_attn_bwd")
+    nv.check_status(q.device)
+    assert bool((dq32[b * t * h * d:] == 7.0).all())
+    f = [x.float().requires_grad_(True) for x in (q, k, v)]
+    exp = torch.autograd.grad(ref.attention(*f, False), f, d_out.float())
+    whole = float(torch.stack([e.norm() for e in exp]).norm())
+    for a, e in zip((dq, dk, dv), exp):       # P and dS in bf16: 2^-9 relative each; dq = dk = 0 at one token
+        assert float((a.float() - e).norm()) <= 3e-2 * float(e.norm()) + 1e-3 * whole
