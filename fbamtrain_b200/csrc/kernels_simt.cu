@@ -502,23 +502,32 @@ __global__ void global_avgpool_fwd_kernel(const elem_t* __restrict__ x, elem_t* 
 // GELU that fed the pool), which folds the activation gradient into the same pass.  A thread stays with one image and
 // one group of 8 channels, so that dy is loaded and unpacked once and no index is divided: the arithmetic of gelu' per
 // 16 bytes is what bounds this kernel (a grid-stride loop with two divisions per group took 245 us for 1024 x 480 x 512,
-// now 183 us).
+// this form 183 us).
+// PACKED: images of fewer positions than one round of a block's threads share blocks, per_block of them each, and dy is
+// loaded per position.  A block of its own would leave most of its threads idle: 66000 images of 2 x 8 took 117 us, the
+// start of the blocks alone.
+template <bool PACKED>
 __global__ void __launch_bounds__(256) global_avgpool_bwd_kernel(const elem_t* __restrict__ dy, const elem_t* __restrict__ z,
-                                                                 elem_t* __restrict__ dx, int pix, int c8, int per_block) {
+                                                                 elem_t* __restrict__ dx, long long images, int pix, int c8,
+                                                                 int per_block) {
   constexpr int kUnroll = 4;
-  const long long n = blockIdx.z;
+  const long long n = PACKED ? (long long)blockIdx.x * per_block : blockIdx.z;
   const int lanes = min(c8, 256);                       // channel groups of a block; the rest of its threads are rows
   const int cg = blockIdx.y * 256 + threadIdx.x % lanes, row = threadIdx.x / lanes, rows = 256 / lanes;
   if (cg >= c8 || row >= rows) return;
   const float inv = 1.0f / (float)pix;
   float d[8];
-  unpack8(reinterpret_cast<const Pack8*>(dy)[n * c8 + cg], d);
+  auto load_d = [&](int image) {
+    unpack8(reinterpret_cast<const Pack8*>(dy)[(n + image) * c8 + cg], d);
 #pragma unroll
-  for (int j = 0; j < 8; ++j) d[j] *= inv;
-  const int p1 = min(pix, (int)(blockIdx.x + 1) * per_block);
+    for (int j = 0; j < 8; ++j) d[j] *= inv;
+  };
+  if (!PACKED) load_d(0);
+  const int first = PACKED ? 0 : blockIdx.x * per_block;
+  const int p1 = PACKED ? (int)min((long long)per_block, images - n) * pix : min(pix, first + per_block);
   const Pack8* zi = reinterpret_cast<const Pack8*>(z) + n * pix * c8 + cg;
   Pack8* xo = reinterpret_cast<Pack8*>(dx) + n * pix * c8 + cg;
-  for (int p0 = blockIdx.x * per_block + row; p0 < p1; p0 += rows * kUnroll) {
+  for (int p0 = first + row; p0 < p1; p0 += rows * kUnroll) {
     Pack8 zr[kUnroll];
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u)
@@ -526,6 +535,7 @@ __global__ void __launch_bounds__(256) global_avgpool_bwd_kernel(const elem_t* _
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
       if (p0 + u * rows >= p1) break;
+      if (PACKED) load_d((p0 + u * rows) / pix);
       float v[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) v[j] = d[j];
@@ -1143,10 +1153,19 @@ int fbam_global_avgpool(const void* in, void* out, long long n, int pix, int c, 
     dim3 grid((unsigned)n, (c / 8 + 31) / 32);
     global_avgpool_fwd_kernel<<<grid, 256, 0, STREAM(stream)>>>((const elem_t*)in, (elem_t*)out, pix, c);
   } else {
-    // images on the slowest grid dimension, 65535 at a time; positions are split until the machine is full
     const int c8 = c / 8, gy = (c8 + 255) / 256;
     if (n <= 0 || pix <= 0 || c8 <= 0) return 0;
     const int rows = c8 < 256 ? 256 / c8 : 1, round = rows * 4;
+    if (pix < round) {
+      // images share blocks: at least one round of positions each, more while 16 blocks per SM are left
+      const long long least = (round + pix - 1) / pix, spread = n / (148 * 16);
+      const long long per_block = least > spread ? least : spread;
+      const dim3 grid((unsigned)((n + per_block - 1) / per_block), gy);
+      global_avgpool_bwd_kernel<true><<<grid, 256, 0, STREAM(stream)>>>((const elem_t*)in, (const elem_t*)gelu_z,
+                                                                       (elem_t*)out, n, pix, c8, (int)per_block);
+      return CHECK_LAUNCH();
+    }
+    // images on the slowest grid dimension, 65535 at a time; positions are split until the machine is full
     for (long long n0 = 0; n0 < n; n0 += 65535) {
       const long long images = n - n0 < 65535 ? n - n0 : 65535;
       long long gx = (148 * 16 + images * gy - 1) / (images * gy);
@@ -1155,9 +1174,9 @@ int fbam_global_avgpool(const void* in, void* out, long long n, int pix, int c, 
       const int per_block = (int)(((pix + gx - 1) / gx + round - 1) / round * round);
       const dim3 grid((pix + per_block - 1) / per_block, gy, (unsigned)images);
       const long long at = n0 * pix * c;
-      global_avgpool_bwd_kernel<<<grid, 256, 0, STREAM(stream)>>>(
-          (const elem_t*)in + n0 * c, gelu_z == nullptr ? nullptr : (const elem_t*)gelu_z + at, (elem_t*)out + at, pix, c8,
-          per_block);
+      global_avgpool_bwd_kernel<false><<<grid, 256, 0, STREAM(stream)>>>(
+          (const elem_t*)in + n0 * c, gelu_z == nullptr ? nullptr : (const elem_t*)gelu_z + at, (elem_t*)out + at, images, pix,
+          c8, per_block);
     }
   }
   return CHECK_LAUNCH();
