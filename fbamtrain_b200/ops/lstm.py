@@ -10,8 +10,8 @@ the gates in the backward pass (reference: ``tensorlib/src/streaming_lstm_fwd.cp
 ``streaming_lstm_bwd.cpp:1218-1307``); here the activated gates are kept (in the buffer that held the
 pre-activations), so nothing is recomputed.
 
-Shapes beyond the persistent kernels' limits (hidden > 2048 or not a multiple of 16) run step by step: a GEMM
-per step against ``W_hh`` followed by the same gate arithmetic.
+Shapes beyond the persistent kernels' limits (hidden > 2048 or not a multiple of 16) and batches of many hundreds of
+rows run step by step: a GEMM per step against ``W_hh`` followed by the same gate arithmetic.
 """
 from __future__ import annotations
 
@@ -25,10 +25,21 @@ from . import reference as ref
 from .native_ops import gemm, gemm_nn, gemm_tn
 
 
+def persistent_shape(hidden: int) -> bool:
+    """Hidden sizes the persistent kernels take, at any batch."""
+    return hidden > 0 and hidden % 16 == 0 and hidden <= nv.lib().fbam_lstm_persistent_max_hidden()
+
+
 def persistent_ok(batch: int, hidden: int) -> bool:
-    """Any batch: 32 rows per launch.  (Batch 32, 256 steps, H 1024, forward + backward: 2.9 ms against 107.9 ms
-    with a GEMM per step.)"""
-    return hidden % 16 == 0 and hidden <= nv.lib().fbam_lstm_persistent_max_hidden()
+    """Where the persistent kernels are the faster path.  They cover 32 rows per launch and the launches follow one
+    another, so their time grows with the batch; a GEMM per step costs about 140 us per step (host and launches) until
+    its product is large.  The line is where the forward pass alone breaks even at its worst, a single step:
+    us, persistent | GEMM per step, forward, 1 step and 16:
+      H  256, batch 1024   191 |  247     836 | 2192        batch 2048   299 |  246    1855 | 2181
+      H 1024, batch  256   126 |  259     579 | 2193        batch 1024   373 |  247    2201 | 2244
+      H 2048, batch  256   259 |  253    1896 | 2168        batch 1024   818 |  268    7412 | 3204
+    (Batch 32, 256 steps, H 1024, forward and backward: 2.9 ms against 107.9 ms.)"""
+    return persistent_shape(hidden) and batch <= min(1024, (1 << 19) // hidden)
 
 
 def recurrent_weight(w_hh: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
@@ -96,7 +107,7 @@ class _LstmSequence(torch.autograd.Function):
 
 
 def _stepwise(x, w_ih, w_hh, b_ih, b_hh, h0, c0):
-    """Fallback for shapes the persistent kernels do not cover: tensor-core GEMM per step, autograd."""
+    """For shapes the persistent kernels do not cover, or not as fast: tensor-core GEMM per step, autograd."""
     from .native_ops import linear
     t_len, b, _ = x.shape
     hdim = w_hh.shape[1]
@@ -117,6 +128,9 @@ def lstm_sequence(x, w_ih, w_hh, b_ih, b_hh, h0, c0, compute_dtype):
     if compute_dtype not in nv.ELEM_DTYPES:
         raise TypeError("native LSTM computes in bf16 or fp16")
     x = x.to(compute_dtype)
-    if not persistent_ok(x.shape[1], w_hh.shape[1]) or x.shape[2] % 8 != 0:
+    b, hidden = x.shape[1], w_hh.shape[1]
+    # a state per sample is something only the persistent kernels take
+    persistent = persistent_shape(hidden) if h0.dim() == 2 else persistent_ok(b, hidden)
+    if not persistent or x.shape[2] % 8 != 0:
         return _stepwise(x, w_ih, w_hh, b_ih, b_hh, h0, c0)
     return _LstmSequence.apply(x, w_ih, w_hh, b_ih, b_hh, h0, c0)

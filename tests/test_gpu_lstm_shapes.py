@@ -55,6 +55,31 @@ def test_batch_and_hidden_edges(t_len, b, h, dtype):
         assert _rel(a, e) < 4e-2, (name, _rel(a, e))
 
 
+@pytest.mark.parametrize("t_len,b,h,persistent", [
+    (3, 70, 1024, True), (2, 100, 2048, True), (3, 97, 64, True),       # three and four launches, ragged last ones
+    (2, 256, 2048, True), (2, 264, 2048, False),                        # both sides of the line
+    (2, 1024, 64, True), (2, 1025, 64, False),
+])
+def test_batches_of_several_launches(t_len, b, h, persistent):
+    from fbamtrain_b200.ops import lstm as L
+    assert L.persistent_ok(b, h) is persistent
+    params, g = _problem(t_len, b, 64, h, torch.bfloat16)
+    y, _, c_n = L.lstm_sequence(*params, torch.bfloat16)
+    dy = torch.randn(y.shape, device=DEV, generator=g).bfloat16()
+    got = torch.autograd.grad(y, params, dy)
+    fp = [p.detach().float().requires_grad_(True) for p in params]
+    yf, _, cf = ref.lstm_sequence(*fp, torch.float32)
+    exp = torch.autograd.grad(yf, fp, dy.float())
+    assert _rel(y, yf) < 1e-2 and _rel(c_n, cf) < 1e-2
+    for name, a, e in zip(["dx", "dw_ih", "dw_hh", "db_ih", "db_hh", "dh0", "dc0"], got, exp):
+        assert _rel(a, e) < 4e-2, (name, _rel(a, e))
+    # a state per sample is accepted on both sides
+    head = [p.detach() for p in params]
+    full = [s.expand(b, h).contiguous() for s in head[5:]]
+    ys, _, _ = L.lstm_sequence(*head[:5], *full, torch.bfloat16)
+    assert _rel(ys, yf) < 1e-2
+
+
 @pytest.mark.parametrize("b,h", [(3, 64), (12, 528)])
 def test_carried_state_per_sample(b, h):
     from fbamtrain_b200.ops import lstm as L
