@@ -592,7 +592,8 @@ class _CellConvGeluStackPool(torch.autograd.Function):
 
 def cell_conv_gelu_stack_pool(cells, cp_embed, pos_embed, colour, rows, cols, weights, stride, paddings, dilations):
     _need_elem(*weights)
-    # what only a backward pass reads (pre-activations, colour features) is not written without one
+    # without a backward pass the pre-activations are not written and nothing is kept (the colour features are computed
+    # either way: they are an operand of the forward)
     need_grad = torch.is_grad_enabled() and any(t.requires_grad for t in (cp_embed, pos_embed, colour, *weights))
     return _CellConvGeluStackPool.apply(need_grad, cells, cp_embed, pos_embed, colour, rows, cols, stride,
                                         tuple(paddings), tuple(dilations), *weights)
