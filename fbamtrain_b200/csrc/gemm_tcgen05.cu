@@ -568,12 +568,17 @@ int pick_bn(int n, int requested) {
 extern "C" int fbam_last_driver_error() { return g_fbam_last_driver_error; }
 extern "C" int fbam_pending_runtime_error() { return (int)cudaPeekAtLastError(); }
 
+// Revision of the C interface: raised whenever an entry point's arguments, the size of a buffer it is given or a struct
+// changes.  The ctypes binding refuses a library of another revision (a stale build): offsets alone do not tell when a
+// field takes the place of padding, and say nothing about arguments.
+extern "C" int fbam_interface_revision() { return FBAM_INTERFACE_REVISION; }
+
 // Layout of GemmParams as this library was compiled: total size, then the offsets of a few fields spread over
 // the struct.  Callers that mirror the struct (the ctypes binding) compare these with their own layout at load.
 extern "C" void fbam_gemm_params_layout(long long* out) {
   out[0] = (long long)sizeof(GemmParams);
   out[1] = (long long)offsetof(GemmParams, status);
-  out[2] = (long long)offsetof(GemmParams, split_workspace);
+  out[2] = (long long)offsetof(GemmParams, out_fp32);  // behind the floats: a field in padding moves it
   out[3] = (long long)offsetof(GemmParams, rs_out);
   out[4] = (long long)offsetof(GemmParams, rs_row_stores);
   out[5] = (long long)offsetof(GemmParams, mode);

@@ -77,12 +77,20 @@ def available(dtype: torch.dtype = torch.bfloat16) -> bool:
     return os.path.exists(LIB_PATH_FP16 if dtype == torch.float16 else LIB_PATH)
 
 
+INTERFACE_REVISION = 2        # FBAM_INTERFACE_REVISION of csrc/gemm_tcgen05.h
+
+
 def _check_struct_layout(library: C.CDLL, path: str) -> None:
-    """The parameter struct is mirrored by hand above: refuse a library whose layout differs (a stale build)."""
+    """Arguments and the parameter struct are mirrored by hand here: refuse a library of another revision of the
+    interface or with another layout (a stale build)."""
+    revision = library.fbam_interface_revision() if hasattr(library, "fbam_interface_revision") else 0
+    if revision != INTERFACE_REVISION:
+        raise RuntimeError(f"{path} was built from different sources than this binding (interface revision {revision}, "
+                           f"expected {INTERFACE_REVISION}); run `python -m fbamtrain_b200.build`")
     got = (C.c_longlong * 8)()
     library.fbam_gemm_params_layout.restype = None
     library.fbam_gemm_params_layout(got)
-    mine = [C.sizeof(GemmParams), GemmParams.status.offset, GemmParams.split_workspace.offset,
+    mine = [C.sizeof(GemmParams), GemmParams.status.offset, GemmParams.out_fp32.offset,
             GemmParams.rs_out.offset, GemmParams.rs_row_stores.offset, GemmParams.mode.offset,
             GemmParams.conv.offset, C.sizeof(ConvGeom)]
     if list(got) != mine:
