@@ -30,16 +30,29 @@ def persistent_shape(hidden: int) -> bool:
     return hidden > 0 and hidden % 16 == 0 and hidden <= nv.lib().fbam_lstm_persistent_max_hidden()
 
 
-def persistent_ok(batch: int, hidden: int) -> bool:
+# us of one launch of the persistent kernels (32 rows): hidden up to, launch, each step; forward, forward + backward
+_LAUNCH_US = ((64, 3.3, 1.05, 5.0, 3.0), (256, 3.0, 1.7, 6.0, 4.0), (512, 4.0, 2.2, 8.0, 5.5), (1024, 7.0, 3.9, 15.0, 11.0),
+              (2048, 10.0, 14.0, 45.0, 33.0))
+
+
+def persistent_ok(batch: int, hidden: int, steps: int = 1024, grad: bool = True) -> bool:
     """Where the persistent kernels are the faster path.  They cover 32 rows per launch and the launches follow one
-    another, so their time grows with the batch; a GEMM per step costs about 140 us per step (host and launches) until
-    its product is large.  The line is where the forward pass alone breaks even at its worst, a single step:
-    us, persistent | GEMM per step, forward, 1 step and 16:
-      H  256, batch 1024   191 |  247     836 | 2192        batch 2048   299 |  246    1855 | 2181
-      H 1024, batch  256   126 |  259     579 | 2193        batch 1024   373 |  247    2201 | 2244
-      H 2048, batch  256   259 |  253    1896 | 2168        batch 1024   818 |  268    7412 | 3204
+    another, so their time grows with the batch; a GEMM per step costs about 140 us a step forward and 450 us with the
+    backward (host and launches) until its product is large, and more the longer the sequence, since the gradient of the
+    pre-activations is summed step by step: from 32 steps on it was not ahead at any batch.  Measured, us, persistent |
+    GEMM per step:
+      forward  H  256, batch 1536: 1 step 232 | 271, 64 steps 5070 | 9068      batch 2048: 1 step 299 | 246
+      forward  H 1024, batch  512: 1 step 209 | 269, 64 steps 4019 | 9011      batch 2048: 1 step 719 | 250, 16 steps 4370 | 2819
+      forward  H 2048, batch  256: 1 step 260 | 268, 64 steps 7193 | 9141      batch 1024: 1 step 818 | 268, 16 steps 7412 | 3204
+      training H 1024, batch  768: 1 step 819 | 1037, 64 steps 17083 | 47717   batch 2048: 1 step 1855 | 1130, 16 steps 12260 | 11204
     (Batch 32, 256 steps, H 1024, forward and backward: 2.9 ms against 107.9 ms.)"""
-    return persistent_shape(hidden) and batch <= min(1024, (1 << 19) // hidden)
+    if not persistent_shape(hidden):
+        return False
+    _, fwd_0, fwd, both_0, both = next(row for row in _LAUNCH_US if hidden <= row[0])
+    launches = (batch + 31) // 32
+    if not grad:
+        return launches * (fwd_0 + fwd * steps) <= 140.0 * steps + 90.0
+    return steps >= 32 or launches * (both_0 + both * steps) <= 450.0 * steps + 500.0
 
 
 def recurrent_weight(w_hh: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
@@ -128,9 +141,11 @@ def lstm_sequence(x, w_ih, w_hh, b_ih, b_hh, h0, c0, compute_dtype):
     if compute_dtype not in nv.ELEM_DTYPES:
         raise TypeError("native LSTM computes in bf16 or fp16")
     x = x.to(compute_dtype)
-    b, hidden = x.shape[1], w_hh.shape[1]
+    t_len, b, _ = x.shape
+    hidden = w_hh.shape[1]
+    grad = torch.is_grad_enabled() and any(t.requires_grad for t in (x, w_ih, w_hh, b_ih, b_hh, h0, c0))
     # a state per sample is something only the persistent kernels take
-    persistent = persistent_shape(hidden) if h0.dim() == 2 else persistent_ok(b, hidden)
+    persistent = persistent_shape(hidden) if h0.dim() == 2 else persistent_ok(b, hidden, t_len, grad)
     if not persistent or x.shape[2] % 8 != 0:
         return _stepwise(x, w_ih, w_hh, b_ih, b_hh, h0, c0)
     return _LstmSequence.apply(x, w_ih, w_hh, b_ih, b_hh, h0, c0)

@@ -57,12 +57,12 @@ def test_batch_and_hidden_edges(t_len, b, h, dtype):
 
 @pytest.mark.parametrize("t_len,b,h,persistent", [
     (3, 70, 1024, True), (2, 100, 2048, True), (3, 97, 64, True),       # three and four launches, ragged last ones
-    (2, 256, 2048, True), (2, 264, 2048, False),                        # both sides of the line
-    (2, 1024, 64, True), (2, 1025, 64, False),
+    (2, 384, 2048, True), (2, 480, 2048, False),                        # both sides of the line with gradients
+    (1, 3744, 64, True), (1, 3800, 64, False),
 ])
 def test_batches_of_several_launches(t_len, b, h, persistent):
     from fbamtrain_b200.ops import lstm as L
-    assert L.persistent_ok(b, h) is persistent
+    assert L.persistent_ok(b, h, t_len) is persistent
     params, g = _problem(t_len, b, 64, h, torch.bfloat16)
     y, _, c_n = L.lstm_sequence(*params, torch.bfloat16)
     dy = torch.randn(y.shape, device=DEV, generator=g).bfloat16()

@@ -19,3 +19,31 @@ def test_dense_rows_at_four_bytes(dtype):
     assert recurrent_weight(w, dtype).data_ptr() == w.data_ptr()          # nothing to do: no copy
     with pytest.raises(ValueError):
         recurrent_weight(w[:-1], dtype)
+
+
+def test_rule_for_large_batches(monkeypatch):
+    """Pure rule (no GPU): the sizes it was measured at, and those no rule is to touch."""
+    from fbamtrain_b200.ops import lstm as L
+
+    class Lib:
+        fbam_lstm_persistent_max_hidden = staticmethod(lambda: 2048)
+
+    monkeypatch.setattr(L.nv, "lib", lambda *a: Lib)
+    for hidden in range(16, 2049, 16):
+        for batch in (1, 8, 9, 32, 64, 128):
+            for steps in (1, 2, 16, 256):
+                for grad in (True, False):
+                    assert L.persistent_ok(batch, hidden, steps, grad)
+    assert not L.persistent_ok(1, 2064) and not L.persistent_ok(1, 24) and not L.persistent_ok(1, 0)
+    # batch, hidden, steps, grad -> persistent was the faster one
+    measured = [((512, 1024, 1, False), True), ((2048, 1024, 1, False), False), ((2048, 1024, 16, False), False),
+                ((768, 1024, 64, False), True), ((256, 2048, 1, False), True), ((1024, 2048, 1, False), False),
+                ((1024, 2048, 16, False), False), ((256, 2048, 64, False), True), ((1536, 256, 1, False), True),
+                ((2048, 256, 1, False), False), ((1024, 64, 16, False), True), ((4096, 256, 16, False), False),
+                ((1024, 512, 1, False), True), ((1536, 512, 1, False), False), ((1536, 512, 4, False), True),
+                ((768, 1024, 1, True), True), ((2048, 1024, 1, True), False), ((1024, 1024, 16, True), True),
+                ((768, 1024, 64, True), True), ((320, 2048, 1, True), True), ((1024, 2048, 1, True), False),
+                ((1024, 2048, 16, True), False), ((320, 2048, 64, True), True), ((4096, 64, 1, True), False),
+                ((1536, 256, 4, True), True), ((2048, 64, 16, False), True), ((4096, 64, 16, False), False)]
+    for args, faster in measured:
+        assert L.persistent_ok(*args) is faster, args
