@@ -135,20 +135,25 @@ __global__ void rmsnorm_fwd_kernel(const elem_t* __restrict__ x, const elem_t* _
 // rows keep as many bytes in flight, and holds its part of the dgamma sum in registers over all of them: one add per column
 // and block at the end, and a grid that fits the machine once.  With a block per 64 rows, shared-memory atomics by every
 // warp and a global one per column and block: 2.93 ms at 983040 rows of 1024, now 1.25 ms (4.8 TB/s).
-template <int VEC_PER_LANE, int ROWS, int BLOCKS>
+// LANES: lanes that share a row, 8 or 16 where it is narrow (a warp per row leaves most lanes idle there, and the
+// instructions per row are what counts: 100000 rows of 64 took 31 us).
+template <int VEC_PER_LANE, int ROWS, int BLOCKS, int LANES = 32>
 __global__ void __launch_bounds__(256, BLOCKS)
 rmsnorm_bwd_kernel(const elem_t* __restrict__ dy, const elem_t* __restrict__ x, const elem_t* __restrict__ w,
                    const float* __restrict__ rstd, elem_t* __restrict__ dx, float* __restrict__ dgamma, long long rows,
                    int dim) {
+  constexpr int kWarpRows = 32 / LANES * ROWS;
   extern __shared__ float sm_dg[];  // [dim]
-  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const int lane = threadIdx.x % LANES, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int sub_row = (threadIdx.x & 31) / LANES * ROWS;
   float acc[VEC_PER_LANE][8];
 #pragma unroll
   for (int i = 0; i < VEC_PER_LANE; ++i)
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
-  const long long step = (long long)gridDim.x * warps * ROWS;
-  for (long long row0 = ((long long)blockIdx.x * warps + (threadIdx.x >> 5)) * ROWS; row0 < rows; row0 += step) {
+  const long long step = (long long)gridDim.x * warps * kWarpRows;
+  for (long long base = ((long long)blockIdx.x * warps + warp) * kWarpRows; base < rows; base += step) {
+    const long long row0 = base + sub_row;
     Pack8 xp[ROWS][VEC_PER_LANE], dp[ROWS][VEC_PER_LANE];
     float r[ROWS];
 #pragma unroll
@@ -156,7 +161,7 @@ rmsnorm_bwd_kernel(const elem_t* __restrict__ dy, const elem_t* __restrict__ x, 
       r[u] = row0 + u < rows ? rstd[row0 + u] : 0.0f;
 #pragma unroll
       for (int i = 0; i < VEC_PER_LANE; ++i) {
-        const int c = (i * 32 + lane) * 8;
+        const int c = (i * LANES + lane) * 8;
         if (c < dim && row0 + u < rows) {
           xp[u][i] = *reinterpret_cast<const Pack8*>(x + (row0 + u) * dim + c);
           dp[u][i] = *reinterpret_cast<const Pack8*>(dy + (row0 + u) * dim + c);
@@ -165,12 +170,13 @@ rmsnorm_bwd_kernel(const elem_t* __restrict__ dy, const elem_t* __restrict__ x, 
     }
 #pragma unroll
     for (int u = 0; u < ROWS; ++u) {
-      if (row0 + u >= rows) break;
+      if (base + u >= rows) break;  // the same for the whole warp
+      const bool on = row0 + u < rows;
       float dot = 0.0f;
 #pragma unroll
       for (int i = 0; i < VEC_PER_LANE; ++i) {
-        const int c = (i * 32 + lane) * 8;
-        if (c < dim) {
+        const int c = (i * LANES + lane) * 8;
+        if (c < dim && on) {
           float xv[8], dv[8], g[8];
           unpack8(xp[u][i], xv);
           unpack8(dp[u][i], dv);
@@ -183,11 +189,13 @@ rmsnorm_bwd_kernel(const elem_t* __restrict__ dy, const elem_t* __restrict__ x, 
           }
         }
       }
-      dot = warp_sum(dot) / dim;  // not times a rounded 1 / dim: one rounding, also when dim is no power of two
+#pragma unroll
+      for (int o = LANES / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+      dot /= dim;  // not times a rounded 1 / dim: one rounding, also when dim is no power of two
 #pragma unroll
       for (int i = 0; i < VEC_PER_LANE; ++i) {
-        const int c = (i * 32 + lane) * 8;
-        if (c < dim) {
+        const int c = (i * LANES + lane) * 8;
+        if (c < dim && on) {
           float xv[8], dv[8], g[8], o[8];
           unpack8(xp[u][i], xv);
           unpack8(dp[u][i], dv);
@@ -199,11 +207,20 @@ rmsnorm_bwd_kernel(const elem_t* __restrict__ dy, const elem_t* __restrict__ x, 
       }
     }
   }
-  for (int k = 0; k < warps; ++k) {  // the warps add their sums one after the other: no atomics in shared memory
-    if ((threadIdx.x >> 5) == k) {
+#pragma unroll
+  for (int o = LANES; o < 32; o <<= 1)  // the rows of a warp, where it has several
+#pragma unroll
+    for (int i = 0; i < VEC_PER_LANE; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[i][j] += __shfl_xor_sync(0xffffffffu, acc[i][j], o);
+  // the warps that had rows add their sums one after the other: no atomics in shared memory
+  const long long block_rows = rows - (long long)blockIdx.x * warps * kWarpRows;
+  const int active = (int)min((long long)warps, (block_rows + kWarpRows - 1) / kWarpRows);
+  for (int k = 0; k < active; ++k) {
+    if (warp == k && (threadIdx.x & 31) < LANES) {
 #pragma unroll
       for (int i = 0; i < VEC_PER_LANE; ++i) {
-        const int c = (i * 32 + lane) * 8;
+        const int c = (i * LANES + lane) * 8;
         if (c < dim)
 #pragma unroll
           for (int j = 0; j < 8; ++j) sm_dg[c + j] = (k == 0 ? 0.0f : sm_dg[c + j]) + acc[i][j];
@@ -963,12 +980,12 @@ int launch_rms_fwd(const elem_t* x, const elem_t* w, elem_t* y, float* rstd, lon
   rmsnorm_fwd_kernel<V><<<(unsigned)((rows + warps - 1) / warps), warps * 32, 0, s>>>(x, w, y, rstd, rows, dim, eps);
   return cudaGetLastError() == cudaSuccess ? 0 : 5;
 }
-template <int V, int ROWS, int BLOCKS>
+template <int V, int ROWS, int BLOCKS, int LANES = 32>
 int launch_rms_bwd(const elem_t* dy, const elem_t* x, const elem_t* w, const float* rstd, elem_t* dx, float* dg, long long rows,
                    int dim, cudaStream_t s) {
-  const long long need = (rows + 8 * ROWS - 1) / (8 * ROWS), fit = 148ll * BLOCKS;
-  rmsnorm_bwd_kernel<V, ROWS, BLOCKS><<<(unsigned)(need < fit ? need : fit), 256, dim * sizeof(float), s>>>(dy, x, w, rstd, dx,
-                                                                                                         dg, rows, dim);
+  const long long block_rows = 8 * (32 / LANES) * ROWS, need = (rows + block_rows - 1) / block_rows, fit = 148ll * BLOCKS;
+  rmsnorm_bwd_kernel<V, ROWS, BLOCKS, LANES>
+      <<<(unsigned)(need < fit ? need : fit), 256, dim * sizeof(float), s>>>(dy, x, w, rstd, dx, dg, rows, dim);
   return cudaGetLastError() == cudaSuccess ? 0 : 5;
 }
 
@@ -1060,6 +1077,8 @@ int fbam_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* 
                      long long rows, int dim, void* stream) {
   if (dim % 8 != 0 || dim > 4096) return 1;
   const elem_t *DY = (const elem_t*)dy, *X = (const elem_t*)x, *W = (const elem_t*)w;
+  if (dim <= 64) return launch_rms_bwd<1, 2, 4, 8>(DY, X, W, rstd, (elem_t*)dx, dgamma, rows, dim, STREAM(stream));
+  if (dim <= 128) return launch_rms_bwd<1, 2, 4, 16>(DY, X, W, rstd, (elem_t*)dx, dgamma, rows, dim, STREAM(stream));
   if (dim <= 256) return launch_rms_bwd<1, 2, 4>(DY, X, W, rstd, (elem_t*)dx, dgamma, rows, dim, STREAM(stream));
   if (dim <= 512) return launch_rms_bwd<2, 2, 2>(DY, X, W, rstd, (elem_t*)dx, dgamma, rows, dim, STREAM(stream));
   if (dim <= 1024) return launch_rms_bwd<4, 1, 2>(DY, X, W, rstd, (elem_t*)dx, dgamma, rows, dim, STREAM(stream));

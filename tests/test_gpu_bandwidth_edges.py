@@ -15,7 +15,8 @@ def _rel(a, e):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("rows,dim", [(1, 8), (3, 64), (65, 256), (9, 264), (700, 512), (33, 1000), (20000, 128), (9001, 1024),
-                                      (17, 2048), (5, 4096)])
+                                      (17, 2048), (5, 4096), (2, 64), (7, 72), (31, 56), (65, 128), (40001, 64),
+                                      (20003, 120), (1, 2048), (2, 1536), (9, 136)])
 def test_rmsnorm_backward(rows, dim, dtype):
     from fbamtrain_b200.ops import native_ops as no
     g = torch.Generator(device=DEV).manual_seed(rows + dim)
