@@ -439,8 +439,8 @@ __global__ void avgpool2x2_kernel(const elem_t* __restrict__ in, elem_t* __restr
 }
 
 // GELU followed by the 2x2 average, NHWC, in one pass over z: forward y[oh, ow] = mean of gelu(z) (y given, dy null);
-// backward dz = dy / 4 * gelu'(z) (dy given).  Bound by DRAM: 10 bytes per input pair forward and 18 backward instead of
-// 26 and 34 with the activation (or its gradient) written out and read back in between, and the activation is not kept.  512 frames
+// backward dz = dy / 4 * gelu'(z) (dy given).  Bound by DRAM: 10 bytes per output value (four inputs) forward and 18 backward
+// instead of 26 and 34 with the activation (or its gradient) written out and read back in between, and the activation is not kept.  512 frames
 // of 48 x 160 and 24 x 80 positions x 1024 channels, forward and backward: 14.3 -> 9.2 ms.
 __global__ void __launch_bounds__(256) gelu_avgpool2x2_kernel(const elem_t* __restrict__ z, const elem_t* __restrict__ dy,
                                                               elem_t* __restrict__ out, long long n, int oh, int ow, int c) {

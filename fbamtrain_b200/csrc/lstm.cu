@@ -20,7 +20,8 @@
 //  * One block-wide barrier per step (partial sums over the K slices; two buffers take turns).  A quad of lanes owns
 //    one (unit, batch row), one lane per gate, and exchanges the gates by shuffles.
 //  * More than 8 batch rows are groups of 8 that have nothing to do with one another: they go to different CTAs while
-//    the machine has room, then take turns inside a CTA, so that one group's exchange is covered by another's work.
+//    the machine has room, then take turns inside a CTA.  A turn is a whole step of its group: poll, products, barrier
+//    and publication of one group are over before the next one is looked at, so two turns cost about twice one.
 //
 // Forward: CTA j owns U = 8 or 16 hidden units (4U gate rows of W_hh).  The buffer of gate pre-activations is
 // overwritten in place with the activated gates, which is exactly what the backward pass needs.
@@ -546,7 +547,8 @@ extern "C" {
 int fbam_lstm_persistent_max_hidden() { return 2048; }
 
 // gates: (T, B, 4H) fp32, pre-activations incl. bias on entry, activated gates on exit.
-// hbuf and counter: not used any more (y itself is what the CTAs exchange); may be null.
+// hbuf and counter: ignored, may be null (y itself is what the CTAs exchange; the arguments stay for callers of the C
+// interface).  whh: 4-byte aligned.
 int fbam_lstm_fwd_ex(float* gates, const void* whh, const float* h0, const float* c0, void* y, float* c_all,
                      void* hbuf, unsigned* counter, int* status, int T, int B, int H, int per_sample, void* stream) {
   (void)hbuf;
@@ -572,7 +574,7 @@ int fbam_lstm_fwd(float* gates, const void* whh, const float* h0, const float* c
   return fbam_lstm_fwd_ex(gates, whh, h0, c0, y, c_all, hbuf, counter, status, T, B, H, 0, stream);
 }
 
-// whh_t: (H, 4H) bf16 = W_hh transposed.  dgates: (T, B, 4H) bf16 out.  dh0/dc0: (B, H) fp32 out.
+// whh_t: (H, 4H) bf16 = W_hh transposed, 4-byte aligned.  counter: ignored, may be null.  dgates: (T, B, 4H) bf16 out.  dh0/dc0: (B, H) fp32 out.
 int fbam_lstm_bwd_ex(const float* gates, const float* c_all, const float* c0, const void* dy, const void* whh_t,
                      void* dgates, float* dh0, float* dc0, const float* dh_last, const float* dc_last,
                      unsigned* counter, int* status, int T, int B, int H, int per_sample, void* stream) {

@@ -2,8 +2,8 @@
 //
 // Bound by DRAM.  As separate tensor operations (cast of the gradient, decay and add of the momentum, Nesterov
 // combination, cast, cast back, norm, division, cast; scale, decay, add, cast into the parameter) one step of a
-// 4096 x 2048 matrix moved about 60 bytes per element in sixteen launches; the three kernels move 28 (fp32 gradient and
-// parameter) or 24 (16-bit).  The one-billion-parameter model with two action blocks: 95.3 -> 87.3 ms of GPU time per
+// 4096 x 2048 matrix moves about 60 bytes per element in sixteen launches; the three kernels move 28, with fp32 gradient and
+// parameter (4 + 8 + 2, 2 + 2, 2 + 8) as with 16-bit ones and a master (2 + 8 + 2, 2 + 2, 2 + 8 + 2).  The one-billion-parameter model with two action blocks: 95.3 -> 87.3 ms of GPU time per
 // step, 1315 -> 924 launches (with the affine terms of the iterations moved into the GEMM epilogue).
 //
 // Sums of squares go through per-block partial sums that every block of the next kernel adds in the same order: no
