@@ -29,11 +29,13 @@
 // reads gate r of dGates[t] only (a quarter of what a CTA without partners would have to read), and sends its partial
 // sums of dh_{t-1} through distributed shared memory to the CTA that owns the unit.
 //
-// Measured on a B200, bf16, us per step, before (grid-wide counter barrier, staged vectors, no clusters) -> now:
-//   H 1024, batch 8:  forward 2.93 -> 1.85, backward 5.08 -> 2.06
-//   H 2048, batch 4:  forward 4.18 -> 3.18, backward 6.24 -> 3.68
-//   H  256, batch 8:  forward 2.30 -> 1.07, backward 2.59 -> 1.73
-//   H 1024, batch 32: forward 3.48, backward 6.40 (before: a GEMM launch and point-wise kernels per step)
+// Measured on a B200, bf16, us per step over 1024 steps, with a grid-wide counter barrier, staged vectors and no clusters
+// -> in this form:
+//   H 1024, batch 8:  forward 2.93 -> 1.88, backward 5.08 -> 2.06
+//   H 2048, batch 4:  forward 4.18 -> 3.32, backward 6.24 -> 3.75
+//   H  256, batch 8:  forward 2.30 -> 1.03, backward 2.59 -> 1.66
+//   H 1024, batch 32 (two groups, two turns): forward 3.49, backward 6.30
+//   H 2048, batch 32 (one group, four turns): forward 12.9, backward 16.2
 // A wider form of the cluster for the forward pass too (each CTA a quarter of h, partial sums through distributed
 // shared memory) was 2.24 us at H = 1024: the cluster barrier costs more than the fewer polls give.
 //
@@ -492,7 +494,7 @@ int coop_launch(K kernel, int grid, int threads, int cluster, void** args, size_
 // How a launch covers `rows` (<= 32) batch rows at hidden size H.
 // 16 units per CTA (half the CTAs of a group of 8 rows, so half the pollers, and the machine holds two groups at
 // H = 1024, four at 512) against 8 units (less work in each CTA), 8 rows:
-//   H = 1024 forward   1.85 us per step with 16 units, 2.33 with 8: fewer pollers of each line win;
+//   H = 1024 forward   1.88 us per step with 16 units, 2.33 with 8: fewer pollers of each line win;
 //   H = 1024 backward  2.85 us with 16 units, 2.06 with 8: polls are a quarter already, the smaller share wins;
 //   H <= 512           8 units while there is one group; more groups fit beside one another with 16 (H > 256).
 // Above 1024 the weights need 16 units per CTA on all SMs.  What does not fit side by side takes turns.

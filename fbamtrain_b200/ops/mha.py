@@ -37,8 +37,8 @@ class _FlashAttention(torch.autograd.Function):
         lse = torch.empty(b, h, t, dtype=torch.float32, device=q.device)
         scale = 1.0 / math.sqrt(d)
         sb, st, sh = q.stride(0), q.stride(1), q.stride(2)
-        # Two query tiles per CTA (one tile's softmax overlaps the other's MMAs): 0.055 ms against 0.215 ms for one
-        # tile per CTA at B8 H8 T1024 D128 causal.  FBAMTRAIN_ATTENTION_FWD2=0 selects the one-tile kernel (same results).
+        # Two query tiles per CTA (one tile's softmax overlaps the other's MMAs) against one: 0.057 and 0.215 ms at
+        # B8 H8 T1024 D128, 0.060 and 0.158 ms causal.  FBAMTRAIN_ATTENTION_FWD2=0 selects the one-tile kernel (same results).
         fwd = nv.lib(q).fbam_attn_fwd if os.environ.get("FBAMTRAIN_ATTENTION_FWD2", "1") == "0" else nv.lib(q).fbam_attn_fwd2
         nv.check(fwd(nv.ptr(q), nv.ptr(k), nv.ptr(v), C.c_longlong(sb), C.c_longlong(st), C.c_longlong(sh),
                      nv.ptr(out), nv.ptr(lse), b, t, h, d, int(causal), C.c_float(scale),
