@@ -520,9 +520,10 @@ __global__ void global_avgpool_fwd_kernel(const elem_t* __restrict__ x, elem_t* 
 // one group of 8 channels, so that dy is loaded and unpacked once and no index is divided: the arithmetic of gelu' per
 // 16 bytes is what bounds this kernel (a grid-stride loop with two divisions per group took 245 us for 1024 x 480 x 512,
 // this form 183 us).
-// PACKED: images of fewer positions than one round of a block's threads share blocks, per_block of them each, and dy is
-// loaded per position.  A block of its own would leave most of its threads idle: 66000 images of 2 x 8 take 117 us that way,
-// the start of the blocks alone, and 5 us packed; 8192 of 12 x 64 18.5 and 10.3.
+// PACKED: images that leave threads of a block without a position share blocks, per_block of them each, and dy is loaded per
+// position.  A block of its own would leave most of its threads idle: 66000 images of 2 x 8 take 117 us that way,
+// the start of the blocks alone, and 5 us packed; 8192 of 12 x 64 18.5 and 10.3.  Where every thread has a position, packing
+// costs a division for each: 1024 images of 24 x 128 6.3 us without and 8.2 with.
 template <bool PACKED>
 __global__ void __launch_bounds__(256) global_avgpool_bwd_kernel(const elem_t* __restrict__ dy, const elem_t* __restrict__ z,
                                                                  elem_t* __restrict__ dx, long long images, int pix, int c8,
@@ -1175,7 +1176,7 @@ int fbam_global_avgpool(const void* in, void* out, long long n, int pix, int c, 
     const int c8 = c / 8, gy = (c8 + 255) / 256;
     if (n <= 0 || pix <= 0 || c8 <= 0) return 0;
     const int rows = c8 < 256 ? 256 / c8 : 1, round = rows * 4;
-    if (pix < round) {
+    if (pix < rows) {
       // images share blocks: at least one round of positions each, more while 16 blocks per SM are left
       const long long least = (round + pix - 1) / pix, spread = n / (148 * 16);
       const long long per_block = least > spread ? least : spread;

@@ -66,6 +66,7 @@ def test_gelu_backward_with_column_sums(rows, cols, dtype):
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("n,pix,c", [(1, 1, 8), (3, 7, 64), (5, 480, 512), (2, 33, 528), (1, 1000, 2048), (2, 5, 2056),
                                      (66000, 2, 8), (70001, 1, 8), (5, 127, 64), (5, 128, 64), (5, 129, 64), (3001, 3, 72),
+                                     (9, 31, 64), (9, 32, 64), (700, 33, 64), (5000, 27, 72), (5000, 28, 72),
                                      (7, 3, 2048), (7, 4, 2048), (2500, 3, 2056), (40000, 24, 64)])
 def test_mean_pool_backward_with_gelu(n, pix, c, dtype):
     import ctypes as C
