@@ -64,6 +64,11 @@ def recurrent_weight(w_hh: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
     return w if w.data_ptr() % 4 == 0 else w.clone()
 
 
+def _fit(t: torch.Tensor, shape) -> torch.Tensor:
+    """``t`` dense in ``shape`` (broadcast, or refused); most calls are host-bound, so nothing is called without need."""
+    return (t if t.shape == shape else t.expand(shape)).contiguous()
+
+
 class _LstmSequence(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w_ih, w_hh, b_ih, b_hh, h0, c0):
@@ -72,13 +77,13 @@ class _LstmSequence(torch.autograd.Function):
         dev = x.device
         x2 = x.reshape(t_len * b, i_dim).contiguous()
         wi, wh = w_ih.to(x.dtype), recurrent_weight(w_hh, x.dtype)
-        bias = (b_ih.float() + b_hh.float()).expand(4 * h).contiguous()
+        bias = _fit(b_ih.float() + b_hh.float(), (4 * h,))
         gates = gemm(x2, wi, bias=bias, out_dtype=torch.float32).view(t_len, b, 4 * h)
         y = torch.empty(t_len, b, h, dtype=x.dtype, device=dev)
         c_all = torch.empty(t_len, b, h, dtype=torch.float32, device=dev)
         per_sample = int(h0.dim() == 2)
         shape = (b, h) if per_sample else (h,)
-        h0f, c0f = h0.float().expand(shape).contiguous(), c0.float().expand(shape).contiguous()
+        h0f, c0f = _fit(h0.float(), shape), _fit(c0.float(), shape)
         nv.check(nv.lib(wh).fbam_lstm_fwd_ex(nv.ptr(gates), nv.ptr(wh), nv.ptr(h0f), nv.ptr(c0f), nv.ptr(y),
                                            nv.ptr(c_all), None, None,
                                            nv.ptr(nv.status_word(dev)), t_len, b, h, per_sample, nv.stream_ptr()),
@@ -143,9 +148,10 @@ def lstm_sequence(x, w_ih, w_hh, b_ih, b_hh, h0, c0, compute_dtype):
     x = x.to(compute_dtype)
     t_len, b, _ = x.shape
     hidden = w_hh.shape[1]
-    grad = torch.is_grad_enabled() and any(t.requires_grad for t in (x, w_ih, w_hh, b_ih, b_hh, h0, c0))
-    # a state per sample is something only the persistent kernels take
-    persistent = persistent_shape(hidden) if h0.dim() == 2 else persistent_ok(b, hidden, t_len, grad)
+    persistent = persistent_shape(hidden)
+    if persistent and b > 32 and h0.dim() == 1:      # a state per sample is something only the persistent kernels take
+        grad = torch.is_grad_enabled() and any(t.requires_grad for t in (x, w_ih, w_hh, b_ih, b_hh, h0, c0))
+        persistent = persistent_ok(b, hidden, t_len, grad)
     if not persistent or x.shape[2] % 8 != 0:
         return _stepwise(x, w_ih, w_hh, b_ih, b_hh, h0, c0)
     return _LstmSequence.apply(x, w_ih, w_hh, b_ih, b_hh, h0, c0)
