@@ -17,33 +17,35 @@
 //  * A warp owns a K slice and reads only that slice of the vector, straight into its MMA fragments (the 32 columns of
 //    a K block are dealt to the lanes 8 at a time, with the weights permuted alike, so that a fragment is one 16-byte
 //    load): no staging in shared memory, and a warp starts when its own slice has arrived.
-//  * One block-wide barrier per step (partial sums over the K slices; two buffers take turns).  A quad of lanes owns
-//    one (unit, batch row), one lane per gate, and exchanges the gates by shuffles.
-//  * More than 8 batch rows are groups of 8 that have nothing to do with one another: they go to different CTAs while
-//    the machine has room, then take turns inside a CTA.  A turn is a whole step of its group: poll, products, barrier
-//    and publication of one group are over before the next one is looked at, so two turns cost about twice one.
+//  * Polls start when the vector can be there and not before (`hold`): polls of lines that are being written delay the
+//    stores they wait for.  Reading 16 KB that nobody writes takes every CTA of a full machine 540 to 680 cycles, whether
+//    they read the same lines or not; copies of the vector for different readers only cost more stores.
+//  * All groups of 8 batch rows of a CTA go through a step together: the chain of latencies is paid once, not once per
+//    group.  Groups go to different CTAs while the machine has room.
 //
-// Forward: CTA j owns U = 8 or 16 hidden units (4U gate rows of W_hh).  The buffer of gate pre-activations is
-// overwritten in place with the activated gates, which is exactly what the backward pass needs.
-// Backward (BPTT): a cluster of four CTAs owns 4U units; CTA r of the cluster holds the columns of gate r of W_hhᵀ,
-// reads gate r of dGates[t] only (a quarter of what a CTA without partners would have to read), and sends its partial
-// sums of dh_{t-1} through distributed shared memory to the CTA that owns the unit.
+// Forward: CTA j owns 8·UT hidden units (32·UT gate rows of W_hh).  A quad of lanes owns one (unit, batch row), one lane
+// per gate, and exchanges the gates by shuffles.  The buffer of gate pre-activations is overwritten in place with the
+// activated gates, which is exactly what the backward pass needs.
+// Backward (BPTT): a cluster of four CTAs owns 32·UT units; CTA r of the cluster holds the columns of gate r of W_hhᵀ,
+// reads gate r of dGates[t] only (a quarter of what a CTA without partners would have to read), adds its warps' partial
+// sums of dh_{t-1} and sends them to the CTA that owns the unit: st.async on an mbarrier there, 267 cycles one way, where
+// an idle cluster barrier takes 400 and one behind the stores of unsummed partials took about 1000.  One thread owns one
+// (unit, batch row) with its four gates, and what does not depend on dh is computed while the sums are on their way.
 //
-// Measured on a B200, bf16, us per step over 1024 steps, with a grid-wide counter barrier, staged vectors and no clusters
-// -> in this form:
-//   H 1024, batch 8:  forward 2.93 -> 1.88, backward 5.08 -> 2.06
-//   H 2048, batch 4:  forward 4.18 -> 3.32, backward 6.24 -> 3.75
-//   H  256, batch 8:  forward 2.30 -> 1.03, backward 2.59 -> 1.66
-//   H 1024, batch 32 (two groups, two turns): forward 3.49, backward 6.30
-//   H 2048, batch 32 (one group, four turns): forward 12.9, backward 16.2
-// A wider form of the cluster for the forward pass too (each CTA a quarter of h, partial sums through distributed
-// shared memory) was 2.24 us at H = 1024: the cluster barrier costs more than the fewer polls give.
+// Measured on a B200, bf16, us per step, before (polls at once, IEEE gate functions, groups of rows in turn, cluster
+// barrier) -> in this form:
+//   H 1024, batch 8:    forward 1.80 -> 1.49, backward 2.05 -> 1.74
+//   H 2048, batch 4:    forward 3.09 -> 2.44, backward 3.75 -> 2.70
+//   H  256, batch 8:    forward 1.06 -> 0.95, backward 1.68 -> 1.29
+//   H 1024, batch 32:   forward 3.47 -> 2.73, backward 6.27 -> 3.06
+//   H 2048, batch 32:   forward 12.9 -> 11.1, backward 16.1 -> 9.8
+// (At H = 1024 a forward cluster that divides K, with partial sums sent as in the backward pass, takes 1.75 us at batch 8,
+// 1.50 without: its second hop costs more than the smaller share of the vector gives.)
 //
 // The reference runs the recurrence as one GEMM launch plus a point-wise cell kernel per time step (reference:
 // kernel_gen/kernel_gen/kernels/lstm_cell.py:6-144, kernels/lstm_cell_bwd.py:6-273 for the cell arithmetic and the
 // recompute / backward point-wise kernels; tensorlib/src/streaming_lstm.cpp and streaming_lstm_bwd.cpp for the loop
-// around them); gate order i, f, g, o, fp32 gates and cell state as there (tanh is tanhf here; the reference
-// writes it as 2·sigmoid(2x) - 1, the same function).
+// around them); gate order i, f, g, o, fp32 gates and cell state as there.
 #include "elem16.cuh"
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -51,9 +53,9 @@
 namespace {
 
 constexpr unsigned kSpinLimit = 1u << 22;  // polls of at least an L2 round trip each: seconds
+constexpr unsigned kTestLimit = 1u << 26;  // tests of a barrier in shared memory, some tens of cycles each: seconds
 constexpr uint32_t kEmpty = 0xffffffffu;   // a word of the exchange buffer that has not been written yet
-constexpr int kCluster = 4;                // CTAs of a backward cluster: one per gate
-constexpr int kLaunchRows = 32;            // batch rows of one launch
+constexpr int kCluster = 4;                // CTAs of a cluster
 enum { LSTM_ERR_EXCHANGE_TIMEOUT = 201 };
 
 __device__ __forceinline__ uint4 ld_relaxed_v4(const elem_t* p) {
@@ -81,8 +83,89 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-__device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + __expf(-x)); }
+// -------------------------------------------------------------------------------------------------
+// gate functions
+// -------------------------------------------------------------------------------------------------
+// One path through the hardware's 2^x and 1/x for both functions, no branch: sigmoid(x) = 1 / (1 + e^-x), tanh(x) =
+// 2 sigmoid(2x) - 1, and x + x³·p(x²) where that would cancel (p: a least-squares fit in the relative error, 2.6e-9 at
+// most on |x| < 0.6).  Errors against 64 bits over [-8, 8], relative, largest | rms, of 1 / (1 + __expf(-x)) and tanhf and
+// of these: sigmoid 5.1e-7 | 9.7e-8 and 5.3e-7 | 9.9e-8, tanh 1.9e-7 | 2.6e-8 and 1.8e-7 | 2.1e-8.  With an IEEE division
+// and tanhf, which a quad went through one after the other, the gates of a forward step took 743 cycles; now 330.
+__device__ __forceinline__ float ex2_f(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float rcp_f(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+// tanh(x), given `far`, its value where |x| is not small.
+__device__ __forceinline__ float tanh_from(float x, float far) {
+  const float s = x * x;
+  float p = fmaf(-0.005905978847295046f, s, 0.020805491134524345f);
+  p = fmaf(p, s, -0.05378672108054161f);
+  p = fmaf(p, s, 0.13331958651542664f);
+  p = fmaf(p, s, -0.33333298563957214f);
+  return fabsf(x) < 0.6f ? fmaf(x * s, p, x) : far;
+}
+__device__ __forceinline__ float tanh_f(float x) {
+  return tanh_from(x, fmaf(2.0f, rcp_f(1.0f + ex2_f(-2.88539008f * x)), -1.0f));
+}
 
+// -------------------------------------------------------------------------------------------------
+// cluster
+// -------------------------------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t smem_address(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ uint32_t map_to_rank(const void* p, int rank) {
+  uint32_t remote;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_address(p)), "r"(rank));
+  return remote;
+}
+// Stores that count towards the transaction bytes of the receiver's barrier.
+__device__ __forceinline__ void st_async_v4(uint32_t at, const float (&v)[4], uint32_t bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1,%2,%3,%4}, [%5];" ::"r"(at), "f"(v[0]),
+               "f"(v[1]), "f"(v[2]), "f"(v[3]), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void bar_init(uint64_t* bar) {
+  asm volatile("mbarrier.init.shared.b64 [%0], 1;" ::"r"(smem_address(bar)) : "memory");
+}
+// Opens the barrier's phase for `bytes`; what has arrived before this counts.
+__device__ __forceinline__ void bar_expect(uint64_t* bar, int bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(smem_address(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool bar_wait(uint64_t* bar, int parity) {  // false: the wait ran out
+  const uint32_t at = smem_address(bar);
+  for (unsigned spins = 0; spins < kTestLimit; ++spins) {
+    uint32_t done;
+    asm volatile(
+        "{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+        : "=r"(done) : "r"(at), "r"(parity) : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The last thing a CTA does: its shared memory stays until its partners have stopped sending.  After a wait that ran out
+// some of their stores may still be on the way when all have arrived here, hence the pause (the stores take well under a
+// microsecond).
+__device__ __forceinline__ void leave(bool failed, int* status) {
+  if (failed && threadIdx.x == 0) atomicExch(status, LSTM_ERR_EXCHANGE_TIMEOUT);
+  cluster_barrier();
+  if (failed) {
+    const long long t0 = clock64();
+    while (clock64() - t0 < 40000) {
+    }
+  }
+}
+
+// -------------------------------------------------------------------------------------------------
+// weights
+// -------------------------------------------------------------------------------------------------
 // 8 consecutive elements of a weight row (4-byte loads: the weights need no more than 4-byte alignment).
 __device__ __forceinline__ uint4 load_row8(const elem_t* p, bool on) {
   uint4 v = make_uint4(0, 0, 0, 0);
@@ -93,30 +176,32 @@ __device__ __forceinline__ uint4 load_row8(const elem_t* p, bool on) {
   return v;
 }
 
-// The K slice of a warp: K blocks kb = warp + WARPS·j (32 columns each); lane q of a quad owns columns 8q..8q+7 of a
-// block.  The two k-steps of a block use elements (0,1 | 2,3) and (4,5 | 6,7) of those for the two K halves of the
-// MMA, in the weights and in the vector alike, so the order of the sum is all that changes.
+// A warp's MMA tiles (16 rows) times its K blocks (32 columns).  Lane q of a quad owns columns 8q..8q+7 of a block, so
+// that a fragment of the vector is one 16-byte piece.  The two k-steps of a block use elements (0,1 | 2,3) and
+// (4,5 | 6,7) of those for the two K halves of the MMA, in the weights and in the vector alike, so the order of the sum
+// is all that changes.
 // The first RB blocks of a warp have their weights in registers, the remaining SB in shared memory.
-template <int WARPS, int TILES, int RB, int SB>
+template <int THREADS, int TILES, int RB, int SB>
 struct Weights {
   uint4 lo[RB][TILES], hi[RB][TILES];
 
-  template <typename RowPtr>  // row(tile, r): pointer to row r of an MMA tile, or nullptr
-  __device__ __forceinline__ void load(RowPtr row, int H, uint4* wsm) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  // row(tile, r): pointer to row r of an MMA tile, or nullptr; col(j): first column of block j, or one past the end
+  template <typename RowPtr, typename Col>
+  __device__ __forceinline__ void load(RowPtr row, Col col, int end, uint4* wsm) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
 #pragma unroll
     for (int j = 0; j < RB + SB; ++j)
 #pragma unroll
       for (int tile = 0; tile < TILES; ++tile) {
-        const int k = (warp + WARPS * j) * 32 + q * 8;
+        const int k = col(j) + q * 8;
         const elem_t *p = row(tile, g), *p8 = row(tile, g + 8);
-        const uint4 a = load_row8(p + k, p != nullptr && k < H), b = load_row8(p8 + k, p8 != nullptr && k < H);
+        const uint4 a = load_row8(p + k, p != nullptr && k < end), b = load_row8(p8 + k, p8 != nullptr && k < end);
         if (j < RB) {
           lo[j < RB ? j : 0][tile] = a;
           hi[j < RB ? j : 0][tile] = b;
         } else {  // read back by the same thread only: no barrier
-          wsm[(((j - RB) * TILES + tile) * 2) * (WARPS * 32) + threadIdx.x] = a;
-          wsm[(((j - RB) * TILES + tile) * 2 + 1) * (WARPS * 32) + threadIdx.x] = b;
+          wsm[(((j - RB) * TILES + tile) * 2) * THREADS + threadIdx.x] = a;
+          wsm[(((j - RB) * TILES + tile) * 2 + 1) * THREADS + threadIdx.x] = b;
         }
       }
   }
@@ -132,13 +217,7 @@ struct Weights {
 #pragma unroll
       for (int tile = 0; tile < TILES; ++tile) {
         uint4 a, b;
-        if (j < RB) {
-          a = lo[j < RB ? j : 0][tile];
-          b = hi[j < RB ? j : 0][tile];
-        } else {
-          a = wsm[(((j - RB) * TILES + tile) * 2) * (WARPS * 32) + threadIdx.x];
-          b = wsm[(((j - RB) * TILES + tile) * 2 + 1) * (WARPS * 32) + threadIdx.x];
-        }
+        get(j, tile, a, b, wsm);
         mma_16816(acc[tile], a.x, b.x, a.y, b.y, v[j].x, v[j].y);
         mma_16816(TILES > 2 ? acc[tile] : odd[tile], a.z, b.z, a.w, b.w, v[j].z, v[j].w);
       }
@@ -149,168 +228,226 @@ struct Weights {
         for (int i = 0; i < 4; ++i) acc[tile][i] += odd[tile][i];
     }
   }
+
+  __device__ __forceinline__ void get(int j, int tile, uint4& a, uint4& b, const uint4* wsm) const {
+    if (j < RB) {
+      a = lo[j < RB ? j : 0][tile];
+      b = hi[j < RB ? j : 0][tile];
+    } else {
+      a = wsm[(((j - RB) * TILES + tile) * 2) * THREADS + threadIdx.x];
+      b = wsm[(((j - RB) * TILES + tile) * 2 + 1) * THREADS + threadIdx.x];
+    }
+  }
 };
 
+// -------------------------------------------------------------------------------------------------
+// exchange
+// -------------------------------------------------------------------------------------------------
 __device__ __forceinline__ bool written(const uint4& v) {
   return v.x != kEmpty && v.y != kEmpty && v.z != kEmpty && v.w != kEmpty;
 }
 
-// Waits until the lane's columns of the vector at `p` (row start + 8q) have been written and returns them; false when
-// the wait ran out.  `vec`: 16-byte aligned rows; otherwise element by element.  KEEP: a round loads only what was not
-// ready in the round before.  The forward pass needs that: every CTA polls the whole vector, and the polls themselves
-// delay the stores they wait for (H = 1024, 128 CTAs: 2.89 us per step without, 2.33 with it).  In the backward pass a
-// CTA polls a quarter, and the plain form is the faster one (2.06 against 2.12 us).
-template <int WARPS, bool KEEP, int NB>
-__device__ __forceinline__ bool poll_vector(uint4 (&v)[NB], const elem_t* p, bool row_ok, int H, int vec) {
-  const int warp = threadIdx.x >> 5, q = threadIdx.x & 3;
+// Loads the lane's N pieces of 8 elements again and again until every one that is `on` has been written (piece i at
+// p + i·stride; what is not on reads as zeros); false when the wait ran out.  `vec`: 16-byte aligned pieces; otherwise
+// element by element.  KEEP: a round loads only what was not ready in the round before.
+template <bool KEEP, int N>
+__device__ __forceinline__ bool poll(uint4 (&v)[N], const elem_t* p, long long stride, const bool (&on)[N], int vec) {
   for (unsigned spins = 0;; ++spins) {
     bool ready = true;
 #pragma unroll
-    for (int j = 0; j < NB; ++j) {
-      const int kb = (warp + WARPS * j) * 32;
-      if (!KEEP || spins == 0) v[j] = make_uint4(0, 0, 0, 0);
-      if (row_ok && kb + q * 8 < H) {
-        if (vec) {
-          if (!KEEP || spins == 0 || !written(v[j])) v[j] = ld_relaxed_v4(p + kb);
-        } else {
-          uint32_t e[8];
+    for (int i = 0; i < N; ++i) {
+      if (!KEEP || spins == 0) v[i] = make_uint4(0, 0, 0, 0);
+      if (!on[i]) continue;
+      if (vec) {
+        if (!KEEP || spins == 0 || !written(v[i])) v[i] = ld_relaxed_v4(p + i * stride);
+      } else {
+        uint32_t e[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            e[i] = ld_relaxed_u16(p + kb + i);
-            ready = ready && e[i] != 0xffffu;
-          }
-          v[j] = make_uint4(e[0] | e[1] << 16, e[2] | e[3] << 16, e[4] | e[5] << 16, e[6] | e[7] << 16);
+        for (int k = 0; k < 8; ++k) {
+          e[k] = ld_relaxed_u16(p + i * stride + k);
+          ready = ready && e[k] != 0xffffu;
         }
+        v[i] = make_uint4(e[0] | e[1] << 16, e[2] | e[3] << 16, e[4] | e[5] << 16, e[6] | e[7] << 16);
       }
     }
 #pragma unroll
-    for (int j = 0; j < NB; ++j)
-      ready = ready && written(v[j]);
+    for (int i = 0; i < N; ++i) ready = ready && written(v[i]);
     if (__all_sync(0xffffffffu, ready)) return true;
     if (spins > kSpinLimit) return false;
   }
 }
 
-// Publishes the values of two neighbouring units (lanes 4 apart; `writer` lanes hold the even one) as one word.
-__device__ __forceinline__ void publish_pair(elem_t* p, float value, bool even_unit, bool on, int vec) {
+// The 16 bits under which a value is published.
+__device__ __forceinline__ uint32_t publish_bits(float value) {
   const elem_t e = f2e(value);
-  uint32_t bits = *reinterpret_cast<const uint16_t*>(&e);
-  if (bits == 0xffffu) bits = 0x7fffu;  // NaN stays NaN
-  const uint32_t other = __shfl_xor_sync(0xffffffffu, bits, 4);
-  if (!on) return;
-  if (!vec) {
-    st_relaxed_u16(p, bits);
-  } else if (even_unit) {
-    st_relaxed_u32(p, bits | other << 16);
+  const uint32_t bits = *reinterpret_cast<const uint16_t*>(&e);
+  return bits == 0xffffu ? 0x7fffu : bits;  // NaN stays NaN
+}
+
+// The lines a CTA writes `kAhead` steps later come back into L2 meanwhile: over long sequences the other streams have
+// pushed out the 0xFF bytes, and polls and partial writes would wait for DRAM.  H = 1024, batch 8, 1024 steps: forward
+// 1.54 -> 1.49, backward 1.90 -> 1.74 us a step; nothing up to H = 512; 1 % slower above 1024, where it is left out.
+constexpr int kAhead = 8;
+__device__ __forceinline__ void prefetch_l2(const elem_t* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+__device__ __forceinline__ long long clock_now() {
+  long long c;
+  asm volatile("mov.u64 %0, %%clock64;" : "=l"(c)::"memory");
+  return c;
+}
+// Waits until `cycles` after `since`.  A vector cannot be there before about 900 cycles after its publication (one store to
+// L2 and one load from it), and polls of a line that is being written hold the writer up.  us per step of the forward pass
+// at H = 1024, batch 8, with waits of 0, 200, 300 .. 600 cycles: 2.19 2.12 1.71 1.54 1.54 1.58.
+__device__ __forceinline__ void hold(long long since, int cycles) {
+  while (clock_now() - since < cycles) {
   }
 }
+
 
 // -------------------------------------------------------------------------------------------------
 // forward
 // -------------------------------------------------------------------------------------------------
-// U = 8·UT units per CTA, 8·UT warps, H <= 32·8·UT·(RB + SB), P groups of 8 batch rows per CTA.
-template <int UT, int SB>
+// 8·UT warps, 8·UT units per CTA; warp w multiplies K blocks w + 8·UT·j with all 32·UT gate rows of the CTA;
+// H <= 256·UT·(RB + SB); P groups of 8 batch rows per CTA.
+template <int UT, int SB, int P>
 constexpr size_t fwd_smem() {
-  return (size_t)SB * 2 * UT * 2 * (256 * UT) * 16 + (size_t)2 * (8 * UT) * 8 * (32 * UT + 4) * sizeof(float);
+  return (size_t)SB * 2 * UT * 2 * (256 * UT) * 16 + (size_t)2 * P * (8 * UT) * 8 * (32 * UT + 4) * sizeof(float);
 }
 
 template <int UT, int RB, int SB, int P>
 __global__ void __launch_bounds__(256 * UT, 1)
 lstm_fwd_kernel(float* __restrict__ gates, const elem_t* __restrict__ whh, const float* __restrict__ h0,
                 const float* __restrict__ c0, elem_t* y, float* __restrict__ c_all, int* status, int T, int B, int H,
-                int per_sample, int b0, int groups, int vec) {
-  constexpr int kWarps = 8 * UT, kTiles = 2 * UT, kLd = 32 * UT + 4;  // row pitch: conflict-free both ways
+                int per_sample, int b0, int groups, int vec, int wait) {
+  constexpr int kWarps = 8 * UT, kThreads = 32 * kWarps, kTiles = 2 * UT, kBlocks = RB + SB;
+  constexpr int kLd = 32 * UT + 4;  // row pitch of the partial sums: conflict-free both ways
   extern __shared__ uint4 dyn_smem[];
   uint4* wsm = dyn_smem;
-  float* part = reinterpret_cast<float*>(dyn_smem + SB * kTiles * 2 * kWarps * 32);  // [2][warp][8 batch][kLd]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = lane >> 2, q = lane & 3;
+  float* part = reinterpret_cast<float*>(dyn_smem + SB * kTiles * 2 * kThreads);  // [2][P][warp][8 batch][kLd]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
   const int unit_ctas = H / (8 * UT);
   const int unit0 = (blockIdx.x % unit_ctas) * 8 * UT, grp = blockIdx.x / unit_ctas;
+  const int row_base = b0 + 8 * grp, row_step = 8 * groups;  // first row of group p: row_base + p·row_step
 
   // MMA tile = (unit group of 8) * 2 + {i|f, g|o}; rows 0-7 the first gate, 8-15 the second
-  Weights<kWarps, kTiles, RB, SB> w;
+  Weights<kThreads, kTiles, RB, SB> w;
   w.load([&](int tile, int r) { return whh + ((long long)((tile & 1) * 2 + (r >> 3)) * H + unit0 + (tile >> 1) * 8 + (r & 7)) * H; },
-         H, wsm);
+         [&](int j) { return (warp + kWarps * j) * 32; }, H, wsm);
 
-  // this thread's gate value: batch row ob of a group, unit `unit`, gate q (a quad of lanes owns one unit and row)
+  // this quad's cells: batch row ob of each group, unit `unit`; a lane has gate q
   const int ob = warp / UT, unit = unit0 + (warp % UT) * 8 + g;
   const int prow = (warp % UT) * 32 + q * 8 + g;  // its row among the CTA's gate rows
+  const float act_scale = (q == 2 ? 2.0f : 1.0f) * -1.44269504f;
+  const bool writes = q == 0 && (!vec || (g & 1) == 0);
+  const long long step = (long long)B * H;
+  // Element of y and c_all at the step at hand, group 0 (the lane's gate lies at 4·at + gate_at), and what the lane polls.
+  // With weights in shared memory too there is no register to spare and both come from t each time (2.44 against 2.58 us a
+  // step with running addresses at H = 2048, batch 4); the other forms are up to 8 % faster with running addresses.
+  long long at = (long long)(row_base + ob) * H + unit;
+  const int gate_at = q * H - 3 * unit;
+  const elem_t* src = y + (long long)(row_base + g) * H + warp * 32 + q * 8;
   float c[P], xg[P];
 #pragma unroll
   for (int p = 0; p < P; ++p) {
-    const int row = b0 + 8 * (p * groups + grp) + ob;
+    const int row = row_base + p * row_step + ob;
     c[p] = xg[p] = 0.0f;
     if (row < B) {
       // initial state: one learned vector broadcast over the batch, or (per_sample) a (B, H) state carried over
       c[p] = c0[per_sample ? (long long)row * H + unit : unit];
-      xg[p] = gates[(long long)row * 4 * H + (long long)q * H + unit];
+      xg[p] = gates[((long long)row * 4 + q) * H + unit];
     }
   }
 
-  int par = 0;
+  bool bad = false;
+  long long published = clock_now();
   for (int t = 0; t < T; ++t) {
+    const int par = t & 1;
+    if (t > 0) hold(published, wait);
 #pragma unroll
     for (int p = 0; p < P; ++p) {
-      const int row0 = b0 + 8 * (p * groups + grp);
+      const int row0 = row_base + p * row_step;
       if (row0 >= B) continue;  // the same for the whole block
-      uint4 v[RB + SB];
-      int bad = 0;
-      {
-        const int row = row0 + g;  // the MMA's batch column of this lane
-        if (t > 0) {
-          bad = !poll_vector<kWarps, true>(v, y + ((long long)(t - 1) * B + row) * H + q * 8, row < B, H, vec);
-        } else {
+      uint4 v[kBlocks];
+      bool on[kBlocks];
 #pragma unroll
-          for (int j = 0; j < RB + SB; ++j) {
-            const int k = (warp + kWarps * j) * 32 + q * 8;
-            elem2_t e[4] = {ff2e2(0, 0), ff2e2(0, 0), ff2e2(0, 0), ff2e2(0, 0)};
-            if (row < B && k < H) {
-              const float* hp = h0 + (per_sample ? (long long)row * H : 0) + k;
+      for (int j = 0; j < kBlocks; ++j) on[j] = row0 + g < B && (warp + kWarps * j) * 32 + q * 8 < H;
+      if (t > 0) {
+        const elem_t* from = SB > 0 ? y + ((long long)(t - 1) * B + row0 + g) * H + warp * 32 + q * 8 : src + p * row_step * H;
+        bad = !poll<true>(v, from, kWarps * 32, on, vec) || bad;
+      } else {
 #pragma unroll
-              for (int i = 0; i < 4; ++i) e[i] = ff2e2(hp[2 * i], hp[2 * i + 1]);
-            }
-            const uint32_t* eb = reinterpret_cast<const uint32_t*>(e);
-            v[j] = make_uint4(eb[0], eb[1], eb[2], eb[3]);
+        for (int j = 0; j < kBlocks; ++j) {
+          elem2_t e[4] = {ff2e2(0, 0), ff2e2(0, 0), ff2e2(0, 0), ff2e2(0, 0)};
+          if (on[j]) {
+            const float* hp = h0 + (per_sample ? (long long)(row0 + g) * H : 0) + (warp + kWarps * j) * 32 + q * 8;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) e[i] = ff2e2(hp[2 * i], hp[2 * i + 1]);
           }
+          const uint32_t* eb = reinterpret_cast<const uint32_t*>(e);
+          v[j] = make_uint4(eb[0], eb[1], eb[2], eb[3]);
         }
       }
       float acc[kTiles][4];
       w.multiply(acc, v, wsm);
-      float* pp = part + (par * kWarps + warp) * 8 * kLd;
+      float* pp = part + ((par * P + p) * kWarps + warp) * 8 * kLd + g;
 #pragma unroll
       for (int tile = 0; tile < kTiles; ++tile) {
-        pp[(2 * q) * kLd + tile * 16 + g] = acc[tile][0];
-        pp[(2 * q + 1) * kLd + tile * 16 + g] = acc[tile][1];
-        pp[(2 * q) * kLd + tile * 16 + g + 8] = acc[tile][2];
-        pp[(2 * q + 1) * kLd + tile * 16 + g + 8] = acc[tile][3];
+        pp[(2 * q) * kLd + tile * 16] = acc[tile][0];
+        pp[(2 * q + 1) * kLd + tile * 16] = acc[tile][1];
+        pp[(2 * q) * kLd + tile * 16 + 8] = acc[tile][2];
+        pp[(2 * q + 1) * kLd + tile * 16 + 8] = acc[tile][3];
       }
-      if (__syncthreads_or(bad)) {  // a wait ran out: the whole block leaves at the same step
-        if (threadIdx.x == 0) atomicExch(status, LSTM_ERR_EXCHANGE_TIMEOUT);
-        return;
-      }
-      float s0 = 0.0f, s1 = 0.0f;
-      const float* ps = part + (par * kWarps * 8 + ob) * kLd + prow;
+    }
+    if (__syncthreads_or(bad)) {  // a wait ran out: the whole block leaves at the same step
+      if (threadIdx.x == 0) atomicExch(status, LSTM_ERR_EXCHANGE_TIMEOUT);
+      return;
+    }
+    float a[P];
 #pragma unroll
-      for (int i = 0; i < kWarps; i += 2) {
-        s0 += ps[i * 8 * kLd];
-        s1 += ps[(i + 1) * 8 * kLd];
+    for (int p = 0; p < P; ++p) {
+      float s0 = 0.0f, s1 = 0.0f;
+      const float* ps = part + ((par * P + p) * kWarps * 8 + ob) * kLd + prow;
+#pragma unroll
+      for (int k = 0; k < kWarps; k += 2) {
+        s0 += ps[k * 8 * kLd];
+        s1 += ps[(k + 1) * 8 * kLd];
       }
-      par ^= 1;  // the next barrier separates these reads from the writes of the step after the next
-      const float pre = (s0 + s1) + xg[p];
-      const float a = q == 2 ? tanhf(pre) : sigmoid_f(pre);
-      const float ig = __shfl_sync(0xffffffffu, a, lane & ~3), fg = __shfl_sync(0xffffffffu, a, (lane & ~3) + 1);
-      const float gg = __shfl_sync(0xffffffffu, a, (lane & ~3) + 2), og = __shfl_sync(0xffffffffu, a, (lane & ~3) + 3);
+      a[p] = (s0 + s1) + xg[p];
+    }
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      const float pre = a[p], s = rcp_f(1.0f + ex2_f(act_scale * pre));
+      a[p] = q == 2 ? tanh_from(pre, fmaf(2.0f, s, -1.0f)) : s;
+      const float ig = __shfl_sync(0xffffffffu, a[p], lane & ~3), fg = __shfl_sync(0xffffffffu, a[p], (lane & ~3) + 1);
+      const float gg = __shfl_sync(0xffffffffu, a[p], (lane & ~3) + 2), og = __shfl_sync(0xffffffffu, a[p], (lane & ~3) + 3);
       c[p] = fg * c[p] + ig * gg;
-      const float h = og * tanhf(c[p]);
-      const int row = row0 + ob;
-      const long long at = (long long)t * B + row;
-      publish_pair(y + at * H + unit, h, (g & 1) == 0, row < B && q == 0, vec);
-      if (row < B) {
-        gates[at * 4 * H + (long long)q * H + unit] = a;
-        if (q == 0) c_all[at * H + unit] = c[p];
-        if (t + 1 < T) xg[p] = gates[(at + B) * 4 * H + (long long)q * H + unit];  // needed after the next exchange
+      const uint32_t bits = publish_bits(og * tanh_f(c[p])), other = __shfl_xor_sync(0xffffffffu, bits, 4);
+      const int row = row_base + p * row_step + ob;
+      if (writes && row < B) {
+        elem_t* yp = SB > 0 ? y + ((long long)t * B + row) * H + unit : y + at + p * row_step * H;
+        if (vec)
+          st_relaxed_u32(yp, bits | other << 16);
+        else
+          st_relaxed_u16(yp, bits);
       }
+    }
+    published = clock_now();
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      const int row = row_base + p * row_step + ob;
+      if (row < B) {
+        const long long from_t = (long long)t * B + row;
+        const long long cell = SB > 0 ? from_t * H + unit : at + p * row_step * H;
+        const long long gate = SB > 0 ? (from_t * 4 + q) * H + unit : 4 * cell + gate_at;
+        gates[gate] = a[p];
+        if (q == 0) c_all[cell] = c[p];
+        if (t + 1 < T) xg[p] = gates[gate + 4 * step];  // needed after the next exchange
+        if (SB == 0 && writes && t + kAhead < T) prefetch_l2(y + cell + kAhead * step);
+      }
+    }
+    if (SB == 0) {
+      at += step;
+      if (t > 0) src += step;
     }
   }
 }
@@ -318,28 +455,24 @@ lstm_fwd_kernel(float* __restrict__ gates, const elem_t* __restrict__ whh, const
 // -------------------------------------------------------------------------------------------------
 // backward
 // -------------------------------------------------------------------------------------------------
-// [2][source rank][warp][8·UT units][8 batch] floats; the pitch of a source keeps the four lanes of a quad, which
-// read from the four sources, on different banks.
+// Warp w multiplies K blocks w + 8·UT·j of gate `rank` with the rows of all 32·UT units of the cluster.
+// H <= 256·UT·(RB + SB); P groups of 8 batch rows per CTA.
+//
+// The gate gradients belong to cells: 8·UT units x 8 batch rows x P groups of a CTA, one thread each, 8·UT neighbouring
+// lanes on one batch row.  H is a multiple of 16, so a CTA's units are all there or none of them is.
+struct Cell {
+  int p, unit, row;  // group; unit and row within the CTA
+};
 template <int UT>
-__host__ __device__ constexpr int bwd_src_pitch() { return 8 * UT * UT * 64 + 2; }
-template <int UT, int SB>
-constexpr size_t bwd_smem() {
-  return (size_t)SB * 2 * UT * 2 * (256 * UT) * 16 + (size_t)2 * kCluster * bwd_src_pitch<UT>() * sizeof(float) + 16;
+__device__ __forceinline__ Cell my_cell() {
+  const int rest = threadIdx.x % (64 * UT);
+  return {(int)threadIdx.x / (64 * UT), rest % (8 * UT), rest / (8 * UT)};
 }
 
-__device__ __forceinline__ uint32_t map_to_rank(const void* p, int rank) {
-  uint32_t local = (uint32_t)__cvta_generic_to_shared(p), remote;
-  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
-  return remote;
-}
-__device__ __forceinline__ void st_cluster_v2(uint32_t addr, float a, float b) {
-  asm volatile("st.shared::cluster.v2.f32 [%0], {%1,%2};" ::"r"(addr), "f"(a), "f"(b) : "memory");
-}
-__device__ __forceinline__ void st_cluster_u32(uint32_t addr, uint32_t v) {
-  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
-}
-__device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+template <int UT, int SB, int P>
+constexpr size_t bwd_smem() {
+  return (size_t)SB * 2 * UT * 2 * (256 * UT) * 16 + ((size_t)2 * 8 * UT * 256 * UT + (size_t)2 * kCluster * P * 64 * UT) * sizeof(float) +
+         2 * P * 8;
 }
 
 template <int UT, int RB, int SB, int P>
@@ -347,120 +480,194 @@ __global__ void __launch_bounds__(256 * UT, 1)
 lstm_bwd_kernel(const float* __restrict__ gates, const float* __restrict__ c_all, const float* __restrict__ c0,
                 const elem_t* __restrict__ dy, const elem_t* __restrict__ whh_t, elem_t* dgates, float* __restrict__ dh0,
                 float* __restrict__ dc0, const float* __restrict__ dh_last, const float* __restrict__ dc_last,
-                int* status, int T, int B, int H, int per_sample, int b0, int groups, int vec) {
-  constexpr int kWarps = 8 * UT, kTiles = 2 * UT, kSrc = bwd_src_pitch<UT>();
+                int* status, int T, int B, int H, int per_sample, int b0, int groups, int vec, int wait) {
+  constexpr int kThreads = 256 * UT, kWarps = 8 * UT, kTiles = 2 * UT, kBlocks = RB + SB, kUnits = 8 * UT, kBox = 64 * UT;
   extern __shared__ uint4 dyn_smem[];
   uint4* wsm = dyn_smem;
-  float* inbox = reinterpret_cast<float*>(dyn_smem + SB * kTiles * 2 * kWarps * 32);
-  uint32_t* gave_up = reinterpret_cast<uint32_t*>(inbox + 2 * kCluster * kSrc);  // [2]: a wait of the cluster ran out
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = lane >> 2, q = lane & 3;
+  float* part = reinterpret_cast<float*>(wsm + SB * kTiles * 2 * kThreads);     // [2][warp][32·UT units][8 rows]
+  // [2][P][source][8·UT units][8 rows]; two boxes take turns from step to step.  A partner fills a box again two steps
+  // later, and by then it has been read: the partner's sums of that step need the dGates that this CTA's cells made of it.
+  float* inbox = part + 2 * kWarps * kThreads;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(inbox + 2 * kCluster * P * kBox);  // [2][P]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
   const int rank = blockIdx.x % kCluster, K = 4 * H;
-  const int unit_clusters = (H + kCluster * 8 * UT - 1) / (kCluster * 8 * UT);
+  const int unit_clusters = (H + kCluster * kUnits - 1) / (kCluster * kUnits);
   const int cluster = blockIdx.x / kCluster;
-  const int cunit0 = (cluster % unit_clusters) * kCluster * 8 * UT, grp = cluster / unit_clusters;
-  if (threadIdx.x < 2) gave_up[threadIdx.x] = 0;
+  const int cunit0 = (cluster % unit_clusters) * kCluster * kUnits, grp = cluster / unit_clusters;
+  const int row_base = b0 + 8 * grp, row_step = 8 * groups;
 
   // rows: the cluster's 32·UT units in order; columns: gate `rank`
-  Weights<kWarps, kTiles, RB, SB> w;
+  Weights<kThreads, kTiles, RB, SB> w;
   w.load([&](int tile, int r) {
     const int u = cunit0 + tile * 16 + r;
     return u < H ? whh_t + (long long)u * K + (long long)rank * H : nullptr;
-  }, H, wsm);
-  uint32_t box[kCluster], flag[kCluster];
-#pragma unroll
-  for (int r = 0; r < kCluster; ++r) {
-    box[r] = map_to_rank(inbox + rank * kSrc + warp * UT * 64 + g * 8 + 2 * q, r);
-    flag[r] = map_to_rank(gave_up, r);
+  }, [&](int j) { return (warp + kWarps * j) * 32; }, H, wsm);
+
+  // the sums this thread makes: unit threadIdx / 2 of the cluster, four batch rows of a group; they go out as one 16-byte
+  // store (every store costs the receiver's barrier an update: 256 of 4 bytes took 200 cycles longer than 64 of 16)
+  const int sum_unit = threadIdx.x >> 1, sum_row = (threadIdx.x & 1) * 4, owner = (sum_unit / kUnits) % kCluster;
+  const uint32_t box = map_to_rank(inbox + rank * kBox + threadIdx.x * 4 % kBox, owner), box_bar = map_to_rank(bars, owner);
+  const bool sum_on = threadIdx.x < 64 * UT && cunit0 + sum_unit < H;
+
+  const Cell cell = my_cell<UT>();
+  const int unit = cunit0 + rank * kUnits + cell.unit, row = row_base + cell.p * row_step + cell.row;
+  const bool live = cell.p < P && row < B && unit < H;
+  const bool warp_live = __any_sync(0xffffffffu, live);
+  const bool writes = live && (!vec || (lane & 1) == 0);
+  const bool opens = live && threadIdx.x % (64 * UT) == 0;  // opens the phases of its group's barriers
+  const int expected = kCluster * kUnits * ((min(8, B - (row_base + cell.p * row_step)) + 3) / 4) * 16;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 2 * P; ++i) bar_init(bars + i);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  if (opens) {
+    bar_expect(bars + cell.p, expected);
+    bar_expect(bars + P + cell.p, expected);
   }
 
-  // this thread's value: batch row ob of a group, unit `unit`, gate q (a quad of lanes owns one unit and row)
-  const int ob = warp / UT, ug = warp % UT, unit = cunit0 + rank * 8 * UT + ug * 8 + g;
-  float dc[P] = {}, n_a[P] = {}, n_ct[P] = {}, n_cp[P] = {}, n_dy[P] = {};
-
-  auto fetch = [&](int p, int t, int row, float ct) {  // point-wise inputs of step t
-    const long long at = (long long)t * B + row;
-    n_a[p] = gates[at * K + (long long)q * H + unit];
-    n_ct[p] = ct;
-    n_cp[p] = t > 0 ? c_all[(at - B) * H + unit] : c0[per_sample ? (long long)row * H + unit : unit];
-    n_dy[p] = e2f(dy[at * H + unit]);
-  };
-  // gate gradients of step t from dh, published as dGates[t]
-  auto pointwise = [&](int p, int t, int row, float dh_in) {
-    const float a = n_a[p];
-    const float ig = __shfl_sync(0xffffffffu, a, lane & ~3), fg = __shfl_sync(0xffffffffu, a, (lane & ~3) + 1);
-    const float gg = __shfl_sync(0xffffffffu, a, (lane & ~3) + 2), og = __shfl_sync(0xffffffffu, a, (lane & ~3) + 3);
-    const float dh = n_dy[p] + dh_in;
-    const float tc = tanhf(n_ct[p]);
-    const float dcv = dh * og * (1.0f - tc * tc) + dc[p];
-    float d = dcv * gg * ig * (1.0f - ig);
-    if (q == 1) d = dcv * n_cp[p] * fg * (1.0f - fg);
-    if (q == 2) d = dcv * ig * (1.0f - gg * gg);
-    if (q == 3) d = dh * tc * og * (1.0f - og);
-    dc[p] = dcv * fg;
-    const bool on = row < B && unit < H;
-    publish_pair(dgates + ((long long)t * B + row) * K + (long long)q * H + unit, d, (g & 1) == 0, on, vec);
-    if (on && t > 0) fetch(p, t - 1, row, n_cp[p]);
-  };
-
-  cluster_barrier();  // the partners' shared memory exists and their flags are clear
+  const long long t_step = (long long)B * H;
+  const float* gp = gates + ((long long)(T - 1) * B + row) * K + unit;    // point-wise inputs of the step at hand
+  const float* cp = c_all + ((long long)(T - 1) * B + row) * H + unit;
+  const elem_t* dyp = dy + ((long long)(T - 1) * B + row) * H + unit;
+  elem_t* dgp = dgates + ((long long)(T - 1) * B + row) * K + unit;
+  float dc = 0.0f, gate[4] = {}, ct = 0.0f, c_prev = 0.0f;  // ct, c_prev: cell state of the step at hand and of the one before
+  uint16_t dy_bits = 0;
+  auto fetch = [&](int t) {  // moves on to step t, whose cell state is the c_prev of the step before
 #pragma unroll
-  for (int p = 0; p < P; ++p) {
-    const int row = b0 + 8 * (p * groups + grp) + ob;
-    const bool on = row < B && unit < H;
-    float dh = 0.0f;
-    if (on) {
-      if (dh_last != nullptr) dh = dh_last[(long long)row * H + unit];
-      if (dc_last != nullptr) dc[p] = dc_last[(long long)row * H + unit];
-      fetch(p, T - 1, row, c_all[((long long)(T - 1) * B + row) * H + unit]);
+    for (int i = 0; i < 4; ++i) gate[i] = gp[(long long)i * H];
+    c_prev = *(t > 0 ? cp - t_step : c0 + (per_sample ? (long long)row * H + unit : unit));
+    dy_bits = *reinterpret_cast<const uint16_t*>(dyp);
+    gp -= 4 * t_step;
+    cp -= t_step;
+    dyp -= t_step;
+  };
+  // What the gate gradients of a step need besides dh: computed while the partial sums are on their way.
+  float to_c, to_o, to_i, to_f, to_g;
+  auto factors = [&] {
+    const float tc = tanh_f(ct);
+    to_c = gate[3] * (1.0f - tc * tc);
+    to_o = tc * gate[3] * (1.0f - gate[3]);
+    to_i = gate[2] * gate[0] * (1.0f - gate[0]);
+    to_f = c_prev * gate[1] * (1.0f - gate[1]);
+    to_g = gate[0] * (1.0f - gate[2] * gate[2]);
+  };
+  // gate gradients from dh, published as dGates of the step at hand
+  auto pointwise = [&](float dh_in) {
+    // the move keeps the conversion here: next to its load it would wait for that load, in front of the next exchange
+    uint16_t now;
+    asm volatile("mov.u16 %0, %1;" : "=h"(now) : "h"(dy_bits));
+    const float dh = e2f(*reinterpret_cast<const elem_t*>(&now)) + dh_in;
+    const float dcv = dh * to_c + dc;
+    uint32_t bits[4] = {publish_bits(dcv * to_i), publish_bits(dcv * to_f), publish_bits(dcv * to_g), publish_bits(dh * to_o)};
+    if (vec) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) bits[i] |= __shfl_xor_sync(0xffffffffu, bits[i], 1) << 16;
+      if (writes)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) st_relaxed_u32(dgp + i * H, bits[i]);
+    } else if (writes) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) st_relaxed_u16(dgp + i * H, bits[i]);
     }
-    pointwise(p, T - 1, row, dh);
-  }
+    dc = dcv * gate[1];
+    ct = c_prev;
+    dgp -= 4 * t_step;
+  };
 
-  int par = 0;
-  for (int t = T - 1; t >= 0; --t) {
+  if (warp_live) {
+    float dh = 0.0f;
+    if (live) {
+      if (dh_last != nullptr) dh = dh_last[(long long)row * H + unit];
+      if (dc_last != nullptr) dc = dc_last[(long long)row * H + unit];
+      ct = *cp;
+      fetch(T - 1);
+    }
+    factors();
+    pointwise(dh);
+    if (live && T > 1) fetch(T - 2);
+  }
+  const elem_t* src = dgates + ((long long)(T - 1) * B + row_base + g) * K + (long long)rank * H + warp * 32 + q * 8;
+  bool cols[kBlocks];
+#pragma unroll
+  for (int j = 0; j < kBlocks; ++j) cols[j] = (warp + kWarps * j) * 32 + q * 8 < H;
+
+  cluster_barrier();  // the partners' barriers exist
+  bool bad = false, failed = false;
+  int buf = 0;
+  long long published = clock_now();
+  for (int t = T - 1; t >= 0 && !failed; --t) {
+    const int n = T - 1 - t, par = n & 1;
 #pragma unroll
     for (int p = 0; p < P; ++p) {
-      const int row0 = b0 + 8 * (p * groups + grp);
-      if (row0 >= B) continue;  // the same for the whole cluster
+      const int row0 = row_base + p * row_step;
+      if (row0 >= B || failed) continue;  // the same for the whole cluster, and for the whole block
       // partial dh_{t-1}[b, unit] = sum over the columns of gate `rank` of dGates[t][b, k] * W_hh[k, unit]
-      uint4 v[RB + SB];
-      if (!poll_vector<kWarps, false>(v, dgates + ((long long)t * B + row0 + g) * K + (long long)rank * H + q * 8, row0 + g < B, H, vec)) {
+      uint4 v[kBlocks];
+      bool on[kBlocks];
 #pragma unroll
-        for (int r = 0; r < kCluster; ++r) st_cluster_u32(flag[r] + par * 4, 1);
-      }
+      for (int j = 0; j < kBlocks; ++j) on[j] = cols[j] && row0 + g < B;
+      if (p == 0) hold(published, wait);
+      bad = !poll<false>(v, src + (long long)p * row_step * K, kWarps * 32, on, vec) || bad;
       float acc[kTiles][4];
       w.multiply(acc, v, wsm);
+      float* pp = part + (buf * kWarps + warp) * kThreads + g * 8 + 2 * q;
 #pragma unroll
-      for (int half = 0; half < 2 * kTiles; ++half) {  // 8 units each: the ones of rank half / UT, group half % UT
-        const uint32_t at = box[half / UT] + (par * kCluster * kSrc + (half % UT) * 64) * 4;
-        st_cluster_v2(at, acc[half >> 1][(half & 1) * 2], acc[half >> 1][(half & 1) * 2 + 1]);
+      for (int tile = 0; tile < kTiles; ++tile) {
+        *reinterpret_cast<float2*>(pp + tile * 128) = make_float2(acc[tile][0], acc[tile][1]);
+        *reinterpret_cast<float2*>(pp + tile * 128 + 64) = make_float2(acc[tile][2], acc[tile][3]);
       }
-      cluster_barrier();
-      if (reinterpret_cast<volatile uint32_t*>(gave_up)[par]) {  // written before the barrier, for all four alike
-        if (threadIdx.x == 0) atomicExch(status, LSTM_ERR_EXCHANGE_TIMEOUT);
-        return;
+      if (__syncthreads_or(bad)) {  // a wait ran out: the whole block leaves at the same step
+        failed = true;
+        continue;
       }
-      float s0 = 0.0f, s1 = 0.0f;
-      const float* ps = inbox + (par * kCluster + q) * kSrc + ug * 64 + g * 8 + ob;
+      if (sum_on && row0 + sum_row < B) {
+        float s[4] = {}, s1[4] = {};
+        const float4* ps = reinterpret_cast<const float4*>(part + buf * kWarps * kThreads) + threadIdx.x;
 #pragma unroll
-      for (int i = 0; i < kWarps; i += 2) {
-        s0 += ps[i * UT * 64];
-        s1 += ps[(i + 1) * UT * 64];
+        for (int i = 0; i < kWarps; i += 2) {
+          const float4 a = ps[i * (kThreads / 4)], b = ps[(i + 1) * (kThreads / 4)];
+          const float even[4] = {a.x, a.y, a.z, a.w}, odd[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            s[r] += even[r];
+            s1[r] += odd[r];
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s[i] += s1[i];
+        st_async_v4(box + ((par * P + p) * kCluster * kBox) * 4, s, box_bar + (par * P + p) * 8);
       }
-      par ^= 1;  // the next barrier separates these reads from the writes of the step after the next
-      float dh = s0 + s1;
-      dh += __shfl_xor_sync(0xffffffffu, dh, 1);
-      dh += __shfl_xor_sync(0xffffffffu, dh, 2);
-      const int row = row0 + ob;
+      buf ^= 1;  // the next barrier separates these reads from the writes after the next ones
+    }
+    src -= 4 * t_step;
+    if (warp_live && !failed) {
+      if (t > 0) factors();
+      if (!bar_wait(bars + par * P + (cell.p < P ? cell.p : 0), (n >> 1) & 1)) bad = true;
+      if (opens) bar_expect(bars + par * P + cell.p, expected);
+      float dh = 0.0f;
+      if (live) {
+        const float* in = inbox + (par * P + cell.p) * kCluster * kBox + cell.unit * 8 + cell.row;
+        dh = (in[0] + in[kBox]) + (in[2 * kBox] + in[3 * kBox]);
+      }
       if (t > 0) {
-        pointwise(p, t - 1, row, dh);
-      } else if (row < B && unit < H && q == 0) {
+        pointwise(dh);
+      } else if (live) {
         dh0[(long long)row * H + unit] = dh;
-        dc0[(long long)row * H + unit] = dc[p];
+        dc0[(long long)row * H + unit] = dc;
+      }
+    }
+    if (t > 0 && !failed) {
+      __syncthreads();  // no warp polls before the CTA has published
+      published = clock_now();
+      if (live && t > 1) fetch(t - 2);
+      if (SB == 0 && writes && t > kAhead) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) prefetch_l2(dgp - 4 * kAhead * t_step + i * H);
       }
     }
   }
+  leave(__syncthreads_or(failed || bad), status);
 }
 
 // -------------------------------------------------------------------------------------------------
@@ -491,54 +698,68 @@ int coop_launch(K kernel, int grid, int threads, int cluster, void** args, size_
   return e == cudaErrorCooperativeLaunchTooLarge ? 1 : 5;
 }
 
-// How a launch covers `rows` (<= 32) batch rows at hidden size H.
-// 16 units per CTA (half the CTAs of a group of 8 rows, so half the pollers, and the machine holds two groups at
-// H = 1024, four at 512) against 8 units (less work in each CTA), 8 rows:
-//   H = 1024 forward   1.88 us per step with 16 units, 2.33 with 8: fewer pollers of each line win;
-//   H = 1024 backward  2.85 us with 16 units, 2.06 with 8: polls are a quarter already, the smaller share wins;
-//   H <= 512           8 units while there is one group; more groups fit beside one another with 16 (H > 256).
-// Above 1024 the weights need 16 units per CTA on all SMs.  What does not fit side by side takes turns.
+// How a launch covers `rows` (<= max_rows) batch rows at hidden size H.  us per step, forward | backward:
+//   H <= 512, to 16 rows    8 units per CTA: H = 512, 8 rows 1.19 | 1.41; with 16 units 1.47 | 1.57
+//   H <= 512, 17 to 32      16 units, so that four groups fit beside one another: H = 512, 32 rows 1.45 | 1.84; with 8 units
+//                           and two groups per CTA 2.07 | 2.60
+//   H <= 1024, to 8 rows    8 units: 8 rows 1.49 | 1.74; with 16 units 1.65 | 2.15
+//   H <= 1024, more         16 units, two groups beside one another, up to two in a CTA: 16 rows 1.75 | 1.91, 32 rows
+//                           2.73 | 3.06; with 8 units 2.40 | 2.97 and 4.9 | 5.1
+//   above                   16 units on all SMs, groups in a CTA: H = 2048, 8 rows 2.78 | 3.00, 32 rows - | 9.8.  The
+//                           forward pass has no shared memory for a second group beside the weights: 8 rows per launch
+//                           (a launch for 32 rows whose groups took turns needed 12.9).
 struct Shape {
   bool wide;   // 16 units per CTA instead of 8
   int groups;  // groups of 8 rows on different CTAs
-  int turns;   // groups of 8 rows per CTA (1, 2 or 4)
+  int shared;  // groups of 8 rows per CTA
+  int wait;    // cycles from a CTA's publication to its first poll
 };
 Shape lstm_shape(int rows, int H, bool forward) {
   const int sub = (rows + 7) / 8;
   Shape s;
-  s.wide = H > 1024 || (H > 256 && sub > 1) || (H > 512 && forward);
-  const int fit = H <= 512 ? 4 : H <= 1024 ? 2 : 1;
+  s.wide = H > 1024 || (H > 512 ? sub > 1 : H > 256 && sub > 2);
+  const int fit = H <= 256 || (H <= 512 && s.wide) ? 4 : H <= 512 || (H <= 1024 && s.wide) ? 2 : 1;
   s.groups = sub < fit ? sub : fit;
-  const int turns = (sub + s.groups - 1) / s.groups;
-  s.turns = turns > 2 ? 4 : turns;
+  s.shared = (sub + s.groups - 1) / s.groups;
+  // Lowest time per step over waits of 0, 100 .. 1400 cycles; flat around it, except in the backward pass at H = 1024:
+  // 8 rows 2.23 us with 400, 1.74 with 800; 3 rows 1.78 and 1.95.
+  if (forward)
+    s.wait = H <= 256 ? 150 : H <= 512 ? (s.wide ? 450 : 300) : s.shared > 1 ? 300 : 450;
+  else
+    s.wait = H <= 256 ? 150 : H > 512 && H <= 1024 && rows > 3 && !s.wide ? 800 : 400;
   return s;
 }
+// Rows of one launch.
+int max_rows(int H, bool forward) { return forward && H > 1024 ? 8 : 32; }
 
 // SIDE: 0 forward, 1 backward.
 template <int SIDE, int UT, int RB, int SB, int P>
 int launch_one(int H, int groups, void** args, cudaStream_t s) {
   if constexpr (SIDE == 0)
-    return coop_launch(lstm_fwd_kernel<UT, RB, SB, P>, H / (8 * UT) * groups, 256 * UT, 1, args, fwd_smem<UT, SB>(), s);
+    return coop_launch(lstm_fwd_kernel<UT, RB, SB, P>, H / (8 * UT) * groups, 256 * UT, 1, args, fwd_smem<UT, SB, P>(), s);
   else
     return coop_launch(lstm_bwd_kernel<UT, RB, SB, P>, (H + kCluster * 8 * UT - 1) / (kCluster * 8 * UT) * kCluster * groups,
-                       256 * UT, kCluster, args, bwd_smem<UT, SB>(), s);
+                       256 * UT, kCluster, args, bwd_smem<UT, SB, P>(), s);
 }
 
 template <int SIDE>
 int launch_shape(const Shape& sh, int H, void** args, cudaStream_t s) {
-  if (!sh.wide) {
-    if (H <= 256) return launch_one<SIDE, 1, 1, 0, 1>(H, sh.groups, args, s);
-    if (H <= 512) return launch_one<SIDE, 1, 2, 0, 1>(H, sh.groups, args, s);
-    if constexpr (SIDE == 1) return launch_one<SIDE, 1, 4, 0, 1>(H, sh.groups, args, s);
+  if (H <= 256) return launch_one<SIDE, 1, 1, 0, 1>(H, sh.groups, args, s);
+  if (H <= 512) {
+    if (!sh.wide) return launch_one<SIDE, 1, 2, 0, 1>(H, sh.groups, args, s);
+    return launch_one<SIDE, 2, 1, 0, 1>(H, sh.groups, args, s);
   }
-  if (H <= 512) return launch_one<SIDE, 2, 1, 0, 1>(H, sh.groups, args, s);
   if (H <= 1024) {
-    if (sh.turns == 1) return launch_one<SIDE, 2, 2, 0, 1>(H, sh.groups, args, s);
+    if (!sh.wide) return launch_one<SIDE, 1, 4, 0, 1>(H, sh.groups, args, s);
+    if (sh.shared == 1) return launch_one<SIDE, 2, 2, 0, 1>(H, sh.groups, args, s);
     return launch_one<SIDE, 2, 2, 0, 2>(H, sh.groups, args, s);
   }
-  if (sh.turns == 1) return launch_one<SIDE, 2, 2, 2, 1>(H, sh.groups, args, s);
-  if (sh.turns == 2) return launch_one<SIDE, 2, 2, 2, 2>(H, sh.groups, args, s);
-  return launch_one<SIDE, 2, 2, 2, 4>(H, sh.groups, args, s);
+  if (sh.shared == 1) return launch_one<SIDE, 2, 2, 2, 1>(H, sh.groups, args, s);
+  if constexpr (SIDE == 1) {
+    if (sh.shared == 2) return launch_one<SIDE, 2, 2, 2, 2>(H, sh.groups, args, s);
+    return launch_one<SIDE, 2, 2, 2, 4>(H, sh.groups, args, s);
+  }
+  return 1;
 }
 
 }  // namespace
@@ -561,9 +782,9 @@ int fbam_lstm_fwd_ex(float* gates, const void* whh, const float* h0, const float
   const size_t exchanged = (size_t)(T - 1) * B * H * sizeof(elem_t);  // nobody reads the last step's y
   if (exchanged != 0 && cudaMemsetAsync(y, 0xff, exchanged, s) != cudaSuccess) return 5;
   int vec = reinterpret_cast<uintptr_t>(y) % 16 == 0;
-  for (int b0 = 0; b0 < B; b0 += kLaunchRows) {
-    Shape sh = lstm_shape(B - b0 < kLaunchRows ? B - b0 : kLaunchRows, H, true);
-    void* args[] = {&gates, &whh, &h0, &c0, &y, &c_all, &status, &T, &B, &H, &per_sample, &b0, &sh.groups, &vec};
+  for (int b0 = 0, most = max_rows(H, true); b0 < B; b0 += most) {
+    Shape sh = lstm_shape(B - b0 < most ? B - b0 : most, H, true);
+    void* args[] = {&gates, &whh, &h0, &c0, &y, &c_all, &status, &T, &B, &H, &per_sample, &b0, &sh.groups, &vec, &sh.wait};
     const int rc = launch_shape<0>(sh, H, args, s);
     if (rc != 0) return rc;
   }
@@ -586,10 +807,10 @@ int fbam_lstm_bwd_ex(const float* gates, const float* c_all, const float* c0, co
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (cudaMemsetAsync(dgates, 0xff, (size_t)T * B * 4 * H * sizeof(elem_t), s) != cudaSuccess) return 5;
   int vec = reinterpret_cast<uintptr_t>(dgates) % 16 == 0;
-  for (int b0 = 0; b0 < B; b0 += kLaunchRows) {
-    Shape sh = lstm_shape(B - b0 < kLaunchRows ? B - b0 : kLaunchRows, H, false);
+  for (int b0 = 0, most = max_rows(H, false); b0 < B; b0 += most) {
+    Shape sh = lstm_shape(B - b0 < most ? B - b0 : most, H, false);
     void* args[] = {&gates, &c_all, &c0, &dy, &whh_t, &dgates, &dh0, &dc0, &dh_last, &dc_last, &status,
-                    &T, &B, &H, &per_sample, &b0, &sh.groups, &vec};
+                    &T, &B, &H, &per_sample, &b0, &sh.groups, &vec, &sh.wait};
     const int rc = launch_shape<1>(sh, H, args, s);
     if (rc != 0) return rc;
   }

@@ -155,3 +155,55 @@ def test_operand_layouts_and_sizes(b):
                   (w_ih, w_hh, b_ih, b_hh, h0[:-1], c0), (w_ih, w_hh, b_ih, b_hh, h0, c0[:-1])):
         with pytest.raises((ValueError, RuntimeError)):
             L.lstm_sequence(x, *wrong, dtype)
+
+
+@pytest.mark.parametrize("t_len,b,h", [(9, 8, 1024), (10, 4, 1024), (17, 3, 560), (18, 9, 2048), (19, 24, 512), (33, 32, 1024)])
+def test_steps_around_the_prefetch_distance_and_many_phases(t_len, b, h):
+    """More steps than the distance at which lines are fetched ahead, and enough for every barrier of a backward cluster
+    to go through several phases, with groups that share a block and rows that fill a group partly."""
+    from fbamtrain_b200.ops import lstm as L, native as nv
+    params, g = _problem(t_len, b, 64, h, torch.bfloat16)
+    y, _, c_n = L.lstm_sequence(*params, torch.bfloat16)
+    dy = torch.randn(y.shape, device=DEV, generator=g).bfloat16()
+    got = torch.autograd.grad(y, params, dy)
+    nv.check_status(y.device)
+    fp = [p.detach().float().requires_grad_(True) for p in params]
+    yf, _, cf = ref.lstm_sequence(*fp, torch.float32)
+    exp = torch.autograd.grad(yf, fp, dy.float())
+    # 16-bit weights, h and gate gradients: 2^-9 relative each, as above
+    assert _rel(y, yf) < 1e-2 and _rel(c_n, cf) < 1e-2
+    for name, a, e in zip(["dx", "dw_ih", "dw_hh", "db_ih", "db_hh", "dh0", "dc0"], got, exp):
+        assert _rel(a, e) < 4e-2, (name, _rel(a, e))
+
+
+def test_gate_functions_against_64_bits():
+    """One step with a recurrent weight of zeros: the activated gates and the cell state are functions of the given
+    pre-activations alone.  Bounds, relative: 2^x within 2^-22 of an argument that is off by 2^-24 of |x| log2(e), 1/x
+    within 2^-23, and a rounding of 2^-24 for each of the operations around them."""
+    from fbamtrain_b200.ops import native as nv
+    b, h = 8, 512
+    x = torch.cat([torch.linspace(-30, 30, 2 * b * h), torch.linspace(-0.7, 0.7, 2 * b * h)]).to(DEV)
+    x[torch.arange(0, 40, 4)] = torch.tensor([0.0, -0.0, 1e-30, -1e-30, 100.0, -100.0, math.inf, -math.inf, math.nan, 1e-8],
+                                             device=DEV)
+    x = x[torch.randperm(x.numel(), device=DEV, generator=torch.Generator(device=DEV).manual_seed(0))]
+    gates = x.view(1, b, 4 * h).clone()
+    whh = torch.zeros(4 * h, h, device=DEV, dtype=torch.bfloat16)
+    h0 = torch.zeros(h, device=DEV)
+    c0 = torch.randn(h, device=DEV, generator=torch.Generator(device=DEV).manual_seed(1))
+    y = torch.empty(1, b, h, dtype=torch.bfloat16, device=DEV)
+    c_all = torch.empty(1, b, h, device=DEV)
+    assert nv.lib().fbam_lstm_fwd(nv.ptr(gates), nv.ptr(whh), nv.ptr(h0), nv.ptr(c0), nv.ptr(y), nv.ptr(c_all), None, None,
+                                  nv.ptr(nv.status_word(y.device)), 1, b, h, nv.stream_ptr()) == 0
+    pre = x.view(b, 4, h).double()
+    expected = torch.sigmoid(pre)
+    expected[:, 2] = torch.tanh(pre[:, 2])
+    got = gates.view(b, 4, h).double()
+    assert torch.equal(got.isnan(), pre.isnan())
+    ok = ~pre.isnan()
+    bound = expected.abs() * (2.0 ** -22 + 2.0 ** -23 + 3 * 2.0 ** -24 + pre.abs().clamp_max(104.0) * 1.45 * 2.0 ** -24) + 1e-37
+    # tanh is 2 s - 1 above 0.6: the error of s counts twice, relative to at least 0.53
+    bound[:, 2] *= 2.0
+    assert bool(((got - expected).abs() <= bound)[ok].all()), float(((got - expected).abs() / bound)[ok].max())
+    c = got[:, 1] * c0.double() + got[:, 0] * got[:, 2]
+    live = ~c.isnan()
+    assert bool(((c_all[0].double() - c).abs() <= 2.0 ** -23 * (c0.abs() + 1.0))[live].all())
