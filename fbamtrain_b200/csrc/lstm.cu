@@ -38,7 +38,7 @@
 //   H 2048, batch 4:    forward 3.09 -> 2.44, backward 3.75 -> 2.70
 //   H  256, batch 8:    forward 1.06 -> 0.95, backward 1.68 -> 1.29
 //   H 1024, batch 32:   forward 3.47 -> 2.73, backward 6.27 -> 3.06
-//   H 2048, batch 32:   forward 12.9 -> 11.1, backward 16.1 -> 9.8
+//   H 2048, batch 32:   forward 12.9 -> 11.4, backward 16.1 -> 9.8
 // (At H = 1024 a forward cluster that divides K, with partial sums sent as in the backward pass, takes 1.75 us at batch 8,
 // 1.50 without: its second hop costs more than the smaller share of the vector gives.)
 //
@@ -308,13 +308,13 @@ __device__ __forceinline__ void hold(long long since, int cycles) {
 // forward
 // -------------------------------------------------------------------------------------------------
 // 8·UT warps, 8·UT units per CTA; warp w multiplies K blocks w + 8·UT·j with all 32·UT gate rows of the CTA;
-// H <= 256·UT·(RB + SB); P groups of 8 batch rows per CTA.
+// H <= 256·UT·(RB + SB); P groups of 8 batch rows per CTA go through a step together, TURNS times in turn.
 template <int UT, int SB, int P>
 constexpr size_t fwd_smem() {
   return (size_t)SB * 2 * UT * 2 * (256 * UT) * 16 + (size_t)2 * P * (8 * UT) * 8 * (32 * UT + 4) * sizeof(float);
 }
 
-template <int UT, int RB, int SB, int P>
+template <int UT, int RB, int SB, int P, int TURNS>
 __global__ void __launch_bounds__(256 * UT, 1)
 lstm_fwd_kernel(float* __restrict__ gates, const elem_t* __restrict__ whh, const float* __restrict__ h0,
                 const float* __restrict__ c0, elem_t* y, float* __restrict__ c_all, int* status, int T, int B, int H,
@@ -346,26 +346,27 @@ lstm_fwd_kernel(float* __restrict__ gates, const elem_t* __restrict__ whh, const
   long long at = (long long)(row_base + ob) * H + unit;
   const int gate_at = q * H - 3 * unit;
   const elem_t* src = y + (long long)(row_base + g) * H + warp * 32 + q * 8;
-  float c[P], xg[P];
+  float c_of[TURNS][P], xg_of[TURNS][P];
 #pragma unroll
-  for (int p = 0; p < P; ++p) {
-    const int row = row_base + p * row_step + ob;
-    c[p] = xg[p] = 0.0f;
+  for (int i = 0; i < TURNS * P; ++i) {
+    const int row = row_base + i * row_step + ob;
+    float &c = c_of[i / P][i % P], &xg = xg_of[i / P][i % P];
+    c = xg = 0.0f;
     if (row < B) {
       // initial state: one learned vector broadcast over the batch, or (per_sample) a (B, H) state carried over
-      c[p] = c0[per_sample ? (long long)row * H + unit : unit];
-      xg[p] = gates[((long long)row * 4 + q) * H + unit];
+      c = c0[per_sample ? (long long)row * H + unit : unit];
+      xg = gates[((long long)row * 4 + q) * H + unit];
     }
   }
 
   bool bad = false;
   long long published = clock_now();
-  for (int t = 0; t < T; ++t) {
-    const int par = t & 1;
-    if (t > 0) hold(published, wait);
+  // One step of P groups from batch row `base` on.
+  auto advance = [&](int t, int base, int par, float (&c)[P], float (&xg)[P]) {
+    if (t > 0 && TURNS == 1) hold(published, wait);  // another group's turn is longer than any wait
 #pragma unroll
     for (int p = 0; p < P; ++p) {
-      const int row0 = row_base + p * row_step;
+      const int row0 = base + p * row_step;
       if (row0 >= B) continue;  // the same for the whole block
       uint4 v[kBlocks];
       bool on[kBlocks];
@@ -398,10 +399,7 @@ lstm_fwd_kernel(float* __restrict__ gates, const elem_t* __restrict__ whh, const
         pp[(2 * q + 1) * kLd + tile * 16 + 8] = acc[tile][3];
       }
     }
-    if (__syncthreads_or(bad)) {  // a wait ran out: the whole block leaves at the same step
-      if (threadIdx.x == 0) atomicExch(status, LSTM_ERR_EXCHANGE_TIMEOUT);
-      return;
-    }
+    if (__syncthreads_or(bad)) return false;  // a wait ran out: the whole block leaves at the same step
     float a[P];
 #pragma unroll
     for (int p = 0; p < P; ++p) {
@@ -422,7 +420,7 @@ lstm_fwd_kernel(float* __restrict__ gates, const elem_t* __restrict__ whh, const
       const float gg = __shfl_sync(0xffffffffu, a[p], (lane & ~3) + 2), og = __shfl_sync(0xffffffffu, a[p], (lane & ~3) + 3);
       c[p] = fg * c[p] + ig * gg;
       const uint32_t bits = publish_bits(og * tanh_f(c[p])), other = __shfl_xor_sync(0xffffffffu, bits, 4);
-      const int row = row_base + p * row_step + ob;
+      const int row = base + p * row_step + ob;
       if (writes && row < B) {
         elem_t* yp = SB > 0 ? y + ((long long)t * B + row) * H + unit : y + at + p * row_step * H;
         if (vec)
@@ -434,7 +432,7 @@ lstm_fwd_kernel(float* __restrict__ gates, const elem_t* __restrict__ whh, const
     published = clock_now();
 #pragma unroll
     for (int p = 0; p < P; ++p) {
-      const int row = row_base + p * row_step + ob;
+      const int row = base + p * row_step + ob;
       if (row < B) {
         const long long from_t = (long long)t * B + row;
         const long long cell = SB > 0 ? from_t * H + unit : at + p * row_step * H;
@@ -448,6 +446,20 @@ lstm_fwd_kernel(float* __restrict__ gates, const elem_t* __restrict__ whh, const
     if (SB == 0) {
       at += step;
       if (t > 0) src += step;
+    }
+    return true;
+  };
+  int turns = 0;
+  for (int t = 0; t < T; ++t) {
+#pragma unroll
+    for (int i = 0; i < TURNS; ++i) {
+      const int base = row_base + i * P * row_step;
+      if (TURNS > 1 && base >= B) continue;  // the same for the whole block
+      // two buffers of partial sums take turns: a barrier lies between the reads of one and its next writes
+      if (!advance(t, base, TURNS == 1 ? t & 1 : turns++ & 1, c_of[i], xg_of[i])) {
+        if (threadIdx.x == 0) atomicExch(status, LSTM_ERR_EXCHANGE_TIMEOUT);
+        return;
+      }
     }
   }
 }
@@ -698,16 +710,15 @@ int coop_launch(K kernel, int grid, int threads, int cluster, void** args, size_
   return e == cudaErrorCooperativeLaunchTooLarge ? 1 : 5;
 }
 
-// How a launch covers `rows` (<= max_rows) batch rows at hidden size H.  us per step, forward | backward:
+// How a launch covers `rows` (at most 32) batch rows at hidden size H.  us per step, forward | backward:
 //   H <= 512, to 16 rows    8 units per CTA: H = 512, 8 rows 1.19 | 1.41; with 16 units 1.47 | 1.57
 //   H <= 512, 17 to 32      16 units, so that four groups fit beside one another: H = 512, 32 rows 1.45 | 1.84; with 8 units
 //                           and two groups per CTA 2.07 | 2.60
 //   H <= 1024, to 8 rows    8 units: 8 rows 1.49 | 1.74; with 16 units 1.65 | 2.15
 //   H <= 1024, more         16 units, two groups beside one another, up to two in a CTA: 16 rows 1.75 | 1.91, 32 rows
 //                           2.73 | 3.06; with 8 units 2.40 | 2.97 and 4.9 | 5.1
-//   above                   16 units on all SMs, groups in a CTA: H = 2048, 8 rows 2.78 | 3.00, 32 rows - | 9.8.  The
-//                           forward pass has no shared memory for a second group beside the weights: 8 rows per launch
-//                           (a launch for 32 rows whose groups took turns needed 12.9).
+//   above                   16 units on all SMs, groups in a CTA: H = 2048, 8 rows 2.78 | 3.00, 32 rows - | 9.8.  In the
+//                           forward pass they take turns: the weights leave no shared memory for their partial sums.
 struct Shape {
   bool wide;   // 16 units per CTA instead of 8
   int groups;  // groups of 8 rows on different CTAs
@@ -729,14 +740,16 @@ Shape lstm_shape(int rows, int H, bool forward) {
     s.wait = H <= 256 ? 150 : H > 512 && H <= 1024 && rows > 3 && !s.wide ? 800 : 400;
   return s;
 }
-// Rows of one launch.
-int max_rows(int H, bool forward) { return forward && H > 1024 ? 8 : 32; }
+// Batch rows of one launch.  Above H = 1024 a forward step of four groups in turn takes 12.3 us and one of a group alone
+// 2.80, but each launch loads the weights (11 us): a launch per group pays from about 30 steps on (16 steps of 32 rows in
+// turn 12.3 us a step, 13.8 in four launches; 256 steps 12.7 and 11.4).
+int launch_rows(int H, int T, bool forward) { return forward && H > 1024 && T >= 32 ? 8 : 32; }
 
 // SIDE: 0 forward, 1 backward.
-template <int SIDE, int UT, int RB, int SB, int P>
+template <int SIDE, int UT, int RB, int SB, int P, int TURNS = 1>
 int launch_one(int H, int groups, void** args, cudaStream_t s) {
   if constexpr (SIDE == 0)
-    return coop_launch(lstm_fwd_kernel<UT, RB, SB, P>, H / (8 * UT) * groups, 256 * UT, 1, args, fwd_smem<UT, SB, P>(), s);
+    return coop_launch(lstm_fwd_kernel<UT, RB, SB, P, TURNS>, H / (8 * UT) * groups, 256 * UT, 1, args, fwd_smem<UT, SB, P>(), s);
   else
     return coop_launch(lstm_bwd_kernel<UT, RB, SB, P>, (H + kCluster * 8 * UT - 1) / (kCluster * 8 * UT) * kCluster * groups,
                        256 * UT, kCluster, args, bwd_smem<UT, SB, P>(), s);
@@ -755,11 +768,9 @@ int launch_shape(const Shape& sh, int H, void** args, cudaStream_t s) {
     return launch_one<SIDE, 2, 2, 0, 2>(H, sh.groups, args, s);
   }
   if (sh.shared == 1) return launch_one<SIDE, 2, 2, 2, 1>(H, sh.groups, args, s);
-  if constexpr (SIDE == 1) {
-    if (sh.shared == 2) return launch_one<SIDE, 2, 2, 2, 2>(H, sh.groups, args, s);
-    return launch_one<SIDE, 2, 2, 2, 4>(H, sh.groups, args, s);
-  }
-  return 1;
+  constexpr int kTurn2 = SIDE == 0 ? 2 : 1, kTurn4 = SIDE == 0 ? 4 : 1;
+  if (sh.shared == 2) return launch_one<SIDE, 2, 2, 2, 2 / kTurn2, kTurn2>(H, sh.groups, args, s);
+  return launch_one<SIDE, 2, 2, 2, 4 / kTurn4, kTurn4>(H, sh.groups, args, s);
 }
 
 }  // namespace
@@ -782,7 +793,7 @@ int fbam_lstm_fwd_ex(float* gates, const void* whh, const float* h0, const float
   const size_t exchanged = (size_t)(T - 1) * B * H * sizeof(elem_t);  // nobody reads the last step's y
   if (exchanged != 0 && cudaMemsetAsync(y, 0xff, exchanged, s) != cudaSuccess) return 5;
   int vec = reinterpret_cast<uintptr_t>(y) % 16 == 0;
-  for (int b0 = 0, most = max_rows(H, true); b0 < B; b0 += most) {
+  for (int b0 = 0, most = launch_rows(H, T, true); b0 < B; b0 += most) {
     Shape sh = lstm_shape(B - b0 < most ? B - b0 : most, H, true);
     void* args[] = {&gates, &whh, &h0, &c0, &y, &c_all, &status, &T, &B, &H, &per_sample, &b0, &sh.groups, &vec, &sh.wait};
     const int rc = launch_shape<0>(sh, H, args, s);
@@ -807,7 +818,7 @@ int fbam_lstm_bwd_ex(const float* gates, const float* c_all, const float* c0, co
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (cudaMemsetAsync(dgates, 0xff, (size_t)T * B * 4 * H * sizeof(elem_t), s) != cudaSuccess) return 5;
   int vec = reinterpret_cast<uintptr_t>(dgates) % 16 == 0;
-  for (int b0 = 0, most = max_rows(H, false); b0 < B; b0 += most) {
+  for (int b0 = 0, most = launch_rows(H, T, false); b0 < B; b0 += most) {
     Shape sh = lstm_shape(B - b0 < most ? B - b0 : most, H, false);
     void* args[] = {&gates, &c_all, &c0, &dy, &whh_t, &dgates, &dh0, &dc0, &dh_last, &dc_last, &status,
                     &T, &B, &H, &per_sample, &b0, &sh.groups, &vec, &sh.wait};

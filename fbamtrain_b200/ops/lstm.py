@@ -31,8 +31,8 @@ def persistent_shape(hidden: int) -> bool:
 
 
 # us of one launch of the persistent kernels (32 rows): hidden up to, launch, each step; forward, forward + backward
-_LAUNCH_US = ((64, 3.3, 1.05, 5.0, 3.0), (256, 3.0, 1.7, 6.0, 4.0), (512, 4.0, 2.2, 8.0, 5.5), (1024, 7.0, 3.9, 15.0, 11.0),
-              (2048, 10.0, 14.0, 45.0, 33.0))
+_LAUNCH_US = ((64, 3.3, 0.95, 5.9, 2.1), (256, 3.0, 1.4, 6.0, 3.3), (512, 4.0, 1.6, 8.0, 3.6), (1024, 7.0, 3.0, 15.0, 6.9),
+              (2048, 10.0, 12.4, 60.0, 23.0))
 
 
 def persistent_ok(batch: int, hidden: int, steps: int = 1024, grad: bool = True) -> bool:
@@ -41,11 +41,11 @@ def persistent_ok(batch: int, hidden: int, steps: int = 1024, grad: bool = True)
     backward (host and launches) until its product is large, and more the longer the sequence, since the gradient of the
     pre-activations is summed step by step: from 32 steps on it was not ahead at any batch.  Measured, us, persistent |
     GEMM per step:
-      forward  H  256, batch 1536: 1 step 232 | 271, 64 steps 5070 | 9068      batch 2048: 1 step 299 | 246
-      forward  H 1024, batch  512: 1 step 209 | 269, 64 steps 4019 | 9011      batch 2048: 1 step 719 | 250, 16 steps 4370 | 2819
-      forward  H 2048, batch  256: 1 step 260 | 268, 64 steps 7193 | 9141      batch 1024: 1 step 818 | 268, 16 steps 7412 | 3204
-      training H 1024, batch  768: 1 step 819 | 1037, 64 steps 17083 | 47717   batch 2048: 1 step 1855 | 1130, 16 steps 12260 | 11204
-    (Batch 32, 256 steps, H 1024, forward and backward: 2.9 ms against 107.9 ms.)"""
+      forward  H  256, batch 1536: 1 step 329 | 360, 64 steps 4702 | 8010      batch 2048: 1 step 351 | 254
+      forward  H 1024, batch  512: 1 step 251 | 257, 64 steps 3263 | 8025      batch 2048: 1 step 757 | 285, 16 steps 3652 | 2793
+      forward  H 2048, batch  256: 1 step 260 | 262, 64 steps 6511 | 8061      batch 1024: 1 step 818 | 300, 16 steps 6340 | 3007
+      training H 1024, batch  768: 1 step 868 | 1152, 64 steps 10860 | 49738   batch 2048: 1 step 1742 | 996, 16 steps 8176 | 11191
+    (Batch 32, 256 steps, H 1024, forward and backward: 1.9 ms against 107.9 ms.)"""
     if not persistent_shape(hidden):
         return False
     _, fwd_0, fwd, both_0, both = next(row for row in _LAUNCH_US if hidden <= row[0])
