@@ -137,12 +137,18 @@ __global__ void rmsnorm_fwd_kernel(const elem_t* __restrict__ x, const elem_t* _
 // warp and a global one per column and block: 2.93 ms at 983040 rows of 1024, now 1.25 ms (4.8 TB/s).
 // LANES: lanes that share a row, 8 or 16 where it is narrow (a warp per row leaves most lanes idle there, and the
 // instructions per row are what counts: 100000 rows of 64 take 31 us with 32 lanes and 12.6 with 8, of 128 31 and 20.8).
-template <int VEC_PER_LANE, int ROWS, int BLOCKS, int LANES = 32>
+// RES: a gradient that reaches x beside the norm (the residual path) is added to dx in fp32 before the one rounding; as an
+// addition of its own it reads both and writes the sum once more (8192 x 1024, all launches of a backward pass: 44.0 us ->
+// 33.6; 245760 x 1024: 548 -> 384).
+// work != nullptr: the block's part of the dgamma sum goes there, [block][dim], for `partial_sum_kernel`; else it is added
+// to dgamma.
+template <int VEC_PER_LANE, int ROWS, int BLOCKS, int LANES, bool RES>
 __global__ void __launch_bounds__(256, BLOCKS)
-rmsnorm_bwd_kernel(const elem_t* __restrict__ dy, const elem_t* __restrict__ x, const elem_t* __restrict__ w,
-                   const float* __restrict__ rstd, elem_t* __restrict__ dx, float* __restrict__ dgamma, long long rows,
-                   int dim) {
+rmsnorm_bwd_kernel(const elem_t* __restrict__ dy, const elem_t* __restrict__ res, const elem_t* __restrict__ x,
+                   const elem_t* __restrict__ w, const float* __restrict__ rstd, elem_t* __restrict__ dx,
+                   float* __restrict__ dgamma, float* __restrict__ work, long long rows, int dim) {
   constexpr int kWarpRows = 32 / LANES * ROWS;
+  constexpr bool kResEarly = RES && VEC_PER_LANE <= 4;  // wider rows have no registers for a third tensor in flight
   extern __shared__ float sm_dg[];  // [dim]
   const int lane = threadIdx.x % LANES, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int sub_row = (threadIdx.x & 31) / LANES * ROWS;
@@ -154,7 +160,7 @@ rmsnorm_bwd_kernel(const elem_t* __restrict__ dy, const elem_t* __restrict__ x, 
   const long long step = (long long)gridDim.x * warps * kWarpRows;
   for (long long base = ((long long)blockIdx.x * warps + warp) * kWarpRows; base < rows; base += step) {
     const long long row0 = base + sub_row;
-    Pack8 xp[ROWS][VEC_PER_LANE], dp[ROWS][VEC_PER_LANE];
+    Pack8 xp[ROWS][VEC_PER_LANE], dp[ROWS][VEC_PER_LANE], rp[kResEarly ? ROWS : 1][kResEarly ? VEC_PER_LANE : 1];
     float r[ROWS];
 #pragma unroll
     for (int u = 0; u < ROWS; ++u) {
@@ -165,6 +171,7 @@ rmsnorm_bwd_kernel(const elem_t* __restrict__ dy, const elem_t* __restrict__ x, 
         if (c < dim && row0 + u < rows) {
           xp[u][i] = *reinterpret_cast<const Pack8*>(x + (row0 + u) * dim + c);
           dp[u][i] = *reinterpret_cast<const Pack8*>(dy + (row0 + u) * dim + c);
+          if (kResEarly) rp[kResEarly ? u : 0][kResEarly ? i : 0] = *reinterpret_cast<const Pack8*>(res + (row0 + u) * dim + c);
         }
       }
     }
@@ -202,6 +209,13 @@ rmsnorm_bwd_kernel(const elem_t* __restrict__ dy, const elem_t* __restrict__ x, 
           unpack8(*reinterpret_cast<const Pack8*>(w + c), g);
 #pragma unroll
           for (int j = 0; j < 8; ++j) o[j] = r[u] * (dv[j] * g[j] - xv[j] * r[u] * dot);
+          if (RES) {
+            float e[8];
+            unpack8(kResEarly ? rp[kResEarly ? u : 0][kResEarly ? i : 0]
+                              : *reinterpret_cast<const Pack8*>(res + (row0 + u) * dim + c), e);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o[j] += e[j];
+          }
           *reinterpret_cast<Pack8*>(dx + (row0 + u) * dim + c) = pack8(o);
         }
       }
@@ -228,7 +242,35 @@ rmsnorm_bwd_kernel(const elem_t* __restrict__ dy, const elem_t* __restrict__ x, 
     }
     __syncthreads();
   }
-  for (int c = threadIdx.x; c < dim; c += blockDim.x) atomicAdd(&dgamma[c], sm_dg[c]);
+  for (int c = threadIdx.x; c < dim; c += blockDim.x) {
+    if (work != nullptr)
+      work[(long long)blockIdx.x * dim + c] = sm_dg[c];
+    else
+      atomicAdd(&dgamma[c], sm_dg[c]);
+  }
+}
+
+// out[c] = sum of n partial sums work[i][c], in a fixed order, as fp32 or as an element.  A block has 32 columns and 32
+// warps, so that the few hundred rows that there are take some ten loads a thread.
+__global__ void __launch_bounds__(1024) partial_sum_kernel(const float* __restrict__ work, void* __restrict__ out, int out_elem,
+                                                           int n, int cols) {
+  __shared__ float part[32][33];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = blockIdx.x * 32 + lane;
+  float s = 0.0f;
+  if (c < cols) {
+#pragma unroll 4
+    for (int i = warp; i < n; i += 32) s += work[(long long)i * cols + c];
+  }
+  part[warp][lane] = s;
+  __syncthreads();
+  s = warp_sum(part[lane][warp]);
+  const int oc = blockIdx.x * 32 + warp;
+  if (lane == 0 && oc < cols) {
+    if (out_elem)
+      reinterpret_cast<elem_t*>(out)[oc] = f2e(s);
+    else
+      reinterpret_cast<float*>(out)[oc] = s;
+  }
 }
 
 // LayerNorm forward (block per row).
@@ -575,10 +617,11 @@ __global__ void __launch_bounds__(256) global_avgpool_bwd_kernel(const elem_t* _
 // warps per SM at 8192 x 1024).  GELU: the activation gradient in the same pass, dz = dy * gelu'(z), summed as rounded
 // (the other products use that dz, and as a kernel of its own it goes through DRAM once more).
 // 8192 x 8192: 30 us alone (54 before), 77 us with the activation gradient (two kernels: 134 us).
+// work != nullptr: a slab's sums go there, [slab][cols], for `partial_sum_kernel`; else they are added to `out`.
 template <bool GELU>
 __global__ void __launch_bounds__(256, 4) colsum_kernel(const elem_t* __restrict__ x, const elem_t* __restrict__ dy,
-                                                     elem_t* __restrict__ dz, float* __restrict__ out, long long rows,
-                                                     int cols, int rows_per_block) {
+                                                     elem_t* __restrict__ dz, float* __restrict__ out,
+                                                     float* __restrict__ work, long long rows, int cols, int rows_per_block) {
   constexpr int U = GELU ? 2 : 4;
   __shared__ float part[8][32][9];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -623,8 +666,92 @@ __global__ void __launch_bounds__(256, 4) colsum_kernel(const elem_t* __restrict
     float t = 0.0f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) t += part[k][threadIdx.x >> 3][threadIdx.x & 7];
-    atomicAdd(out + oc, t);
+    if (work != nullptr)
+      work[(long long)blockIdx.y * cols + oc] = t;
+    else
+      atomicAdd(out + oc, t);
   }
+}
+
+// The same sums in one launch, for matrices of few rows, where the launches of a fill, the kernel and a conversion are what
+// counts: a cluster owns 64 columns, its CTAs share the rows (a warp takes four at a time), and each CTA adds up the
+// cluster's sums of its part of the columns through distributed shared memory and writes them as fp32 or as elements.
+// us of the launches together (fill, sums by atomics, conversion | this): 256 x 256 11.3 | 8.2, 999 x 4096 15.4 | 10.2,
+// 8192 x 1024 15.6 | 14.4, 30000 x 64 15.3 | 20.5; with the activation gradient 999 x 4096 19.5 | 14.4, 8192 x 1024
+// 23.6 | 28.7.
+template <bool GELU>
+__global__ void __launch_bounds__(512, 2) cluster_colsum_kernel(const elem_t* __restrict__ x, const elem_t* __restrict__ dy,
+                                                               elem_t* __restrict__ dz, void* __restrict__ out, int out_elem,
+                                                               long long rows, int cols) {
+  constexpr int U = GELU ? 2 : 4, kWarps = 16;
+  __shared__ float part[kWarps][64], sums[64];
+  uint32_t ranks, rank;
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, col0 = blockIdx.x / ranks * 64;
+  const int c = col0 + (lane & 7) * 8;
+  const long long step = (long long)ranks * kWarps * 4;
+  float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  if (c < cols) {
+    for (long long r = ((long long)rank * kWarps + warp) * 4 + (lane >> 3); r < rows; r += step * U) {
+      Pack8 p[U], d[GELU ? U : 1];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (r + step * u < rows) {
+          p[u] = *reinterpret_cast<const Pack8*>(x + (r + step * u) * cols + c);
+          if (GELU) d[GELU ? u : 0] = *reinterpret_cast<const Pack8*>(dy + (r + step * u) * cols + c);
+        }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (r + step * u >= rows) break;
+        float v[8];
+        unpack8(p[u], v);
+        if (GELU) {
+          float g[8], e[8];
+          unpack8(d[GELU ? u : 0], e);
+          gelu_grad8(v, g);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) g[j] *= e[j];
+          const Pack8 q = pack8(g);
+          *reinterpret_cast<Pack8*>(dz + (r + step * u) * cols + c) = q;
+          unpack8(q, v);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s[j] += v[j];
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    s[j] += __shfl_xor_sync(0xffffffffu, s[j], 8);
+    s[j] += __shfl_xor_sync(0xffffffffu, s[j], 16);
+    if (lane < 8) part[warp][lane * 8 + j] = s[j];
+  }
+  __syncthreads();
+  if (threadIdx.x < 64) {
+    float t = 0.0f;
+#pragma unroll
+    for (int k = 0; k < kWarps; ++k) t += part[k][threadIdx.x];
+    sums[threadIdx.x] = t;
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  const int per = 64 / ranks, mine = rank * per + threadIdx.x;
+  if (threadIdx.x < per && col0 + mine < cols) {
+    float t = 0.0f;
+    for (uint32_t k = 0; k < ranks; ++k) {
+      uint32_t at;
+      float v;
+      asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(&sums[mine])), "r"(k));
+      asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at));
+      t += v;
+    }
+    if (out_elem)
+      reinterpret_cast<elem_t*>(out)[col0 + mine] = f2e(t);
+    else
+      reinterpret_cast<float*>(out)[col0 + mine] = t;
+  }
+  // no CTA leaves while another may still read its sums
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -981,12 +1108,46 @@ int launch_rms_fwd(const elem_t* x, const elem_t* w, elem_t* y, float* rstd, lon
   rmsnorm_fwd_kernel<V><<<(unsigned)((rows + warps - 1) / warps), warps * 32, 0, s>>>(x, w, y, rstd, rows, dim, eps);
   return cudaGetLastError() == cudaSuccess ? 0 : 5;
 }
+// Rows a block takes at once, and blocks per SM, by width (fbam_rmsnorm_bwd's table).
+struct RmsBwdShape { int rows, blocks; };
+RmsBwdShape rms_bwd_shape(int dim) {
+  return dim <= 64 ? RmsBwdShape{64, 4} : dim <= 128 ? RmsBwdShape{32, 4} : dim <= 256 ? RmsBwdShape{16, 4}
+       : dim <= 512 ? RmsBwdShape{16, 2} : dim <= 2048 ? RmsBwdShape{8, 2} : RmsBwdShape{8, 1};
+}
+int rms_bwd_blocks(long long rows, int dim) {
+  const RmsBwdShape sh = rms_bwd_shape(dim);
+  const long long need = (rows + sh.rows - 1) / sh.rows, fit = 148ll * sh.blocks;
+  return (int)(need < fit ? need : fit);
+}
+struct RmsBwdArgs {
+  const elem_t *dy, *res, *x, *w;
+  const float* rstd;
+  elem_t* dx;
+  float *dgamma, *work;
+  long long rows;
+  int dim;
+};
 template <int V, int ROWS, int BLOCKS, int LANES = 32>
-int launch_rms_bwd(const elem_t* dy, const elem_t* x, const elem_t* w, const float* rstd, elem_t* dx, float* dg, long long rows,
-                   int dim, cudaStream_t s) {
-  const long long block_rows = 8 * (32 / LANES) * ROWS, need = (rows + block_rows - 1) / block_rows, fit = 148ll * BLOCKS;
-  rmsnorm_bwd_kernel<V, ROWS, BLOCKS, LANES>
-      <<<(unsigned)(need < fit ? need : fit), 256, dim * sizeof(float), s>>>(dy, x, w, rstd, dx, dg, rows, dim);
+int launch_rms_bwd(const RmsBwdArgs& a, cudaStream_t s) {
+  const int grid = rms_bwd_blocks(a.rows, a.dim), smem = a.dim * (int)sizeof(float);
+  if (a.res != nullptr)
+    rmsnorm_bwd_kernel<V, ROWS, BLOCKS, LANES, true><<<grid, 256, smem, s>>>(a.dy, a.res, a.x, a.w, a.rstd, a.dx, a.dgamma, a.work, a.rows, a.dim);
+  else
+    rmsnorm_bwd_kernel<V, ROWS, BLOCKS, LANES, false><<<grid, 256, smem, s>>>(a.dy, a.res, a.x, a.w, a.rstd, a.dx, a.dgamma, a.work, a.rows, a.dim);
+  return cudaGetLastError() == cudaSuccess ? 0 : 5;
+}
+int rms_bwd(const RmsBwdArgs& a, cudaStream_t s) {
+  if (a.dim % 8 != 0 || a.dim > 4096) return 1;
+  if (a.dim <= 64) return launch_rms_bwd<1, 2, 4, 8>(a, s);
+  if (a.dim <= 128) return launch_rms_bwd<1, 2, 4, 16>(a, s);
+  if (a.dim <= 256) return launch_rms_bwd<1, 2, 4>(a, s);
+  if (a.dim <= 512) return launch_rms_bwd<2, 2, 2>(a, s);
+  if (a.dim <= 1024) return launch_rms_bwd<4, 1, 2>(a, s);
+  if (a.dim <= 2048) return launch_rms_bwd<8, 1, 2>(a, s);
+  return launch_rms_bwd<16, 1, 1>(a, s);
+}
+int launch_partial_sum(const float* work, void* out, int out_elem, int n, int cols, cudaStream_t s) {
+  partial_sum_kernel<<<(cols + 31) / 32, 1024, 0, s>>>(work, out, out_elem, n, cols);
   return cudaGetLastError() == cudaSuccess ? 0 : 5;
 }
 
@@ -1074,17 +1235,21 @@ int fbam_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, long lo
   return launch_rms_fwd<32>(X, W, (elem_t*)y, rstd, rows, dim, eps, STREAM(stream));
 }
 
+// dgamma: fp32 [dim], added to.
 int fbam_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx, float* dgamma,
                      long long rows, int dim, void* stream) {
-  if (dim % 8 != 0 || dim > 4096) return 1;
-  const elem_t *DY = (const elem_t*)dy, *X = (const elem_t*)x, *W = (const elem_t*)w;
-  if (dim <= 64) return launch_rms_bwd<1, 2, 4, 8>(DY, X, W, rstd, (elem_t*)dx, dgamma, rows, dim, STREAM(stream));
-  if (dim <= 128) return launch_rms_bwd<1, 2, 4, 16>(DY, X, W, rstd, (elem_t*)dx, dgamma, rows, dim, STREAM(stream));
-  if (dim <= 256) return launch_rms_bwd<1, 2, 4>(DY, X, W, rstd, (elem_t*)dx, dgamma, rows, dim, STREAM(stream));
-  if (dim <= 512) return launch_rms_bwd<2, 2, 2>(DY, X, W, rstd, (elem_t*)dx, dgamma, rows, dim, STREAM(stream));
-  if (dim <= 1024) return launch_rms_bwd<4, 1, 2>(DY, X, W, rstd, (elem_t*)dx, dgamma, rows, dim, STREAM(stream));
-  if (dim <= 2048) return launch_rms_bwd<8, 1, 2>(DY, X, W, rstd, (elem_t*)dx, dgamma, rows, dim, STREAM(stream));
-  return launch_rms_bwd<16, 1, 1>(DY, X, W, rstd, (elem_t*)dx, dgamma, rows, dim, STREAM(stream));
+  return rms_bwd({(const elem_t*)dy, nullptr, (const elem_t*)x, (const elem_t*)w, rstd, (elem_t*)dx, dgamma, nullptr, rows, dim},
+                 STREAM(stream));
+}
+
+// The same with the gradient of a residual path added to dx (res, may be null) and dgamma written as elements; work: fp32
+// [fbam_rmsnorm_bwd_partials(rows, dim)][dim].
+int fbam_rmsnorm_bwd_partials(long long rows, int dim) { return rms_bwd_blocks(rows, dim); }
+int fbam_rmsnorm_bwd_to(const void* dy, const void* res, const void* x, const void* w, const float* rstd, void* dx, void* dgamma,
+                        float* work, long long rows, int dim, void* stream) {
+  const int rc = rms_bwd({(const elem_t*)dy, (const elem_t*)res, (const elem_t*)x, (const elem_t*)w, rstd, (elem_t*)dx, nullptr, work,
+                          rows, dim}, STREAM(stream));
+  return rc != 0 ? rc : launch_partial_sum(work, dgamma, 1, rms_bwd_blocks(rows, dim), dim, STREAM(stream));
 }
 
 // partial: fp32 [rows][slots][2] (maximum, sum of exp) from the head GEMM's statistics epilogue; tgt_logit: fp32 [rows];
@@ -1216,7 +1381,7 @@ int fbam_colsum(const void* x, float* out, long long rows, int cols, void* strea
   if (cols % 8 != 0) return 1;
   int rpb;
   const dim3 grid = colsum_grid(rows, cols, &rpb);
-  colsum_kernel<false><<<grid, 256, 0, STREAM(stream)>>>((const elem_t*)x, nullptr, nullptr, out, rows, cols, rpb);
+  colsum_kernel<false><<<grid, 256, 0, STREAM(stream)>>>((const elem_t*)x, nullptr, nullptr, out, nullptr, rows, cols, rpb);
   return CHECK_LAUNCH();
 }
 
@@ -1225,9 +1390,52 @@ int fbam_gelu_bwd_colsum(const void* z, const void* dy, void* dz, float* out, lo
   if (cols % 8 != 0) return 1;
   int rpb;
   const dim3 grid = colsum_grid(rows, cols, &rpb);
-  colsum_kernel<true><<<grid, 256, 0, STREAM(stream)>>>((const elem_t*)z, (const elem_t*)dy, (elem_t*)dz, out, rows, cols,
+  colsum_kernel<true><<<grid, 256, 0, STREAM(stream)>>>((const elem_t*)z, (const elem_t*)dy, (elem_t*)dz, out, nullptr, rows, cols,
                                                         rpb);
   return CHECK_LAUNCH();
+}
+
+// Column sums written to `out` (fp32, or elements with out_elem), with the activation gradient in the same pass where z is
+// given (x is then dy).  work: fp32 [fbam_colsum_partials(rows, cols, z != null)][cols]; 0 of them: not used.
+// One launch of clusters up to 8192 rows, 2048 with the activation gradient (whose loads a cluster has half as many of in
+// flight); above, and for what is narrower than two clusters, slabs over the whole machine and a launch that adds them up.
+static bool colsum_by_clusters(long long rows, int cols, int gelu) { return rows <= (gelu || cols <= 128 ? 2048 : 8192); }
+int fbam_colsum_partials(long long rows, int cols, int gelu) {
+  int rpb;
+  return colsum_by_clusters(rows, cols, gelu) ? 0 : (int)colsum_grid(rows, cols, &rpb).y;
+}
+int fbam_colsum_to(const void* x, const void* z, void* dz, void* out, int out_elem, float* work, long long rows, int cols,
+                   void* stream) {
+  if (cols % 8 != 0) return 1;
+  cudaStream_t s = STREAM(stream);
+  const bool gelu = z != nullptr;
+  if (!colsum_by_clusters(rows, cols, gelu)) {
+    int rpb;
+    const dim3 grid = colsum_grid(rows, cols, &rpb);
+    if (gelu)
+      colsum_kernel<true><<<grid, 256, 0, s>>>((const elem_t*)z, (const elem_t*)x, (elem_t*)dz, nullptr, work, rows, cols, rpb);
+    else
+      colsum_kernel<false><<<grid, 256, 0, s>>>((const elem_t*)x, nullptr, nullptr, nullptr, work, rows, cols, rpb);
+    if (cudaGetLastError() != cudaSuccess) return 5;
+    return launch_partial_sum(work, out, out_elem, grid.y, cols, s);
+  }
+  // as many CTAs per cluster as keep the grid within two CTAs per SM
+  const int groups = (cols + 63) / 64, ranks = groups * 8 <= 296 ? 8 : groups * 4 <= 296 ? 4 : groups * 2 <= 296 ? 2 : 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(groups * ranks);
+  cfg.blockDim = dim3(512);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = ranks;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = gelu ? cudaLaunchKernelEx(&cfg, cluster_colsum_kernel<true>, (const elem_t*)z, (const elem_t*)x, (elem_t*)dz,
+                                                  out, out_elem, rows, cols)
+                             : cudaLaunchKernelEx(&cfg, cluster_colsum_kernel<false>, (const elem_t*)x, (const elem_t*)nullptr,
+                                                  (elem_t*)nullptr, out, out_elem, rows, cols);
+  return e == cudaSuccess ? 0 : 5;
 }
 
 static int embed_threads(int e8) { return (256 / e8 > 0 ? 256 / e8 : 1) * e8; }

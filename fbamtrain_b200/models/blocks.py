@@ -22,7 +22,10 @@ class RmsNorm(nn.Module):
         self.eps = eps
         self.weight = nn.Parameter(torch.ones(dim, dtype=dtype))
 
-    def forward(self, x: torch.Tensor) -> torch.Tensor:
+    def forward(self, x: torch.Tensor, with_input: bool = False):
+        """``with_input``: returns ``x`` too, for a residual path beside the norm (see ``ops.rms_norm_residual``)."""
+        if with_input:
+            return ops.rms_norm_residual(x, self.weight, self.eps)
         return ops.rms_norm(x, self.weight, self.eps)
 
 
@@ -125,7 +128,8 @@ class AttentionBlock(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         # the residual additions ride in the epilogues of the output-projection and second MLP GEMMs
-        x = self.attn(self.ln1(x), residual=x)
+        y, x = self.ln1(x, with_input=True)
+        x = self.attn(y, residual=x)
         b, t, e = x.shape
-        x2 = x.reshape(b * t, e)
-        return self.mlp(self.ln2(x).reshape(b * t, e), residual=x2).view(b, t, e)
+        y, x2 = self.ln2(x.reshape(b * t, e), with_input=True)
+        return self.mlp(y, residual=x2).view(b, t, e)

@@ -99,6 +99,14 @@ def rms_norm(x, weight, eps: float):
     return ref.rms_norm(x, weight, eps)
 
 
+def rms_norm_residual(x, weight, eps: float):
+    """``(rms_norm(x), x)``, for a block that goes on with both: their gradients are added in one kernel."""
+    if _native(x):
+        from .native_ops import rms_norm_residual as f
+        return f(x, weight, eps)
+    return ref.rms_norm(x, weight, eps), x
+
+
 def layer_norm(x, weight, bias, eps: float):
     if _native(x):
         from .native_ops import layer_norm as f

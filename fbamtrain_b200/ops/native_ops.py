@@ -239,10 +239,23 @@ def gemm_tn(a_km, b_kn, **kw):
     return gemm(_t(a_km), _t(b_kn), **kw)
 
 
-def _colsum(x2d: torch.Tensor) -> torch.Tensor:
-    out = torch.zeros(x2d.shape[1], dtype=torch.float32, device=x2d.device)
-    nv.check(nv.lib(x2d).fbam_colsum(nv.ptr(x2d), nv.ptr(out), C.c_longlong(x2d.shape[0]), x2d.shape[1],
-                                  nv.stream_ptr()), "fbam_colsum")
+@functools.lru_cache(maxsize=4096)
+def _sum_partials(entry: str, *sizes) -> int:
+    """Rows of the fp32 workspace that a reduction over ``sizes`` needs."""
+    return getattr(nv.lib(), entry)(C.c_longlong(sizes[0]), *sizes[1:])
+
+
+def _sum_work(entry: str, cols: int, device, *sizes) -> Optional[torch.Tensor]:
+    n = _sum_partials(entry, *sizes)
+    return torch.empty(n * cols, dtype=torch.float32, device=device) if n else None
+
+
+def _colsum(x2d: torch.Tensor, dtype: torch.dtype = torch.float32) -> torch.Tensor:
+    rows, cols = x2d.shape
+    out = torch.empty(cols, dtype=dtype, device=x2d.device)
+    work = _sum_work("fbam_colsum_partials", cols, x2d.device, rows, cols, 0)
+    nv.check(nv.lib(x2d).fbam_colsum_to(nv.ptr(x2d), None, None, nv.ptr(out), int(dtype != torch.float32), nv.ptr(work),
+                                        C.c_longlong(rows), cols, nv.stream_ptr()), "fbam_colsum")
     return out
 
 
@@ -253,13 +266,14 @@ def _gelu_bwd(preact: torch.Tensor, dy: torch.Tensor) -> torch.Tensor:
     return out
 
 
-def _gelu_bwd_colsum(preact: torch.Tensor, dy: torch.Tensor):
-    """``dz = dy · gelu'(preact)`` and its fp32 column sums in one pass."""
+def _gelu_bwd_colsum(preact: torch.Tensor, dy: torch.Tensor, dtype: torch.dtype = torch.float32):
+    """``dz = dy · gelu'(preact)`` and its column sums (added in fp32) in one pass."""
     rows, cols = preact.shape
     dz = torch.empty_like(dy)
-    out = torch.zeros(cols, dtype=torch.float32, device=dy.device)
-    nv.check(nv.lib(preact).fbam_gelu_bwd_colsum(nv.ptr(preact), nv.ptr(dy), nv.ptr(dz), nv.ptr(out),
-                                                 C.c_longlong(rows), cols, nv.stream_ptr()), "fbam_gelu_bwd_colsum")
+    out = torch.empty(cols, dtype=dtype, device=dy.device)
+    work = _sum_work("fbam_colsum_partials", cols, dy.device, rows, cols, 1)
+    nv.check(nv.lib(preact).fbam_colsum_to(nv.ptr(dy), nv.ptr(preact), nv.ptr(dz), nv.ptr(out), int(dtype != torch.float32),
+                                           nv.ptr(work), C.c_longlong(rows), cols, nv.stream_ptr()), "fbam_gelu_bwd_colsum")
     return dz, out
 
 
@@ -293,7 +307,7 @@ class _Linear(torch.autograd.Function):
         want_db = ctx.has_bias and ctx.needs_input_grad[2]
         dx = dw = db = None
         if ctx.act == "gelu" and want_db:
-            dy2, db = _gelu_bwd_colsum(preact, dy2)
+            dy2, db = _gelu_bwd_colsum(preact, dy2, dy2.dtype)
         elif ctx.act == "gelu":
             dy2 = _gelu_bwd(preact, dy2)
         elif ctx.act == "relu":
@@ -303,8 +317,8 @@ class _Linear(torch.autograd.Function):
         if ctx.needs_input_grad[1]:
             n_out, n_in = dy2.shape[1], x2.shape[1]
             dw = gemm_tn(dy2, x2, splits=weight_grad_splits(n_out, n_in, dy2.shape[0]) if USE_MN_MAJOR else 0)
-        if want_db:
-            db = (_colsum(dy2) if db is None else db).to(dy2.dtype)
+        if want_db and db is None:
+            db = _colsum(dy2, dy2.dtype)
         d_res = dy if len(ctx.needs_input_grad) > 4 and ctx.needs_input_grad[4] else None
         return dx, dw, db, None, d_res
 
@@ -655,11 +669,52 @@ class _RmsNorm(torch.autograd.Function):
     def backward(ctx, dy):
         x2, weight, rstd = ctx.saved_tensors
         dy2 = dy.reshape(x2.shape).contiguous()
-        dx = torch.empty_like(x2)
-        dg = torch.zeros(x2.shape[1], dtype=torch.float32, device=x2.device)
-        nv.check(nv.lib(dy2).fbam_rmsnorm_bwd(nv.ptr(dy2), nv.ptr(x2), nv.ptr(weight), nv.ptr(rstd), nv.ptr(dx), nv.ptr(dg),
-                                           C.c_longlong(x2.shape[0]), x2.shape[1], nv.stream_ptr()), "fbam_rmsnorm_bwd")
-        return dx.view(dy.shape), dg.to(weight.dtype), None
+        dx, dg = _rms_norm_bwd(dy2, None, x2, weight, rstd)
+        return dx.view(dy.shape), dg, None
+
+
+def _rms_norm_bwd(dy2, res2, x2, weight, rstd):
+    """``(dx, dgamma)``; ``res2``: a further gradient of ``x2``, added to ``dx`` before it is rounded."""
+    rows, dim = x2.shape
+    dx, dg = torch.empty_like(x2), torch.empty(dim, dtype=weight.dtype, device=weight.device)
+    work = _sum_work("fbam_rmsnorm_bwd_partials", dim, x2.device, rows, dim)
+    nv.check(nv.lib(dy2).fbam_rmsnorm_bwd_to(nv.ptr(dy2), nv.ptr(res2), nv.ptr(x2), nv.ptr(weight), nv.ptr(rstd), nv.ptr(dx),
+                                             nv.ptr(dg), nv.ptr(work), C.c_longlong(rows), dim, nv.stream_ptr()),
+             "fbam_rmsnorm_bwd")
+    return dx, dg
+
+
+# Above this width a row's third tensor finds no registers for its loads to be in flight with the others'.  us with the
+# addition in the kernel | on its own, at 8192 rows: 1024 33.6 | 44.0, 2048 72.7 | 72.8, 4096 158.7 | 140.2.
+RESIDUAL_NORM_MAX_DIM = 2048
+
+
+class _RmsNormResidual(torch.autograd.Function):
+    """``(rms_norm(x), x)``: the second output is for what continues beside the norm, so that both gradients of ``x`` meet
+    in one kernel."""
+
+    @staticmethod
+    def forward(ctx, x, weight, eps):
+        y = _RmsNorm.forward(ctx, x, weight, eps)
+        return y, x.view_as(x)
+
+    @staticmethod
+    def backward(ctx, dy, dres):
+        x2, weight, rstd = ctx.saved_tensors
+        dy2 = dy.reshape(x2.shape).contiguous()
+        if x2.shape[1] > RESIDUAL_NORM_MAX_DIM:
+            dx, dg = _rms_norm_bwd(dy2, None, x2, weight, rstd)
+            return dx.view(dres.shape) + dres, dg, None
+        res2 = dres.reshape(x2.shape).contiguous()
+        if res2.data_ptr() % 16:
+            res2 = res2.clone()
+        dx, dg = _rms_norm_bwd(dy2, res2, x2, weight, rstd)
+        return dx.view(dres.shape), dg, None
+
+
+def rms_norm_residual(x, weight, eps):
+    _need_elem(x, weight)
+    return _RmsNormResidual.apply(x, weight, eps)
 
 
 def rms_norm(x, weight, eps):

@@ -64,6 +64,52 @@ def test_gelu_backward_with_column_sums(rows, cols, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,cols", [(1, 8), (3, 72), (513, 64), (2047, 136), (2048, 128), (2049, 128), (2049, 2368), (300, 2376),
+                                       (200, 4744), (70, 9480), (8192, 200), (8193, 200), (20000, 8)])
+def test_column_sums_of_both_kinds_of_launch(rows, cols, dtype):
+    """One launch of clusters of 8, 4, 2 or 1 CTAs up to a number of rows, slabs and an adding launch above; written as fp32
+    and as elements."""
+    from fbamtrain_b200.ops import native_ops as no
+    g = torch.Generator(device=DEV).manual_seed(rows + cols)
+    z, dy = (torch.randn(rows, cols, device=DEV, generator=g).to(dtype) for _ in range(2))
+    dz, sums = no._gelu_bwd_colsum(z, dy)
+    assert torch.equal(dz, no._gelu_bwd(z, dy))
+    # fp32 sums of the rounded values: at most rows roundings of a partial sum
+    for got, of in ((sums, dz), (no._colsum(dy), dy)):
+        bound = rows * 2.0 ** -24 * of.double().abs().sum(0) + 1e-6
+        assert bool(((got.double() - of.double().sum(0)).abs() <= bound).all())
+    assert torch.equal(no._colsum(dy, dtype), no._colsum(dy).to(dtype))
+    assert torch.equal(no._gelu_bwd_colsum(z, dy, dtype)[1], sums.to(dtype))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,dim", [(1, 8), (5, 64), (70, 72), (333, 128), (17, 256), (300, 264), (40, 512), (9, 1024), (700, 1032),
+                                      (5, 2048), (150, 2056), (3, 4096), (5000, 256)])
+def test_rmsnorm_backward_with_a_residual_gradient(rows, dim, dtype):
+    from fbamtrain_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(rows + dim)
+    x, dy, dres = (torch.randn(rows, dim, device=DEV, generator=g).to(dtype) for _ in range(3))
+    x.requires_grad_(True)
+    w = (1 + 0.1 * torch.randn(dim, device=DEV, generator=g)).to(dtype).requires_grad_(True)
+    y, same = ops.rms_norm_residual(x, w, 1e-5)
+    assert torch.equal(same, x) and torch.equal(y, ops.rms_norm(x, w, 1e-5))
+    dx, dw = torch.autograd.grad((y, same), (x, w), (dy, dres))
+    xd, wd = x.detach().double().requires_grad_(True), w.detach().double().requires_grad_(True)
+    exp = torch.autograd.grad((ref.rms_norm(xd, wd, 1e-5), xd * 1.0), (xd, wd), (dy.double(), dres.double()))
+    # one rounding to the 16-bit type; fp32 sums behind it
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    assert _rel(dx, exp[0]) < eps and _rel(dw, exp[1]) < 1.5 * eps
+    # the gradients alone give the same as the two together, up to the rounding of the sum
+    plain, dw_plain = torch.autograd.grad(ops.rms_norm(x, w, 1e-5), (x, w), dy)
+    assert torch.equal(dw, dw_plain)
+    assert float((dx.float() - (plain.float() + dres.float())).norm() / exp[0].norm()) < 2 * eps
+    # an upstream gradient whose rows start two bytes off a 16-byte boundary
+    odd = torch.empty(rows * dim + 1, device=DEV, dtype=dtype)[1:].view(rows, dim).copy_(dres)
+    y, same = ops.rms_norm_residual(x, w, 1e-5)
+    assert torch.equal(torch.autograd.grad((y, same), x, (dy, odd))[0], dx)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("n,pix,c", [(1, 1, 8), (3, 7, 64), (5, 480, 512), (2, 33, 528), (1, 1000, 2048), (2, 5, 2056),
                                      (66000, 2, 8), (70001, 1, 8), (5, 127, 64), (5, 128, 64), (5, 129, 64), (3001, 3, 72),
                                      (9, 31, 64), (9, 32, 64), (700, 33, 64), (5000, 27, 72), (5000, 28, 72),
