@@ -136,7 +136,9 @@ struct WorkIter {
 };
 
 // p.tiles_m counts PAIR tiles (256 rows); K is never split in this variant.
-template <int BN>
+// POOL: the epilogue of GemmParams::pool_partial.  The activation of the last convolution of the frame head was written
+// (503 MB per 1024 frames of 48 x 160), read by the pool and dropped; what leaves now is 4 / pool_seg bytes per value.
+template <int BN, bool POOL>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
              const __grid_constant__ CUtensorMap map_d, const __grid_constant__ CUtensorMap map_pre, const GemmParams p) {
@@ -326,7 +328,15 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
       // the side input (gelu_grad_in or residual) of the first chunk is requested before the accumulator is waited
       // for, and that of every later chunk before the previous one is processed
       const int c_first = col_half * (BN / 2), c_last = (col_half + 1) * (BN / 2);
-      const elem_t* aux_row = gemm_epi::aux_row_ptr(p, roff);
+      float* pool_row = nullptr;       // this lane's segment sums
+      if constexpr (POOL) {
+        const ConvGeom& g = p.conv;
+        const int per_image = g.th * g.tw, tile_pos = half % (g.tiles_w * g.tiles_h);
+        const int n = half / (g.tiles_w * g.tiles_h) * g.tn + row / per_image;
+        const int part = tile_pos * (per_image / p.pool_seg) + row % per_image / p.pool_seg;
+        if (n < g.batch) pool_row = p.pool_partial + ((long long)n * p.pool_parts + part) * p.N;
+      }
+      const elem_t* aux_row = POOL ? nullptr : gemm_epi::aux_row_ptr(p, roff);
       uint4 aux[4] = {};
       gemm_epi::aux_prefetch(aux_row, tile_n * BN + c_first, p.N, aux);
       if (!mbar_wait(&tmem_full[acc], acc_phase)) { ok = false; break; }
@@ -343,6 +353,23 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
         if (c0 + 32 < c_last) gemm_epi::aux_prefetch(aux_row, n0 + 32, p.N, aux);
         tmem_ld_wait();
         if (n0 >= p.N) continue;                               // the same for the whole warp
+        if constexpr (POOL) {                                  // N is a multiple of 32
+          uint8_t* out_buf = (stage_turn++ & 1) ? stage_out : stage_pre;
+          if (p.tma_store) {
+            if (lane == 0) bulk_wait_group_read<1>();
+            __syncwarp();
+          }
+          gemm_epi::pool_chunk(p, roff >= 0, pool_row ? pool_row + n0 : nullptr, r, p.tma_store ? out_buf : nullptr);
+          if (p.tma_store) {
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              if (box_in) tma_store_4d(&map_d, out_buf, n0, sx1, sx2, sx3);
+              bulk_commit_group();
+            }
+          }
+          continue;
+        }
         if (p.tma_store && n0 + 32 <= p.N) {
           // A staging buffer is free once the copy that read it is done (tracked by lane 0, which issued it).  Without
           // preact_out the two buffers take turns (stage_turn counts this warp's stored chunks across tiles), so only
@@ -439,12 +466,12 @@ int enc_nhwc(CUtensorMap* map, const void* base, int n, int h, int w, int c, int
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : GEMM_ERR_TENSORMAP;
 }
 
-template <int BN>
+template <int BN, bool POOL = false>
 int launch2(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams& p, cudaStream_t stream) {
   using L = Smem2<BN>;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(gemm2_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal) != cudaSuccess)
+    if (cudaFuncSetAttribute(gemm2_kernel<BN, POOL>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal) != cudaSuccess)
       return GEMM_ERR_LAUNCH;
     configured = true;
   }
@@ -461,7 +488,8 @@ int launch2(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams& p, cudaStr
   CUtensorMap md, mpre;
   const int e = fbam_encode_out_maps(encode_fn2(), &md, &mpre, p);
   if (e) return e;
-  gemm2_kernel<BN><<<2 * clusters, kThreads, L::kTotal, stream>>>(ma, mb, md, mpre, p);
+  if (POOL && p.D != nullptr && !p.tma_store) return GEMM_ERR_SHAPE;
+  gemm2_kernel<BN, POOL><<<2 * clusters, kThreads, L::kTotal, stream>>>(ma, mb, md, mpre, p);
   return cudaGetLastError() == cudaSuccess ? 0 : GEMM_ERR_LAUNCH;
 }
 
@@ -529,5 +557,17 @@ extern "C" int fbam_conv2(const void* X, int in_h, int in_w, int C, const void* 
   e = enc2d(&mb, Wmat, N, p.K, ldw, bn / 2);
   if (e) return e;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (p.pool_partial != nullptr) {
+    int seg;
+    const int parts = fbam_pool_geometry(g.grid_h, g.grid_w, g.th, g.tw, &seg);
+    if (parts == 0 || p.pool_seg != seg || p.pool_parts != parts || bn != 256 || N % 32 != 0 || p.num_classes != 0 || p.preact_out != nullptr ||
+        (g.th & (g.th - 1)) || (g.tw & (g.tw - 1)) || (reinterpret_cast<uintptr_t>(p.pool_partial) & 15))
+      return GEMM_ERR_SHAPE;
+    return launch2<256, true>(ma, mb, p, s);
+  }
   return bn == 128 ? launch2<128>(ma, mb, p, s) : launch2<256>(ma, mb, p, s);
+}
+
+extern "C" int fbam_conv_pool_parts(int grid_h, int grid_w, int th, int tw, int* seg) {
+  return fbam_pool_geometry(grid_h, grid_w, th, tw, seg);
 }

@@ -324,6 +324,49 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, long long roff,
 
 }
 
+// Sums of 32 columns over segments of SEG lanes: with every exchange a lane keeps half of its columns, so 32 columns cost 31
+// shuffles at most.  Afterwards lane l holds columns (l % SEG)·(32 / SEG) onwards of its segment in v[0 .. 32 / SEG).
+template <int SEG>
+__device__ __forceinline__ void segment_sums(float (&v)[32], float* out) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = SEG / 2, w = 16; o > 0; o >>= 1, w >>= 1) {
+    const bool upper = (lane & o) != 0;
+#pragma unroll
+    for (int j = 0; j < w; ++j) {
+      const float send = upper ? v[j] : v[j + w], keep = upper ? v[j + w] : v[j];
+      v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  if (out == nullptr) return;
+  out += (lane % SEG) * (32 / SEG);
+#pragma unroll
+  for (int j = 0; j < 32 / SEG; ++j) out[j] = v[j];
+}
+
+// One chunk of a convolution whose activation is only averaged (GemmParams::pool_partial): the pre-activation goes to
+// `stage_out` where it is wanted, GELU of it is summed over segments; `valid`: the row lies in the output.
+__device__ __forceinline__ void pool_chunk(const GemmParams& p, bool valid, float* sums, const uint32_t (&r)[32], uint8_t* stage_out) {
+  float v[32];
+#pragma unroll
+  for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * p.alpha;
+  if (stage_out != nullptr) stage_row64(stage_out, v);
+#pragma unroll
+  for (int j = 0; j < 32; j += 2) {
+    const float2 g = gelu_math::gelu2(make_float2(v[j], v[j + 1]));
+    v[j] = valid ? g.x : 0.0f;
+    v[j + 1] = valid ? g.y : 0.0f;
+  }
+  if (p.pool_seg == 32)
+    segment_sums<32>(v, sums);
+  else if (p.pool_seg == 16)
+    segment_sums<16>(v, sums);
+  else if (p.pool_seg == 8)
+    segment_sums<8>(v, sums);
+  else
+    segment_sums<4>(v, sums);
+}
+
 template <bool CE = false>
 __device__ __forceinline__ void store_chunk(const GemmParams& p, long long roff, int n0, const uint32_t (&r)[32]) {
   const uint4 none[4] = {};

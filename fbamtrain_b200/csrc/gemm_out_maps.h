@@ -18,7 +18,7 @@ static inline int fbam_encode_out_maps(EncFn enc, CUtensorMap* md, CUtensorMap* 
   p.st_bn = 32;
   std::memset(md, 0, sizeof(CUtensorMap));
   std::memset(mpre, 0, sizeof(CUtensorMap));
-  if (p.out_fp32 || p.accumulate != 0 || p.rs_rows_per_rank > 0 || !p.vec_ok || p.N < 32 || (p.ldd * 2) % 16 != 0) return 0;
+  if (p.D == nullptr || p.out_fp32 || p.accumulate != 0 || p.rs_rows_per_rank > 0 || !p.vec_ok || p.N < 32 || (p.ldd * 2) % 16 != 0) return 0;
   if ((reinterpret_cast<uintptr_t>(p.D) & 15) || (p.preact_out && (reinterpret_cast<uintptr_t>(p.preact_out) & 15))) return 0;
   if (!enc) return GEMM_ERR_DRIVER;
   fbam_bind_context_to_thread();

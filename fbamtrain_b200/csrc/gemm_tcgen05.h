@@ -105,7 +105,23 @@ struct GemmParams {
   // that one epilogue warp owns, as a box of output positions (w, h, n) of a convolution brick (1, 1, 32 rows of a
   // plain matrix).
   int tma_store, st_bw, st_bh, st_bn;
+  // Convolution with GELU whose activation is wanted only as a mean over positions (CTA-pair kernel, 256 columns per tile;
+  // act, out_fp32 and the side inputs are not looked at).  D receives the pre-activation, or is null; of the activation only
+  // fp32 sums over segments of positions leave the kernel: pool_partial[image][pool_parts][N].  pool_seg and pool_parts
+  // are what fbam_conv_pool_parts gives for the brick.
+  float* pool_partial;
+  int pool_seg, pool_parts;
 };
+
+// How the rows of a brick divide into segments of one image each, within the 32 rows of an epilogue warp: returns the
+// segments of an image over all bricks and sets the rows of a segment (4 to 32); 0 where a segment would have fewer rows
+// (then the sums are no smaller than the activation).  th and tw are powers of two.
+static inline int fbam_pool_geometry(int grid_h, int grid_w, int th, int tw, int* seg) {
+  const int per_image = th * tw;
+  *seg = per_image < 32 ? per_image : 32;
+  if (*seg < 4) return 0;
+  return ((grid_w + tw - 1) / tw) * ((grid_h + th - 1) / th) * (per_image / *seg);
+}
 
 // Driver entry points (tensor-map encoding) need a context that is current on the CALLING thread.  A thread that
 // has only inherited "device 0" by default (an autograd worker whose first CUDA work is one of these launchers)

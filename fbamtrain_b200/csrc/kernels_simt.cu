@@ -526,6 +526,25 @@ __global__ void __launch_bounds__(256) gelu_avgpool2x2_kernel(const elem_t* __re
   }
 }
 
+// y[n, c] = (sum of the image's partial sums, in order) / pix, for the pooled epilogue of the CTA-pair convolution.
+__global__ void __launch_bounds__(256) pool_finish_kernel(const float* __restrict__ partial, elem_t* __restrict__ y, long long n,
+                                                          int parts, int pix, int c) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int c4 = c / 4;
+  if (i >= n * c4) return;
+  const float4* p = reinterpret_cast<const float4*>(partial) + i / c4 * parts * c4 + i % c4;
+  float s[4] = {0, 0, 0, 0};
+  for (int k = 0; k < parts; ++k) {
+    const float4 t = p[(long long)k * c4];
+    s[0] += t.x;
+    s[1] += t.y;
+    s[2] += t.z;
+    s[3] += t.w;
+  }
+  elem2_t h[2] = {ff2e2(s[0] / pix, s[1] / pix), ff2e2(s[2] / pix, s[3] / pix)};
+  *reinterpret_cast<uint2*>(y + i * 4) = *reinterpret_cast<uint2*>(h);
+}
+
 // Global average pool over `pix` positions: x [n, pix, c] -> y [n, c].  One block per (n, 8-channel-group
 // slab of 32 groups); threads stride over positions.
 __global__ void global_avgpool_fwd_kernel(const elem_t* __restrict__ x, elem_t* __restrict__ y, int pix, int c) {
@@ -1328,6 +1347,12 @@ int fbam_gelu_avgpool2x2(const void* z, const void* dy, void* out, long long n, 
   const long long total = n * oh * ow * (c / 8);
   gelu_avgpool2x2_kernel<<<(unsigned)((total + 255) / 256), 256, 0, STREAM(stream)>>>((const elem_t*)z, (const elem_t*)dy,
                                                                                      (elem_t*)out, n, oh, ow, c);
+  return CHECK_LAUNCH();
+}
+
+int fbam_pool_finish(const float* partial, void* y, long long n, int parts, int pix, int c, void* stream) {
+  if (c % 4 != 0) return 1;
+  pool_finish_kernel<<<(unsigned)((n * (c / 4) + 255) / 256), 256, 0, STREAM(stream)>>>(partial, (elem_t*)y, n, parts, pix, c);
   return CHECK_LAUNCH();
 }
 

@@ -70,7 +70,8 @@ class GemmParams(C.Structure):
                 ("k_blocks", C.c_int), ("a_mn_major", C.c_int), ("b_mn_major", C.c_int), ("vec_ok", C.c_int),
                 ("conv", ConvGeom),
                 ("num_classes", C.c_int), ("cls", ConvClass * 4),
-                ("tma_store", C.c_int), ("st_bw", C.c_int), ("st_bh", C.c_int), ("st_bn", C.c_int)]
+                ("tma_store", C.c_int), ("st_bw", C.c_int), ("st_bh", C.c_int), ("st_bn", C.c_int),
+                ("pool_partial", C.c_void_p), ("pool_seg", C.c_int), ("pool_parts", C.c_int)]
 
 
 def available(dtype: torch.dtype = torch.bfloat16) -> bool:

@@ -348,19 +348,22 @@ def _brick(n: int, h: int, w: int, total: int = 128) -> Tuple[int, int, int]:
     return best
 
 
-def conv_pass(x: torch.Tensor, wmat: torch.Tensor, n_out: int, out: torch.Tensor, *, grid_hw, in_mul, taps,
+def conv_pass(x: torch.Tensor, wmat: torch.Tensor, n_out: int, out: Optional[torch.Tensor], *, grid_hw, in_mul, taps,
               out_mul=1, out_off=(0, 0), accumulate=0, bn: int = 0, act: str = "none",
               preact_out: Optional[torch.Tensor] = None, gelu_grad_in: Optional[torch.Tensor] = None,
-              tile_rows: int = 0, two_cta=None, classes=None) -> None:
+              tile_rows: int = 0, two_cta=None, classes=None, pool=None) -> None:
     """One implicit-GEMM pass (see ``ConvGeom`` in csrc/gemm_tcgen05.h).  ``x`` NHWC bf16 or fp16, ``wmat``
     ``(n_out, taps·C)`` of the same type, ``out`` NHWC with ``n_out`` channels.
 
     ``classes`` (CTA-pair kernel only): a list of ``(taps, out_off)`` — parity classes of a strided data gradient
     that share the iteration grid.  ``taps`` is then the concatenation of the classes' taps and ``wmat`` holds the
     classes' filter columns side by side in that order; every tile is computed once per class by the same CTA pair,
-    so the input tile is read from DRAM once for all classes."""
+    so the input tile is read from DRAM once for all classes.
+
+    ``pool`` (CTA-pair kernel only): ``(partial, seg, parts)`` of :func:`_pool_plan`; ``out`` receives the
+    pre-activation, or is ``None``, and ``partial`` the segment sums of GELU of it."""
     b, ih, iw, c = x.shape
-    if classes is not None:
+    if classes is not None or pool is not None:
         two_cta, tile_rows, bn = True, 0, 0
     elif bn == 0 and tile_rows == 0 and two_cta is None and tuning.active():
         tuned = tuning.lookup(tuning.conv_key(b, grid_hw[0], grid_hw[1], c, n_out, len(taps), in_mul, out_mul),
@@ -387,7 +390,7 @@ def conv_pass(x: torch.Tensor, wmat: torch.Tensor, n_out: int, out: torch.Tensor
     g.tn, g.th, g.tw = tn, th, tw
     g.in_mul, g.out_mul = in_mul, out_mul
     g.out_off_h, g.out_off_w = out_off
-    g.out_h, g.out_w = out.shape[1], out.shape[2]
+    g.out_h, g.out_w = (out.shape[1], out.shape[2]) if out is not None else grid_hw
     g.num_taps = len(taps)
     for i, (dh, dw) in enumerate(taps):
         g.tap_dh[i], g.tap_dw[i] = dh, dw
@@ -400,12 +403,15 @@ def conv_pass(x: torch.Tensor, wmat: torch.Tensor, n_out: int, out: torch.Tensor
             for i, (dh, dw) in enumerate(ctaps):
                 cl.tap_dh[i], cl.tap_dw[i] = dh, dw
             base += len(ctaps)
-    p.D, p.ldd = out.data_ptr(), out.shape[3]
+    if out is not None:
+        p.D, p.out_fp32 = out.data_ptr(), int(out.dtype == torch.float32)
+    p.ldd = n_out if out is None else out.shape[3]
     p.status = nv.status_word(x.device).data_ptr()
     p.alpha = 1.0
-    p.out_fp32 = int(out.dtype == torch.float32)
     p.accumulate = accumulate
     p.bn = bn
+    if pool is not None:
+        p.pool_partial, p.pool_seg, p.pool_parts = pool[0].data_ptr(), pool[1], pool[2]
     p.act = nv.GEMM_ACT[act]
     if preact_out is not None:
         p.preact_out = preact_out.data_ptr()
@@ -431,6 +437,44 @@ def conv2d_fprop(x, w_ohwi, stride, padding, dilation, act: str = "none", preact
     conv_pass(x, w_ohwi.reshape(o, 9 * c), o, out, grid_hw=(oh, ow), in_mul=stride, taps=taps, act=act,
               preact_out=preact_out)
     return out
+
+
+@functools.lru_cache(maxsize=4096)
+def _pool_plan(n: int, oh: int, ow: int, channels: int):
+    """``(segment, segments per image)`` of a convolution whose activation is only averaged over positions, or ``None``
+    where that runs as a convolution and a pool: the CTA-pair kernel is not the one for the size (as in ``conv_pass``),
+    or a brick has fewer than four neighbouring positions of an image, so that the sums would be no smaller than the
+    activation."""
+    tn, th, tw = _brick(n, oh, ow, 256)
+    tiles = math.ceil(n / tn) * math.ceil(oh / th) * math.ceil(ow / tw)
+    if TWO_CTA not in ("auto", True) or channels < 256 or channels % 32 or tiles < 148:
+        return None
+    _, th, tw = _brick(n, oh, ow, 128)
+    seg = C.c_int()
+    parts = nv.lib().fbam_conv_pool_parts(oh, ow, th, tw, C.byref(seg))
+    return (seg.value, parts) if parts else None
+
+
+def conv2d_gelu_mean(x, w_ohwi, stride, padding, dilation, z):
+    """Mean over the positions of GELU(conv3x3(x)), ``(n, channels)``; ``z`` (or ``None``) receives the pre-activation."""
+    n, ih, iw, c = x.shape
+    o = w_ohwi.shape[0]
+    oh, ow = conv_out_hw(ih, iw, stride, padding, dilation)
+    plan = None if tuning.active() else _pool_plan(n, oh, ow, o)
+    vec = torch.empty(n, o, dtype=x.dtype, device=x.device)
+    if plan is None:
+        y = conv2d_fprop(x, w_ohwi, stride, padding, dilation, act="gelu", preact_out=z)
+        nv.check(nv.lib(y).fbam_global_avgpool(nv.ptr(y), nv.ptr(vec), C.c_longlong(n), oh * ow, o, 0, None,
+                                               nv.stream_ptr()), "fbam_global_avgpool")
+        return vec
+    seg, parts = plan
+    partial = torch.empty(n, parts, o, dtype=torch.float32, device=x.device)
+    taps = [(r * dilation - padding, s * dilation - padding) for r in range(3) for s in range(3)]
+    conv_pass(x, w_ohwi.reshape(o, 9 * c), o, z, grid_hw=(oh, ow), in_mul=stride, taps=taps, act="gelu",
+              pool=(partial, seg, parts))
+    nv.check(nv.lib(x).fbam_pool_finish(nv.ptr(partial), nv.ptr(vec), C.c_longlong(n), parts, oh * ow, o, nv.stream_ptr()),
+             "fbam_pool_finish")
+    return vec
 
 
 def conv_out_hw(ih, iw, stride, padding, dilation):
@@ -510,14 +554,12 @@ class _ConvGeluStackPool(torch.autograd.Function):
         for w, pad, dil in zip(weights, paddings, dilations):
             oh, ow = conv_out_hw(ys[-1].shape[1], ys[-1].shape[2], stride, pad, dil)
             z = debug.fresh((x.shape[0], oh, ow, w.shape[0]), x.dtype, x.device)
-            ys.append(conv2d_fprop(ys[-1], w, stride, pad, dil, act="gelu", preact_out=z))
             zs.append(z)
-        last = ys[-1]
-        n, h, wd, c = last.shape
-        vec = torch.empty(n, c, dtype=last.dtype, device=x.device)
-        nv.check(nv.lib(last).fbam_global_avgpool(nv.ptr(last), nv.ptr(vec), C.c_longlong(n), h * wd, c, 0, None,
-                                              nv.stream_ptr()), "fbam_global_avgpool")
-        ctx.save_for_backward(*ys[:-1], *zs, *weights)
+            if len(zs) < len(weights):
+                ys.append(conv2d_fprop(ys[-1], w, stride, pad, dil, act="gelu", preact_out=z))
+            else:
+                vec = conv2d_gelu_mean(ys[-1], w, stride, pad, dil, z)
+        ctx.save_for_backward(*ys, *zs, *weights)
         ctx.cfg = (stride, tuple(paddings), tuple(dilations), len(weights))
         return vec
 
@@ -563,17 +605,20 @@ class _CellConvGeluStackPool(torch.autograd.Function):
             if need_grad:
                 oh, ow = conv_out_hw(ys[-1].shape[1], ys[-1].shape[2], stride, pad, dil)
                 z = debug.fresh((cells.shape[0], oh, ow, w.shape[0]), y1.dtype, cells.device)
+            zs.append(z)
+            if len(zs) == len(weights):
+                vec = conv2d_gelu_mean(ys[-1], w, stride, pad, dil, z)
+                break
             ys.append(conv2d_fprop(ys[-1], w, stride, pad, dil, act="gelu", preact_out=z))
             if not need_grad:
                 ys = ys[-1:]
-            zs.append(z)
-        last = ys[-1]
-        n, h, wd, c = last.shape
-        vec = torch.empty(n, c, dtype=last.dtype, device=cells.device)
-        nv.check(nv.lib(last).fbam_global_avgpool(nv.ptr(last), nv.ptr(vec), C.c_longlong(n), h * wd, c, 0, None,
-                                              nv.stream_ptr()), "fbam_global_avgpool")
+        if len(weights) == 1:
+            n, h, wd, c = y1.shape
+            vec = torch.empty(n, c, dtype=y1.dtype, device=cells.device)
+            nv.check(nv.lib(y1).fbam_global_avgpool(nv.ptr(y1), nv.ptr(vec), C.c_longlong(n), h * wd, c, 0, None,
+                                                    nv.stream_ptr()), "fbam_global_avgpool")
         if need_grad:
-            ctx.save_for_backward(cells, feat, cp_embed, pos_embed, colour, *ys[:-1], *zs, *weights)
+            ctx.save_for_backward(cells, feat, cp_embed, pos_embed, colour, *ys[:len(weights) - 1], *zs, *weights)
         ctx.cfg = (rows, cols, stride, tuple(paddings), tuple(dilations), len(weights))
         return vec
 
