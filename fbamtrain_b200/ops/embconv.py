@@ -171,6 +171,10 @@ def set_cache_token(token: Optional[int]) -> None:
     _cache_token = token
 
 
+def cache_token() -> Optional[int]:
+    return _cache_token
+
+
 def _tables_native(cp_embed, pos_embed, colour, w, rows, cols, stride, pad, dil):
     """→ ``ext`` bf16 ``(V + 6, C)`` (code-point rows then the six colour vectors), ``w_p`` bf16 ``(9·O, C)`` (filter
     rows ordered tap-major), ``table`` bf16 ``(V, 9, O)``, ``cc_t`` bf16 ``(O, 64)``, ``pos_out`` fp32 ``(P_out, O)``,

@@ -34,6 +34,7 @@ from .utils.flat import FlatGroup, build_groups
 from .utils.logging import LOG, enabled as log_enabled
 from .utils.metrics import AsyncStepLogger, LossRingBuffer, ProgressRecord, StepRecord
 from .utils.nvtx import gputx_range
+from .utils.step_graph import StepGraph
 
 
 def _is_muon_param(name: str, p: torch.nn.Parameter) -> bool:
@@ -122,6 +123,8 @@ class Trainer:
         self._warned_recompute = False
         self._upload_slot, self._slot_in_use, self._fresh_buffer = 0, 0, False
         self._slot_free: List[Optional[torch.cuda.Event]] = [None, None]
+        # data-parallel steps start collectives from gradient hooks, which a graph would pass by
+        self._step_graph = StepGraph(self.model, self.device) if self._cuda and dp is None else None
 
     @property
     def rank(self) -> int:
@@ -195,6 +198,22 @@ class Trainer:
             return self._forward_backward_replayed(cells, targets, loss_scale)
         dev_cells, dev_targets, events, chunk = self._upload(cells, targets)
         b, t, p, _ = dev_cells.shape
+        if self._step_graph is not None and (events is None or len(events) == 1):
+            def run(step_cells, step_targets):
+                with gputx_range("fbamtrain::forward"):
+                    emb = self.model.frame_embeddings(step_cells)
+                    with gputx_range("fbamtrain::action_model_fwd_bwd"):
+                        loss = self.model.action_model(emb, step_targets, loss_scale)
+                with gputx_range("fbamtrain::backward"):
+                    loss.backward()
+                return loss.detach()
+
+            if events is not None:
+                torch.cuda.current_stream().wait_event(events[0])
+            loss = self._step_graph.forward_backward(dev_cells, dev_targets, loss_scale, run)
+            if loss is not None:
+                self._upload_read(events)
+                return loss
         progress = log_enabled("INFO")          # per-chunk progress lines cost two events per chunk: only when shown
         phase0 = self._mark() if progress else None
         with gputx_range("fbamtrain::forward"):
@@ -239,11 +258,15 @@ class Trainer:
             loss.backward()
         if progress:
             self.logger.progress(ProgressRecord("Backward: frames", b * t, b * t, phase1, self._mark()))
-        if events is not None:          # the backward was the last reader of this micro-batch's device buffers
+        self._upload_read(events)
+        return loss.detach()
+
+    def _upload_read(self, events) -> None:
+        """The backward was the last reader of the micro-batch's device buffers, where it was uploaded."""
+        if events is not None:
             done = torch.cuda.Event()
             done.record()
             self._slot_free[self._slot_in_use] = done
-        return loss.detach()
 
     def _forward_backward_replayed(self, cells: torch.Tensor, targets: torch.Tensor, loss_scale: float) -> torch.Tensor:
         """Model key ``frame_replay``: the frames stay in host memory, the frame head sees one chunk at a time and

@@ -33,6 +33,14 @@ def add(flops: float) -> None:
         recording.on_flops(flops, useful)
 
 
+def add_counted(total: float, useful: float) -> None:
+    """Adds a count that was taken before (the launches of a replayed graph)."""
+    global _total, _useful
+    with _lock:
+        _total += total
+        _useful += useful
+
+
 @contextmanager
 def not_useful():
     """FLOPs added inside this block (on this thread) are recomputation."""

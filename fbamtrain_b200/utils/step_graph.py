@@ -1,0 +1,192 @@
+"""Forward and backward of a launch-bound training step as a CUDA graph.
+
+A step of a small configuration is some two hundred launches of a few microseconds each, which take the host several
+times as long to issue as the GPU to run (toy configuration, 4 x 64 frames of 24 x 80: 4.5 ms a step, GPU busy for 1.1).
+:class:`StepGraph` watches the steps of a trainer; where the host is what a step waits for, forward and backward of the
+next step of that shape are captured once and replayed from then on.  Gradients are added to the flat buffers and the
+parameters read where they lie, so the optimizer, gradient accumulation and checkpoints see no difference; inputs are
+copied into the graph's own buffers, the loss out of them.
+
+What is captured is what the host would have done for the step at hand.  Whatever can change that is compared or asked
+for before every replay (:meth:`_setting`); with anything out of the ordinary — hooks, saved-tensor hooks, dispatch modes,
+anomaly detection, debug switches, a recording of launches or shapes — the step runs as usual.
+``FBAMTRAIN_STEP_GRAPH=0`` keeps every step that way.
+
+The reference has no counterpart: its executor launches kernel by kernel (reference:
+``tensorlib/src/execution_backend.cpp``).
+"""
+from __future__ import annotations
+
+import gc
+import os
+import time
+from collections import OrderedDict
+from typing import Optional
+
+import torch
+from torch.nn.modules import module as _module
+
+from ..ops import dispatch, embconv, native, native_ops, tuning
+from . import debug, flops, plan
+from .logging import LOG, enabled as log_enabled
+
+# Cells of a step (frames x positions) up to which steps are watched: a step of the headline configuration has 63 million
+# and keeps the GPU busy three times as long as the host; its graph would hold 28 GB of activations.
+MAX_CELLS = 8 << 20
+WATCHED_STEPS = 2        # steps of a shape that run as usual before one may be captured
+HOST_SHARE = 0.7         # captured where the host takes at least this share of the step's time on the GPU's clock
+MAX_GRAPHS = 2           # per trainer; the least recently used one is given back
+
+
+class _Watch:
+    """Host and GPU time of the steps of one shape that ran as usual (the smallest of each)."""
+
+    def __init__(self) -> None:
+        self.steps, self.host_ms, self.gpu_ms, self.pending = 0, float("inf"), float("inf"), []
+
+    def launch_bound(self) -> bool:
+        """Asked after ``WATCHED_STEPS``; looks at finished events only, so it never waits for the device."""
+        while self.pending and self.pending[0][1].query():
+            start, end = self.pending.pop(0)
+            self.gpu_ms = min(self.gpu_ms, start.elapsed_time(end))
+        return self.steps >= WATCHED_STEPS and self.gpu_ms < float("inf") and self.host_ms >= HOST_SHARE * self.gpu_ms
+
+
+class _Captured:
+    def __init__(self, cells, targets):
+        self.cells, self.targets = torch.empty_like(cells), torch.empty_like(targets)
+        self.graph = torch.cuda.CUDAGraph()
+        self.loss: Optional[torch.Tensor] = None
+        self.flops = (0.0, 0.0)
+        self.launches = 0
+
+
+class StepGraph:
+    def __init__(self, model: torch.nn.Module, device: torch.device):
+        self.model = model
+        self.device = torch.device("cuda", torch.cuda.current_device() if device.index is None else device.index)
+        self._watches: "OrderedDict[tuple, _Watch]" = OrderedDict()
+        self._graphs: "OrderedDict[tuple, _Captured]" = OrderedDict()
+        self._refused: set = set()
+        self._stream: Optional[torch.cuda.Stream] = None
+
+    # ------------------------------------------------------------------------------------------
+    def _ordinary(self) -> bool:
+        """Nothing is active that a replay would pass by."""
+        if (os.environ.get("FBAMTRAIN_STEP_GRAPH", "1") == "0" or dispatch.get_backend() != "auto" or tuning.active()
+                or plan.active() is not None or debug.SYNC_EVERY_OP or debug.POISON_ALLOC or debug.DEBUG_KERNEL_LAUNCH
+                or debug.PROFILE_LABELS or debug.BREAK_ON_LAUNCH or log_enabled("INFO")):
+            return False
+        if (not torch.is_grad_enabled() or torch.is_inference_mode_enabled() or torch.is_anomaly_enabled()
+                or torch.is_autocast_enabled("cuda") or torch._C._len_torch_dispatch_stack()
+                or torch._C._len_torch_function_stack() or torch._C._autograd._top_saved_tensors_default_hooks(True)
+                or torch.cuda.is_current_stream_capturing() or torch.cuda.current_device() != self.device.index):
+            return False
+        if (_module._global_forward_hooks or _module._global_forward_pre_hooks or _module._global_backward_hooks
+                or _module._global_backward_pre_hooks):
+            return False
+        for m in self.model.modules():
+            if (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
+                    or "forward" in m.__dict__):
+                return False
+        for p in self.model.parameters():
+            if p._backward_hooks or p._post_accumulate_grad_hooks:
+                return False
+        cfg, action = self.model.cfg, self.model.action_model
+        # recomputed chunks and the streamed recurrence (which reads a value back) run as usual
+        return not (cfg.frame_head_recompute or cfg.frame_replay or action.streaming or action.host_offload)
+
+    def _setting(self, cells: torch.Tensor, targets: torch.Tensor, loss_scale: float) -> tuple:
+        """What the launches of a step depend on besides the values of its inputs and parameters."""
+        no = native_ops
+        return (tuple(cells.shape), cells.dtype, tuple(targets.shape), targets.dtype, loss_scale, self.model.frame_chunk,
+                no.TWO_CTA, no.USE_MN_MAJOR, no.WEIGHT_GRAD_SPLIT_K, no.FUSE_DGRAD_CLASSES, no.FUSED_LM_HEAD_CE,
+                no.LM_HEAD_CHUNK_ROWS, no.RESIDUAL_NORM_MAX_DIM,
+                tuple(dispatch._prefer.values()), os.environ.get("FBAMTRAIN_EMBCONV"),
+                os.environ.get("FBAMTRAIN_ATTENTION_FWD2"), torch.are_deterministic_algorithms_enabled(),
+                tuple((p.data_ptr(), p.requires_grad, -1 if p.grad is None else p.grad.data_ptr())
+                      for p in self.model.parameters()))
+
+    # ------------------------------------------------------------------------------------------
+    def forward_backward(self, cells: torch.Tensor, targets: torch.Tensor, loss_scale: float, run) -> Optional[torch.Tensor]:
+        """The loss of ``run(cells, targets)`` (forward and backward on device tensors), or ``None`` where the step is not
+        one to watch."""
+        chunk = self.model.frame_chunk
+        frames = cells.shape[0] * cells.shape[1]
+        if frames * cells.shape[2] > MAX_CELLS or (chunk and frames > chunk) or not self._ordinary():
+            return None
+        if not (cells.is_contiguous() and targets.is_contiguous()) or any(p.grad is None for p in self.model.parameters()):
+            return None
+        key = self._setting(cells, targets, loss_scale)
+        captured = self._graphs.get(key)
+        if captured is None:
+            watch = self._watches.get(key)
+            if watch is None:
+                watch = self._watches[key] = _Watch()
+                while len(self._watches) > 8:
+                    self._watches.popitem(last=False)
+            if key in self._refused or not watch.launch_bound():
+                return self._watched(watch, cells, targets, run)
+            try:
+                captured = self._capture(cells, targets, run)
+            except RuntimeError as e:        # nothing of a capture has run: the step does now, as usual
+                LOG("WARN", f"step graph: capture failed, steps of this shape run launch by launch ({e})")
+                self._refused.add(key)
+                return self._watched(watch, cells, targets, run)
+            self._graphs[key] = captured
+            while len(self._graphs) > MAX_GRAPHS:
+                # its kernels may still be running: the memory goes back to the allocator only behind them
+                torch.cuda.current_stream().synchronize()
+                self._graphs.popitem(last=False)
+        self._graphs.move_to_end(key)
+        captured.cells.copy_(cells)
+        captured.targets.copy_(targets)
+        captured.graph.replay()
+        flops.add_counted(*captured.flops)
+        native.add_launches(captured.launches)
+        return captured.loss.clone()
+
+    def _watched(self, watch: _Watch, cells, targets, run) -> torch.Tensor:
+        start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        start.record()
+        t0 = time.perf_counter()
+        loss = run(cells, targets)
+        watch.host_ms = min(watch.host_ms, 1e3 * (time.perf_counter() - t0))
+        end.record()
+        watch.steps += 1
+        watch.pending = (watch.pending + [(start, end)])[-4:]
+        return loss
+
+    def _capture(self, cells, targets, run) -> _Captured:
+        captured = _Captured(cells, targets)
+        if self._stream is None:
+            self._stream = torch.cuda.Stream(self.device)
+        token = embconv.cache_token()
+        before, launches = flops.snapshot(), native.launches()
+        # tables that depend on parameters are built inside the graph, in every replay, and none of its memory is
+        # left to calls outside
+        embconv.set_cache_token(("graph", id(captured)))
+        compute = torch.cuda.current_stream()
+        self._stream.wait_stream(compute)
+        collecting = gc.isenabled()
+        gc.disable()                     # what a collection frees may not be freed during a capture
+        try:
+            with torch.cuda.stream(self._stream):
+                # other threads (logger, prefetch) may use CUDA meanwhile: only this thread's calls are looked at.  Not
+                # torch.cuda.graph(), which waits for the device and gives the allocator's cache back first.
+                captured.graph.capture_begin(capture_error_mode="thread_local")
+                try:
+                    captured.loss = run(captured.cells, captured.targets)
+                finally:
+                    captured.graph.capture_end()
+        finally:
+            if collecting:
+                gc.enable()
+            embconv.set_cache_token(token)
+            after = flops.snapshot()
+            captured.flops = (after[0] - before[0], after[1] - before[1])
+            captured.launches = native.launches() - launches
+            flops.add_counted(-captured.flops[0], -captured.flops[1])     # counted with each replay
+            native.add_launches(-captured.launches)
+        compute.wait_stream(self._stream)
+        return captured
