@@ -56,11 +56,16 @@ constexpr int kThreads = 32 * (2 + kNumEpilogueWarps);
 //           tensor-core cycle instead of 96 — at the price of using both accumulators for one tile.
 template <int BM, int BN>
 struct SmemLayout {
-  static constexpr int kStageRaw = (BM + BN) * BK * 2;
-  static constexpr int kStages = (200 * 1024 / kStageRaw) > 6 ? 6 : (200 * 1024 / kStageRaw);
+  // K blocks per stage.  The one thread that issues the loads needs some 70 to 110 cycles per load and 250 for the barrier of
+  // a stage, and the MMAs of a K block take 256 (BN = 128) or 128 cycles (64): two blocks share a stage there.  Cycles per K
+  // block, one block per stage -> two: BN = 128 390 -> 310, 64 390 -> 280 (460 before the loop of plain products was one of
+  // its own); four blocks and two stages: no change.
+  static constexpr int kSub = BM == 128 && BN <= 128 ? 2 : 1;
   static constexpr int kABytes = BM * BK * 2;
   static constexpr int kBBytes = BN * BK * 2;
-  static constexpr int kStageBytes = kABytes + kBBytes;
+  static constexpr int kBlockBytes = kABytes + kBBytes;
+  static constexpr int kStageBytes = kSub * kBlockBytes;
+  static constexpr int kStages = (200 * 1024 / kStageBytes) > 6 ? 6 : (200 * 1024 / kStageBytes);
   static constexpr int kBarrierBytes = 256;
   static constexpr int kEpiStage = 8 * 2 * 2048;   // per epilogue warp: two 32-row x 64-byte buffers for TMA stores
   static constexpr int kTotal = kStages * kStageBytes + kEpiStage + kBarrierBytes + 1024;  // +1024: manual alignment slack
@@ -186,50 +191,76 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
           if (!ok) break;
           asm volatile("fence.proxy.async;" ::: "memory");   // generic-proxy acquire -> async-proxy (TMA) reads
         }
-        for (int kb = wk.k_begin; kb < wk.k_end; kb += wk.k_step) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1)) { ok = false; break; }
-          uint8_t* sa = smem + stage * L::kStageBytes;
-          uint8_t* sb = sa + L::kABytes;
-          mbar_expect_tx(&full_bar[stage], L::kStageBytes);
-          if (p.mode == GEMM_MODE_WGRAD) {
-            // K block = brick of 64 output pixels; A = dY panel pair, B = gathered input for this tile's tap
-            const ConvGeom& g = p.conv;
-            const int bw = (kb % g.tiles_w) * g.tw;
-            const int bh = ((kb / g.tiles_w) % g.tiles_h) * g.th;
-            const int bn = (kb / (g.tiles_w * g.tiles_h)) * g.tn;
-            const int C = g.c_blocks * 64;
+        if (p.mode == GEMM_MODE_PLAIN) {
+          // a loop of its own: with the cases of the other modes in it an iteration takes 70 cycles more
+          const bool a_mn = p.a_mn_major != 0, b_mn = p.b_mn_major != 0;
+          const int a_row = tile_m * BM, b_row = tile_n * BN;
+          auto load_block = [&](uint8_t* sa, int kb) {
+            uint8_t* sb = sa + L::kABytes;
+            if (a_mn) {
 #pragma unroll
-            for (int j = 0; j < BM / 64; ++j)
-              tma_load_4d(sa + j * BK * 128, &map_a, &full_bar[stage], tile_m * BM + j * 64, bw, bh, bn);
+              for (int j = 0; j < BM / 64; ++j) tma_load_2d(sa + j * BK * 128, &map_a, &full_bar[stage], a_row + j * 64, kb * BK);
+            } else {
+              tma_load_2d(sa, &map_a, &full_bar[stage], kb * BK, a_row);
+            }
+            if (b_mn) {
 #pragma unroll
-            for (int j = 0; j < BN / 64; ++j) {
-              // column panel j of the tile: its filter tap and channel offset (past the last tap: channel
-              // coordinate C, i.e. out of range, which TMA fills with zeros)
-              const int col = tile_n * BN + j * 64;
-              int tap = col / C, c0 = col % C;
-              if (tap >= g.num_taps) { tap = 0; c0 = C; }
-              tma_load_4d(sb + j * BK * 128, &map_b, &full_bar[stage], c0, bw * g.in_mul + g.tap_dw[tap],
-                          bh * g.in_mul + g.tap_dh[tap], bn);
+              for (int j = 0; j < BN / 64; ++j) tma_load_2d(sb + j * BK * 128, &map_b, &full_bar[stage], b_row + j * 64, kb * BK);
+            } else {
+              tma_load_2d(sb, &map_b, &full_bar[stage], kb * BK, b_row);
+            }
+          };
+          for (int kb = wk.k_begin; kb < wk.k_end; kb += L::kSub * wk.k_step) {
+            if (!mbar_wait(&empty_bar[stage], phase ^ 1)) { ok = false; break; }
+            uint8_t* sa = smem + stage * L::kStageBytes;
+            if (kb + (L::kSub - 1) * wk.k_step < wk.k_end) {   // whole stages without a branch per block
+              mbar_expect_tx(&full_bar[stage], L::kStageBytes);
+#pragma unroll
+              for (int sub = 0; sub < L::kSub; ++sub) load_block(sa + sub * L::kBlockBytes, kb + sub * wk.k_step);
+            } else {
+              const int blocks = (wk.k_end - kb + wk.k_step - 1) / wk.k_step;
+              mbar_expect_tx(&full_bar[stage], blocks * L::kBlockBytes);
+#pragma unroll 1
+              for (int sub = 0; sub < blocks; ++sub) load_block(sa + sub * L::kBlockBytes, kb + sub * wk.k_step);
             }
             if (++stage == L::kStages) { stage = 0; phase ^= 1; }
-            continue;
           }
-          if (p.mode == GEMM_MODE_CONV) {
+          continue;
+        }
+        for (int kb0 = wk.k_begin; kb0 < wk.k_end; kb0 += L::kSub * wk.k_step) {
+          if (!mbar_wait(&empty_bar[stage], phase ^ 1)) { ok = false; break; }
+          const int blocks = min(L::kSub, (wk.k_end - kb0 + wk.k_step - 1) / wk.k_step);
+          mbar_expect_tx(&full_bar[stage], blocks * L::kBlockBytes);
+#pragma unroll 1
+          for (int sub = 0; sub < blocks; ++sub) {
+            const int kb = kb0 + sub * wk.k_step;
+            uint8_t* sa = smem + stage * L::kStageBytes + sub * L::kBlockBytes;
+            uint8_t* sb = sa + L::kABytes;
+            if (p.mode == GEMM_MODE_WGRAD) {
+              // K block = brick of 64 output pixels; A = dY panel pair, B = gathered input for this tile's tap
+              const ConvGeom& g = p.conv;
+              const int bw = (kb % g.tiles_w) * g.tw;
+              const int bh = ((kb / g.tiles_w) % g.tiles_h) * g.th;
+              const int bn = (kb / (g.tiles_w * g.tiles_h)) * g.tn;
+              const int C = g.c_blocks * 64;
+#pragma unroll
+              for (int j = 0; j < BM / 64; ++j)
+                tma_load_4d(sa + j * BK * 128, &map_a, &full_bar[stage], tile_m * BM + j * 64, bw, bh, bn);
+#pragma unroll
+              for (int j = 0; j < BN / 64; ++j) {
+                // column panel j of the tile: its filter tap and channel offset (past the last tap: channel
+                // coordinate C, i.e. out of range, which TMA fills with zeros)
+                const int col = tile_n * BN + j * 64;
+                int tap = col / C, c0 = col % C;
+                if (tap >= g.num_taps) { tap = 0; c0 = C; }
+                tma_load_4d(sb + j * BK * 128, &map_b, &full_bar[stage], c0, bw * g.in_mul + g.tap_dw[tap],
+                            bh * g.in_mul + g.tap_dh[tap], bn);
+              }
+              continue;
+            }
             const ConvGeom& g = p.conv;
             const int tap = kb / g.c_blocks, cb = kb % g.c_blocks;
             tma_load_4d(sa, &map_a, &full_bar[stage], cb * BK, cw + g.tap_dw[tap], ch + g.tap_dh[tap], cn);
-          } else if (p.a_mn_major) {
-#pragma unroll
-            for (int j = 0; j < BM / 64; ++j)
-              tma_load_2d(sa + j * BK * 128, &map_a, &full_bar[stage], tile_m * BM + j * 64, kb * BK);
-          } else {
-            tma_load_2d(sa, &map_a, &full_bar[stage], kb * BK, tile_m * BM);
-          }
-          if (p.b_mn_major) {
-#pragma unroll
-            for (int j = 0; j < BN / 64; ++j)
-              tma_load_2d(sb + j * BK * 128, &map_b, &full_bar[stage], tile_n * BN + j * 64, kb * BK);
-          } else {
             tma_load_2d(sb, &map_b, &full_bar[stage], kb * BK, tile_n * BN);
           }
           if (++stage == L::kStages) { stage = 0; phase ^= 1; }
@@ -258,18 +289,22 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         if (!mbar_wait(&tmem_empty[acc], acc_phase ^ 1)) { ok = false; break; }
         fence_after_sync();
         const uint32_t d_tmem = tmem_base + (MH == 1 ? acc * BN : 0);
-        for (int kb = wk.k_begin; kb < wk.k_end; kb += wk.k_step) {
+        for (int kb = wk.k_begin; kb < wk.k_end; kb += L::kSub * wk.k_step) {
           if (!mbar_wait(&full_bar[stage], phase)) { ok = false; break; }
           fence_after_sync();
-          const uint32_t sa = smem_u32(smem + stage * L::kStageBytes);
-          const uint32_t sb = sa + L::kABytes;
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint64_t db = make_smem_desc_sw128(sb + k * b_kstep, b_lbo, 1024);
+          for (int sub = 0; sub < L::kSub; ++sub) {
+            if (sub > 0 && kb + sub * wk.k_step >= wk.k_end) continue;
+            const uint32_t sa = smem_u32(smem + stage * L::kStageBytes + sub * L::kBlockBytes);
+            const uint32_t sb = sa + L::kABytes;
 #pragma unroll
-            for (int h = 0; h < MH; ++h) {   // M half h: rows [128h, 128h+128) = 16 KB further in either layout
-              const uint64_t da = make_smem_desc_sw128(sa + h * 128 * 128 + k * a_kstep, a_lbo, 1024);
-              mma_f16_ss(d_tmem + h * BN, da, db, idesc, ((kb - wk.k_begin) | k) != 0);   // first block overwrites
+            for (int k = 0; k < BK / UMMA_K; ++k) {
+              const uint64_t db = make_smem_desc_sw128(sb + k * b_kstep, b_lbo, 1024);
+#pragma unroll
+              for (int h = 0; h < MH; ++h) {   // M half h: rows [128h, 128h+128) = 16 KB further in either layout
+                const uint64_t da = make_smem_desc_sw128(sa + h * 128 * 128 + k * a_kstep, a_lbo, 1024);
+                mma_f16_ss(d_tmem + h * BN, da, db, idesc, ((kb - wk.k_begin) | sub | k) != 0);   // first block overwrites
+              }
             }
           }
           mma_commit(&empty_bar[stage]);  // frees the smem stage once these MMAs have read it
@@ -551,6 +586,17 @@ int pick_bm(long long m, int n, int bn, int requested) {
   return tiles256 >= 2 * 148 ? 256 : 128;
 }
 
+// Columns of a tile of a plain product: the narrowest tile that still leaves one tile per SM at most.  us, 256 | chosen:
+// 1000 x 1024 x 1024 11.5 | 7.2 (64), x 4096 24.9 | 14.2, 512 x 4096 x 1024 11.5 | 8.4 (128), 256 x 256 x 256 7.6 | 5.2.
+// Above one tile per SM the wide tile wins: 1000 x 3072 x 1024 11.8 with 256, 13 with 128.
+int pick_bn_plain(long long m, int n, int requested) {
+  if (requested == 64 || requested == 128 || requested == 256) return requested;
+  const long long tiles_m = (m + 127) / 128;
+  for (int bn = 64; bn < 256; bn *= 2)
+    if (tiles_m * ((n + bn - 1) / bn) <= 148) return bn;
+  return n <= 128 ? 128 : 256;
+}
+
 int pick_bn(int n, int requested) {
   if (requested == 64 || requested == 128 || requested == 256) return requested;
   if (n <= 64) return 64;
@@ -610,7 +656,8 @@ extern "C" int fbam_gemm(const void* A, long long lda, int a_mn_major, const voi
   if (p.splits > p.k_blocks) p.splits = p.k_blocks;
   if (p.splits > 1 && p.split_workspace == nullptr && !(p.out_fp32 && p.accumulate == GEMM_ACC_ATOMIC))
     return GEMM_ERR_SHAPE;
-  int bn = pick_bn(N, p.bn);
+  // a split product divides K until its wide tiles fill the machine
+  int bn = p.splits > 1 || p.bm == 256 ? pick_bn(N, p.bn) : pick_bn_plain(M, N, p.bn);
   int BM = pick_bm(M, N, bn, p.bm);
   if (p.ce_mode != 0) {
     // fused cross-entropy epilogues: one tile shape, no split-K, the buffers of the mode present
