@@ -222,6 +222,8 @@ def bench_embconv(a):
     tag = f"n{n} {rows}x{cols} v{a.vocab} ->{o} change{a.change}"
     feat = embconv.features_native(cells, *geom)
     pix = n * oh * ow
+    report("embconv_fwd_colour " + tag, timeit(lambda: embconv.forward_colour_native(cells, table, pos, cc_t, feat, z, y, *geom)),
+           bytes_moved=2 * pix * o * 2 + pix * 128 + cells.numel() * 4)
     report("embconv_features " + tag, timeit(lambda: embconv.features_native(cells, *geom)),
            bytes_moved=cells.numel() * 4 + pix * 128)
     report("embconv_colour_gemm " + tag, timeit(lambda: no.gemm(feat.view(pix, 64), cc_t, out=z.view(pix, o))),

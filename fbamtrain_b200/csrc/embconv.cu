@@ -14,13 +14,15 @@
 // (kernel_gen/kernel_gen/kernels/build_cell_embeds.py:74-134, build_cell_embeds_bwd.py:6-322,
 // src/framehead_model.cpp:126-175, 601-731) is covered here by
 //
-//   fbam_embconv_features    colour features F[n, p, tap*6 + c] = rgb_c(cell(p, tap)) / 255 (bf16, 64 per pixel):
-//                            the colour term is the GEMM F . CC (forward) and F^T . dZ (backward) on the tensor cores
+//   fbam_embconv_fwd_colour  Z = POS + table rows + F . CC; Y = GELU(Z), with the colour features
+//                            F[n, p, tap*6 + c] = rgb_c(cell(p, tap)) / 255 (bf16, 64 per pixel) made on the way and
+//                            kept for the backward, whose colour term is the product F^T . dZ
+//   fbam_embconv_features    F alone
 //   fbam_embconv_fwd         Z += POS + table rows; Y = GELU(Z)
 //   fbam_embconv_bwd_reduce  S[v][tap][:] += dZ rows by code point and tap;  D[p][:] += dZ summed over frames
 //
-// A warp owns one output pixel (32 lanes x 8 channels = a 256-channel block) and walks a run of consecutive frames.
-// Terminal frames change little from one frame to the next, and both kernels use that without depending on it:
+// A warp owns one output pixel (32 lanes x 8 channels = a 256-channel block; 4 in the backward) and walks a run of
+// consecutive frames.  Terminal frames change little from one frame to the next, and both kernels use that without depending on it:
 // the forward kernel keeps the sum of the nine table rows and, when a few of the nine code points changed, subtracts
 // the old rows and adds the new ones (it rebuilds the sum from scratch when more than four changed and at the start
 // of every run, which also bounds the rounding drift); the backward kernel accumulates dZ in registers per tap
@@ -87,118 +89,324 @@ __global__ void __launch_bounds__(256) embconv_features_kernel(const int* __rest
 }
 
 // ------------------------------------------------------------------------------------------------
-// forward: Z += POS + sum of table rows, Y = GELU(Z)
+// forward: Z = [colour term or Z] + POS + sum of table rows, Y = GELU(Z)
 // ------------------------------------------------------------------------------------------------
-constexpr int kPrefetch = 4;       // frames whose cell words / rows are fetched before any of them is used (forward)
-constexpr int kPrefetchBwd = 16;   // same in the backward reduction (8-byte pieces: 128 bytes in flight per lane)
+constexpr int kPrefetchBwd = 16;   // frames whose cell words / rows the backward reduction fetches before it uses any
+                                   // (8-byte pieces: 128 bytes in flight per lane)
 
 using gelu_math::f2;
 using gelu_math::gelu2;
 
-__device__ __forceinline__ void add_row(float2* acc, const elem_t* row, float sign) {
-  const Pack8 r = *reinterpret_cast<const Pack8*>(row);
-  const float2 s2 = f2(sign);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) acc[j] = __ffma2_rn(s2, e22ff(r.h[j]), acc[j]);
+// Eight warps, eight neighbouring pixels, 256 channels; a pass of the loop takes eight frames:
+//   1  the nine cells under each of the 64 (pixel, frame) pairs, loaded during the previous pass, become code points
+//      and colour features in shared memory;
+//   2  each warp lists the table rows by which the sum of its pixel changes from frame to frame, and multiplies the 64
+//      feature rows with the colour matrix for 32 of the 256 channels (mma.sync; the matrix waits in shared memory in
+//      fragment order, and its columns are permuted so that a lane holds eight neighbouring channels of a row);
+//   3  each warp walks the eight frames of its pixel, a lane with eight channels: rows from the list (the next pair
+//      of rows is always on its way), plus the colour term, GELU, stores.
+// The colour term was a product of its own before (features to memory, a GEMM with K = 64 into Z, Z read back here) and
+// the rows were loaded when a change was met, with the warp waiting for each: 1024 frames of 24 x 80 pixels, 256
+// channels, took 1195 / 1290 / 1570 / 2630 us with 1 / 5 / 15 / 100 % of the cells changing, 1096 / 1214 without Z kept;
+// now 744 / 829 / 1039 / 1774 and 673 / 760.  The 2.2 GB written are 0.34 ms: instructions bound it, 277 a pixel and
+// frame (84 of them GELU, 31 the colour product, 40 at 5 % the changed rows) at 55 % of the issue rate; sixteen warps an
+// SM do as much as twenty-four.
+constexpr int kFwdPix = 8;
+constexpr int kFwdFrames = 8;
+constexpr int kFwdThreads = 32 * kFwdPix;
+constexpr int kFwdBlocks = 2;                             // per SM, 128 registers; three with 80 spill: 395 against 385 us
+                                                          // for 444 frames of 24 x 80 pixels and 256 channels
+constexpr int kFwdRows = kFwdPix * kFwdFrames;            // rows of the colour product
+constexpr int kFwdLoads = 3;                              // cells a thread looks at per pass: taps part, part + 4, part + 8
+constexpr int kRebuild = 4;                               // more changed taps than this: the sum is built anew
+constexpr int kNewPairs = kRebuild + 1;                   // five pairs cover nine rows
+constexpr int kMaxPairs = kFwdFrames * kNewPairs + 1;     // one more marks the end
+
+struct FwdSmem {
+  uint4 cc[kFwdPix][7][32];                               // 28 KB: B fragments of three K = 16 steps and one K = 8 step
+  uint4 term[kFwdRows][32];                               // 32 KB: colour term, 16-bit
+  uint4 feat[kFwdRows][8];                                //  8 KB: features, 54 of 64 columns used
+  int2 pairs[kFwdPix][kMaxPairs];
+  int cp[kFwdPix][kFwdFrames + 1][9];                     // slot 0: the frame before this pass
+};
+
+// 16-byte chunks of a feature row are permuted by pixel and frame: the stores of a warp (eight pixels, four frames) and
+// the fragment loads (eight frames of a pixel) both spread over the banks.
+__device__ __forceinline__ int feat_key(int row) { return (row ^ (row >> 3)) & 7; }
+__device__ __forceinline__ int term_chunk(int row, int chunk) { return chunk ^ ((row & 1) << 2); }
+
+__device__ __forceinline__ void mma_k16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, float c0, float c1,
+                                        float c2, float c3) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32." ELEM_PTX "." ELEM_PTX ".f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+               "{%10,%11,%12,%13};"
+               : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
+}
+__device__ __forceinline__ void mma_k8(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32." ELEM_PTX "." ELEM_PTX ".f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a0), "r"(a1), "r"(b0));
 }
 
-// Blocks of 128 threads, five per SM (no spills; 256 and three: 817 us against 798 per 1024 frames of 24 x 80 pixels and
-// 256 channels with 5 % of the cells changing).
-constexpr int kFwdThreads = 128;
-__global__ void __launch_bounds__(kFwdThreads, 5) embconv_fwd_kernel(const int* __restrict__ cells, const elem_t* __restrict__ table,
-                                                             const float* __restrict__ pos, elem_t* __restrict__ z,
+// three colour bytes of a word as floats: the byte goes into the mantissa of 2^23
+__device__ __forceinline__ float byte_of(uint32_t w, uint32_t selector) {
+  return __uint_as_float(__byte_perm(w, 0x4b000000u, selector)) - 8388608.0f;
+}
+
+template <bool COLOUR>
+__global__ void __launch_bounds__(kFwdThreads, kFwdBlocks) embconv_fwd_kernel(const int* __restrict__ cells, const elem_t* __restrict__ table,
+                                                             const float* __restrict__ pos, const elem_t* __restrict__ cc,
+                                                             elem_t* __restrict__ feat, elem_t* __restrict__ z,
                                                              elem_t* __restrict__ y, long long frames, int vocab, int O,
-                                                             EmbConvGeom g, int seg_len, int nseg, int z_has_input,
+                                                             EmbConvGeom g, int seg_len, int z_has_input,
                                                              int apply_gelu, int write_z) {
+  extern __shared__ __align__(16) char smem_raw[];
+  FwdSmem& sm = *reinterpret_cast<FwdSmem*>(smem_raw);
   const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int p_out = g.oh * g.ow;
-  const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (item >= (long long)p_out * nseg) return;             // the whole warp leaves together
-  const int seg = (int)(item / p_out), p = (int)(item % p_out);
-  const int cell = lane < 9 ? tap_cell(g, p / g.ow, p % g.ow, lane) : -1;
-  const int co = blockIdx.y * 256 + lane * 8;
-  const bool act = co < O;
-  const long long cells_per_frame = (long long)g.rows * g.cols;
-  float2 base[4], sum[4];
+  const int groups = (p_out + kFwdPix - 1) / kFwdPix;
+  const long long seg = blockIdx.x / groups;
+  const int p0 = (int)(blockIdx.x % groups) * kFwdPix, p = p0 + warp;
+  const bool walks = p < p_out;
+  const int cb = blockIdx.y * 256, co = cb + lane * 8;
+  const bool act = walks && co < O;
+  const long long f0 = seg * seg_len, f1 = min(frames, f0 + seg_len);
+  const long long frame_words = (long long)g.rows * g.cols * 3;
+
+  // the cells that this thread fetches: pixel px of the eight, frame fu of a pass, every fourth tap from `part`
+  const int px = tid & 7, fu = (tid >> 3) & 7, part = tid >> 6;
+  const int frow = px * kFwdFrames + fu, fkey = feat_key(frow);
+  int item_off[kFwdLoads];                                // word of the cell within its frame; -1: padding or no such tap
 #pragma unroll
-  for (int j = 0; j < 4; ++j) { base[j] = f2(0.0f); sum[j] = f2(0.0f); }
-  if (act && pos != nullptr) {
-    const float4* pp = reinterpret_cast<const float4*>(pos + (long long)p * O + co);
-    const float4 a = pp[0], b = pp[1];
-    base[0] = make_float2(a.x, a.y); base[1] = make_float2(a.z, a.w);
-    base[2] = make_float2(b.x, b.y); base[3] = make_float2(b.z, b.w);
+  for (int k = 0; k < kFwdLoads; ++k) {
+    const int t = part + 4 * k;
+    item_off[k] = -1;
+    if (t < 9 && p0 + px < p_out) {
+      const int c = tap_cell(g, (p0 + px) / g.ow, (p0 + px) % g.ow, t);
+      if (c >= 0) item_off[k] = c * 3;
+    }
   }
-  int cur = -1;                                            // lanes 0..8: code point of this lane's tap (-1: none)
-  const long long f0 = (long long)seg * seg_len;
-  const long long f1 = min(frames, f0 + seg_len);
-  const long long row9 = 9ll * O;
-  const elem_t* tab = table + (act ? co : 0);
-  const int* cell_ptr = cells + (f0 * cells_per_frame + max(cell, 0)) * 3;
-  const long long cell_step = cells_per_frame * 3, z_step = (long long)p_out * O;
-  long long off = (f0 * p_out + p) * O + (act ? co : 0);
-  for (long long fb = f0; fb < f1; fb += kPrefetch) {
-    int ncp[kPrefetch];
-    Pack8 zin[kPrefetch];
+  const int* cell_ptr = cells + (f0 + fu) * frame_words;
+  int raw[kFwdLoads][3];
+  auto fetch = [&](int left) {                            // left: frames from the pass on
 #pragma unroll
-    for (int u = 0; u < kPrefetch; ++u) {
-      ncp[u] = -1;
-      if (fb + u < f1) {
-        if (cell >= 0) ncp[u] = __ldg(cell_ptr + u * cell_step);
-        if (act && z_has_input) zin[u] = *reinterpret_cast<const Pack8*>(z + off + u * z_step);
+    for (int k = 0; k < kFwdLoads; ++k) {
+      raw[k][0] = -1; raw[k][1] = 0; raw[k][2] = 0;
+      if (item_off[k] >= 0 && fu < left) {
+        raw[k][0] = __ldg(cell_ptr + item_off[k]);
+        if (COLOUR) { raw[k][1] = __ldg(cell_ptr + item_off[k] + 1); raw[k][2] = __ldg(cell_ptr + item_off[k] + 2); }
       }
     }
-    cell_ptr += kPrefetch * cell_step;
+    cell_ptr += kFwdFrames * frame_words;
+  };
+  fetch((int)min(f1 - f0, (long long)kFwdFrames));
+  if (COLOUR && part == 3) {                              // columns 54 to 63 stay zero
 #pragma unroll
-    for (int u = 0; u < kPrefetch; ++u) {
-      const long long f = fb + u;
-      if (f >= f1) break;
-      int nc = ncp[u];
-      if ((unsigned)nc >= (unsigned)vocab) nc = -1;        // outside the table (or padding): contributes nothing
-      const unsigned changed = __ballot_sync(full, nc != cur) & 0x1ffu;
-      if (f == f0 || __popc(changed) > 4) {
+    for (int w = 27; w < 32; ++w) reinterpret_cast<uint32_t*>(sm.feat[frow])[((w >> 2) ^ fkey) * 4 + (w & 3)] = 0u;
+  }
+
+  if (COLOUR) {                                           // colour matrix rows (channels) as B fragments
+    const int n = lane >> 2, kq = (lane & 3) * 2;
+    const int ch0 = cb + warp * 32 + 8 * (n >> 1) + (n & 1);
+    uint32_t w[28];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) sum[j] = f2(0.0f);
+    for (int j = 0; j < 4; ++j) {
+      const int ch = ch0 + 2 * j;
+      const uint32_t* row = reinterpret_cast<const uint32_t*>(cc + (long long)ch * 64);
 #pragma unroll
-        for (int t = 0; t < 9; ++t) {
-          const int c = __shfl_sync(full, nc, t);
-          if (c >= 0 && act) add_row(sum, tab + c * row9 + t * O, 1.0f);
-        }
-      } else {
-        unsigned m = changed;
-        while (m) {
-          const int t = __ffs(m) - 1;
-          m &= m - 1;
-          const int o = __shfl_sync(full, cur, t);
-          const int c = __shfl_sync(full, nc, t);
-          if (act) {
-            if (o >= 0) add_row(sum, tab + o * row9 + t * O, -1.0f);
-            if (c >= 0) add_row(sum, tab + c * row9 + t * O, 1.0f);
+      for (int h = 0; h < 7; ++h) w[j * 7 + h] = ch < O ? __ldg(row + (h * 8 + kq) / 2) : 0u;
+    }
+#pragma unroll
+    for (int i = 0; i < 7; ++i) sm.cc[warp][i][lane] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+  }
+
+  float2 sum[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) sum[j] = f2(0.0f);
+  const char* tab = reinterpret_cast<const char*>(table + (act ? co : 0));
+  const int row_bytes = O * (int)sizeof(elem_t);
+  auto load_row = [&](int row, Pack8& r) {
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (row >= 0 && act) v = __ldg(reinterpret_cast<const uint4*>(tab + (long long)row * row_bytes));
+    r = *reinterpret_cast<Pack8*>(&v);
+  };
+  const long long z_step = (long long)p_out * O;
+  const long long off = (f0 * p_out + p) * O + co;
+  elem_t* z_ptr = z + off;                                // not followed when there is no z or y
+  elem_t* y_ptr = y + off;
+
+  for (long long fb = f0; fb < f1; fb += kFwdFrames) {
+    const int nf = (int)min((long long)kFwdFrames, f1 - fb);
+    // 1: cells -> code points and features
+#pragma unroll
+    for (int k = 0; k < kFwdLoads; ++k) {
+      const int t = part + 4 * k;
+      if (k < 2 || part == 0) {
+        const int c = raw[k][0];
+        sm.cp[px][fu + 1][t] = (unsigned)c >= (unsigned)vocab ? -1 : c;         // outside the table contributes nothing
+        if (COLOUR) {
+          const uint32_t fg = (uint32_t)raw[k][1], bg = (uint32_t)raw[k][2];
+          const float s = 1.0f / 255.0f;
+          const elem2_t v[3] = {ff2e2(byte_of(fg, 0x7542) * s, byte_of(fg, 0x7541) * s),
+                                ff2e2(byte_of(fg, 0x7540) * s, byte_of(bg, 0x7542) * s),
+                                ff2e2(byte_of(bg, 0x7541) * s, byte_of(bg, 0x7540) * s)};
+          uint32_t* dst = reinterpret_cast<uint32_t*>(sm.feat[frow]);
+#pragma unroll
+          for (int h = 0; h < 3; ++h) {
+            const int w = part * 3 + h;                                         // 32-bit word of the row, less 12 k
+            dst[(((w >> 2) + 3 * k) ^ fkey) * 4 + (w & 3)] = *reinterpret_cast<const uint32_t*>(&v[h]);
           }
         }
       }
-      cur = nc;
+    }
+    __syncthreads();
+    // 2a: rows that change this pixel's sum, in pairs: (old, new) of a changed tap, or two taps of a sum built anew
+    uint32_t counts = 0;                                                        // pairs per frame, four bits each; kNewPairs: built anew
+    if (walks) {
+      int npairs = 0;
+      const int t = lane & 15, half = lane >> 4;
+      const bool tap = t < 9;
+      const int* cps = &sm.cp[warp][half][tap ? t : 0];
+      int2* pairs = sm.pairs[warp];
+#pragma unroll
+      for (int r = 0; r < kFwdFrames / 2; ++r) {
+        const bool on = tap && 2 * r + half < nf;
+        const int c = cps[(2 * r + 1) * 9], o = cps[2 * r * 9];
+        unsigned bal = __ballot_sync(full, on && c != o);
+        if (r == 0 && fb == f0) bal |= 0x1ffu;                                  // nothing to change yet: built anew
+        if (bal != 0) {
+          const int c0 = min(__popc(bal & 0xffffu), kNewPairs), c1 = min(__popc(bal >> 16), kNewPairs);
+          const unsigned mine = half ? bal >> 16 : bal & 0xffffu;
+          int2* slot = pairs + npairs + (half ? c0 : 0);
+          if ((half ? c1 : c0) == kNewPairs) {
+            const int n = t < 8 ? cps[(2 * r + 1) * 9 + 1] : -1;                // the next tap
+            if (on && !(t & 1)) slot[t >> 1] = make_int2(c >= 0 ? c * 9 + t : -1, n >= 0 ? n * 9 + t + 1 : -1);
+          } else if ((mine >> t) & 1u) {
+            slot[__popc(mine & ((1u << t) - 1u))] = make_int2(o >= 0 ? o * 9 + t : -1, c >= 0 ? c * 9 + t : -1);
+          }
+          npairs += c0 + c1;
+          counts |= (uint32_t)(c0 | (c1 << 4)) << (8 * r);
+        }
+      }
+      if (lane == 0) pairs[npairs] = make_int2(-1, -1);
+      __syncwarp();
+      if (lane < 9) sm.cp[warp][0][lane] = sm.cp[warp][kFwdFrames][lane];
+    }
+    if (COLOUR) {
+      // features that the backward reads
+      if (feat != nullptr && blockIdx.y == 0) {
+#pragma unroll
+        for (int k = 0; k < kFwdRows * 8 / kFwdThreads; ++k) {
+          const int i = tid + k * kFwdThreads;
+          const int chunk = i & 7, x = (i >> 3) % kFwdPix, u = (i >> 3) / kFwdPix;
+          const int row = x * kFwdFrames + u;
+          if (u < nf && p0 + x < p_out)
+            reinterpret_cast<uint4*>(feat + ((fb + u) * p_out + p0 + x) * 64)[chunk] = sm.feat[row][chunk ^ feat_key(row)];
+        }
+      }
+      // 2b: colour term of 64 rows, 32 channels a warp
+      uint32_t b[28];
+#pragma unroll
+      for (int i = 0; i < 7; ++i) {
+        const uint4 v = sm.cc[warp][i][lane];
+        b[4 * i] = v.x; b[4 * i + 1] = v.y; b[4 * i + 2] = v.z; b[4 * i + 3] = v.w;
+      }
+      const int r = lane & 15, hi = lane >> 4;
+#pragma unroll
+      for (int mt = 0; mt < kFwdRows / 16; ++mt) {
+        float d[4][4];
+        const int row = mt * 16 + r;
+#pragma unroll
+        for (int ks = 0; ks < 3; ++ks) {
+          uint32_t a[4];
+          const uint32_t addr = (uint32_t)__cvta_generic_to_shared(&sm.feat[row][(2 * ks + hi) ^ feat_key(row)]);
+          asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                       : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(addr) : "memory");
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float c = 0.0f;
+            mma_k16(d[j], a, b[j * 7 + 2 * ks], b[j * 7 + 2 * ks + 1], ks == 0 ? c : d[j][0], ks == 0 ? c : d[j][1],
+                    ks == 0 ? c : d[j][2], ks == 0 ? c : d[j][3]);
+          }
+        }
+        uint32_t a0, a1;
+        const uint32_t addr = (uint32_t)__cvta_generic_to_shared(&sm.feat[row][6 ^ feat_key(row)]);
+        asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(a0), "=r"(a1) : "r"(addr) : "memory");
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mma_k8(d[j], a0, a1, b[j * 7 + 6]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int orow = mt * 16 + 8 * h + (lane >> 2);
+          Pack8 v;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) v.h[j] = ff2e2(d[j][2 * h], d[j][2 * h + 1]);
+          sm.term[orow][term_chunk(orow, warp * 4 + (lane & 3))] = *reinterpret_cast<uint4*>(&v);
+        }
+      }
+    }
+    // 3: walk the frames; the next cells and the first pair of rows are on their way meanwhile
+    Pack8 ra, rb;
+    const int2* pair = sm.pairs[warp];
+    auto next_pair = [&]() {
+      const int2 pr = *pair++;
+      load_row(pr.x, ra);
+      load_row(pr.y, rb);
+    };
+    if (walks) next_pair();
+    if (fb + kFwdFrames < f1) fetch((int)min(f1 - fb - kFwdFrames, (long long)kFwdFrames));
+    __syncthreads();
+    if (!walks) continue;
+#pragma unroll 1
+    for (int u = 0; u < nf; ++u) {
+      const int n = counts & 15u;
+      counts >>= 4;
+      if (n != 0) {
+        const bool anew = n == kNewPairs;
+        if (anew) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) sum[j] = f2(0.0f);
+          if (act && pos != nullptr) {
+            const float4* pp = reinterpret_cast<const float4*>(pos + (long long)p * O + co);
+            const float4 a = __ldg(pp), b = __ldg(pp + 1);
+            sum[0] = make_float2(a.x, a.y); sum[1] = make_float2(a.z, a.w);
+            sum[2] = make_float2(b.x, b.y); sum[3] = make_float2(b.z, b.w);
+          }
+        }
+        const float2 sign = f2(anew ? 1.0f : -1.0f);
+#pragma unroll 1
+        for (int i = 0; i < n; ++i) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) sum[j] = __fadd2_rn(__ffma2_rn(sign, e22ff(ra.h[j]), sum[j]), e22ff(rb.h[j]));
+          next_pair();
+        }
+      }
       if (act) {
+        Pack8 term;
+        if (COLOUR) {
+          const int row = warp * kFwdFrames + u;
+          *reinterpret_cast<uint4*>(&term) = sm.term[row][term_chunk(row, lane)];
+        } else if (z_has_input) {
+          term = *reinterpret_cast<const Pack8*>(z_ptr);
+        }
         float2 v[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          v[j] = __fadd2_rn(sum[j], base[j]);
-          if (z_has_input) v[j] = __fadd2_rn(v[j], e22ff(zin[u].h[j]));
-        }
+        for (int j = 0; j < 4; ++j) v[j] = COLOUR || z_has_input ? __fadd2_rn(sum[j], e22ff(term.h[j])) : sum[j];
         Pack8 out;
+        if (write_z) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) out.h[j] = f22e2(v[j]);
-        if (write_z) *reinterpret_cast<Pack8*>(z + off + u * z_step) = out;
-        if (y != nullptr) {
-          if (apply_gelu) {
+          for (int j = 0; j < 4; ++j) out.h[j] = f22e2(v[j]);
+          *reinterpret_cast<Pack8*>(z_ptr) = out;
+        }
+        if (COLOUR || y != nullptr) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) out.h[j] = f22e2(gelu2(v[j]));
-          }
-          *reinterpret_cast<Pack8*>(y + off + u * z_step) = out;
+          for (int j = 0; j < 4; ++j) out.h[j] = f22e2(COLOUR || apply_gelu ? gelu2(v[j]) : v[j]);
+          *reinterpret_cast<Pack8*>(y_ptr) = out;
         }
       }
+      z_ptr += z_step;
+      y_ptr += z_step;
     }
-    off += kPrefetch * z_step;
   }
 }
 
@@ -336,27 +544,51 @@ extern "C" int fbam_embconv_features(const void* cells, void* feat, long long fr
   return launch_result();
 }
 
+namespace {
+template <bool COLOUR>
+int launch_fwd(const void* cells, const void* table, const void* pos, const void* cc, void* feat, void* z, void* y,
+               long long frames, int vocab, int O, const EmbConvGeom& g, int seg_len, int z_has_input, int apply_gelu,
+               int write_z, void* stream) {
+  if (!geom_ok(g) || frames < 0 || vocab < 1 || O < 8 || O % 8 != 0 || seg_len < 1) return 1;
+  for (const void* q : {table, pos, cc, (const void*)feat, (const void*)z, (const void*)y})
+    if (reinterpret_cast<uintptr_t>(q) % 16 != 0) return 2;
+  if (frames == 0) return 0;
+  const long long nseg = (frames + seg_len - 1) / seg_len;
+  const long long blocks = ((long long)g.oh * g.ow + kFwdPix - 1) / kFwdPix * nseg;
+  if (blocks > 0x7fffffffll) return 1;
+  auto kernel = embconv_fwd_kernel<COLOUR>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FwdSmem)) != cudaSuccess) return 5;
+  kernel<<<dim3((unsigned)blocks, (unsigned)((O + 255) / 256)), kFwdThreads, sizeof(FwdSmem),
+           reinterpret_cast<cudaStream_t>(stream)>>>(
+      reinterpret_cast<const int*>(cells), reinterpret_cast<const elem_t*>(table), reinterpret_cast<const float*>(pos),
+      reinterpret_cast<const elem_t*>(cc), reinterpret_cast<elem_t*>(feat), reinterpret_cast<elem_t*>(z),
+      reinterpret_cast<elem_t*>(y), frames, vocab, O, g, seg_len, z_has_input, apply_gelu, write_z);
+  return launch_result();
+}
+}  // namespace
+
 // table: bf16 [vocab][9][O]; pos: fp32 [oh*ow][O] or null; z: bf16 [frames][oh*ow][O], read (when z_has_input) and
 // overwritten with the pre-activation (left alone without write_z); y: bf16 like z or null, receives GELU(z) (or z itself without apply_gelu).
 extern "C" int fbam_embconv_fwd(const void* cells, const void* table, const void* pos, void* z, void* y,
                                 long long frames, int vocab, int O, int rows, int cols, int oh, int ow, int stride,
                                 int pad, int dil, int seg_len, int z_has_input, int apply_gelu, int write_z, void* stream) {
-  const EmbConvGeom g{rows, cols, oh, ow, stride, pad, dil};
-  if (!geom_ok(g) || frames < 0 || vocab < 1 || O < 8 || O % 8 != 0 || seg_len < 1) return 1;
-  if (reinterpret_cast<uintptr_t>(table) % 16 != 0 || reinterpret_cast<uintptr_t>(z) % 16 != 0 ||
-      reinterpret_cast<uintptr_t>(y) % 16 != 0 || reinterpret_cast<uintptr_t>(pos) % 16 != 0)
-    return 2;
-  if (frames == 0) return 0;
-  const int nseg = (int)((frames + seg_len - 1) / seg_len);
-  const long long items = (long long)oh * ow * nseg;
-  const long long blocks = (items + kFwdThreads / 32 - 1) / (kFwdThreads / 32);
-  if (blocks > 0x7fffffffll) return 1;
-  dim3 grid((unsigned)blocks, (unsigned)((O + 255) / 256));
-  embconv_fwd_kernel<<<grid, kFwdThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<const int*>(cells), reinterpret_cast<const elem_t*>(table), reinterpret_cast<const float*>(pos),
-      reinterpret_cast<elem_t*>(z), reinterpret_cast<elem_t*>(y), frames, vocab, O, g, seg_len, nseg, z_has_input,
-      apply_gelu, write_z);
-  return launch_result();
+  return launch_fwd<false>(cells, table, pos, nullptr, nullptr, z, y, frames, vocab, O,
+                           EmbConvGeom{rows, cols, oh, ow, stride, pad, dil}, seg_len, z_has_input, apply_gelu, write_z, stream);
+}
+
+// The same with the colour term computed on the way: cc: bf16 [O][64], colour matrix (54 columns used, the rest
+// ignored); feat: bf16 [frames][oh*ow][64] or null, receives the colour features (what fbam_embconv_features writes);
+// z: written only, or null; y: GELU(z).
+extern "C" int fbam_embconv_fwd_colour(const void* cells, const void* table, const void* pos, const void* cc, void* feat,
+                                       void* z, void* y, long long frames, int vocab, int O, int rows, int cols, int oh,
+                                       int ow, int stride, int pad, int dil, void* stream) {
+  if (cc == nullptr || y == nullptr) return 1;
+  // Runs of 64 frames, or of 16 where that would not give every SM its blocks twice over (256 frames of 12 x 40 pixels:
+  // 80 us against 86 with 64 and 123 with 128; 1024 frames of 24 x 80: 836 with 64 and 128, 873 with 32).
+  const long long groups = ((long long)oh * ow + kFwdPix - 1) / kFwdPix;
+  const int seg_len = groups * ((frames + 63) / 64) >= 2ll * 148 * kFwdBlocks ? 64 : 16;
+  return launch_fwd<true>(cells, table, pos, cc, feat, z, y, frames, vocab, O,
+                          EmbConvGeom{rows, cols, oh, ow, stride, pad, dil}, seg_len, 0, 1, z != nullptr, stream);
 }
 
 // S: fp32 [vocab][9][O] and D: fp32 [oh*ow][O]; both are added to (the caller zeroes them).

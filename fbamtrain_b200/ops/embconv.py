@@ -144,6 +144,17 @@ def forward_native(cells, table, pos, z, y, rows, cols, stride, pad, dil, z_has_
              "fbam_embconv_fwd")
 
 
+def forward_colour_native(cells, table, pos, cc_t, feat, z, y, rows, cols, stride, pad, dil) -> None:
+    """``y (N, P_out, O) = GELU(z)`` with the colour term ``F · cc_tᵀ`` (``cc_t (O, 64)``) added on the way; ``z`` and the
+    features ``feat (N, P_out, 64)`` are written where they are given."""
+    from . import native as nv
+    vocab, _, o = table.shape
+    nv.check(nv.lib(table).fbam_embconv_fwd_colour(nv.ptr(cells), nv.ptr(table), nv.ptr(pos), nv.ptr(cc_t), nv.ptr(feat),
+                                                   nv.ptr(z), nv.ptr(y), C.c_longlong(cells.shape[0]), vocab, o,
+                                                   *_geom_args(rows, cols, stride, pad, dil), nv.stream_ptr()),
+             "fbam_embconv_fwd_colour")
+
+
 def reduce_native(cells, dz, s, d, rows, cols, stride, pad, dil, seg_len: int = SEGMENT_FRAMES) -> None:
     """Adds into ``s`` (fp32, at least ``(V, 9, O)``; rows past ``vocab`` are left alone) and ``d`` (fp32 ``(P_out, O)``)."""
     from . import native as nv
@@ -207,19 +218,19 @@ def _tables_native(cp_embed, pos_embed, colour, w, rows, cols, stride, pad, dil)
 # first layer, forward and backward
 # =================================================================================================
 def first_layer_forward_native(cells, cp_embed, pos_embed, colour, w, rows, cols, stride, pad, dil, need_grad=True):
-    """→ ``y = GELU(z)``, ``z`` (both bf16 ``(N, OH, OW, O)``) and the colour features kept for the backward (``z`` is not
-    the pre-activation without ``need_grad``)."""
-    from . import native_ops as no
+    """→ ``y = GELU(z)`` and, for the backward, ``z`` (both bf16 ``(N, OH, OW, O)``) and the colour features; the last two
+    are ``None`` without ``need_grad``."""
+    from ..utils import debug, flops
     o = w.shape[0]
     n = cells.shape[0]
     oh, ow = out_hw(rows, cols, stride, pad, dil)
     _ext, _w_p, table, cc_t, pos_out, _pos_img = _tables_native(cp_embed, pos_embed, colour, w, rows, cols, stride, pad, dil)
-    feat = features_native(cells, rows, cols, stride, pad, dil, w.dtype)
-    # colour term: K = 64 makes this GEMM all epilogue; the CTA-pair kernel writes its tiles with TMA stores
-    z = no.gemm(feat.view(n * oh * ow, FEATURES), cc_t, two_cta=True)
-    y = torch.empty_like(z)
-    forward_native(cells, table, pos_out, z, y, rows, cols, stride, pad, dil, write_z=need_grad)
-    return y.view(n, oh, ow, o), z.view(n, oh, ow, o), feat
+    y = debug.fresh((n, oh, ow, o), w.dtype, cells.device)
+    z = debug.fresh((n, oh, ow, o), w.dtype, cells.device) if need_grad else None
+    feat = debug.fresh((n, oh * ow, FEATURES), w.dtype, cells.device) if need_grad else None
+    flops.add(2.0 * n * oh * ow * FEATURES * o)
+    forward_colour_native(cells, table, pos_out, cc_t, feat, z, y, rows, cols, stride, pad, dil)
+    return y, z, feat
 
 
 def first_layer_backward_native(cells, feat, dz, cp_embed, pos_embed, colour, w, rows, cols, stride, pad, dil):

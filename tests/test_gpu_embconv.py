@@ -65,6 +65,39 @@ def test_forward_gather_kernel(rows, cols, stride, pad, dil, o, change):
     assert _rel(y, torch.nn.functional.gelu(want)) < 4e-3
 
 
+# frames around one pass of eight, runs of 16 and (the last: enough pixels) of 64; pixels that are no multiple of eight
+@pytest.mark.parametrize("n,geom,o,change", [(1, (9, 15, 2, 1, 1), 64, 0.05), (7, (8, 16, 2, 1, 1), 320, 0.05),
+                                             (8, (8, 12, 1, 1, 1), 256, 1.0), (9, (12, 10, 2, 2, 2), 64, 0.3),
+                                             (33, (9, 15, 2, 1, 1), 256, 0.05), (130, (48, 160, 2, 1, 1), 64, 0.1)])
+@pytest.mark.parametrize("dtype", [BF, torch.float16])
+def test_forward_with_colour_term(n, geom, o, change, dtype):
+    """Rounding to the element type (half an ulp: 2^-8, 2^-11) of the colour term and of the result, and fp32 drift of at
+    most eight additions a frame over a run of 64 frames."""
+    from fbamtrain_b200.ops import embconv, native as nv
+    torch.manual_seed(7)
+    vocab, half_ulp = 50, 2.0 ** (-8 if dtype == BF else -11)
+    cells = _cells(n, geom[0], geom[1], vocab, 8, change)
+    taps = embconv.tap_cells(*geom, DEV)
+    table = torch.randn(vocab, 9, o, device=DEV).to(dtype)
+    cc_t = torch.zeros(o, embconv.FEATURES, device=DEV, dtype=dtype)
+    cc_t[:, :54] = torch.randn(o, 54, device=DEV)
+    pos = torch.randn(taps.shape[0], o, device=DEV)
+    y = torch.full((n, taps.shape[0], o), float("nan"), device=DEV, dtype=dtype)
+    z, alone = torch.full_like(y, float("nan")), torch.full_like(y, float("nan"))
+    feat = torch.full((n, taps.shape[0], embconv.FEATURES), float("nan"), device=DEV, dtype=dtype)
+    embconv.forward_colour_native(cells, table, pos, cc_t, feat, z, y, *geom)
+    embconv.forward_colour_native(cells, table, pos, cc_t, None, None, alone, *geom)
+    nv.check_status(cells.device)
+    assert torch.equal(feat, embconv.features_torch(cells, taps, dtype)) and torch.equal(y, alone)
+    term = feat.double() @ cc_t.double().t()
+    want = embconv.gather_torch(cells, taps, table).double() + pos.double() + term
+    drift = 8 * 64 * 2.0 ** -24 * 32                              # sums stay below 32
+    v_err = half_ulp * term.abs() * 1.01 + drift
+    assert bool(((z.double() - want).abs() <= v_err + half_ulp * 1.01 * want.abs()).all())
+    gelu = torch.nn.functional.gelu(want)
+    assert bool(((y.double() - gelu).abs() <= 1.13 * v_err + half_ulp * 1.01 * gelu.abs() + 1e-6).all())
+
+
 @pytest.mark.parametrize("change", [0.05, 1.0])
 @pytest.mark.parametrize("o", [64, 256, 320])
 @pytest.mark.parametrize("rows,cols,stride,pad,dil", GEOMS)
