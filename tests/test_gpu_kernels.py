@@ -36,6 +36,23 @@ def test_gemm_k_major(m, n, k):
     assert_similar(expect.to(BF), d, 0.02 * math.sqrt(k))
 
 
+# narrow tiles take two K blocks of 64 per stage: odd counts, a last block of 8, fewer blocks than one stage and more than all
+# stages; 148 tiles of 64 or 128 columns and one tile more
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+@pytest.mark.parametrize("m,n", [(128, 64), (2, 200), (4 * 128, 37 * 64), (4 * 128, 37 * 64 + 8), (4 * 128, 37 * 128), (4 * 128, 37 * 128 + 8)])
+@pytest.mark.parametrize("k", [8, 64, 136, 192, 1352])
+def test_gemm_two_k_blocks_per_stage(m, n, k, a_mn, b_mn):
+    """Integers up to 8: every partial sum stays below 2^24 and is exact in fp32, so the result is too."""
+    nv, no = _nops()
+    g = torch.Generator(device=DEV).manual_seed(m + n + k)
+    a = torch.randint(-8, 9, (m, k), device=DEV, generator=g).to(BF)
+    b = torch.randint(-8, 9, (n, k), device=DEV, generator=g).to(BF)
+    d = no.gemm(a.t().contiguous() if a_mn else a, b.t().contiguous() if b_mn else b, a_mn=a_mn, b_mn=b_mn,
+                out_dtype=torch.float32)
+    nv.check_status(a.device)
+    assert torch.equal(d, a.float() @ b.float().t())
+
+
 @pytest.mark.parametrize("a_mn,b_mn", [(False, True), (True, False), (True, True)])
 @pytest.mark.parametrize("m,n,k", [(128, 128, 64), (256, 512, 320), (1024, 4096, 8192), (200, 264, 136)])
 def test_gemm_mn_major_operands(a_mn, b_mn, m, n, k):
