@@ -288,6 +288,11 @@ __device__ __forceinline__ uint32_t publish_bits(float value) {
 // pushed out the 0xFF bytes, and polls and partial writes would wait for DRAM.  H = 1024, batch 8, 1024 steps: forward
 // 1.54 -> 1.49, backward 1.90 -> 1.74 us a step; nothing up to H = 512; 1 % slower above 1024, where it is left out.
 constexpr int kAhead = 8;
+// The step whose lines are fetched when step `published` of T has been, going up (forward) or down (backward); -1: past the
+// last one.  The buffers end there, and what lies behind is another tensor's memory or nobody's.
+__host__ __device__ constexpr int step_ahead(int published, int T, bool down) {
+  return down ? (published >= kAhead ? published - kAhead : -1) : (published + kAhead < T ? published + kAhead : -1);
+}
 __device__ __forceinline__ void prefetch_l2(const elem_t* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 __device__ __forceinline__ long long clock_now() {
@@ -440,7 +445,7 @@ lstm_fwd_kernel(float* __restrict__ gates, const elem_t* __restrict__ whh, const
         gates[gate] = a[p];
         if (q == 0) c_all[cell] = c[p];
         if (t + 1 < T) xg[p] = gates[gate + 4 * step];  // needed after the next exchange
-        if (SB == 0 && writes && t + kAhead < T) prefetch_l2(y + cell + kAhead * step);
+        if (SB == 0 && writes && step_ahead(t, T, false) >= 0) prefetch_l2(y + cell + kAhead * step);
       }
     }
     if (SB == 0) {
@@ -673,9 +678,11 @@ lstm_bwd_kernel(const float* __restrict__ gates, const float* __restrict__ c_all
       __syncthreads();  // no warp polls before the CTA has published
       published = clock_now();
       if (live && t > 1) fetch(t - 2);
-      if (SB == 0 && writes && t > kAhead) {
+      const int ahead = step_ahead(t - 1, T, true);  // t - 1 has just been published, and dgp has moved on to t - 2
+      if (SB == 0 && writes && ahead >= 0) {
+        const elem_t* to = dgp - 4 * (t - 2 - ahead) * t_step;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) prefetch_l2(dgp - 4 * kAhead * t_step + i * H);
+        for (int i = 0; i < 4; ++i) prefetch_l2(to + i * H);
       }
     }
   }
@@ -779,6 +786,9 @@ extern "C" {
 
 // Largest hidden size the persistent kernels accept.
 int fbam_lstm_persistent_max_hidden() { return 2048; }
+
+// For tests: which step's lines the kernels fetch behind the publication of a step, or -1.
+int fbam_lstm_step_ahead(int published, int T, int down) { return step_ahead(published, T, down != 0); }
 
 // gates: (T, B, 4H) fp32, pre-activations incl. bias on entry, activated gates on exit.
 // hbuf and counter: ignored, may be null (y itself is what the CTAs exchange; the arguments stay for callers of the C

@@ -47,3 +47,17 @@ def test_rule_for_large_batches(monkeypatch):
                 ((1536, 256, 4, True), True), ((2048, 64, 16, False), True), ((4096, 64, 16, False), False)]
     for args, faster in measured:
         assert L.persistent_ok(*args) is faster, args
+
+
+@pytest.mark.parametrize("steps", [1, 2, 8, 9, 10, 11, 17, 18, 256])
+@pytest.mark.parametrize("down", [0, 1])
+def test_lines_are_fetched_within_the_sequence(steps, down):
+    """Both directions fetch the lines of the step eight behind the published one while there is one: the backward pass used
+    to reach the step before the first (T = 10 and more)."""
+    from fbamtrain_b200.ops import native as nv
+    if not nv.available():
+        pytest.skip("kernel library not built")
+    ahead = nv.lib().fbam_lstm_step_ahead
+    for published in range(steps):
+        to = published - 8 if down else published + 8
+        assert ahead(published, steps, down) == (to if 0 <= to < steps else -1)
