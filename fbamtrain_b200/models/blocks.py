@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import torch
 from torch import nn
+from torch.nn.modules import module as _module
 
 from .. import ops
 from .init_utils import SeedSequence, fill_uniform_fan_
@@ -27,6 +28,22 @@ class RmsNorm(nn.Module):
         if with_input:
             return ops.rms_norm_residual(x, self.weight, self.eps)
         return ops.rms_norm(x, self.weight, self.eps)
+
+
+_RMS_FORWARD = RmsNorm.forward
+
+
+def _norm_beside_residual(norm: nn.Module, x: torch.Tensor):
+    """``(norm(x), x)`` for a block that goes on with both.  A plain :class:`RmsNorm` gives both from one autograd function,
+    so that their gradients meet in one kernel.  Any other module in its place, and one whose calls something looks at, is
+    called as a module is: with ``x`` alone, for a tensor."""
+    if type(norm) is RmsNorm and "forward" not in vars(norm) and RmsNorm.forward is _RMS_FORWARD:
+        hooked = (norm._forward_hooks or norm._forward_pre_hooks or norm._backward_hooks or norm._backward_pre_hooks
+                  or _module._global_forward_hooks or _module._global_forward_pre_hooks or _module._global_backward_hooks
+                  or _module._global_backward_pre_hooks)
+        if not hooked:
+            return norm(x, with_input=True)
+    return norm(x), x
 
 
 class LayerNorm(nn.Module):
@@ -128,8 +145,8 @@ class AttentionBlock(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         # the residual additions ride in the epilogues of the output-projection and second MLP GEMMs
-        y, x = self.ln1(x, with_input=True)
+        y, x = _norm_beside_residual(self.ln1, x)
         x = self.attn(y, residual=x)
         b, t, e = x.shape
-        y, x2 = self.ln2(x.reshape(b * t, e), with_input=True)
+        y, x2 = _norm_beside_residual(self.ln2, x.reshape(b * t, e))
         return self.mlp(y, residual=x2).view(b, t, e)
