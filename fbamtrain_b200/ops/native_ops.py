@@ -439,15 +439,20 @@ def conv2d_fprop(x, w_ohwi, stride, padding, dilation, act: str = "none", preact
     return out
 
 
-@functools.lru_cache(maxsize=4096)
 def _pool_plan(n: int, oh: int, ow: int, channels: int):
     """``(segment, segments per image)`` of a convolution whose activation is only averaged over positions, or ``None``
     where that runs as a convolution and a pool: the CTA-pair kernel is not the one for the size (as in ``conv_pass``),
     or a brick has fewer than four neighbouring positions of an image, so that the sums would be no smaller than the
     activation."""
+    return _pool_segments(n, oh, ow, channels) if TWO_CTA in ("auto", True) else None
+
+
+@functools.lru_cache(maxsize=4096)
+def _pool_segments(n: int, oh: int, ow: int, channels: int):
+    """The part of :func:`_pool_plan` that follows from the sizes alone."""
     tn, th, tw = _brick(n, oh, ow, 256)
     tiles = math.ceil(n / tn) * math.ceil(oh / th) * math.ceil(ow / tw)
-    if TWO_CTA not in ("auto", True) or channels < 256 or channels % 32 or tiles < 148:
+    if channels < 256 or channels % 32 or tiles < 148:
         return None
     _, th, tw = _brick(n, oh, ow, 128)
     seg = C.c_int()
