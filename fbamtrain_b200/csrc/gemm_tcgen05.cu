@@ -536,6 +536,16 @@ int encode_nhwc(CUtensorMap* map, const void* base, int n, int h, int w, int c, 
 
 int g_num_sms = 0;
 
+// CTAs that a launch of a persistent kernel may use.
+int usable_ctas(int max_ctas) {
+  int dev = 0;
+  if (g_num_sms == 0 && (cudaGetDevice(&dev) != cudaSuccess ||
+                         cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess))
+    g_num_sms = 148;
+  const int sms = g_num_sms > g_fbam_reserved_sms ? g_num_sms - g_fbam_reserved_sms : 1;
+  return max_ctas > 0 && max_ctas < sms ? max_ctas : sms;
+}
+
 template <int BM, int BN, bool CE = false>
 int launch(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams& p, cudaStream_t stream) {
   using L = SmemLayout<BM, BN>;
@@ -546,15 +556,8 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams& p, cudaStre
       return GEMM_ERR_LAUNCH;
     configured = true;
   }
-  if (g_num_sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
-  }
-  const int tiles = p.tiles_m * ((p.N + BN - 1) / BN) * p.splits;
-  const int usable = g_num_sms - g_fbam_reserved_sms > 0 ? g_num_sms - g_fbam_reserved_sms : 1;
-  int grid = tiles < usable ? tiles : usable;
-  if (p.max_ctas > 0 && grid > p.max_ctas) grid = p.max_ctas;
+  const int tiles = p.tiles_m * ((p.N + BN - 1) / BN) * p.splits, usable = usable_ctas(p.max_ctas);
+  const int grid = tiles < usable ? tiles : usable;
   CUtensorMap md, mpre;
   p.tma_store = 0;
   std::memset(&md, 0, sizeof(md));
@@ -586,22 +589,22 @@ int pick_bm(long long m, int n, int bn, int requested) {
   return tiles256 >= 2 * 148 ? 256 : 128;
 }
 
-// Columns of a tile of a plain product: the narrowest tile that still leaves one tile per SM at most.  us, 256 | chosen:
-// 1000 x 1024 x 1024 11.5 | 7.2 (64), x 4096 24.9 | 14.2, 512 x 4096 x 1024 11.5 | 8.4 (128), 256 x 256 x 256 7.6 | 5.2.
-// Above one tile per SM the wide tile wins: 1000 x 3072 x 1024 11.8 with 256, 13 with 128.
-int pick_bn_plain(long long m, int n, int requested) {
-  if (requested == 64 || requested == 128 || requested == 256) return requested;
-  const long long tiles_m = (m + 127) / 128;
-  for (int bn = 64; bn < 256; bn *= 2)
-    if (tiles_m * ((n + bn - 1) / bn) <= 148) return bn;
-  return n <= 128 ? 128 : 256;
-}
-
 int pick_bn(int n, int requested) {
   if (requested == 64 || requested == 128 || requested == 256) return requested;
   if (n <= 64) return 64;
   if (n <= 128) return 128;
   return 256;
+}
+
+// Columns of a tile of a plain product: the narrowest tile that still leaves one tile per CTA that the launch may use at
+// most.  us, 256 | chosen: 1000 x 1024 x 1024 11.5 | 7.2 (64), x 4096 24.9 | 14.2, 512 x 4096 x 1024 11.5 | 8.4 (128),
+// 256 x 256 x 256 7.6 | 5.2.  Above one tile per CTA the wide tile wins: 1000 x 3072 x 1024 11.8 with 256, 13 with 128.
+int pick_bn_plain(long long m, int n, int requested, int ctas) {
+  if (requested == 64 || requested == 128 || requested == 256) return requested;
+  const long long tiles_m = (m + 127) / 128;
+  for (int bn = 64; bn < 256; bn *= 2)
+    if (tiles_m * ((n + bn - 1) / bn) <= ctas) return bn;
+  return n <= 128 ? 128 : 256;
 }
 
 }  // namespace
@@ -644,6 +647,9 @@ extern "C" int fbam_set_reserved_sms(int n) {
   return old;
 }
 
+// Columns of a tile that fbam_gemm picks for an unsplit product (for tests of the rule).
+extern "C" int fbam_gemm_tile_columns(int M, int N, int max_ctas) { return pick_bn_plain(M, N, 0, usable_ctas(max_ctas)); }
+
 extern "C" int fbam_gemm(const void* A, long long lda, int a_mn_major, const void* B, long long ldb,
                               int b_mn_major, int M, int N, int K, GemmParams* params, void* stream) {
   GemmParams p = *params;
@@ -657,7 +663,7 @@ extern "C" int fbam_gemm(const void* A, long long lda, int a_mn_major, const voi
   if (p.splits > 1 && p.split_workspace == nullptr && !(p.out_fp32 && p.accumulate == GEMM_ACC_ATOMIC))
     return GEMM_ERR_SHAPE;
   // a split product divides K until its wide tiles fill the machine
-  int bn = p.splits > 1 || p.bm == 256 ? pick_bn(N, p.bn) : pick_bn_plain(M, N, p.bn);
+  int bn = p.splits > 1 || p.bm == 256 ? pick_bn(N, p.bn) : pick_bn_plain(M, N, p.bn, usable_ctas(p.max_ctas));
   int BM = pick_bm(M, N, bn, p.bm);
   if (p.ce_mode != 0) {
     // fused cross-entropy epilogues: one tile shape, no split-K, the buffers of the mode present

@@ -1,0 +1,27 @@
+"""The rule for the tiles of plain products (the products themselves are tested on the GPU)."""
+import pytest
+
+from fbamtrain_b200.ops import native as nv
+
+
+@pytest.fixture
+def columns():
+    if not nv.available():
+        pytest.skip("kernel library not built")
+    lib = nv.lib()
+    yield lib.fbam_gemm_tile_columns
+    lib.fbam_set_reserved_sms(0)
+
+
+def test_narrow_tiles_fit_the_ctas_of_the_launch(columns):
+    """9 x 16 tiles of 64 columns: one wave of the whole machine, two of what a pipeline rank or a limited launch may use."""
+    assert columns(9 * 128, 16 * 64, 0) == 64
+    assert columns(9 * 128, 16 * 64, 144) == 64
+    assert columns(9 * 128, 16 * 64, 143) == 128
+    assert columns(9 * 128, 16 * 64, 71) == 256
+    assert columns(9 * 128, 16 * 64, 500) == 64
+    assert columns(9 * 128, 32 * 64, 0) == 128 and columns(9 * 128, 64 * 64, 0) == 256
+    assert nv.lib().fbam_set_reserved_sms(16) == 0
+    assert columns(9 * 128, 16 * 64, 0) == 128
+    assert columns(9 * 128, 32 * 64, 0) == 256
+    assert columns(9 * 128, 14 * 64, 0) == 64
