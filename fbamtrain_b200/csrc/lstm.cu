@@ -86,11 +86,16 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a
 // -------------------------------------------------------------------------------------------------
 // gate functions
 // -------------------------------------------------------------------------------------------------
-// One path through the hardware's 2^x and 1/x for both functions, no branch: sigmoid(x) = 1 / (1 + e^-x), tanh(x) =
-// 2 sigmoid(2x) - 1, and x + x³·p(x²) where that would cancel (p: a least-squares fit in the relative error, 2.6e-9 at
-// most on |x| < 0.6).  Errors against 64 bits over [-8, 8], relative, largest | rms, of 1 / (1 + __expf(-x)) and tanhf and
-// of these: sigmoid 5.1e-7 | 9.7e-8 and 5.3e-7 | 9.9e-8, tanh 1.9e-7 | 2.6e-8 and 1.8e-7 | 2.1e-8.  With an IEEE division
-// and tanhf, which a quad went through one after the other, the gates of a forward step took 743 cycles; now 330.
+// One path through the hardware's 2^x and 1/x for both functions, no branch: sigmoid(x) = 1 / (1 + e^-x), tanh(|x|) =
+// 1 - 2 / (1 + e^2|x|), and x + x³·p(x²) where that would cancel (p: a fit of the least largest relative error; with these
+// coefficients 4.8e-9 on |x| < 0.9).  Errors against 64 bits, relative, largest | rms, of 1 / (1 + __expf(-x)) and tanhf
+// -> of these:
+//   sigmoid  [-8, 8] 5.0e-7 | 9.7e-8 -> 2.2e-7 | 4.1e-8   [-1, 1] 1.6e-7 | 4.4e-8 -> 1.7e-7 | 3.5e-8
+//   tanh     [-8, 8] 1.9e-7 | 2.6e-8 -> 1.1e-7 | 2.0e-8   [-1, 1] 2.0e-7 | 5.6e-8 -> 1.1e-7 | 2.8e-8
+// (2 / (1 + e^-2x) - 1 instead is off by up to 3.7e-7 where x is around 1: the rounding of a value near one counts twice.)
+// us per forward step with an IEEE division | uncorrected | as here: H = 1024, 8 rows 1.56 | 1.52 | 1.54, 32 rows 2.86 |
+// 2.74 | 2.80, H = 2048, 8 rows 2.98 | 2.81 | 2.84; with tanhf too, which a quad goes through after the sigmoids, the
+// gates of a step take 743 cycles instead of some 350.
 __device__ __forceinline__ float ex2_f(float x) {
   float r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -101,18 +106,32 @@ __device__ __forceinline__ float rcp_f(float x) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
-// tanh(x), given `far`, its value where |x| is not small.
-__device__ __forceinline__ float tanh_from(float x, float far) {
+// 1 / (1 + 2^(k·x)) for k = ±log2 e or twice that, as the nearest float.  Three roundings are made good where the result is
+// a normal number: that of the exponent, by its error-free product (Dekker; k·x = hi + lo, and what k lacks) and 2^lo = 1 +
+// lo·ln 2; that of the sum, by the part of the smaller addend that it dropped (Dekker's fast two-sum); that of the
+// reciprocal, by one step of Newton's iteration.
+__device__ __forceinline__ float logistic(float x, float k) {
+  const float hi = k * x;
+  const bool normal = fabsf(hi) < 100.0f;  // false for infinities and NaN, which the plain terms carry through
+  const float e0 = ex2_f(hi), lo = fmaf(hi, 1.335e-8f, fmaf(k, x, -hi));
+  const float e = normal ? fmaf(e0, lo * 0.69314718f, e0) : e0;
+  const float d = 1.0f + e, r = rcp_f(d), dropped = fminf(e, 1.0f) - (d - fmaxf(e, 1.0f));
+  return normal ? fmaf(r, fmaf(-dropped, r, fmaf(-d, r, 1.0f)), r) : r;
+}
+// tanh(x), given 1 / (1 + e^2|x|).
+__device__ __forceinline__ float tanh_from(float x, float r) {
   const float s = x * x;
-  float p = fmaf(-0.005905978847295046f, s, 0.020805491134524345f);
-  p = fmaf(p, s, -0.05378672108054161f);
-  p = fmaf(p, s, 0.13331958651542664f);
-  p = fmaf(p, s, -0.33333298563957214f);
-  return fabsf(x) < 0.6f ? fmaf(x * s, p, x) : far;
+  float p = fmaf(-0.0004554584447760135f, s, 0.0025826634373515844f);
+  p = fmaf(p, s, -0.008264538832008839f);
+  p = fmaf(p, s, 0.021663539111614227f);
+  p = fmaf(p, s, -0.053929299116134644f);
+  p = fmaf(p, s, 0.13332977890968323f);
+  p = fmaf(p, s, -0.33333322405815125f);
+  float near = fmaf(x * s, p, x);
+  asm volatile("" : "+f"(near));  // computed by all lanes: as a branch it cost 0.1 us a step
+  return fabsf(x) < 0.9f ? near : copysignf(fmaf(-2.0f, r, 1.0f), x);
 }
-__device__ __forceinline__ float tanh_f(float x) {
-  return tanh_from(x, fmaf(2.0f, rcp_f(1.0f + ex2_f(-2.88539008f * x)), -1.0f));
-}
+__device__ __forceinline__ float tanh_f(float x) { return tanh_from(x, rcp_f(1.0f + ex2_f(2.88539008f * fabsf(x)))); }
 
 // -------------------------------------------------------------------------------------------------
 // cluster
@@ -342,7 +361,7 @@ lstm_fwd_kernel(float* __restrict__ gates, const elem_t* __restrict__ whh, const
   // this quad's cells: batch row ob of each group, unit `unit`; a lane has gate q
   const int ob = warp / UT, unit = unit0 + (warp % UT) * 8 + g;
   const int prow = (warp % UT) * 32 + q * 8 + g;  // its row among the CTA's gate rows
-  const float act_scale = (q == 2 ? 2.0f : 1.0f) * -1.44269504f;
+  const float act_scale = q == 2 ? 2.88539008f : -1.44269504f;
   const bool writes = q == 0 && (!vec || (g & 1) == 0);
   const long long step = (long long)B * H;
   // Element of y and c_all at the step at hand, group 0 (the lane's gate lies at 4·at + gate_at), and what the lane polls.
@@ -419,8 +438,8 @@ lstm_fwd_kernel(float* __restrict__ gates, const elem_t* __restrict__ whh, const
     }
 #pragma unroll
     for (int p = 0; p < P; ++p) {
-      const float pre = a[p], s = rcp_f(1.0f + ex2_f(act_scale * pre));
-      a[p] = q == 2 ? tanh_from(pre, fmaf(2.0f, s, -1.0f)) : s;
+      const float pre = a[p], s = logistic(q == 2 ? fabsf(pre) : pre, act_scale);
+      a[p] = q == 2 ? tanh_from(pre, s) : s;
       const float ig = __shfl_sync(0xffffffffu, a[p], lane & ~3), fg = __shfl_sync(0xffffffffu, a[p], (lane & ~3) + 1);
       const float gg = __shfl_sync(0xffffffffu, a[p], (lane & ~3) + 2), og = __shfl_sync(0xffffffffu, a[p], (lane & ~3) + 3);
       c[p] = fg * c[p] + ig * gg;
