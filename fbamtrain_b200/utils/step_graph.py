@@ -36,20 +36,27 @@ MAX_CELLS = 8 << 20
 WATCHED_STEPS = 2        # steps of a shape that run as usual before one may be captured
 HOST_SHARE = 0.7         # captured where the host takes at least this share of the step's time on the GPU's clock
 MAX_GRAPHS = 2           # per trainer; the least recently used one is given back
+MAX_WATCHES = 8
 
 
 class _Watch:
-    """Host and GPU time of the steps of one shape that ran as usual (the smallest of each)."""
+    """Host and GPU time of the steps of one shape that ran as usual (the smallest of each).  ``wait``: how many there have
+    to be before a capture; it doubles whenever a graph of the shape is given back, so that shapes that take turns and do
+    not fit ``MAX_GRAPHS`` cost some ten captures in a thousand steps each and not one at every turn."""
 
     def __init__(self) -> None:
         self.steps, self.host_ms, self.gpu_ms, self.pending = 0, float("inf"), float("inf"), []
+        self.wait: float = WATCHED_STEPS
+
+    def given_back(self) -> None:
+        self.steps, self.wait = 0, 2 * self.wait
 
     def launch_bound(self) -> bool:
-        """Asked after ``WATCHED_STEPS``; looks at finished events only, so it never waits for the device."""
+        """Looks at finished events only, so it never waits for the device."""
         while self.pending and self.pending[0][1].query():
             start, end = self.pending.pop(0)
             self.gpu_ms = min(self.gpu_ms, start.elapsed_time(end))
-        return self.steps >= WATCHED_STEPS and self.gpu_ms < float("inf") and self.host_ms >= HOST_SHARE * self.gpu_ms
+        return self.steps >= self.wait and self.gpu_ms < float("inf") and self.host_ms >= HOST_SHARE * self.gpu_ms
 
 
 class _Captured:
@@ -67,7 +74,6 @@ class StepGraph:
         self.device = torch.device("cuda", torch.cuda.current_device() if device.index is None else device.index)
         self._watches: "OrderedDict[tuple, _Watch]" = OrderedDict()
         self._graphs: "OrderedDict[tuple, _Captured]" = OrderedDict()
-        self._refused: set = set()
         self._stream: Optional[torch.cuda.Stream] = None
 
     # ------------------------------------------------------------------------------------------
@@ -120,24 +126,20 @@ class StepGraph:
         key = self._setting(cells, targets, loss_scale)
         captured = self._graphs.get(key)
         if captured is None:
-            watch = self._watches.get(key)
-            if watch is None:
-                watch = self._watches[key] = _Watch()
-                while len(self._watches) > 8:
-                    self._watches.popitem(last=False)
-            if key in self._refused or not watch.launch_bound():
+            watch = self._watch(key)
+            if not watch.launch_bound():
                 return self._watched(watch, cells, targets, run)
             try:
                 captured = self._capture(cells, targets, run)
             except RuntimeError as e:        # nothing of a capture has run: the step does now, as usual
                 LOG("WARN", f"step graph: capture failed, steps of this shape run launch by launch ({e})")
-                self._refused.add(key)
+                watch.wait = float("inf")
                 return self._watched(watch, cells, targets, run)
             self._graphs[key] = captured
             while len(self._graphs) > MAX_GRAPHS:
                 # its kernels may still be running: the memory goes back to the allocator only behind them
                 torch.cuda.current_stream().synchronize()
-                self._graphs.popitem(last=False)
+                self._watch(self._graphs.popitem(last=False)[0]).given_back()
         self._graphs.move_to_end(key)
         captured.cells.copy_(cells)
         captured.targets.copy_(targets)
@@ -145,6 +147,14 @@ class StepGraph:
         flops.add_counted(*captured.flops)
         native.add_launches(captured.launches)
         return captured.loss.clone()
+
+    def _watch(self, key: tuple) -> _Watch:
+        """The watch of a shape; those of the last ``MAX_WATCHES`` shapes are kept."""
+        watch = self._watches.setdefault(key, _Watch())
+        self._watches.move_to_end(key)
+        while len(self._watches) > MAX_WATCHES:
+            self._watches.popitem(last=False)
+        return watch
 
     def _watched(self, watch: _Watch, cells, targets, run) -> torch.Tensor:
         start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)

@@ -1,0 +1,77 @@
+"""Which steps a trainer's step graph captures (captures and replays themselves are tested on the GPU)."""
+import pytest
+import torch
+
+from fbamtrain_b200.utils import step_graph as sg
+
+
+class _Model(torch.nn.Module):
+    frame_chunk = 0
+
+
+class _Graph:
+    """Stands in for a captured step: a replay counts."""
+
+    def __init__(self, log):
+        self.cells, self.targets = torch.zeros(0), torch.zeros(0)
+        self.graph, self.log = self, log
+        self.flops, self.launches, self.loss = (0.0, 0.0), 0, torch.zeros(())
+
+    def replay(self):
+        self.log.append("replay")
+
+
+@pytest.fixture
+def graph(monkeypatch):
+    log = []
+    monkeypatch.setattr(sg.torch.cuda, "current_stream", lambda *a: type("S", (), {"synchronize": lambda s: log.append("wait")})())
+    g = sg.StepGraph(_Model(), torch.device("cuda", 0))
+    g.log = log
+    monkeypatch.setattr(g, "_ordinary", lambda: True)
+    monkeypatch.setattr(g, "_setting", lambda cells, targets, scale: tuple(cells.shape))
+
+    def watched(watch, cells, targets, run):
+        watch.steps, watch.host_ms, watch.gpu_ms = watch.steps + 1, 1.0, 1.0
+        log.append("usual")
+        return torch.zeros(())
+
+    def capture(cells, targets, run):
+        log.append("capture")
+        captured = _Graph(log)
+        captured.cells = captured.targets = torch.empty_like(cells)
+        return captured
+
+    monkeypatch.setattr(g, "_watched", watched)
+    monkeypatch.setattr(g, "_capture", capture)
+    return g
+
+
+def _steps(g, shapes, n):
+    for i in range(n):
+        cells = torch.zeros(1, shapes[i % len(shapes)], 1)
+        assert g.forward_backward(cells, cells, 1.0, None) is not None
+    return {what: g.log.count(what) for what in ("usual", "capture", "replay", "wait")}
+
+
+@pytest.mark.parametrize("shapes", [[1], [1, 2]])
+def test_shapes_that_fit_are_captured_once(graph, shapes):
+    seen = _steps(graph, shapes, 60)
+    assert seen["usual"] == 2 * len(shapes) and seen["capture"] == len(shapes) and seen["wait"] == 0
+    assert seen["replay"] == 60 - 2 * len(shapes)
+
+
+@pytest.mark.parametrize("n_shapes", [3, 5, 8, 12])
+def test_shapes_that_take_turns_are_not_captured_at_every_turn(graph, n_shapes):
+    """300 turns: a capture at every turn would be some 290 of each shape; with waits of 2, 4, 8 ... there are at most eight."""
+    seen = _steps(graph, list(range(1, n_shapes + 1)), 300 * n_shapes)
+    assert seen["capture"] <= 8 * n_shapes and seen["wait"] <= seen["capture"]
+    assert len(graph._graphs) <= sg.MAX_GRAPHS and len(graph._watches) <= sg.MAX_WATCHES
+
+
+def test_a_capture_that_fails_is_not_tried_again(graph, monkeypatch):
+    def fails(*a):
+        graph.log.append("capture")
+        raise RuntimeError("no")
+    monkeypatch.setattr(graph, "_capture", fails)
+    seen = _steps(graph, [1], 40)
+    assert seen["capture"] == 1 and seen["usual"] == 40
