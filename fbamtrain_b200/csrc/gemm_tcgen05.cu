@@ -641,6 +641,7 @@ extern "C" int fbam_elem_is_fp16() { return ELEM_IS_FP16; }
 // 1 when the row-store variant of the reduce-scatter epilogue was compiled in (see gemm_epilogue.cuh).
 extern "C" int fbam_has_rs_row_stores() { return FBAM_RS_ROW_STORES; }
 
+extern "C" int fbam_reserved_sms() { return g_fbam_reserved_sms; }
 extern "C" int fbam_set_reserved_sms(int n) {
   const int old = g_fbam_reserved_sms;
   g_fbam_reserved_sms = n < 0 ? 0 : n;

@@ -7,10 +7,10 @@ next step of that shape are captured once and replayed from then on.  Gradients 
 parameters read where they lie, so the optimizer, gradient accumulation and checkpoints see no difference; inputs are
 copied into the graph's own buffers, the loss out of them.
 
-What is captured is what the host would have done for the step at hand.  Whatever can change that is compared or asked
-for before every replay (:meth:`_setting`); with anything out of the ordinary — hooks, saved-tensor hooks, dispatch modes,
-anomaly detection, debug switches, a recording of launches or shapes — the step runs as usual.
-``FBAMTRAIN_STEP_GRAPH=0`` keeps every step that way.
+What is captured is what the host would have done for the step at hand.  Before every replay the settings of the model, of
+this package and of the libraries that this depends on are compared (:meth:`_setting`); with anything out of the ordinary —
+hooks, saved-tensor hooks, dispatch modes, anomaly detection, debug switches, a recording of launches or shapes — the step
+runs as usual.  ``FBAMTRAIN_STEP_GRAPH=0`` keeps every step that way.
 
 The reference has no counterpart: its executor launches kernel by kernel (reference:
 ``tensorlib/src/execution_backend.cpp``).
@@ -37,6 +37,29 @@ WATCHED_STEPS = 2        # steps of a shape that run as usual before one may be 
 HOST_SHARE = 0.7         # captured where the host takes at least this share of the step's time on the GPU's clock
 MAX_GRAPHS = 2           # per trainer; the least recently used one is given back
 MAX_WATCHES = 8
+
+
+_PLAIN = frozenset((bool, int, float, str, torch.dtype))
+
+
+def _module_setting(m: torch.nn.Module) -> tuple:
+    """What a module's part of a step depends on besides parameters: its code, its plain attributes and its buffers."""
+    kind = type(m)
+    setting = [kind, kind.forward, kind.__call__]
+    setting += [item for item in vars(m).items() if type(item[1]) in _PLAIN]
+    if m._buffers:
+        setting += [None if b is None else b.data_ptr() for b in m._buffers.values()]
+    return tuple(setting)
+
+
+def _library_setting() -> tuple:
+    """Switches of the library paths, which fp32 models and the tables of the first layer take."""
+    b = torch.backends
+    return (torch.get_float32_matmul_precision(), b.fp32_precision, b.cuda.matmul.fp32_precision, b.cudnn.fp32_precision,
+            b.cudnn.conv.fp32_precision, b.cudnn.rnn.fp32_precision, b.cuda.matmul.allow_fp16_reduced_precision_reduction,
+            b.cuda.matmul.allow_bf16_reduced_precision_reduction, b.cudnn.enabled, b.cudnn.benchmark, b.cudnn.deterministic,
+            b.cuda.flash_sdp_enabled(), b.cuda.mem_efficient_sdp_enabled(), b.cuda.math_sdp_enabled(),
+            b.cuda.cudnn_sdp_enabled(), b.cuda.preferred_blas_library())
 
 
 class _Watch:
@@ -110,6 +133,8 @@ class StepGraph:
                 no.LM_HEAD_CHUNK_ROWS, no.RESIDUAL_NORM_MAX_DIM,
                 tuple(dispatch._prefer.values()), os.environ.get("FBAMTRAIN_EMBCONV"),
                 os.environ.get("FBAMTRAIN_ATTENTION_FWD2"), torch.are_deterministic_algorithms_enabled(),
+                native.lib(self.model.action_model.head_weight).fbam_reserved_sms(), *_library_setting(),
+                repr(self.model.cfg), tuple([_module_setting(m) for m in self.model.modules()]),
                 tuple((p.data_ptr(), p.requires_grad, -1 if p.grad is None else p.grad.data_ptr())
                       for p in self.model.parameters()))
 
