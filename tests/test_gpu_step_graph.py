@@ -6,12 +6,12 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-def _trainer(kind="toy"):
+def _trainer(kind="toy", dtype="bf16"):
     from fbamtrain_b200 import RunConfiguration, Trainer, presets
     d = presets.fbam_toy()
     if kind == "muon":
         d["optimizer"].update({"type": "muon", "learning_rate": 2e-3, "momentum": 0.9, "nesterov": True})
-    d["model_config"]["dtype"] = "bf16"
+    d["model_config"]["dtype"] = dtype
     d["micro_batch_size"] = d["total_batch_size"] = 2
     d["train_sequence_length"] = 24
     return Trainer(RunConfiguration.from_json(d), device=torch.device("cuda", 0))
@@ -85,7 +85,6 @@ def test_new_inputs_shapes_and_storage(monkeypatch):
         torch.cuda.synchronize()
     assert _graphs(trainer) == 1
     before = [g.data.clone() for g in trainer.all_groups()]
-    state = [g.data.clone() for g in trainer.all_groups()]
     trainer.zero_grad()
     loss_a = float(trainer._forward_backward(*a))
     grads_a = [g.grad.clone() for g in trainer.all_groups()]
@@ -97,6 +96,7 @@ def test_new_inputs_shapes_and_storage(monkeypatch):
     trainer._forward_backward(*a)                           # gradients add up, as launch by launch
     for g, one in zip(trainer.all_groups(), grads_a):
         assert float((g.grad.float() - 2 * one.float()).norm()) <= 2e-2 * float(one.float().norm()) + 1e-6
+    assert all(torch.equal(g.data, x) for g, x in zip(trainer.all_groups(), before))     # forward and backward alone
     short = [(c[:, :16].contiguous(), t[:, :16].contiguous()) for c, t in (a, b)]
     for i in range(4):
         trainer.train_step(*short[i % 2])
@@ -111,7 +111,6 @@ def test_new_inputs_shapes_and_storage(monkeypatch):
     monkeypatch.setenv("FBAMTRAIN_STEP_GRAPH", "0")
     trainer.zero_grad()
     assert changed == pytest.approx(float(trainer._forward_backward(*a)), rel=1e-3)
-    assert all(torch.equal(x, y) for x, y in zip(before, state))
     trainer.close()
 
 
