@@ -199,11 +199,13 @@ class Trainer:
         dev_cells, dev_targets, events, chunk = self._upload(cells, targets)
         b, t, p, _ = dev_cells.shape
         if self._step_graph is not None and (events is None or len(events) == 1):
-            def run(step_cells, step_targets):
+            def run(step_cells, step_targets, after_forward):
                 with gputx_range("fbamtrain::forward"):
                     emb = self.model.frame_embeddings(step_cells)
                     with gputx_range("fbamtrain::action_model_fwd_bwd"):
                         loss = self.model.action_model(emb, step_targets, loss_scale)
+                if after_forward is not None:
+                    after_forward()
                 with gputx_range("fbamtrain::backward"):
                     loss.backward()
                 return loss.detach()
@@ -238,11 +240,7 @@ class Trainer:
                             # the rest would not fit, the remaining chunks keep only their inputs and are run
                             # again in the backward (the alternative is running out of memory).
                             grown = torch.cuda.memory_allocated(self.device) - before
-                            cached = torch.cuda.memory_reserved(self.device) - torch.cuda.memory_allocated(self.device)
-                            # The driver is asked only when what the allocator holds is not enough by itself (the
-                            # first step): its answer takes 0.1 ms to 0.2 s, during which nothing is launched.
-                            need = grown * (n_chunks - i - 1)
-                            if need > 0.9 * cached and need > 0.9 * (torch.cuda.mem_get_info(self.device)[0] + cached):
+                            if not self._memory_for(grown * (n_chunks - i - 1)):
                                 recompute = True
                                 if not self._warned_recompute:
                                     self._warned_recompute = True
@@ -262,6 +260,22 @@ class Trainer:
             self.logger.progress(ProgressRecord("Backward: frames", b * t, b * t, phase1, self._mark()))
         self._upload_read(events)
         return loss.detach()
+
+    def _memory_for(self, need: int) -> bool:
+        """Whether ``need`` more bytes of activations fit.  What the allocator holds for captured steps is no room for other
+        allocations; the graphs are given back where their memory decides."""
+        graphs = self._step_graph
+        cached = torch.cuda.memory_reserved(self.device) - torch.cuda.memory_allocated(self.device)
+        if graphs is not None:
+            cached -= graphs.pool_bytes
+        # The driver is asked only when what the allocator holds is not enough by itself (the first step): its answer takes
+        # 0.1 ms to 0.2 s, during which nothing is launched.
+        if need <= 0.9 * cached:
+            return True
+        free = torch.cuda.mem_get_info(self.device)[0] + cached
+        if need > 0.9 * free and graphs is not None and graphs.pool_bytes:
+            free += graphs.release()
+        return need <= 0.9 * free
 
     def _upload_read(self, events) -> None:
         """The backward was the last reader of the micro-batch's device buffers, where it was uploaded."""

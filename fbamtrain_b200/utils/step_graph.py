@@ -12,6 +12,10 @@ this package and of the libraries that this depends on are compared (:meth:`_set
 hooks, saved-tensor hooks, dispatch modes, anomaly detection, debug switches, a recording of launches or shapes — the step
 runs as usual.  ``FBAMTRAIN_STEP_GRAPH=0`` keeps every step that way.
 
+The activations of the captured steps stay with the graphs, in one pool of memory that is as large as the largest step
+needs and goes to nobody else.  It is at most ``MEMORY_SHARE`` of the memory that is free at a capture, and is given back
+(:meth:`StepGraph.release`) where a large step of the trainer would otherwise have to recompute its activations.
+
 The reference has no counterpart: its executor launches kernel by kernel (reference:
 ``tensorlib/src/execution_backend.cpp``).
 """
@@ -37,6 +41,9 @@ WATCHED_STEPS = 2        # steps of a shape that run as usual before one may be 
 HOST_SHARE = 0.7         # captured where the host takes at least this share of the step's time on the GPU's clock
 MAX_GRAPHS = 2           # per trainer; the least recently used one is given back
 MAX_WATCHES = 8
+# Part of the device memory that is free at a capture which the graphs of a trainer may hold: what they hold is lost to
+# everything else for as long as they live.
+MEMORY_SHARE = 0.125
 
 
 _PLAIN = frozenset((bool, int, float, str, torch.dtype))
@@ -70,6 +77,7 @@ class _Watch:
     def __init__(self) -> None:
         self.steps, self.host_ms, self.gpu_ms, self.pending = 0, float("inf"), float("inf"), []
         self.wait: float = WATCHED_STEPS
+        self.kept = 0              # bytes that the forward leaves for the backward
 
     def given_back(self) -> None:
         self.steps, self.wait = 0, 2 * self.wait
@@ -98,6 +106,7 @@ class StepGraph:
         self._watches: "OrderedDict[tuple, _Watch]" = OrderedDict()
         self._graphs: "OrderedDict[tuple, _Captured]" = OrderedDict()
         self._stream: Optional[torch.cuda.Stream] = None
+        self.pool_bytes = 0        # device memory that the allocator holds for the graphs and gives to nobody else
 
     # ------------------------------------------------------------------------------------------
     def _ordinary(self) -> bool:
@@ -140,8 +149,8 @@ class StepGraph:
 
     # ------------------------------------------------------------------------------------------
     def forward_backward(self, cells: torch.Tensor, targets: torch.Tensor, loss_scale: float, run) -> Optional[torch.Tensor]:
-        """The loss of ``run(cells, targets)`` (forward and backward on device tensors), or ``None`` where the step is not
-        one to watch."""
+        """The loss of ``run(cells, targets, after_forward)`` (forward and backward on device tensors, with a call between the
+        two where one is given), or ``None`` where the step is not one to watch."""
         chunk = self.model.frame_chunk
         frames = cells.shape[0] * cells.shape[1]
         if frames * cells.shape[2] > MAX_CELLS or (chunk and frames > chunk) or not self._ordinary():
@@ -153,6 +162,9 @@ class StepGraph:
         if captured is None:
             watch = self._watch(key)
             if not watch.launch_bound():
+                return self._watched(watch, cells, targets, run)
+            if not self._room(watch):
+                watch.given_back()
                 return self._watched(watch, cells, targets, run)
             try:
                 captured = self._capture(cells, targets, run)
@@ -173,6 +185,20 @@ class StepGraph:
         native.add_launches(captured.launches)
         return captured.loss.clone()
 
+    def _room(self, watch: _Watch) -> bool:
+        """Gradients of activations come to less than the activations, hence the two."""
+        more = max(0, 2 * watch.kept + (64 << 20) - self.pool_bytes)
+        return self.pool_bytes + more <= MEMORY_SHARE * (torch.cuda.mem_get_info(self.device)[0] + self.pool_bytes)
+
+    def release(self) -> int:
+        """Gives all graphs back, for a step that needs their memory; the bytes that are free for it now."""
+        if self._graphs:
+            torch.cuda.current_stream().synchronize()
+        while self._graphs:
+            self._watch(self._graphs.popitem(last=False)[0]).given_back()
+        freed, self.pool_bytes = self.pool_bytes, 0
+        return freed
+
     def _watch(self, key: tuple) -> _Watch:
         """The watch of a shape; those of the last ``MAX_WATCHES`` shapes are kept."""
         watch = self._watches.setdefault(key, _Watch())
@@ -183,9 +209,15 @@ class StepGraph:
 
     def _watched(self, watch: _Watch, cells, targets, run) -> torch.Tensor:
         start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        after_forward = None
+        if watch.steps > 0:              # not in the first step of a shape, which may be its only one
+            before = torch.cuda.memory_allocated(self.device)
+
+            def after_forward():
+                watch.kept = max(watch.kept, torch.cuda.memory_allocated(self.device) - before)
         start.record()
         t0 = time.perf_counter()
-        loss = run(cells, targets)
+        loss = run(cells, targets, after_forward)
         watch.host_ms = min(watch.host_ms, 1e3 * (time.perf_counter() - t0))
         end.record()
         watch.steps += 1
@@ -209,11 +241,15 @@ class StepGraph:
             with torch.cuda.stream(self._stream):
                 # other threads (logger, prefetch) may use CUDA meanwhile: only this thread's calls are looked at.  Not
                 # torch.cuda.graph(), which waits for the device and gives the allocator's cache back first.
-                captured.graph.capture_begin(capture_error_mode="thread_local")
+                # Graphs share a pool: what a step leaves behind in it is its loss, which is copied out at once, and replays
+                # follow one another on the trainer's stream.
+                pool = next((c.graph.pool() for c in self._graphs.values()), None) or torch.cuda.graph_pool_handle()
+                captured.graph.capture_begin(pool=pool, capture_error_mode="thread_local")
                 try:
-                    captured.loss = run(captured.cells, captured.targets)
+                    captured.loss = run(captured.cells, captured.targets, None)
                 finally:
                     captured.graph.capture_end()
+            self.pool_bytes = sum(s["total_size"] for s in torch.cuda.memory_snapshot(pool, include_traces=False))
         finally:
             if collecting:
                 gc.enable()

@@ -28,6 +28,7 @@ def graph(monkeypatch):
     g = sg.StepGraph(_Model(), torch.device("cuda", 0))
     g.log = log
     monkeypatch.setattr(g, "_ordinary", lambda: True)
+    monkeypatch.setattr(sg.torch.cuda, "mem_get_info", lambda *a: (64 << 30, 180 << 30))
     monkeypatch.setattr(g, "_setting", lambda cells, targets, scale: tuple(cells.shape))
 
     def watched(watch, cells, targets, run):
@@ -75,3 +76,39 @@ def test_a_capture_that_fails_is_not_tried_again(graph, monkeypatch):
     monkeypatch.setattr(graph, "_capture", fails)
     seen = _steps(graph, [1], 40)
     assert seen["capture"] == 1 and seen["usual"] == 40
+
+
+def test_graphs_hold_a_part_of_the_free_memory_at_most(graph, monkeypatch):
+    """An eighth of what is free: with 8 GB free no graph whose step leaves 0.5 GB for its backward, with 10 GB one; then
+    none while it is given back more often than it is replayed."""
+    free = [8 << 30]
+    monkeypatch.setattr(sg.torch.cuda, "mem_get_info", lambda *a: (free[0], 180 << 30))
+    _steps(graph, [1], 2)
+    graph._watch((1, 1, 1)).kept = 512 << 20
+    assert _steps(graph, [1], 10)["capture"] == 0
+    free[0] = 10 << 30
+    assert _steps(graph, [1], 60)["capture"] == 1
+    graph.pool_bytes = 1 << 30
+    assert graph.release() == 1 << 30 and not graph._graphs and graph.pool_bytes == 0
+    assert _steps(graph, [1], 4)["capture"] == 1          # it has to earn another
+
+
+@pytest.mark.parametrize("pool,need,fits,released", [
+    (0, 80, True, False), (0, 100, True, False), (0, 190, False, False),
+    (60, 30, True, False),        # the allocator's own cache, less the graphs', is enough
+    (60, 80, True, False),        # with what the driver has free
+    (60, 150, True, True),        # with the graphs' memory too
+    (60, 190, False, True),
+])
+def test_memory_of_graphs_is_no_room_for_a_step(pool, need, fits, released, monkeypatch):
+    """100 bytes in the allocator's cache, of which the graphs hold ``pool``, and 100 free."""
+    from types import SimpleNamespace
+    from fbamtrain_b200.train import Trainer
+    cuda, gave = torch.cuda, []
+    monkeypatch.setattr(cuda, "memory_reserved", lambda *a: 150)
+    monkeypatch.setattr(cuda, "memory_allocated", lambda *a: 50)
+    monkeypatch.setattr(cuda, "mem_get_info", lambda *a: (100, 1000))
+    graphs = SimpleNamespace(pool_bytes=pool, release=lambda: gave.append(pool) or pool)
+    assert Trainer._memory_for(SimpleNamespace(_step_graph=graphs, device=None), need) is fits
+    assert bool(gave) is released
+    assert Trainer._memory_for(SimpleNamespace(_step_graph=None, device=None), need) is (need <= 180)
