@@ -598,13 +598,14 @@ int pick_bn(int n, int requested) {
 
 // Columns of a tile of a plain product: the narrowest tile that still leaves one tile per CTA that the launch may use at
 // most.  us, 256 | chosen: 1000 x 1024 x 1024 11.5 | 7.2 (64), x 4096 24.9 | 14.2, 512 x 4096 x 1024 11.5 | 8.4 (128),
-// 256 x 256 x 256 7.6 | 5.2.  Above one tile per CTA the wide tile wins: 1000 x 3072 x 1024 11.8 with 256, 13 with 128.
+// 256 x 256 x 256 7.6 | 5.2.  Above one tile per CTA the widest tile that N fills wins: 1000 x 3072 x 1024 11.8 with 256, 13
+// with 128; 20000 x 64 x 4096 51 with 64, 55 with 128, 200000 x 64 x 1024 84 and 90.
 int pick_bn_plain(long long m, int n, int requested, int ctas) {
   if (requested == 64 || requested == 128 || requested == 256) return requested;
   const long long tiles_m = (m + 127) / 128;
   for (int bn = 64; bn < 256; bn *= 2)
     if (tiles_m * ((n + bn - 1) / bn) <= ctas) return bn;
-  return n <= 128 ? 128 : 256;
+  return pick_bn(n, 0);
 }
 
 }  // namespace

@@ -25,3 +25,9 @@ def test_narrow_tiles_fit_the_ctas_of_the_launch(columns):
     assert columns(9 * 128, 16 * 64, 0) == 128
     assert columns(9 * 128, 32 * 64, 0) == 256
     assert columns(9 * 128, 14 * 64, 0) == 64
+
+
+@pytest.mark.parametrize("n,wide", [(8, 64), (64, 64), (72, 128), (128, 128), (136, 256), (4096, 256)])
+def test_many_rows_take_the_tile_that_the_columns_fill(columns, n, wide):
+    """More tiles than CTAs: 64 columns and fewer used to be padded to 128 there."""
+    assert columns(200 * 128, n, 0) == wide
