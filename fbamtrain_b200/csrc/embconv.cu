@@ -17,8 +17,8 @@
 //   fbam_embconv_fwd_colour  Z = POS + table rows + F . CC; Y = GELU(Z), with the colour features
 //                            F[n, p, tap*6 + c] = rgb_c(cell(p, tap)) / 255 (bf16, 64 per pixel) made on the way and
 //                            kept for the backward, whose colour term is the product F^T . dZ
-//   fbam_embconv_features    F alone
-//   fbam_embconv_fwd         Z += POS + table rows; Y = GELU(Z)
+//   fbam_embconv_features    F alone, and
+//   fbam_embconv_fwd         Z += POS + table rows; Y = GELU(Z): the parts of the above, for tests and measurements
 //   fbam_embconv_bwd_reduce  S[v][tap][:] += dZ rows by code point and tap;  D[p][:] += dZ summed over frames
 //
 // A warp owns one output pixel (32 lanes x 8 channels = a 256-channel block; 4 in the backward) and walks a run of

@@ -636,11 +636,11 @@ __global__ void __launch_bounds__(256) global_avgpool_bwd_kernel(const elem_t* _
 // warps per SM at 8192 x 1024).  GELU: the activation gradient in the same pass, dz = dy * gelu'(z), summed as rounded
 // (the other products use that dz, and as a kernel of its own it goes through DRAM once more).
 // 8192 x 8192: 30 us alone (54 before), 77 us with the activation gradient (two kernels: 134 us).
-// work != nullptr: a slab's sums go there, [slab][cols], for `partial_sum_kernel`; else they are added to `out`.
+// A slab's sums go to work, [slab][cols], for `partial_sum_kernel`.
 template <bool GELU>
 __global__ void __launch_bounds__(256, 4) colsum_kernel(const elem_t* __restrict__ x, const elem_t* __restrict__ dy,
-                                                     elem_t* __restrict__ dz, float* __restrict__ out,
-                                                     float* __restrict__ work, long long rows, int cols, int rows_per_block) {
+                                                     elem_t* __restrict__ dz, float* __restrict__ work, long long rows, int cols,
+                                                     int rows_per_block) {
   constexpr int U = GELU ? 2 : 4;
   __shared__ float part[8][32][9];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -685,10 +685,7 @@ __global__ void __launch_bounds__(256, 4) colsum_kernel(const elem_t* __restrict
     float t = 0.0f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) t += part[k][threadIdx.x >> 3][threadIdx.x & 7];
-    if (work != nullptr)
-      work[(long long)blockIdx.y * cols + oc] = t;
-    else
-      atomicAdd(out + oc, t);
+    work[(long long)blockIdx.y * cols + oc] = t;
   }
 }
 
@@ -1127,7 +1124,7 @@ int launch_rms_fwd(const elem_t* x, const elem_t* w, elem_t* y, float* rstd, lon
   rmsnorm_fwd_kernel<V><<<(unsigned)((rows + warps - 1) / warps), warps * 32, 0, s>>>(x, w, y, rstd, rows, dim, eps);
   return cudaGetLastError() == cudaSuccess ? 0 : 5;
 }
-// Rows a block takes at once, and blocks per SM, by width (fbam_rmsnorm_bwd's table).
+// Rows a block takes at once, and blocks per SM, by width (as `rms_bwd` chooses).
 struct RmsBwdShape { int rows, blocks; };
 RmsBwdShape rms_bwd_shape(int dim) {
   return dim <= 64 ? RmsBwdShape{64, 4} : dim <= 128 ? RmsBwdShape{32, 4} : dim <= 256 ? RmsBwdShape{16, 4}
@@ -1254,7 +1251,8 @@ int fbam_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, long lo
   return launch_rms_fwd<32>(X, W, (elem_t*)y, rstd, rows, dim, eps, STREAM(stream));
 }
 
-// dgamma: fp32 [dim], added to.
+// dgamma: fp32 [dim], added to.  The package's own backward is fbam_rmsnorm_bwd_to; this form is for sums that a caller
+// keeps, and for tests of the kernel alone.
 int fbam_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx, float* dgamma,
                      long long rows, int dim, void* stream) {
   return rms_bwd({(const elem_t*)dy, nullptr, (const elem_t*)x, (const elem_t*)w, rstd, (elem_t*)dx, dgamma, nullptr, rows, dim},
@@ -1393,31 +1391,13 @@ int fbam_global_avgpool(const void* in, void* out, long long n, int pix, int c, 
 }
 
 // Rows per block of the column sums: about eight blocks per SM, in whole rounds of the eight warps (64 to 512 rows, so
-// that the adds to `out` stay a small part of the work).
+// that adding the slabs up stays a small part of the work).
 static dim3 colsum_grid(long long rows, int cols, int* rows_per_block) {
   const int gx = (cols + 255) / 256;
   const long long want = (148 * 8 + gx - 1) / gx;
   const long long rpb = ((rows + want - 1) / want + 63) / 64 * 64;
   *rows_per_block = (int)(rpb < 64 ? 64 : rpb > 512 ? 512 : rpb);
   return dim3(gx, (unsigned)((rows + *rows_per_block - 1) / *rows_per_block));
-}
-
-int fbam_colsum(const void* x, float* out, long long rows, int cols, void* stream) {
-  if (cols % 8 != 0) return 1;
-  int rpb;
-  const dim3 grid = colsum_grid(rows, cols, &rpb);
-  colsum_kernel<false><<<grid, 256, 0, STREAM(stream)>>>((const elem_t*)x, nullptr, nullptr, out, nullptr, rows, cols, rpb);
-  return CHECK_LAUNCH();
-}
-
-// z, dy, dz: bf16 [rows][cols]; out: fp32 [cols], added to (the caller zeroes it).
-int fbam_gelu_bwd_colsum(const void* z, const void* dy, void* dz, float* out, long long rows, int cols, void* stream) {
-  if (cols % 8 != 0) return 1;
-  int rpb;
-  const dim3 grid = colsum_grid(rows, cols, &rpb);
-  colsum_kernel<true><<<grid, 256, 0, STREAM(stream)>>>((const elem_t*)z, (const elem_t*)dy, (elem_t*)dz, out, nullptr, rows, cols,
-                                                        rpb);
-  return CHECK_LAUNCH();
 }
 
 // Column sums written to `out` (fp32, or elements with out_elem), with the activation gradient in the same pass where z is
@@ -1438,9 +1418,9 @@ int fbam_colsum_to(const void* x, const void* z, void* dz, void* out, int out_el
     int rpb;
     const dim3 grid = colsum_grid(rows, cols, &rpb);
     if (gelu)
-      colsum_kernel<true><<<grid, 256, 0, s>>>((const elem_t*)z, (const elem_t*)x, (elem_t*)dz, nullptr, work, rows, cols, rpb);
+      colsum_kernel<true><<<grid, 256, 0, s>>>((const elem_t*)z, (const elem_t*)x, (elem_t*)dz, work, rows, cols, rpb);
     else
-      colsum_kernel<false><<<grid, 256, 0, s>>>((const elem_t*)x, nullptr, nullptr, nullptr, work, rows, cols, rpb);
+      colsum_kernel<false><<<grid, 256, 0, s>>>((const elem_t*)x, nullptr, nullptr, work, rows, cols, rpb);
     if (cudaGetLastError() != cudaSuccess) return 5;
     return launch_partial_sum(work, out, out_elem, grid.y, cols, s);
   }

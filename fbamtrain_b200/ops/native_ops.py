@@ -255,7 +255,7 @@ def _colsum(x2d: torch.Tensor, dtype: torch.dtype = torch.float32) -> torch.Tens
     out = torch.empty(cols, dtype=dtype, device=x2d.device)
     work = _sum_work("fbam_colsum_partials", cols, x2d.device, rows, cols, 0)
     nv.check(nv.lib(x2d).fbam_colsum_to(nv.ptr(x2d), None, None, nv.ptr(out), int(dtype != torch.float32), nv.ptr(work),
-                                        C.c_longlong(rows), cols, nv.stream_ptr()), "fbam_colsum")
+                                        C.c_longlong(rows), cols, nv.stream_ptr()), "fbam_colsum_to")
     return out
 
 
@@ -273,7 +273,7 @@ def _gelu_bwd_colsum(preact: torch.Tensor, dy: torch.Tensor, dtype: torch.dtype 
     out = torch.empty(cols, dtype=dtype, device=dy.device)
     work = _sum_work("fbam_colsum_partials", cols, dy.device, rows, cols, 1)
     nv.check(nv.lib(preact).fbam_colsum_to(nv.ptr(dy), nv.ptr(preact), nv.ptr(dz), nv.ptr(out), int(dtype != torch.float32),
-                                           nv.ptr(work), C.c_longlong(rows), cols, nv.stream_ptr()), "fbam_gelu_bwd_colsum")
+                                           nv.ptr(work), C.c_longlong(rows), cols, nv.stream_ptr()), "fbam_colsum_to")
     return dz, out
 
 
@@ -730,7 +730,7 @@ def _rms_norm_bwd(dy2, res2, x2, weight, rstd):
     work = _sum_work("fbam_rmsnorm_bwd_partials", dim, x2.device, rows, dim)
     nv.check(nv.lib(dy2).fbam_rmsnorm_bwd_to(nv.ptr(dy2), nv.ptr(res2), nv.ptr(x2), nv.ptr(weight), nv.ptr(rstd), nv.ptr(dx),
                                              nv.ptr(dg), nv.ptr(work), C.c_longlong(rows), dim, nv.stream_ptr()),
-             "fbam_rmsnorm_bwd")
+             "fbam_rmsnorm_bwd_to")
     return dx, dg
 
 
