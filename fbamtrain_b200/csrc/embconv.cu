@@ -108,9 +108,8 @@ using gelu_math::gelu2;
 // The colour term was a product of its own before (features to memory, a GEMM with K = 64 into Z, Z read back here) and
 // the rows were loaded when a change was met, with the warp waiting for each: 1024 frames of 24 x 80 pixels, 256
 // channels, took 1195 / 1290 / 1570 / 2630 us with 1 / 5 / 15 / 100 % of the cells changing, 1096 / 1214 without Z kept;
-// now 744 / 829 / 1039 / 1774 and 673 / 760.  The 2.2 GB written are 0.34 ms: instructions bound it, 277 a pixel and
-// frame (84 of them GELU, 31 the colour product, 40 at 5 % the changed rows) at 55 % of the issue rate; sixteen warps an
-// SM do as much as twenty-four.
+// now 744 / 829 / 1039 / 1774 and 673 / 760.  The 2.2 GB written are 0.34 ms: instructions bound it, 255 a pixel and
+// frame at 5 % of the cells changing, at 55 % of the issue rate (256 frames); sixteen warps an SM do as much as twenty-four.
 constexpr int kFwdPix = 8;
 constexpr int kFwdFrames = 8;
 constexpr int kFwdThreads = 32 * kFwdPix;
