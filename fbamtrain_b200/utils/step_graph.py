@@ -75,9 +75,13 @@ class _Watch:
     not fit ``MAX_GRAPHS`` cost some ten captures in a thousand steps each and not one at every turn."""
 
     def __init__(self) -> None:
-        self.steps, self.host_ms, self.gpu_ms, self.pending = 0, float("inf"), float("inf"), []
         self.wait: float = WATCHED_STEPS
         self.kept = 0              # bytes that the forward leaves for the backward
+        self.restart(None)
+
+    def restart(self, setting: Optional[tuple]) -> None:
+        self.steps, self.host_ms, self.gpu_ms, self.pending = 0, float("inf"), float("inf"), []
+        self.setting = setting     # what the steps run under; asked for from the last one before a capture on
 
     def given_back(self) -> None:
         self.steps, self.wait = 0, 2 * self.wait
@@ -123,29 +127,32 @@ class StepGraph:
         if (_module._global_forward_hooks or _module._global_forward_pre_hooks or _module._global_backward_hooks
                 or _module._global_backward_pre_hooks):
             return False
-        for m in self.model.modules():
-            if (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
-                    or "forward" in m.__dict__):
-                return False
-        for p in self.model.parameters():
-            if p._backward_hooks or p._post_accumulate_grad_hooks:
-                return False
         cfg, action = self.model.cfg, self.model.action_model
         # recomputed chunks and the streamed recurrence (which reads a value back) run as usual
         return not (cfg.frame_head_recompute or cfg.frame_replay or action.streaming or action.host_offload)
 
-    def _setting(self, cells: torch.Tensor, targets: torch.Tensor, loss_scale: float) -> tuple:
-        """What the launches of a step depend on besides the values of its inputs and parameters."""
+    def _setting(self) -> Optional[tuple]:
+        """What the launches of a step depend on besides its shape and the values of inputs and parameters; ``None`` where
+        the model has something that a replay would pass by."""
         no = native_ops
-        return (tuple(cells.shape), cells.dtype, tuple(targets.shape), targets.dtype, loss_scale, self.model.frame_chunk,
-                no.TWO_CTA, no.USE_MN_MAJOR, no.WEIGHT_GRAD_SPLIT_K, no.FUSE_DGRAD_CLASSES, no.FUSED_LM_HEAD_CE,
-                no.LM_HEAD_CHUNK_ROWS, no.RESIDUAL_NORM_MAX_DIM,
-                tuple(dispatch._prefer.values()), os.environ.get("FBAMTRAIN_EMBCONV"),
-                os.environ.get("FBAMTRAIN_ATTENTION_FWD2"), torch.are_deterministic_algorithms_enabled(),
-                native.lib(self.model.action_model.head_weight).fbam_reserved_sms(), *_library_setting(),
-                repr(self.model.cfg), tuple([_module_setting(m) for m in self.model.modules()]),
-                tuple((p.data_ptr(), p.requires_grad, -1 if p.grad is None else p.grad.data_ptr())
-                      for p in self.model.parameters()))
+        setting = [self.model.frame_chunk, no.TWO_CTA, no.USE_MN_MAJOR, no.WEIGHT_GRAD_SPLIT_K, no.FUSE_DGRAD_CLASSES,
+                   no.FUSED_LM_HEAD_CE, no.LM_HEAD_CHUNK_ROWS, no.RESIDUAL_NORM_MAX_DIM,
+                   tuple(dispatch._prefer.values()), os.environ.get("FBAMTRAIN_EMBCONV"),
+                   os.environ.get("FBAMTRAIN_ATTENTION_FWD2"), torch.are_deterministic_algorithms_enabled(),
+                   native.lib(self.model.action_model.head_weight).fbam_reserved_sms(), *_library_setting(),
+                   repr(self.model.cfg)]
+        for m in self.model.modules():       # one walk: 0.2 ms for the headline model, in which nothing is launched
+            if (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
+                    or "forward" in m.__dict__):
+                return None
+            setting.append(_module_setting(m))
+            for p in m._parameters.values():
+                if p is not None:
+                    grad = p.grad
+                    if grad is None or p._backward_hooks or p._post_accumulate_grad_hooks:
+                        return None
+                    setting += (p.data_ptr(), grad.data_ptr(), p.requires_grad)
+        return tuple(setting)
 
     # ------------------------------------------------------------------------------------------
     def forward_backward(self, cells: torch.Tensor, targets: torch.Tensor, loss_scale: float, run) -> Optional[torch.Tensor]:
@@ -155,12 +162,27 @@ class StepGraph:
         frames = cells.shape[0] * cells.shape[1]
         if frames * cells.shape[2] > MAX_CELLS or (chunk and frames > chunk) or not self._ordinary():
             return None
-        if not (cells.is_contiguous() and targets.is_contiguous()) or any(p.grad is None for p in self.model.parameters()):
+        if not (cells.is_contiguous() and targets.is_contiguous()):
             return None
-        key = self._setting(cells, targets, loss_scale)
+        shape = (tuple(cells.shape), cells.dtype, tuple(targets.shape), targets.dtype, loss_scale)
+        watch = self._watch(shape)
+        # The setting of the model is looked at where a graph may be replayed or captured now or in the next step: the first
+        # step of a shape, which may be its only one, and steps that the GPU bounds go without.
+        if (not any(of == shape for of, _ in self._graphs) and watch.steps + 1 != watch.wait
+                and not watch.launch_bound()):
+            return self._watched(watch, cells, targets, run)
+        setting = self._setting()
+        if setting is None:
+            return None
+        key = (shape, setting)
         captured = self._graphs.get(key)
         if captured is None:
-            watch = self._watch(key)
+            if watch.setting != setting:
+                if watch.setting is None:
+                    watch.setting = setting
+                else:
+                    watch.restart(setting)
+                return self._watched(watch, cells, targets, run)
             if not watch.launch_bound():
                 return self._watched(watch, cells, targets, run)
             if not self._room(watch):
@@ -176,7 +198,7 @@ class StepGraph:
             while len(self._graphs) > MAX_GRAPHS:
                 # its kernels may still be running: the memory goes back to the allocator only behind them
                 torch.cuda.current_stream().synchronize()
-                self._watch(self._graphs.popitem(last=False)[0]).given_back()
+                self._give_back()
         self._graphs.move_to_end(key)
         captured.cells.copy_(cells)
         captured.targets.copy_(targets)
@@ -195,14 +217,20 @@ class StepGraph:
         if self._graphs:
             torch.cuda.current_stream().synchronize()
         while self._graphs:
-            self._watch(self._graphs.popitem(last=False)[0]).given_back()
+            self._give_back()
         freed, self.pool_bytes = self.pool_bytes, 0
         return freed
 
-    def _watch(self, key: tuple) -> _Watch:
+    def _give_back(self) -> None:
+        (shape, _), _graph = self._graphs.popitem(last=False)
+        self._watch(shape).given_back()
+
+    def _watch(self, shape: tuple) -> _Watch:
         """The watch of a shape; those of the last ``MAX_WATCHES`` shapes are kept."""
-        watch = self._watches.setdefault(key, _Watch())
-        self._watches.move_to_end(key)
+        watch = self._watches.get(shape)
+        if watch is None:
+            watch = self._watches[shape] = _Watch()
+        self._watches.move_to_end(shape)
         while len(self._watches) > MAX_WATCHES:
             self._watches.popitem(last=False)
         return watch

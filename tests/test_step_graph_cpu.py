@@ -29,7 +29,8 @@ def graph(monkeypatch):
     g.log = log
     monkeypatch.setattr(g, "_ordinary", lambda: True)
     monkeypatch.setattr(sg.torch.cuda, "mem_get_info", lambda *a: (64 << 30, 180 << 30))
-    monkeypatch.setattr(g, "_setting", lambda cells, targets, scale: tuple(cells.shape))
+    g.setting = ("a",)
+    monkeypatch.setattr(g, "_setting", lambda: log.append("asked") or g.setting)
 
     def watched(watch, cells, targets, run):
         watch.steps, watch.host_ms, watch.gpu_ms = watch.steps + 1, 1.0, 1.0
@@ -84,7 +85,7 @@ def test_graphs_hold_a_part_of_the_free_memory_at_most(graph, monkeypatch):
     free = [8 << 30]
     monkeypatch.setattr(sg.torch.cuda, "mem_get_info", lambda *a: (free[0], 180 << 30))
     _steps(graph, [1], 2)
-    graph._watch((1, 1, 1)).kept = 512 << 20
+    next(iter(graph._watches.values())).kept = 512 << 20
     assert _steps(graph, [1], 10)["capture"] == 0
     free[0] = 10 << 30
     assert _steps(graph, [1], 60)["capture"] == 1
@@ -112,3 +113,32 @@ def test_memory_of_graphs_is_no_room_for_a_step(pool, need, fits, released, monk
     assert Trainer._memory_for(SimpleNamespace(_step_graph=graphs, device=None), need) is fits
     assert bool(gave) is released
     assert Trainer._memory_for(SimpleNamespace(_step_graph=None, device=None), need) is (need <= 180)
+
+
+def test_the_first_step_of_a_shape_asks_for_no_setting(graph):
+    """Walking the model takes the host 0.3 ms and more, in which nothing is launched."""
+    _steps(graph, [1, 2, 3, 4, 5], 5)
+    assert "asked" not in graph.log
+    _steps(graph, [1], 1)
+    assert graph.log.count("asked") == 1
+
+
+def test_another_setting_is_watched_anew_and_the_old_graph_comes_back(graph):
+    assert _steps(graph, [1], 4)["capture"] == 1
+    graph.setting = ("b",)
+    graph.log.clear()
+    assert _steps(graph, [1], 2) == {"usual": 2, "capture": 0, "replay": 0, "wait": 0}
+    assert _steps(graph, [1], 1)["capture"] == 1
+    graph.setting = ("a",)
+    graph.log.clear()
+    assert _steps(graph, [1], 3) == {"usual": 0, "capture": 0, "replay": 3, "wait": 0}
+    graph.setting = None                      # hooks on the model: the caller runs the step
+    cells = torch.zeros(1, 1, 1)
+    assert graph.forward_backward(cells, cells, 1.0, None) is None
+
+
+def test_settings_in_turn_are_not_captured(graph):
+    for i in range(60):
+        graph.setting = (i % 3,)
+        _steps(graph, [1], 1)
+    assert graph.log.count("capture") == 0
