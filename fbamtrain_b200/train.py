@@ -448,6 +448,8 @@ class Trainer:
         self.ckpt.wait()
         self.logger.drain()
         self.logger.close()
+        if self._step_graph is not None:
+            self._step_graph.release()
         if self.cursor is not None:
             self.cursor.close()
 

@@ -65,6 +65,7 @@ def test_given_back_and_captured_again(monkeypatch):
     assert len(graphs._graphs) == 1
     _same(_losses(trainer, batches), expected)
     trainer.close()
+    assert not graphs._graphs and graphs.pool_bytes == 0     # a closed trainer holds none, also while somebody holds it
 
 
 def test_a_capture_that_fails_leaves_the_step(monkeypatch):
