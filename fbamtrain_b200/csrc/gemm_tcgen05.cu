@@ -618,8 +618,8 @@ int pick_bn_plain(long long m, int n, int requested, int ctas) {
 extern "C" int fbam_last_driver_error() { return g_fbam_last_driver_error; }
 extern "C" int fbam_pending_runtime_error() { return (int)cudaPeekAtLastError(); }
 
-// Revision of the C interface: raised whenever an entry point's arguments, the size of a buffer it is given or a struct
-// changes.  The ctypes binding refuses a library of another revision (a stale build): offsets alone do not tell when a
+// Revision of the C interface: raised whenever an entry point comes, goes or changes its arguments, or the size of a buffer
+// it is given or a struct changes.  The ctypes binding refuses a library of another revision (a stale build): offsets alone do not tell when a
 // field takes the place of padding, and say nothing about arguments.
 extern "C" int fbam_interface_revision() { return FBAM_INTERFACE_REVISION; }
 

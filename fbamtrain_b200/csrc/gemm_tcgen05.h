@@ -36,7 +36,7 @@ struct ConvClass {
   int k_block_base;
 };
 
-#define FBAM_INTERFACE_REVISION 4  // see fbam_interface_revision; INTERFACE_REVISION in ops/native.py
+#define FBAM_INTERFACE_REVISION 5  // see fbam_interface_revision; INTERFACE_REVISION in ops/native.py
 
 struct GemmParams {
   void* D;                          // output, bf16 or fp32, row pitch ldd elements

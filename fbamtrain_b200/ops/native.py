@@ -78,7 +78,7 @@ def available(dtype: torch.dtype = torch.bfloat16) -> bool:
     return os.path.exists(LIB_PATH_FP16 if dtype == torch.float16 else LIB_PATH)
 
 
-INTERFACE_REVISION = 4        # FBAM_INTERFACE_REVISION of csrc/gemm_tcgen05.h
+INTERFACE_REVISION = 5        # FBAM_INTERFACE_REVISION of csrc/gemm_tcgen05.h
 
 
 def _check_struct_layout(library: C.CDLL, path: str) -> None:
