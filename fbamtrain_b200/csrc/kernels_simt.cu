@@ -1402,9 +1402,16 @@ static dim3 colsum_grid(long long rows, int cols, int* rows_per_block) {
 
 // Column sums written to `out` (fp32, or elements with out_elem), with the activation gradient in the same pass where z is
 // given (x is then dy).  work: fp32 [fbam_colsum_partials(rows, cols, z != null)][cols]; 0 of them: not used.
-// One launch of clusters up to 8192 rows, 2048 with the activation gradient (whose loads a cluster has half as many of in
-// flight); above, and for what is narrower than two clusters, slabs over the whole machine and a launch that adds them up.
-static bool colsum_by_clusters(long long rows, int cols, int gelu) { return rows <= (gelu || cols <= 128 ? 2048 : 8192); }
+// One launch of clusters for few rows, slabs over the whole machine and a launch that adds them up for more.  The line lies
+// where clusters of 64 columns leave SMs idle: above 4096 rows, 1024 with the activation gradient (whose loads a cluster has
+// half as many of in flight), they need more than 1024 columns, and twice the rows are the most.  us on the device alone of a
+// fill, sums by atomics and a conversion | clusters | slabs: 4096 x 1024 5.6 | 5.5 | 5.2, 8192 x 1024 7.0 | 8.0 | 6.5, 8192 x
+// 2048 9.4 | 8.1 | 9.2; with the activation gradient 1024 x 1024 7.7 | 5.5 | 7.1, 2048 x 1024 7.8 | 8.1 | 7.4, 2048 x 4096
+// 13.2 | 12.6 | 13.4.  (Slabs are a launch more, which the host takes some 5 us to issue.)
+static bool colsum_by_clusters(long long rows, int cols, int gelu) {
+  const long long most = gelu ? 1024 : cols <= 128 ? 2048 : 4096;
+  return rows <= most || (cols > 1024 && rows <= 2 * most);
+}
 int fbam_colsum_partials(long long rows, int cols, int gelu) {
   int rpb;
   return colsum_by_clusters(rows, cols, gelu) ? 0 : (int)colsum_grid(rows, cols, &rpb).y;

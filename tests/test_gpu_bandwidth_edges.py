@@ -65,7 +65,8 @@ def test_gelu_backward_with_column_sums(rows, cols, dtype):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("rows,cols", [(1, 8), (3, 72), (513, 64), (2047, 136), (2048, 128), (2049, 128), (2049, 2368), (300, 2376),
-                                       (200, 4744), (70, 9480), (8192, 200), (8193, 200), (20000, 8)])
+                                       (200, 4744), (70, 9480), (8192, 200), (8193, 200), (20000, 8), (1024, 1024), (1025, 1024),
+                                       (1025, 1032), (2048, 1032), (4096, 1024), (4097, 1024), (4097, 1032), (8192, 1032)])
 def test_column_sums_of_both_kinds_of_launch(rows, cols, dtype):
     """One launch of clusters of 8, 4, 2 or 1 CTAs up to a number of rows, slabs and an adding launch above; written as fp32
     and as elements."""
