@@ -685,7 +685,9 @@ __global__ void __launch_bounds__(256, 4) colsum_kernel(const elem_t* __restrict
     float t = 0.0f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) t += part[k][threadIdx.x >> 3][threadIdx.x & 7];
-    work[(long long)blockIdx.y * cols + oc] = t;
+    // 32 bits: slabs have 64 rows at least, so there are fewer sums than 2^32 for any matrix that fits the memory.  With a
+    // 64-bit index the loop above takes a register more and 2 % longer (8192 x 8192 with the gradient 71.0 -> 72.5 us).
+    work[blockIdx.y * (unsigned)cols + oc] = t;
   }
 }
 
