@@ -60,7 +60,7 @@ struct SmemLayout {
   // a stage, and the MMAs of a K block take 256 (BN = 128) or 128 cycles (64): two blocks share a stage there.  Cycles per K
   // block, one block per stage -> two: BN = 128 390 -> 310, 64 390 -> 280 (460 before the loop of plain products was one of
   // its own); four blocks and two stages: no change.
-  static constexpr int kSub = BM == 128 && BN <= 128 ? 2 : 1;
+  static constexpr int kSub = BM == 128 && BN <= 128 ? 2 : 1;  // the producer knows of no more than two
   static constexpr int kABytes = BM * BK * 2;
   static constexpr int kBBytes = BN * BK * 2;
   static constexpr int kBlockBytes = kABytes + kBBytes;
@@ -217,11 +217,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
               mbar_expect_tx(&full_bar[stage], L::kStageBytes);
 #pragma unroll
               for (int sub = 0; sub < L::kSub; ++sub) load_block(sa + sub * L::kBlockBytes, kb + sub * wk.k_step);
-            } else {
-              const int blocks = (wk.k_end - kb + wk.k_step - 1) / wk.k_step;
-              mbar_expect_tx(&full_bar[stage], blocks * L::kBlockBytes);
-#pragma unroll 1
-              for (int sub = 0; sub < blocks; ++sub) load_block(sa + sub * L::kBlockBytes, kb + sub * wk.k_step);
+            } else {                                            // the last of an odd number
+              mbar_expect_tx(&full_bar[stage], L::kBlockBytes);
+              load_block(sa, kb);
             }
             if (++stage == L::kStages) { stage = 0; phase ^= 1; }
           }
@@ -229,10 +227,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         }
         for (int kb0 = wk.k_begin; kb0 < wk.k_end; kb0 += L::kSub * wk.k_step) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1)) { ok = false; break; }
-          const int blocks = min(L::kSub, (wk.k_end - kb0 + wk.k_step - 1) / wk.k_step);
-          mbar_expect_tx(&full_bar[stage], blocks * L::kBlockBytes);
+          const bool whole = kb0 + (L::kSub - 1) * wk.k_step < wk.k_end;   // no division here: it costs 80 cycles a stage
+          mbar_expect_tx(&full_bar[stage], whole ? L::kStageBytes : L::kBlockBytes);
 #pragma unroll 1
-          for (int sub = 0; sub < blocks; ++sub) {
+          for (int sub = 0; sub < L::kSub; ++sub) {
+            if (sub > 0 && !whole) break;
             const int kb = kb0 + sub * wk.k_step;
             uint8_t* sa = smem + stage * L::kStageBytes + sub * L::kBlockBytes;
             uint8_t* sb = sa + L::kABytes;
@@ -597,12 +596,16 @@ int pick_bn(int n, int requested) {
 }
 
 // Columns of a tile of a plain product: the narrowest tile that still leaves one tile per CTA that the launch may use at
-// most.  us, 256 | chosen: 1000 x 1024 x 1024 11.5 | 7.2 (64), x 4096 24.9 | 14.2, 512 x 4096 x 1024 11.5 | 8.4 (128),
-// 256 x 256 x 256 7.6 | 5.2.  Above one tile per CTA the widest tile that N fills wins: 1000 x 3072 x 1024 11.8 with 256, 13
-// with 128; 20000 x 64 x 4096 51 with 64, 55 with 128, 200000 x 64 x 1024 84 and 90.
-int pick_bn_plain(long long m, int n, int requested, int ctas) {
+// most.  us, 256 | chosen: 1000 x 1024 x 1024 10.8 | 7.0 (64), x 4096 24.4 | 14.8, 512 x 4096 x 1024 11.3 | 8.6 (128),
+// 256 x 256 x 256 7.3 | 4.8.  Above one tile per CTA the widest tile that N fills wins: 1000 x 3072 x 1024 11.6 with 256,
+// 12.3 with 128; 20000 x 64 x 4096 51 with 64, 55 with 128, 200000 x 64 x 1024 84 and 90.
+// Very few rows of A, which all CTAs then read at once: some 40 CTAs do best.  us with 64 | 128 | 256 columns: 8 x 9472 x
+// 4096 30.1 | 29.5 | 24.2 (16 rows: 14.4 | 16.3 | 24.0), 8 x 4096 x 4096 22.6 | 17.2 | 23.9, 8 x 2048 x 2048 9.0 | 10.4 | 15.1;
+// A stored column by column 8 x 9472 x 1024 18.7 | - | 12.6, 32 rows 12.1 | - | 11.0, 64 rows 7.1 | - | 10.8.
+int pick_bn_plain(long long m, int n, int requested, int ctas, int a_mn_major) {
   if (requested == 64 || requested == 128 || requested == 256) return requested;
   const long long tiles_m = (m + 127) / 128;
+  if (m <= (a_mn_major ? 32 : 8) && ctas > 40) ctas = 40;
   for (int bn = 64; bn < 256; bn *= 2)
     if (tiles_m * ((n + bn - 1) / bn) <= ctas) return bn;
   return pick_bn(n, 0);
@@ -650,7 +653,9 @@ extern "C" int fbam_set_reserved_sms(int n) {
 }
 
 // Columns of a tile that fbam_gemm picks for an unsplit product (for tests of the rule).
-extern "C" int fbam_gemm_tile_columns(int M, int N, int max_ctas) { return pick_bn_plain(M, N, 0, usable_ctas(max_ctas)); }
+extern "C" int fbam_gemm_tile_columns(int M, int N, int max_ctas, int a_mn_major) {
+  return pick_bn_plain(M, N, 0, usable_ctas(max_ctas), a_mn_major);
+}
 
 extern "C" int fbam_gemm(const void* A, long long lda, int a_mn_major, const void* B, long long ldb,
                               int b_mn_major, int M, int N, int K, GemmParams* params, void* stream) {
@@ -665,7 +670,7 @@ extern "C" int fbam_gemm(const void* A, long long lda, int a_mn_major, const voi
   if (p.splits > 1 && p.split_workspace == nullptr && !(p.out_fp32 && p.accumulate == GEMM_ACC_ATOMIC))
     return GEMM_ERR_SHAPE;
   // a split product divides K until its wide tiles fill the machine
-  int bn = p.splits > 1 || p.bm == 256 ? pick_bn(N, p.bn) : pick_bn_plain(M, N, p.bn, usable_ctas(p.max_ctas));
+  int bn = p.splits > 1 || p.bm == 256 ? pick_bn(N, p.bn) : pick_bn_plain(M, N, p.bn, usable_ctas(p.max_ctas), a_mn_major);
   int BM = pick_bm(M, N, bn, p.bm);
   if (p.ce_mode != 0) {
     // fused cross-entropy epilogues: one tile shape, no split-K, the buffers of the mode present

@@ -9,7 +9,7 @@ def columns():
     if not nv.available():
         pytest.skip("kernel library not built")
     lib = nv.lib()
-    yield lib.fbam_gemm_tile_columns
+    yield lambda m, n, max_ctas, a_mn=0: lib.fbam_gemm_tile_columns(m, n, max_ctas, a_mn)
     lib.fbam_set_reserved_sms(0)
 
 
@@ -31,3 +31,10 @@ def test_narrow_tiles_fit_the_ctas_of_the_launch(columns):
 def test_many_rows_take_the_tile_that_the_columns_fill(columns, n, wide):
     """More tiles than CTAs: 64 columns and fewer used to be padded to 128 there."""
     assert columns(200 * 128, n, 0) == wide
+
+
+@pytest.mark.parametrize("m,a_mn,few", [(1, 0, True), (8, 0, True), (9, 0, False), (32, 1, True), (33, 1, False)])
+def test_very_few_rows_take_some_forty_tiles(columns, m, a_mn, few):
+    """148, 64 and 32 tiles of 64 columns."""
+    assert [columns(m, n, 0, a_mn) for n in (9472, 4096, 2048)] == ([256, 128, 64] if few else [64, 64, 64])
+    assert columns(m, 9472, 36, a_mn) == 256
