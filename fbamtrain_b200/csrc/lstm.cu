@@ -751,7 +751,7 @@ struct Shape {
   int shared;  // groups of 8 rows per CTA
   int wait;    // cycles from a CTA's publication to its first poll
 };
-Shape lstm_shape(int rows, int H, bool forward) {
+Shape lstm_shape(int rows, int H, int T, bool forward) {
   const int sub = (rows + 7) / 8;
   Shape s;
   s.wide = H > 1024 || (H > 512 ? sub > 1 : H > 256 && sub > 2);
@@ -760,8 +760,11 @@ Shape lstm_shape(int rows, int H, bool forward) {
   s.shared = (sub + s.groups - 1) / s.groups;
   // Lowest time per step over waits of 0, 100 .. 1400 cycles; flat around it, except in the backward pass at H = 1024:
   // 8 rows 2.23 us with 400, 1.74 with 800; 3 rows 1.78 and 1.95.
+  // Four groups at H <= 512 publish earlier while what a launch reads and writes (22 bytes a unit, row and step) stays in L2:
+  // us per step with 250 | 450 cycles, H = 512, 24 rows, 256 steps (69 MB) 1.32 | 1.42, 32 rows (92 MB) 1.67 | 1.44.
+  const bool in_l2 = 22ll * rows * H * T < 80000000;
   if (forward)
-    s.wait = H <= 256 ? 150 : H <= 512 ? (s.wide ? 450 : 300) : s.shared > 1 ? 300 : 450;
+    s.wait = H <= 256 ? 150 : H <= 512 ? (!s.wide ? 300 : in_l2 ? 250 : 450) : s.shared > 1 ? 300 : 450;
   else
     s.wait = H <= 256 ? 150 : H > 512 && H <= 1024 && rows > 3 && !s.wide ? 800 : 400;
   return s;
@@ -823,7 +826,7 @@ int fbam_lstm_fwd_ex(float* gates, const void* whh, const float* h0, const float
   if (exchanged != 0 && cudaMemsetAsync(y, 0xff, exchanged, s) != cudaSuccess) return 5;
   int vec = reinterpret_cast<uintptr_t>(y) % 16 == 0;
   for (int b0 = 0, most = launch_rows(H, T, true); b0 < B; b0 += most) {
-    Shape sh = lstm_shape(B - b0 < most ? B - b0 : most, H, true);
+    Shape sh = lstm_shape(B - b0 < most ? B - b0 : most, H, T, true);
     void* args[] = {&gates, &whh, &h0, &c0, &y, &c_all, &status, &T, &B, &H, &per_sample, &b0, &sh.groups, &vec, &sh.wait};
     const int rc = launch_shape<0>(sh, H, args, s);
     if (rc != 0) return rc;
@@ -848,7 +851,7 @@ int fbam_lstm_bwd_ex(const float* gates, const float* c_all, const float* c0, co
   if (cudaMemsetAsync(dgates, 0xff, (size_t)T * B * 4 * H * sizeof(elem_t), s) != cudaSuccess) return 5;
   int vec = reinterpret_cast<uintptr_t>(dgates) % 16 == 0;
   for (int b0 = 0, most = launch_rows(H, T, false); b0 < B; b0 += most) {
-    Shape sh = lstm_shape(B - b0 < most ? B - b0 : most, H, false);
+    Shape sh = lstm_shape(B - b0 < most ? B - b0 : most, H, T, false);
     void* args[] = {&gates, &c_all, &c0, &dy, &whh_t, &dgates, &dh0, &dc0, &dh_last, &dc_last, &status,
                     &T, &B, &H, &per_sample, &b0, &sh.groups, &vec, &sh.wait};
     const int rc = launch_shape<1>(sh, H, args, s);
