@@ -32,12 +32,13 @@
 // an idle cluster barrier takes 400 and one behind the stores of unsummed partials took about 1000.  One thread owns one
 // (unit, batch row) with its four gates, and what does not depend on dh is computed while the sums are on their way.
 //
-// Measured on a B200, bf16, us per step, before (polls at once, IEEE gate functions, groups of rows in turn, cluster
+// Measured on a B200, bf16, us per step over 1024 steps, before (polls at once, IEEE gate functions, groups of rows in turn, cluster
 // barrier) -> in this form:
-//   H 1024, batch 8:    forward 1.80 -> 1.49, backward 2.05 -> 1.74
-//   H 2048, batch 4:    forward 3.09 -> 2.44, backward 3.75 -> 2.70
-//   H  256, batch 8:    forward 1.06 -> 0.95, backward 1.68 -> 1.29
-//   H 1024, batch 32:   forward 3.47 -> 2.73, backward 6.27 -> 3.06
+//   H 1024, batch 8:    forward 1.82 -> 1.52, backward 2.06 -> 1.75
+//   H 2048, batch 4:    forward 3.09 -> 2.50, backward 3.72 -> 2.71
+//   H  256, batch 8:    forward 1.02 -> 0.94, backward 1.65 -> 1.27
+//   H  512, batch 32:   forward 1.97 -> 1.47, backward 2.76 -> 1.72
+//   H 1024, batch 32:   forward 3.43 -> 2.79, backward 6.22 -> 2.99
 //   H 2048, batch 32:   forward 12.9 -> 11.4, backward 16.1 -> 9.8
 // (At H = 1024 a forward cluster that divides K, with partial sums sent as in the backward pass, takes 1.75 us at batch 8,
 // 1.50 without: its second hop costs more than the smaller share of the vector gives.)
